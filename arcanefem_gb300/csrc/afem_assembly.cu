@@ -140,20 +140,82 @@ __global__ void __launch_bounds__(256) k_elem_poisson_tri(int cell0, int nb_cell
 // then the other cell nodes increasing); each row is the reference's element
 // vector of its own node, which in the module formulation is not the
 // transpose of the column bit for bit ((vol dx_i) dx_k against (vol dx_k) dx_i),
-// so every row is formed: 4 x 23 + ~130 FP64 instructions per tetrahedron
-// (divisions included) against 72 for the minimal form.  A cell coefficient
-// multiplies each entry as the node-wise loop does (coeff * v).
-// Which stages of the reference-rounding tetrahedron run their products and
-// sums on the integer pipe (afem_fp64_int.cuh) instead of the FP64 pipe, so
-// that both pipes work at once: bit 0 the element rows, bit 1 the gradient
-// numerators, bit 2 the coordinate differences.  The values are the same bit
-// for bit whatever the choice; it is a throughput tuning constant.
-#ifndef AFEM_REF_INT_STAGES
-#define AFEM_REF_INT_STAGES 0
-#endif
-constexpr bool kIntRows = (AFEM_REF_INT_STAGES & 1) != 0;
-constexpr bool kIntNumerators = (AFEM_REF_INT_STAGES & 2) != 0;
-constexpr bool kIntDifferences = (AFEM_REF_INT_STAGES & 4) != 0;
+// so every row is formed.  A cell coefficient multiplies each entry as the
+// node-wise loop does (coeff * v).  On the FP64 pipe alone: triangles, the
+// testlab form, and the tetrahedra that k_elem_poisson_tet_ref leaves out.
+// The element of cell c, its rows written to their incidences.
+template <int NPC, int F>
+__device__ __forceinline__ void elem_p1_cell(int64_t c, const double* __restrict__ xyz, const int32_t* __restrict__ cn,
+                                             const int32_t* __restrict__ inv, const double* __restrict__ coeff,
+                                             double* __restrict__ er, int* __restrict__ bad) {
+  int32_t nid[NPC];
+  if constexpr (NPC == 4) {
+    const int4 q = __ldg(reinterpret_cast<const int4*>(cn) + c);
+    nid[0] = q.x; nid[1] = q.y; nid[2] = q.z; nid[3] = q.w;
+  } else {
+#pragma unroll
+    for (int a = 0; a < NPC; ++a) nid[a] = __ldg(cn + NPC * c + a);
+  }
+  double n[NPC][3];
+#pragma unroll
+  for (int a = 0; a < NPC; ++a) {
+    const double* p = xyz + 3 * (int64_t)nid[a];
+    n[a][0] = __ldg(p);
+    n[a][1] = __ldg(p + 1);
+    n[a][2] = __ldg(p + 2);
+  }
+  double K[NPC][NPC], meas;
+  if constexpr (F == AFEM_FORMULATION_TESTLAB) {
+    if constexpr (NPC == 4) meas = ref::testlab_tet(n, K);
+    else meas = ref::testlab_tri(n, K);
+#pragma unroll
+    for (int i = 0; i < NPC; ++i)
+#pragma unroll
+      for (int k = 0; k < i; ++k) K[i][k] = K[k][i];
+  } else if constexpr (NPC == 4) {
+    double g[3][4], vol;
+    meas = ref::tet_gradients(n, g, &vol);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ref::tet_row(g, vol, i, K[i]);
+  } else {
+    double dx[3], dy[3], area;
+    meas = ref::tri_gradients(n, dx, dy, &area);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) ref::tri_row(dx, dy, area, i, K[i]);
+  }
+  if (bad && !ref::measure_ok(meas)) atomicOr(bad, kFlagDegenerateCell);
+  if (coeff) {
+    const double k = __ldg(coeff + c);
+#pragma unroll
+    for (int i = 0; i < NPC; ++i)
+#pragma unroll
+      for (int j = 0; j < NPC; ++j) K[i][j] = ref::mul(k, K[i][j]);
+  }
+  int32_t pos[NPC];
+  if constexpr (NPC == 4) {
+    const int4 p = __ldg(reinterpret_cast<const int4*>(inv) + c);
+    pos[0] = p.x; pos[1] = p.y; pos[2] = p.z; pos[3] = p.w;
+  } else {
+#pragma unroll
+    for (int a = 0; a < NPC; ++a) pos[a] = __ldg(inv + NPC * c + a);
+  }
+#pragma unroll
+  for (int i = 0; i < NPC; ++i) {
+    double r[NPC];
+    r[0] = K[i][i];
+    int q = 1;
+#pragma unroll
+    for (int j = 0; j < NPC; ++j)
+      if (j != i) r[q++] = K[i][j];
+    double* dst = er + NPC * (int64_t)pos[i];
+    if constexpr (NPC == 4) {
+      st4(dst, r[0], r[1], r[2], r[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NPC; ++j) dst[j] = r[j];
+    }
+  }
+}
 
 template <int NPC, int F>
 __global__ void __launch_bounds__(128) k_elem_poisson_p1_ref(int cell0, int nb_cell, const double* __restrict__ xyz,
@@ -162,70 +224,72 @@ __global__ void __launch_bounds__(128) k_elem_poisson_p1_ref(int cell0, int nb_c
                                                              const double* __restrict__ coeff,
                                                              double* __restrict__ er, int* __restrict__ bad) {
   for (int64_t c = cell0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    int32_t nid[NPC], pos[NPC];
-    if constexpr (NPC == 4) {
+       c += (int64_t)gridDim.x * blockDim.x)
+    elem_p1_cell<NPC, F>(c, xyz, cn, inv, coeff, er, bad);
+}
+
+// A cell whose operands leave the integer path's range, on the FP64 pipe alone.
+__device__ __noinline__ void elem_tet_cell_fp64(int64_t c, const double* xyz, const int32_t* cn, const int32_t* inv,
+                                                const double* coeff, double* er, int* bad) {
+  elem_p1_cell<4, AFEM_FORMULATION_REFERENCE>(c, xyz, cn, inv, coeff, er, bad);
+}
+
+// The reference-rounding tetrahedron, its sums on the FP64 pipe and its
+// products and quotients on the integer pipes (afem_fp64_int.cuh), bit for bit
+// the same.  Bound: the two pipes together.  A warp FP64 instruction occupies
+// its pipe for about 75 cycles of an SM partition, an integer one for 2, so a
+// product of ~20 integer instructions and 4 wide multiply-adds costs less there
+// even alone; of the 230 FP64 instructions a cell 79 are left, and 2500 integer
+// ones come in: measured 73 % of the FP64 pipe and 72 % of the integer ALU at
+// once (93 % and 4 % before).  The cell's coordinates, differences and factors
+// live in shared memory, so that the loops over dimensions and rows stay loops:
+// fully unrolled the kernel needed 168 registers and missed the instruction
+// cache (12 warps an SM, 1.38 ms at 96^3); as loops it runs 20 warps an SM of
+// 96 registers.  Measured (5.3 M / 12.6 M cells): 2.47 / 5.86 -> 0.93 / 2.19 ms;
+// 4 or 6 blocks an SM: 0.96 / 0.94 ms at 96^3.
+constexpr int kTetBlock = 128;
+
+template <bool COEFF>
+__global__ void __launch_bounds__(kTetBlock, 5)
+    k_elem_poisson_tet_ref(int cell0, int nb_cell, const double* __restrict__ xyz, const int32_t* __restrict__ cn,
+                           const int32_t* __restrict__ inv, const double* __restrict__ coeff, double* __restrict__ er,
+                           int* __restrict__ bad) {
+  __shared__ ref::TetScratch<kTetBlock> sh;
+  for (int64_t c = cell0 + blockIdx.x * (int64_t)kTetBlock + threadIdx.x; c < nb_cell;
+       c += (int64_t)gridDim.x * kTetBlock) {
+    bool ok = true;
+    {
       const int4 q = __ldg(reinterpret_cast<const int4*>(cn) + c);
-      const int4 p = __ldg(reinterpret_cast<const int4*>(inv) + c);
-      nid[0] = q.x; nid[1] = q.y; nid[2] = q.z; nid[3] = q.w;
-      pos[0] = p.x; pos[1] = p.y; pos[2] = p.z; pos[3] = p.w;
-    } else {
+      ok = ref::tet_gradients_int(xyz, q, sh, threadIdx.x);
+    }
+    if (!ok) {
+      elem_tet_cell_fp64(c, xyz, cn, inv, coeff, er, bad);
+      continue;
+    }
+    using V = ref::Val;
+    V g[3][4];
 #pragma unroll
-      for (int a = 0; a < NPC; ++a) {
-        nid[a] = __ldg(cn + NPC * c + a);
-        pos[a] = __ldg(inv + NPC * c + a);
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[d][i] = sh.gradient(d, i, threadIdx.x);
+    const V vol = sh.volume(threadIdx.x);
+    const double k = COEFF ? __ldg(coeff + c) : 1.0;
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+      const V sx(ref::mul(vol, sh.gradient(0, i, threadIdx.x))), sy(ref::mul(vol, sh.gradient(1, i, threadIdx.x))),
+          sz(ref::mul(vol, sh.gradient(2, i, threadIdx.x)));
+      double v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        v[j] = ref::add(ref::add(ref::mul(sx, g[0][j]), ref::mul(sy, g[1][j])), ref::mul(sz, g[2][j]));
+      if constexpr (COEFF) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = ref::mul(k, v[j]);
       }
-    }
-    double n[NPC][3];
-#pragma unroll
-    for (int a = 0; a < NPC; ++a) {
-      const double* p = xyz + 3 * (int64_t)nid[a];
-      n[a][0] = __ldg(p);
-      n[a][1] = __ldg(p + 1);
-      n[a][2] = __ldg(p + 2);
-    }
-    double K[NPC][NPC], meas;
-    if constexpr (F == AFEM_FORMULATION_TESTLAB) {
-      if constexpr (NPC == 4) meas = ref::testlab_tet(n, K);
-      else meas = ref::testlab_tri(n, K);
-#pragma unroll
-      for (int i = 0; i < NPC; ++i)
-#pragma unroll
-        for (int k = 0; k < i; ++k) K[i][k] = K[k][i];
-    } else if constexpr (NPC == 4) {
-      double g[3][4], vol;
-      meas = ref::tet_gradients<kIntDifferences, kIntNumerators>(n, g, &vol);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ref::tet_row<kIntRows>(g, vol, i, K[i]);
-    } else {
-      double dx[3], dy[3], area;
-      meas = ref::tri_gradients(n, dx, dy, &area);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) ref::tri_row(dx, dy, area, i, K[i]);
-    }
-    if (bad && !ref::measure_ok(meas)) atomicOr(bad, kFlagDegenerateCell);
-    if (coeff) {
-      const double k = __ldg(coeff + c);
-#pragma unroll
-      for (int i = 0; i < NPC; ++i)
-#pragma unroll
-        for (int j = 0; j < NPC; ++j) K[i][j] = ref::mul(k, K[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < NPC; ++i) {
-      double r[NPC];
-      r[0] = K[i][i];
-      int q = 1;
-#pragma unroll
-      for (int j = 0; j < NPC; ++j)
-        if (j != i) r[q++] = K[i][j];
-      double* dst = er + NPC * (int64_t)pos[i];
-      if constexpr (NPC == 4) {
-        st4(dst, r[0], r[1], r[2], r[3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < NPC; ++j) dst[j] = r[j];
-      }
+      // diagonal first, then the other nodes in increasing order
+      const double d = i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : v[3];
+      st4(er + 4 * (int64_t)__ldg(inv + 4 * c + i), d, i == 0 ? v[1] : v[0], i <= 1 ? v[2] : v[1],
+          i <= 2 ? v[3] : v[2]);
     }
   }
 }
@@ -267,32 +331,16 @@ __device__ __forceinline__ int elast_packed(int i, int m, int a, int b) {
 //   a != b: (lambda P_ab) vol + (mu P_ba) vol
 // with each product rounded as the reference rounds it.  The products commute,
 // so K is symmetric bit for bit.
-// INT: 0 all on the FP64 pipe, 1 all on the integer pipe, 2 the mu (shear)
-// terms and the final sum on the integer pipe, the rest on the FP64 pipe.
-template <int INT>
 __device__ __forceinline__ double elast_ref_entry(int a, int b, const double P[3][3], double l2m, double lambda,
                                                   double mu, double vol) {
-  auto add1 = [](double x, double y) { return ref::xadd<INT == 1>(x, y); };
-  auto mul1 = [](double x, double y) { return ref::xmul<INT == 1>(x, y); };
-  auto add2 = [](double x, double y) { return ref::xadd<INT != 0>(x, y); };
-  auto mul2 = [](double x, double y) { return ref::xmul<INT != 0>(x, y); };
+  using ref::add;
+  using ref::mul;
   if (a == b) {
-    const double z = a == 0 ? add2(P[1][1], P[2][2]) : (a == 1 ? add2(P[0][0], P[2][2]) : add2(P[1][1], P[0][0]));
-    return add2(mul1(mul1(l2m, P[a][a]), vol), mul2(mul2(mu, z), vol));
+    const double z = a == 0 ? add(P[1][1], P[2][2]) : (a == 1 ? add(P[0][0], P[2][2]) : add(P[1][1], P[0][0]));
+    return add(mul(mul(l2m, P[a][a]), vol), mul(mul(mu, z), vol));
   }
-  return add2(mul1(mul1(lambda, P[a][b]), vol), mul2(mul2(mu, P[b][a]), vol));
+  return add(mul(mul(lambda, P[a][b]), vol), mul(mul(mu, P[b][a]), vol));
 }
-
-// Integer-pipe stages of the reference-rounding elasticity element (as
-// AFEM_REF_INT_STAGES for the Poisson tetrahedron): bit 0 the block entries,
-// bit 1 the gradient products P, bit 2 the gradient numerators, bit 3 only
-// the shear terms of the block entries (when bit 0 is clear).
-#ifndef AFEM_ELAST_INT_STAGES
-#define AFEM_ELAST_INT_STAGES 0
-#endif
-constexpr int kElastIntEntries = (AFEM_ELAST_INT_STAGES & 1) ? 1 : ((AFEM_ELAST_INT_STAGES & 8) ? 2 : 0);
-constexpr bool kElastIntProducts = (AFEM_ELAST_INT_STAGES & 2) != 0;
-constexpr bool kElastIntNumerators = (AFEM_ELAST_INT_STAGES & 4) != 0;
 
 template <int F>
 __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cell0, int nb_cell, const double* __restrict__ xyz,
@@ -336,7 +384,7 @@ __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cel
         n[a][2] = __ldg(p + 2);
       }
       double g[3][4], vol;
-      const double v6 = ref::tet_gradients<false, kElastIntNumerators>(n, g, &vol);
+      const double v6 = ref::tet_gradients(n, g, &vol);
       if (bad && !ref::measure_ok(v6)) atomicOr(bad, kFlagDegenerateCell);
       stage_p[threadIdx.x] = __ldg(reinterpret_cast<const int4*>(inv) + c);
       const double l2m = ref::add(lambda, 2.0 * mu);
@@ -349,12 +397,12 @@ __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cel
 #pragma unroll
           for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) P[a][b] = ref::xmul<kElastIntProducts>(g[a][lo], g[b][hi]);
+            for (int b = 0; b < 3; ++b) P[a][b] = ref::mul(g[a][lo], g[b][hi]);
 #pragma unroll
           for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b)
-              my[pair * 9 + a * 3 + b] = elast_ref_entry<kElastIntEntries>(a, b, P, l2m, lambda, mu, vol);
+              my[pair * 9 + a * 3 + b] = elast_ref_entry(a, b, P, l2m, lambda, mu, vol);
         }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -362,13 +410,13 @@ __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cel
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-          for (int b = a; b < 3; ++b) P[a][b] = P[b][a] = ref::xmul<kElastIntProducts>(g[a][i], g[b][i]);
+          for (int b = a; b < 3; ++b) P[a][b] = P[b][a] = ref::mul(g[a][i], g[b][i]);
         int k = 0;
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
           for (int b = a; b < 3; ++b, ++k)
-            my[54 + i * 6 + k] = elast_ref_entry<kElastIntEntries>(a, b, P, l2m, lambda, mu, vol);
+            my[54 + i * 6 + k] = elast_ref_entry(a, b, P, l2m, lambda, mu, vol);
       }
     } else if (c < nb_cell) {
       // cofactors c_1..c_3 of the edges from node 0 and s = 1 / (6 |det|);
@@ -777,14 +825,6 @@ __constant__ double kHexDN[8][3][8] = {
     {{-kHpm, kHpm, kHpp, -kHpp, -kHmm, kHmm, kHpm, -kHpm}, {-kHpm, -kHpp, kHpp, kHpm, -kHmm, -kHpm, kHpm, kHmm}, {-kHmm, -kHpm, -kHpp, -kHpm, kHmm, kHpm, kHpp, kHpm}},
     {{-kHmm, kHmm, kHpm, -kHpm, -kHpm, kHpm, kHpp, -kHpp}, {-kHmm, -kHpm, kHpm, kHmm, -kHpm, -kHpp, kHpp, kHpm}, {-kHmm, -kHpm, -kHpp, -kHpm, kHmm, kHpm, kHpp, kHpm}}};
 
-// Integer-pipe stages of the reference-rounding Hexa8 element: bit 0 the
-// matrix accumulation, bit 1 the Jacobians.
-#ifndef AFEM_HEX_INT_STAGES
-#define AFEM_HEX_INT_STAGES 0
-#endif
-constexpr bool kHexIntRows = (AFEM_HEX_INT_STAGES & 1) != 0;
-constexpr bool kHexIntJacobian = (AFEM_HEX_INT_STAGES & 2) != 0;
-
 template <int F>
 __global__ void __launch_bounds__(128) k_elem_poisson_hexa8(int cell0, int nb_cell, const double* __restrict__ xyz,
                                                             const int32_t* __restrict__ cn,
@@ -803,7 +843,7 @@ __global__ void __launch_bounds__(128) k_elem_poisson_hexa8(int cell0, int nb_ce
     }
     double K[8][8];
     if constexpr (F != AFEM_FORMULATION_MINIMAL) {
-      const bool ok = ref::hexa8_matrix<kHexIntJacobian, kHexIntRows>(x, y, z, kHexDnRef, K);
+      const bool ok = ref::hexa8_matrix(x, y, z, kHexDnRef, K);
       if (bad && !ok) atomicOr(bad, kFlagDegenerateCell);
       if (coeff) scale_upper<8>(K, __ldg(coeff + c));
       write_rows_q1<8>(K, inv + 8 * c, er);
@@ -1147,8 +1187,8 @@ static afem_status launch_elem_p1(afem_context ctx, const afem_mesh_view* m, int
     return f == AFEM_FORMULATION_TESTLAB
                ? launch(ctx, k_elem_poisson_p1_ref<4, AFEM_FORMULATION_TESTLAB>, ge, 128, 0, c0, c1, m->coords_d,
                         m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad)
-               : launch(ctx, k_elem_poisson_p1_ref<4, AFEM_FORMULATION_REFERENCE>, ge, 128, 0, c0, c1, m->coords_d,
-                        m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad);
+               : launch(ctx, coeff ? k_elem_poisson_tet_ref<true> : k_elem_poisson_tet_ref<false>, ge, kTetBlock, 0, c0,
+                        c1, m->coords_d, m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad);
   return f == AFEM_FORMULATION_TESTLAB
              ? launch(ctx, k_elem_poisson_p1_ref<3, AFEM_FORMULATION_TESTLAB>, ge, 128, 0, c0, c1, m->coords_d,
                       m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad)
@@ -1713,8 +1753,8 @@ extern "C" afem_status afem_assemble_poisson_p1_noalloc(void* cuda_stream, const
   const unsigned gg = (unsigned)((m->nb_node + kGatherBlock - 1) / kGatherBlock);
   int* no_flags = nullptr;
   if (m->dim == 3) {
-    AFEM_TRY(launch_on(s, k_elem_poisson_p1_ref<4, AFEM_FORMULATION_REFERENCE>, ge, 128, 0, m->nb_cell, m->coords_d,
-                       m->cell_nodes_d, m->nc_inverse_d, cell_coeff_d, rows, no_flags));
+    AFEM_TRY(launch_on(s, cell_coeff_d ? k_elem_poisson_tet_ref<true> : k_elem_poisson_tet_ref<false>, ge, kTetBlock, 0,
+                       m->nb_cell, m->coords_d, m->cell_nodes_d, m->nc_inverse_d, cell_coeff_d, rows, no_flags));
     return launch_on(s, k_gather_scalar<4>, gg, kGatherBlock, 0, m->nb_node, m->nc_ptr_d, m->nc_slot_d, row_ptr_d,
                      (const double*)rows, values_d);
   }

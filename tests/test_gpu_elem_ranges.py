@@ -1,0 +1,64 @@
+"""The reference-rounding element kernels whose products run on the integer
+pipe, bit for bit against the oracle where that path has its edges: cells with
+exact zeros (unjittered meshes, coordinates on the axes), coordinates near and
+beyond the range it takes (scaled by powers of two), cells inside and outside
+it in one warp, and cell counts around a warp and a block."""
+import numpy as np
+import pytest
+import torch
+
+from arcanefem_gb300 import fem, meshgen
+from oracle import oracle as O
+from test_gpu_parity import build_format
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def own_ctx():
+    """A context of the test's own: overflowing cells raise its degenerate-cell flag."""
+    ctx = fem.Context()
+    yield ctx
+    ctx.close()
+
+
+def assert_bit_exact(got, ref, what):
+    """Every entry equal; a cell whose products overflow gives NaN in both."""
+    if not np.array_equal(got, ref, equal_nan=True):
+        d = ~((got == ref) | (np.isnan(got) & np.isnan(ref)))
+        k = int(np.argmax(d))
+        raise AssertionError(f"{what}: {int(d.sum())} of {got.size} entries differ; first at {k}: {got[k]!r} vs {ref[k]!r}")
+
+
+def moved_mesh(make, n, jitter, case):
+    m = make(n, jitter=jitter, seed=n)
+    x = m.coords.copy()
+    if case == "mixed":      # scattered tiny and huge coordinates: their cells leave the integer path's range
+        rng = np.random.default_rng(n)
+        some = rng.choice(m.nb_node, max(1, m.nb_node // 12), replace=False)
+        x[some] *= np.where(np.arange(some.size) % 2 == 0, 2.0 ** -104, 2.0 ** 101)[:, None]
+    else:
+        x *= 2.0 ** case
+    return meshgen.Mesh(m.dim, x, m.cells, m.groups)
+
+
+CASES = [(1, 0.15, 0), (3, 0.0, 0), (4, 0.15, -70), (4, 0.0, -97), (4, 0.15, -99), (4, 0.15, 99), (5, 0.15, -120),
+         (5, 0.15, 110), (6, 0.15, "mixed"), (9, 0.15, 0)]
+
+
+def oracle_values(m, kind, coeff=None, **kw):
+    ptr, nc, _ = O.node_cell(m.nb_node, m.cells)
+    rp, cols = O.sparsity(m.nb_node, m.cells)
+    with np.errstate(all="ignore"):
+        return O.assemble(kind, m.coords, m.cells, ptr, nc, rp, cols, cell_coeff=coeff, **kw)
+
+
+@pytest.mark.parametrize("n,jitter,case", CASES)
+def test_tetrahedra_over_the_operand_ranges(own_ctx, n, jitter, case):
+    m = moved_mesh(meshgen.unit_cube_tet, n, jitter, case)
+    f = build_format(own_ctx, m)
+    f.assemble_poisson()
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_TET4), "tetrahedra")
+    k = np.exp(np.random.default_rng(0).standard_normal(m.nb_cell))
+    f.assemble_poisson(torch.as_tensor(k, device="cuda"))
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_TET4, coeff=k), "coefficient")
