@@ -1,0 +1,800 @@
+// Conjugate gradients in one launch, for systems whose vectors fit the
+// register files: a cooperative grid of at most one block per SM, every
+// thread owning up to K rows for the whole solve.
+//
+// What bounds the launches per iteration of the general path is not the work
+// but the gaps: at 66 k rows an iteration took 17.4 us in three kernels,
+// against 1.9 us of FP64 issue.  Here
+//   * x, r, D^-1, p, q of a thread's rows stay in registers (for K > 4 only
+//     r, D^-1 and q do), so that an iteration's vector updates move nothing;
+//   * the matrix sits in shared memory as 32-row slices, as many of a block's
+//     as fit (12 B an entry: 2.8 M entries on the chip); the others are read
+//     from the sliced copy in global memory, or from the CSR rows;
+//   * only the direction (FP64) or z (FP32) goes through global memory, since
+//     other blocks gather it;
+//   * the blocks meet in all-to-all exchanges: a block publishes its partial
+//     sum and the exchange's number in one 16-byte slot, and each block polls
+//     all slots and adds them in the same fixed order.  Every block takes the
+//     same decisions, results are deterministic, and no exchange pays an
+//     atomic's queue or a second trip for a flag.
+// Every wait is bounded; one that runs out sets *err and ends all blocks.
+#pragma once
+#include "afem_krylov.cuh"
+
+namespace afem {
+
+struct CgState {
+  double rz, rr, pq, alpha, beta, bnorm2, tol2, pad0;
+  int done, iter, status, max_iter;
+  unsigned int ticket[4];
+};
+
+constexpr int kResThreads = 512;
+constexpr int kResMaxRows = 6;                 // rows a thread owns at most
+constexpr int kResSpins = 4000000;             // polls of a wait, about 2 s
+constexpr int kSlotStride = 8;                  // slots of 16 B a cache line of its own apart
+constexpr size_t kResSmem = 226 * 1024;        // dynamic shared memory of a block
+
+// A slot: the value's bits and the number of the exchange it belongs to.
+__device__ __forceinline__ void slot_put(ulonglong2* s, unsigned long long v, unsigned long long epoch) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], t;\n\t}"
+               :: "l"(v), "l"(epoch), "l"(s) : "memory");
+}
+__device__ __forceinline__ ulonglong2 slot_get(const ulonglong2* s) {
+  ulonglong2 r;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(r.x), "=l"(r.y) : "l"(s) : "memory");
+  return r;
+}
+
+// The blocks' exchanges.  Slots are double-buffered by the exchange's parity:
+// a block can be one exchange ahead of another's polling, never two.  FENCE:
+// what the block's threads wrote before is visible to every block afterwards
+// (a release before the put, an acquire after the polls).
+struct Grid {
+  ulonglong2* slots;          // [2 parities][2 values][gridDim.x] lines, zero at the launch
+  double* sh;                 // shared, res_scratch(gridDim.x) doubles
+  int* err;
+  unsigned long long epoch = 0;
+
+  // Publish the values that threads 0 (and 32 for the second) of the block hold, poll everyone's into sh.
+  // Returns false in every thread if a wait ran out.  Ends with a block barrier.
+  template <int V, bool FENCE>
+  __device__ __forceinline__ bool meet(double v) {
+    ++epoch;
+    const int nb = gridDim.x;
+    ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
+    if constexpr (FENCE) __syncthreads();
+    if (threadIdx.x < 32 * V && (threadIdx.x & 31) == 0) {
+      if constexpr (FENCE) __threadfence();
+      slot_put(at + ((threadIdx.x >> 5) * nb + blockIdx.x) * kSlotStride, __double_as_longlong(v), epoch);
+    }
+    int bad = 0;
+    for (int i = threadIdx.x; i < V * nb; i += kResThreads) {
+      ulonglong2 s = slot_get(at + i * kSlotStride);
+      int spins = 0;
+      while (s.y != epoch) {
+        if (++spins >= kResSpins || ((spins & 1023) == 0 && *(volatile int*)err)) {
+          atomicCAS(err, 0, (int)AFEM_ERR_TIMEOUT);
+          bad = 1;
+          break;
+        }
+        s = slot_get(at + i * kSlotStride);
+      }
+      sh[i] = __longlong_as_double(s.x);
+    }
+    if constexpr (FENCE)
+      if (threadIdx.x < V * nb) __threadfence();   // the pollers acquire for the block
+    return __syncthreads_or(bad) == 0;
+  }
+
+  // total of sh[v * gridDim.x ..] for the warp v that calls it, in every lane
+  __device__ __forceinline__ double total(int v) const {
+    const int nb = gridDim.x, lane = threadIdx.x & 31;
+    double s = 0.0;
+    for (int i = lane; i < nb; i += 32) s += sh[v * nb + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  }
+};
+
+inline size_t res_scratch_doubles(unsigned grid) { return std::max<size_t>(2 * kResThreads, 2 * grid); }
+
+// Block sums of V FP64 values a thread; value v's ends in the lanes of warp v.
+// GB300 takes as long for a warp's FP64 instruction however many lanes take
+// part, so the sums go through shared memory with full warps first.
+template <int V>
+__device__ __forceinline__ double res_block_sum(const double (&v)[V], double* sh) {
+  constexpr int T = kResThreads, W = 128 / V;   // four warps add, 128 / V threads per value
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < V; ++j) sh[j * T + t] = v[j];
+  __syncthreads();
+  double s = 0.0;
+  if (t < 128) {
+    const double* p = sh + (t / W) * T + t % W;
+    s = p[0];
+#pragma unroll
+    for (int m = 1; m < T / W; ++m) s += p[m * W];
+  }
+  __syncthreads();
+  if (t < 128) sh[t] = s;
+  __syncthreads();
+  if (t < 32 * V) {
+    const double* p = sh + (t >> 5) * W + (t & 31);
+    s = p[0];
+#pragma unroll
+    for (int m = 1; m < W / 32; ++m) s += p[m * 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
+  __syncthreads();   // meet() writes sh
+  return s;
+}
+
+// The same of FP32 values, warps summed in FP32 and their totals in FP64.
+template <int V>
+__device__ __forceinline__ double res_block_sum_f(const float (&v)[V], double* sh) {
+  constexpr int NW = kResThreads / 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    float s = v[j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) sh[j * NW + w] = (double)s;
+  }
+  __syncthreads();
+  double s = 0.0;
+  if (w < V) {
+    s = sh[w * NW + (lane & (NW - 1))];
+#pragma unroll
+    for (int o = NW / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
+  __syncthreads();
+  return s;
+}
+
+struct ResCtl {
+  double alpha, beta;
+  int done, status;
+};
+
+// The slices of a block's rows that its shared memory holds, filled from the
+// CSR rows (a negative column is an unused slot and becomes a zero weight on
+// the row itself, as past the end of a row).
+template <class T>
+struct ResMatrix {
+  int32_t* off;    // [slices + 1] first step of each slice
+  T* vals;
+  int32_t* cols;
+  int steps;       // steps of 32 entries that fit
+
+  __device__ __forceinline__ bool resident(int s) const { return off[s + 1] <= steps; }
+
+  // off[] from the row lengths; every thread calls it
+  __device__ __forceinline__ void offsets(int nslice, int r0, int r1, const int32_t* __restrict__ rp) {
+    for (int s = threadIdx.x >> 5; s < nslice; s += kResThreads / 32) {
+      const int row = r0 + 32 * s + (threadIdx.x & 31);
+      const int len = row < r1 ? __ldg(rp + row + 1) - __ldg(rp + row) : 0;
+      const int m = __reduce_max_sync(0xffffffffu, len);
+      if ((threadIdx.x & 31) == 0) off[s + 1] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      off[0] = 0;
+      for (int s = 0; s < nslice; ++s) off[s + 1] += off[s];
+    }
+    __syncthreads();
+  }
+  __device__ __forceinline__ void fill(int s, int row, int r1, const int32_t* __restrict__ rp,
+                                       const int32_t* __restrict__ gcols, const double* __restrict__ gvals) {
+    const int m = off[s + 1] - off[s], at = 32 * off[s] + (threadIdx.x & 31);
+    const int32_t b = row < r1 ? __ldg(rp + row) : 0, e = row < r1 ? __ldg(rp + row + 1) : 0;
+    for (int k = 0; k < m; ++k) {
+      const int32_t c = b + k < e ? __ldg(gcols + b + k) : -1;
+      cols[at + 32 * k] = c >= 0 ? c : (row < r1 ? row : 0);
+      vals[at + 32 * k] = c >= 0 ? (T)__ldg(gvals + b + k) : T(0);
+    }
+  }
+};
+
+// Sum of a row's products in CSR order.  x is written by other blocks between
+// the exchanges: plain loads, not the read-only path.  STEP: entries of a row
+// are that many apart.
+// A chunk's gathers are issued with the next chunk's columns and values, so
+// that a row pays one memory latency a chunk.
+constexpr int kResChunk = 8;
+template <int STEP, bool SHARED, class T>
+__device__ __forceinline__ T res_row_dot(const int32_t* c, const T* a, int m, const T* x) {
+  T acc = T(0);
+  int32_t cc[kResChunk];
+  T aa[kResChunk];
+  auto load = [&](int k) {
+#pragma unroll
+    for (int u = 0; u < kResChunk; ++u) {
+      const int e = (k + u < m ? k + u : 0) * STEP;
+      cc[u] = SHARED ? c[e] : __ldg(c + e);
+      aa[u] = SHARED ? a[e] : __ldg(a + e);
+    }
+  };
+  if (m > 0) load(0);
+  for (int k = 0; k < m; k += kResChunk) {
+    T xx[kResChunk], av[kResChunk];
+#pragma unroll
+    for (int u = 0; u < kResChunk; ++u) {
+      xx[u] = x[cc[u]];
+      av[u] = aa[u];
+    }
+    if (k + kResChunk < m) load(k + kResChunk);
+#pragma unroll
+    for (int u = 0; u < kResChunk; ++u)
+      if (k + u < m) acc = fma(av[u], xx[u], acc);
+  }
+  return acc;
+}
+// straight from the CSR row (slices that do not fit where no sliced copy was made)
+template <class T>
+__device__ __forceinline__ T res_row_dot_csr(int row, const int32_t* __restrict__ rp,
+                                             const int32_t* __restrict__ cols, const double* __restrict__ vals,
+                                             const T* x) {
+  T acc = T(0);
+  const int32_t e = __ldg(rp + row + 1);
+  for (int32_t k = __ldg(rp + row); k < e; ++k) {
+    const int32_t c = __ldg(cols + k);
+    if (c >= 0) acc = fma((T)__ldg(vals + k), x[c], acc);
+  }
+  return acc;
+}
+
+// FP64 CG, up to `iters` iterations: the arithmetic of k_cg_spmv_sl,
+// k_cg_update and k_cg_dir row by row; the dot products' partial sums are
+// per thread, block and grid.  x, r, p carry the state in and out (with st),
+// so that a long solve is a few launches.
+struct CgResident {
+  int n, rows_pb, iters, steps;          // rows of a block (a multiple of 32), steps of shared memory
+  const int32_t *rp, *cols;              // CSR
+  const double* vals;
+  const int32_t *soff, *scols;           // sliced copy, or null
+  const double* svals;
+  const double* dinv;                    // or null
+  const uint8_t* skip;                   // or null
+  double *x, *r, *p;
+  ulonglong2* slots;
+  int* err;
+  CgState* st;
+};
+
+template <int K>
+__global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident a) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ ResCtl ctl;
+  __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
+  if (((volatile CgState*)a.st)->done) return;
+  const int nb = gridDim.x, lane = threadIdx.x & 31;
+  Grid grid;
+  grid.slots = a.slots;
+  grid.sh = reinterpret_cast<double*>(dyn);
+  grid.err = a.err;
+  ResMatrix<double> mat;
+  mat.off = soff_sh;
+  mat.vals = grid.sh + (2 * kResThreads > 2 * nb ? 2 * kResThreads : 2 * nb);
+  mat.cols = reinterpret_cast<int32_t*>(mat.vals + 32 * (size_t)a.steps);
+  mat.steps = a.steps;
+  const int r0 = blockIdx.x * a.rows_pb, r1 = min(a.n, r0 + a.rows_pb);
+  mat.offsets(a.rows_pb / 32, r0, r1, a.rp);
+
+  constexpr bool kAll = K <= 4;          // x and p in registers too
+  double r[K], d[K], q[K], x[kAll ? K : 1], p[kAll ? K : 1];
+  unsigned counted = 0;                  // bit k: the row enters the stop test's norm
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = k * kResThreads + threadIdx.x, row = r0 + i;
+    r[k] = d[k] = q[k] = 0.0;
+    if constexpr (kAll) x[k] = p[k] = 0.0;
+    if (i < a.rows_pb && mat.resident(i >> 5)) mat.fill(i >> 5, row, r1, a.rp, a.cols, a.vals);
+    if (i < a.rows_pb && row < r1) {
+      r[k] = a.r[row];
+      d[k] = a.dinv ? __ldg(a.dinv + row) : 1.0;
+      if constexpr (kAll) {
+        x[k] = a.x[row];
+        p[k] = a.p[row];
+      }
+      if (!(a.skip && a.skip[row])) counted |= 1u << k;
+    }
+  }
+  __syncthreads();
+  double rz = a.st->rz;                  // thread 0's is the one in use
+  const double tol2 = a.st->tol2;
+  const int max_iter = a.st->max_iter, iter0 = a.st->iter;
+  int it = 0;
+  for (;;) {
+    // q = A p ; <p, q> -> alpha
+    double pq[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = k * kResThreads + threadIdx.x, row = r0 + i;
+      if (i < a.rows_pb) {
+        const int s = i >> 5, m = mat.off[s + 1] - mat.off[s];   // 0 past the matrix's last slice
+        if (mat.resident(s) || m == 0)
+          q[k] = res_row_dot<32, true>(mat.cols + 32 * mat.off[s] + lane, mat.vals + 32 * mat.off[s] + lane, m, a.p);
+        else if (a.scols) {
+          const int64_t at = (int64_t)kSlice * __ldg(a.soff + (row >> 5)) + lane;
+          q[k] = res_row_dot<kSlice, false>(a.scols + at, a.svals + at, m, a.p);
+        } else if (row < r1)
+          q[k] = res_row_dot_csr<double>(row, a.rp, a.cols, a.vals, a.p);
+        if (row < r1) pq[0] += (kAll ? p[kAll ? k : 0] : a.p[row]) * q[k];
+      }
+    }
+    const double bpq = res_block_sum<1>(pq, grid.sh);
+    if (!grid.template meet<1, false>(bpq)) return;
+    if (threadIdx.x < 32) {
+      const double t = grid.total(0);
+      if (threadIdx.x == 0) {
+        const bool ok = t > 0.0 && isfinite(t);
+        ctl.alpha = ok ? rz / t : 0.0;
+        ctl.status = ok ? AFEM_OK : AFEM_ERR_BREAKDOWN;
+        ctl.done = !ok;
+        if (blockIdx.x == 0) a.st->pq = t;
+      }
+    }
+    __syncthreads();
+    if (ctl.done) break;
+    // x += alpha p ; r -= alpha q ; z = D^-1 r ; <r, z>, <r, r> -> beta, stop test
+    const double alpha = ctl.alpha;
+    double rs[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = k * kResThreads + threadIdx.x, row = r0 + i;
+      if (i < a.rows_pb && row < r1) {
+        if constexpr (kAll) x[k] += alpha * p[k];
+        else a.x[row] += alpha * a.p[row];
+        r[k] = r[k] - alpha * q[k];
+        q[k] = d[k] * r[k];
+        rs[0] += r[k] * q[k];
+        if (counted >> k & 1) rs[1] += r[k] * r[k];
+      }
+    }
+    const double brs = res_block_sum<2>(rs, grid.sh);
+    if (!grid.template meet<2, false>(brs)) return;
+    ++it;
+    if (threadIdx.x < 64) {
+      const double t = grid.total(threadIdx.x >> 5);
+      if (threadIdx.x == 0) {
+        ctl.beta = t / rz;
+        rz = t;
+      } else if (threadIdx.x == 32) {
+        int done = 0, status = AFEM_OK;
+        if (!isfinite(t)) {
+          status = AFEM_ERR_BREAKDOWN;
+          done = 1;
+        } else if (t <= tol2) {
+          done = 1;
+        } else if (iter0 + it >= max_iter) {
+          status = AFEM_ERR_NOT_CONVERGED;
+          done = 1;
+        }
+        ctl.done = done;
+        ctl.status = status;
+        if (blockIdx.x == 0) a.st->rr = t;
+      }
+    }
+    __syncthreads();
+    if (ctl.done) break;
+    // p = z + beta p
+    const double beta = ctl.beta;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = k * kResThreads + threadIdx.x, row = r0 + i;
+      if (i < a.rows_pb && row < r1) {
+        const double pn = q[k] + beta * (kAll ? p[kAll ? k : 0] : a.p[row]);
+        if constexpr (kAll) p[k] = pn;
+        a.p[row] = pn;
+      }
+    }
+    if (it == a.iters) break;
+    if (!grid.template meet<1, true>(0.0)) return;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = k * kResThreads + threadIdx.x, row = r0 + i;
+    if (i < a.rows_pb && row < r1) {
+      a.r[row] = r[k];
+      if constexpr (kAll) a.x[row] = x[k];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.st->rz = rz;
+    a.st->iter = iter0 + it;
+    a.st->status = ctl.status;
+    a.st->done = ctl.done;
+  }
+}
+
+// A 3x3-block matrix in FP32 as k_cgf_spmv_b3s reads it: slices of 32 block
+// rows, one column index and nine value planes a step.
+struct ResMatrix3 {
+  int32_t* off;
+  float* vals;
+  int32_t* cols;
+  int steps;
+
+  __device__ __forceinline__ bool resident(int s) const { return off[s + 1] <= steps; }
+  __device__ __forceinline__ void offsets(int nslice, int I0, int I1, const int32_t* __restrict__ rp) {
+    for (int s = threadIdx.x >> 5; s < nslice; s += kResThreads / 32) {
+      const int I = I0 + 32 * s + (threadIdx.x & 31);
+      const int len = I < I1 ? (__ldg(rp + 3 * I + 1) - __ldg(rp + 3 * I)) / 3 : 0;
+      const int m = __reduce_max_sync(0xffffffffu, len);
+      if ((threadIdx.x & 31) == 0) off[s + 1] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      off[0] = 0;
+      for (int s = 0; s < nslice; ++s) off[s + 1] += off[s];
+    }
+    __syncthreads();
+  }
+  // component c's planes of slice s, and the columns with component 0
+  __device__ __forceinline__ void fill(int s, int c, int I, int I1, const int32_t* __restrict__ rp,
+                                       const int32_t* __restrict__ bcols, const double* __restrict__ gvals) {
+    const int m = off[s + 1] - off[s], lane = threadIdx.x & 31;
+    const int32_t b0 = I < I1 ? __ldg(rp + 3 * I) : 0, bc = I < I1 ? __ldg(rp + 3 * I + c) : 0;
+    const int nbk = I < I1 ? (__ldg(rp + 3 * I + 1) - b0) / 3 : 0;
+    for (int k = 0; k < m; ++k) {
+      const bool in = k < nbk;
+      const size_t e = 32 * (size_t)(off[s] + k);
+      if (c == 0) cols[e + lane] = in ? __ldg(bcols + b0 / 9 + k) : (I < I1 ? I : 0);
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+        vals[e * 9 + (3 * c + b) * 32 + lane] = in ? (float)__ldg(gvals + bc + 3 * k + b) : 0.f;
+    }
+  }
+};
+
+// One scalar row of a block slice (c: its first block column, v: the first
+// value plane of its component), in the order of k_cgf_spmv_b3s.
+template <bool SHARED>
+__device__ __forceinline__ float res_row_dot3(const int32_t* c, const float* v, int m, const float* z) {
+  constexpr int kChunk = 3;
+  float acc = 0.f;
+  for (int kb = 0; kb < m; kb += kChunk) {
+    int32_t j[kChunk];
+    float x[3 * kChunk], zz[3 * kChunk];
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      const int e = kb + u < m ? kb + u : 0;
+      j[u] = 3 * (SHARED ? c[32 * e] : __ldg(c + 32 * e));
+#pragma unroll
+      for (int b = 0; b < 3; ++b) x[3 * u + b] = SHARED ? v[288 * e + 32 * b] : __ldg(v + 288 * (int64_t)e + 32 * b);
+    }
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) zz[3 * u + b] = z[j[u] + b];
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u)
+      if (kb + u < m)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) acc = fmaf(x[3 * u + b], zz[3 * u + b], acc);
+  }
+  return acc;
+}
+
+__device__ __forceinline__ float res_row_dot3_csr(int I, int c, const int32_t* __restrict__ rp,
+                                                  const int32_t* __restrict__ bcols, const double* __restrict__ vals,
+                                                  const float* z) {
+  float acc = 0.f;
+  const int32_t b0 = __ldg(rp + 3 * I), b = __ldg(rp + 3 * I + c), len = __ldg(rp + 3 * I + 1) - b0;
+  for (int32_t k = 0; k < len; ++k)
+    acc = fmaf((float)__ldg(vals + b + k), z[3 * __ldg(bcols + b0 / 9 + k / 3) + k % 3], acc);
+  return acc;
+}
+
+// The FP32 inner CG of the mixed solver, up to `iters` iterations: the
+// arithmetic of k_cgf_spmv_sl / k_cgf_spmv_b3s (w = A z, p = z + beta p,
+// q = w + beta q) and k_cgf_update row by row.  B3: a warp takes one
+// component of 32 block rows, and rows_pb counts block rows.
+struct CgfResident {
+  int n, rows_pb, iters, steps;
+  const int32_t *rp, *cols;              // CSR; B3: the block columns
+  const double* vals;
+  const int32_t *soff, *scols;           // sliced copy, or null
+  const float* svals;
+  const float* dinv;
+  const uint8_t* skip;
+  float *x, *r, *z, *p, *q;
+  ulonglong2* slots;
+  int* err;
+  CgState* st;
+};
+
+template <int K, bool B3>
+__global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfResident a) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ ResCtl ctl;
+  __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
+  if (((volatile CgState*)a.st)->done) return;
+  const int nb = gridDim.x, lane = threadIdx.x & 31;
+  Grid grid;
+  grid.slots = a.slots;
+  grid.sh = reinterpret_cast<double*>(dyn);
+  grid.err = a.err;
+  std::conditional_t<B3, ResMatrix3, ResMatrix<float>> mat;
+  mat.off = soff_sh;
+  mat.vals = reinterpret_cast<float*>(grid.sh + (2 * kResThreads > 2 * nb ? 2 * kResThreads : 2 * nb));
+  mat.cols = reinterpret_cast<int32_t*>(mat.vals + (B3 ? 288 : 32) * (size_t)a.steps);
+  mat.steps = a.steps;
+  constexpr int C = B3 ? 3 : 1;
+  const int rows = a.n / C;              // rows, or block rows
+  const int r0 = blockIdx.x * a.rows_pb, r1 = min(rows, r0 + a.rows_pb);
+  mat.offsets(a.rows_pb / 32, r0, r1, a.rp);
+  const int units = C * a.rows_pb / 32;  // warps' worth of rows
+
+  // unit of slot k: (slice, component) and the lane's row or block row
+  auto unit = [&](int k) { return k * (kResThreads / 32) + (int)(threadIdx.x >> 5); };
+  float r[K], d[K], x[K], p[K], q[K], z[K];
+  unsigned counted = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int u = unit(k), s = u / C, c = u - C * s, I = r0 + 32 * s + lane, row = C * I + c;
+    r[k] = d[k] = x[k] = p[k] = q[k] = z[k] = 0.f;
+    if (u < units) {
+      if (mat.resident(s)) {
+        if constexpr (B3) mat.fill(s, c, I, r1, a.rp, a.cols, a.vals);
+        else mat.fill(s, row, r1, a.rp, a.cols, a.vals);
+      }
+      if (I < r1) {
+        r[k] = a.r[row];
+        d[k] = __ldg(a.dinv + row);
+        x[k] = a.x[row];
+        z[k] = a.z[row];
+        p[k] = a.p[row];
+        q[k] = a.q[row];
+        if (!(a.skip && a.skip[row])) counted |= 1u << k;
+      }
+    }
+  }
+  __syncthreads();
+  double rz = a.st->rz, rz_prev = 0.0, rr = 0.0;   // threads 0 (rz) and 32 (rr) keep them
+  float beta = (float)a.st->beta;
+  double beta64 = 0.0;
+  const double tol2 = a.st->tol2;
+  const int max_iter = a.st->max_iter, iter0 = a.st->iter;
+  int it = 0;
+  for (;;) {
+    float pq[1] = {0.f};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int u = unit(k), s = u / C, c = u - C * s, I = r0 + 32 * s + lane;
+      if (u < units) {
+        const int m = mat.off[s + 1] - mat.off[s];
+        float w;
+        if (mat.resident(s) || m == 0) {   // 0: past the matrix's last slice
+          const int32_t* mc = mat.cols + 32 * (size_t)mat.off[s] + lane;
+          if constexpr (B3) w = res_row_dot3<true>(mc, mat.vals + 288 * (size_t)mat.off[s] + 96 * c + lane, m, a.z);
+          else w = res_row_dot<32, true>(mc, mat.vals + 32 * mat.off[s] + lane, m, a.z);
+        } else if (!a.scols) {
+          w = 0.f;
+          if (I < r1) {
+            if constexpr (B3) w = res_row_dot3_csr(I, c, a.rp, a.cols, a.vals, a.z);
+            else w = res_row_dot_csr<float>(I, a.rp, a.cols, a.vals, a.z);
+          }
+        } else {
+          const int64_t at = (int64_t)kSlice * __ldg(a.soff + (r0 >> 5) + s);
+          if constexpr (B3) w = res_row_dot3<false>(a.scols + at + lane, a.svals + 9 * at + 96 * c + lane, m, a.z);
+          else w = res_row_dot<kSlice, false>(a.scols + at + lane, a.svals + at + lane, m, a.z);
+        }
+        if (I < r1) {
+          p[k] = beta != 0.f ? fmaf(beta, p[k], z[k]) : z[k];
+          q[k] = beta != 0.f ? fmaf(beta, q[k], w) : w;
+          pq[0] = fmaf(p[k], q[k], pq[0]);
+        }
+      }
+    }
+    const double bpq = res_block_sum_f<1>(pq, grid.sh);
+    if (!grid.template meet<1, false>(bpq)) return;
+    if (threadIdx.x < 32) {
+      const double t = grid.total(0);
+      if (threadIdx.x == 0) {
+        const bool ok = t > 0.0 && isfinite(t);
+        ctl.alpha = ok ? rz / t : 0.0;
+        ctl.status = ok ? AFEM_OK : AFEM_ERR_BREAKDOWN;
+        ctl.done = !ok;
+      }
+    }
+    __syncthreads();
+    if (ctl.done) break;
+    const float alpha = (float)ctl.alpha;
+    float rs[2] = {0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int u = unit(k), s = u / C, c = u - C * s, I = r0 + 32 * s + lane;
+      if (u < units && I < r1) {
+        x[k] = fmaf(alpha, p[k], x[k]);
+        r[k] = fmaf(-alpha, q[k], r[k]);
+        z[k] = d[k] * r[k];
+        a.z[C * I + c] = z[k];
+        rs[0] = fmaf(r[k], z[k], rs[0]);
+        if (counted >> k & 1) rs[1] = fmaf(r[k], r[k], rs[1]);
+      }
+    }
+    const double brs = res_block_sum_f<2>(rs, grid.sh);
+    if (!grid.template meet<2, true>(brs)) return;
+    ++it;
+    if (threadIdx.x < 64) {
+      const double t = grid.total(threadIdx.x >> 5);
+      if (threadIdx.x == 0) {
+        beta64 = t / rz;
+        ctl.beta = beta64;
+        rz_prev = rz;
+        rz = t;
+      } else if (threadIdx.x == 32) {
+        rr = t;
+        ctl.status = isfinite(t) ? AFEM_OK : AFEM_ERR_BREAKDOWN;
+        ctl.done = !isfinite(t) || t <= tol2 || iter0 + it >= max_iter;
+      }
+    }
+    __syncthreads();
+    beta = (float)ctl.beta;
+    if (ctl.done || it == a.iters) break;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int u = unit(k), s = u / C, c = u - C * s, I = r0 + 32 * s + lane, row = C * I + c;
+    if (u < units && I < r1) {
+      a.x[row] = x[k];
+      a.r[row] = r[k];
+      a.p[row] = p[k];
+      a.q[row] = q[k];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 32 && it > 0) a.st->rr = rr;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (it > 0) {
+      a.st->beta = beta64;
+      a.st->pad0 = rz_prev;
+      a.st->rz = rz;
+    }
+    a.st->iter = iter0 + it;
+    a.st->status = ctl.status;
+    a.st->done = ctl.done;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Host side.
+
+// The split of `rows` rows of C components over the blocks.  At least 128
+// scalar rows a block (one warp for each of an SM's four partitions): below
+// that an exchange costs more than the rows.
+struct ResPlan {
+  unsigned grid = 0;
+  int rows_pb = 0, K = 0, steps = 0;
+  bool fits = false;     // every slice is likely to fit the shared memory
+  bool take = false;     // this form rather than the launches per iteration
+};
+
+// Where the line lies: one block an SM has the loads in flight for what the
+// shared memory leaves over of a matrix up to about 80 MB (L2-resident), and
+// registers for 6 rows a thread.  A solve, three launches an iteration against
+// this form: 2D triangles 256^2 19.2 -> 9.6 ms, 600^2 98.5 -> 43.2; tetrahedra
+// 57^3 8.8 -> 4.3, 75^3 17.7 -> 9.7; hexahedra 69^3 (34 MB left over)
+// 11.2 -> 7.1; elasticity 40^3 (77 MB left over) 50.8 -> 30.1, mixed
+// 35.1 -> 15.1.  Above, with 8 rows a thread: tetrahedra 84^3 23.7 -> 20.2, but
+// renumbered at random 28.1 -> 34.2; hexahedra 84^3 17.9 -> 20.4.
+// A matrix whose rows gather at random lives on what the L1 keeps of the
+// gathered vector, and here shared memory takes most of the L1: with
+// kResScatterEntries and more of them the launches win (random numbering,
+// launches -> this form: triangles 600^2, 2.5 M entries, 105 -> 73 ms;
+// hexahedra 50^3, 3.6 M, mixed 5.1 -> 5.2; 66^3, 8.1 M, 11.2 -> 12.0).
+constexpr int64_t kResScatterEntries = 3300000;
+constexpr int64_t kResStreamBytes = 80ll << 20;
+
+inline ResPlan res_plan(afem_context ctx, int rows, int C, int64_t nnz, size_t step_bytes) {
+  ResPlan p;
+  const int64_t want = std::min<int64_t>(ctx->sm_count, ((int64_t)rows * C + 127) / 128);
+  const int64_t pb = (rows + want - 1) / want;
+  p.rows_pb = (int)((pb + 31) / 32 * 32);
+  p.grid = (unsigned)((rows + p.rows_pb - 1) / p.rows_pb);
+  p.K = (int)(((int64_t)C * p.rows_pb + kResThreads - 1) / kResThreads);
+  p.steps = (int)((kResSmem - sizeof(double) * res_scratch_doubles(p.grid)) / step_bytes);
+  // rows of a slice differ in length and the last block may be short: one step in ten for the padding
+  p.take = p.K <= kResMaxRows &&
+           (int64_t)(nnz / (C * C) * (step_bytes / 32)) - (int64_t)p.grid * (int64_t)kResSmem <= kResStreamBytes;
+  p.fits = (double)nnz / (C * C) <= 0.9 * 32.0 * p.steps * p.grid;
+  return p;
+}
+
+// Samples slices of 32 rows: counts[0] entries seen, counts[1] those more than
+// 64 columns from the same entry of the row before.
+static __global__ void k_scatter_sample(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ cols,
+                                        int32_t* counts) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x / 32);
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  const int64_t row = (int64_t)w * (n / 32) / warps * 32 + lane;
+  const int32_t b = row < n ? __ldg(rp + row) : 0, e = row < n ? __ldg(rp + row + 1) : 0;
+  const int m = __reduce_min_sync(0xffffffffu, e - b);
+  int far = 0;
+  for (int k = 0; k < m; ++k) {
+    const int32_t c = __ldg(cols + b + k), before = __shfl_up_sync(0xffffffffu, c, 1);
+    far += __popc(__ballot_sync(0xffffffffu, lane > 0 && abs(c - before) > 64));
+  }
+  if (lane == 0 && m > 0) {
+    atomicAdd(counts, 31 * m);
+    atomicAdd(counts + 1, far);
+  }
+}
+
+// Whether the gathers of the rows are mostly scattered (one synchronising read).
+inline afem_status res_scattered(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, int32_t* counts,
+                                 bool* scattered) {
+  struct Two {
+    int32_t seen, far;
+  } c{};
+  AFEM_CUDA(cudaMemsetAsync(counts, 0, sizeof(Two), ctx->stream));
+  AFEM_TRY(launch(ctx, k_scatter_sample, 64, 256, 0, n, rp, cols, counts));
+  AFEM_TRY(read_scalar(ctx, reinterpret_cast<const Two*>(counts), &c));
+  *scattered = 2 * (int64_t)c.far > c.seen;
+  return AFEM_OK;
+}
+
+inline size_t res_slots_bytes(const ResPlan& p) { return align256(sizeof(ulonglong2) * 4 * kSlotStride * p.grid); }
+
+// Iterations of one launch, for some 10 ms of work by the largest of the
+// exchanges, the entries and the rows.
+inline int res_launch_iters(int n, int64_t nnz) {
+  return (int)std::max<int64_t>(64, 4000000000ll / (nnz + 20ll * n + 2000000ll));
+}
+
+template <class Args>
+afem_status launch_resident(afem_context ctx, void (*k)(const Args), const ResPlan& p, const Args& a) {
+  AFEM_CUDA(cudaMemsetAsync(a.slots, 0, res_slots_bytes(p), ctx->stream));
+  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(p.grid);
+  lc.blockDim = dim3(kResThreads);
+  lc.dynamicSmemBytes = kResSmem;
+  lc.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  AFEM_CUDA(cudaLaunchKernelEx(&lc, k, a));
+  ++ctx->launches;
+  return AFEM_OK;
+}
+
+template <class F>
+afem_status dispatch_rows(int K, F&& f) {
+  switch (K) {
+    case 1: return f(std::integral_constant<int, 1>{});
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 3: return f(std::integral_constant<int, 3>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    default: return f(std::integral_constant<int, kResMaxRows>{});
+  }
+}
+
+// Launch until the state says done; *hs is the final state.  A wait that ran
+// out leaves the slots' owner with AFEM_ERR_TIMEOUT.
+template <class Launch>
+afem_status run_resident(afem_context ctx, CgState* st, int* err, CgState* hs, Launch&& go) {
+  struct Both {
+    CgState s;
+    int err;
+  };
+  for (;;) {
+    AFEM_TRY(go());
+    auto* h = reinterpret_cast<Both*>(ctx->pinned);
+    AFEM_CUDA(cudaMemcpyAsync(&h->s, st, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+    AFEM_CUDA(cudaMemcpyAsync(&h->err, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    AFEM_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (h->err) return fail((afem_status)h->err, "CG: a grid exchange ran out of time (status %d)", h->err);
+    *hs = h->s;
+    if (hs->done) return AFEM_OK;
+  }
+}
+
+}  // namespace afem

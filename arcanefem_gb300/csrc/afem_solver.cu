@@ -5,8 +5,9 @@
 // femutils/DoFLinearSystem.cc:151-159).  Diagonal (Jacobi) preconditioned CG
 // with HYPRE's two-norm stop ||r|| <= max(rtol ||b||, atol).
 //
-// Layout of one iteration (3 kernels, captured in a CUDA graph per chunk of
-// iterations):
+// Systems whose vectors fit the register files run in one cooperative launch
+// (afem_cg_resident.cuh).  Layout of one iteration of the others (3 kernels,
+// captured in a CUDA graph per chunk of iterations):
 //   K1  q = A p, <p, q>           -> alpha        (last-block finalize)
 //   K2  x += alpha p, r -= alpha q, z = D^-1 r, <r, z>, <r, r> -> beta, stop
 //   K3  p = z + beta p
@@ -30,15 +31,9 @@
 #include <algorithm>
 #include <cmath>
 
-#include "afem_krylov.cuh"
+#include "afem_cg_resident.cuh"
 
 namespace afem {
-
-struct CgState {
-  double rz, rr, pq, alpha, beta, bnorm2, tol2, pad0;
-  int done, iter, status, max_iter;
-  unsigned int ticket[4];
-};
 
 template <int G>
 __global__ void __launch_bounds__(kSolveBlock) k_spmv(int n, const int32_t* __restrict__ rp,
@@ -647,10 +642,25 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
   const unsigned grid_vec = grid_for(ctx, n, kSolveBlock, 8);
   const unsigned nparts = std::max(grid_rows, grid_vec);
   size_t need = 6 * align256(sizeof(double) * (size_t)n) + align256(sizeof(double) * 3 * nparts) +
-                align256(sizeof(CgState)) + slices_scratch_bytes(n);
+                align256(sizeof(CgState)) + slices_scratch_bytes(n) + 256;
+  const ResPlan plan = res_plan(ctx, n, 1, nnz, 32 * (sizeof(double) + sizeof(int32_t)));
+  bool resident = plan.take;
+  if (resident) need += res_slots_bytes(plan);
   AFEM_TRY(scratch_reserve(ctx, need));
   double *r, *z, *p, *q, *dinv, *partials;
   CgState* st;
+  int* err;
+  ulonglong2* slots = nullptr;
+  AFEM_TRY(scratch_take(ctx, 2, &err));
+  if (resident && nnz > kResScatterEntries) {
+    bool scattered = false;
+    AFEM_TRY(res_scattered(ctx, n, rp, cols, err, &scattered));
+    resident = !scattered;
+  }
+  if (resident) {
+    AFEM_TRY(scratch_take(ctx, res_slots_bytes(plan) / sizeof(ulonglong2), &slots));
+    AFEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+  }
   // the iterate lives in an aligned scratch copy (16-byte vector accesses in
   // k_cg_update), copied in here and back to the caller's x at the end
   double* const x_user = x;
@@ -675,7 +685,24 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
                   (const double*)x, dv, skip, r, z, p, partials, st, opt.rtol, opt.atol);
   }));
   SlicedCopy<double> sliced;   // the iteration's SpMV reads the sliced-ELL copy
-  AFEM_TRY(build_slices(ctx, n, rp, cols, vals, sliced));
+  if (!resident || !plan.fits) AFEM_TRY(build_slices(ctx, n, rp, cols, vals, sliced));
+  CgState hs{};
+  if (resident) {
+    const CgResident a{n,    plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, cols, vals, sliced.soff,
+                       sliced.cols, sliced.vals, dv, skip, x, r, p, slots, err, st};
+    AFEM_TRY(run_resident(ctx, st, err, &hs, [&]() {
+      return dispatch_rows(plan.K, [&](auto k) {
+        return launch_resident(ctx, k_cg_resident<decltype(k)::value>, plan, a);
+      });
+    }));
+    AFEM_CUDA(cudaMemcpyAsync(x_user, x, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
+    if (info) {
+      info->iterations = hs.iter;
+      info->refinements = 0;
+      info->status = hs.status;
+    }
+    return (afem_status)hs.status;
+  }
   const unsigned grid_sl = grid_for(ctx, n, kSolveBlock, 8);
   const int chunk = opt.check_every > 0 ? opt.check_every : 16;
   GraphChunk gc;
@@ -689,7 +716,6 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
     }
     return AFEM_OK;
   }));
-  CgState hs{};
   for (int done_chunks = 0;; ++done_chunks) {
     AFEM_CUDA(cudaMemcpyAsync(ctx->pinned, st, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
     AFEM_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -719,8 +745,11 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
   // 3x3-block SpMV: one warp per (slice of 32 block rows, component)
   const unsigned grid_b3 = grid_for(ctx, 3 * (((int64_t)n / 3 + kSlice - 1) / kSlice) * kSlice, kSolveBlock, 8);
   const unsigned nparts = std::max(std::max(std::max(grid_rows, grid_rows64), grid_vec), grid_b3);
+  // a step of the resident form: 32 entries, or 32 blocks of nine values
+  const ResPlan plan = res_plan(ctx, b3 ? n / 3 : n, b3 ? 3 : 1, nnz, b3 ? 32 * 40 : 32 * 8);
+  bool resident = plan.take;
   size_t need = 6 * align256(sizeof(float) * (size_t)n) + align256(sizeof(double) * 3 * nparts) +
-                2 * align256(sizeof(CgState)) +
+                2 * align256(sizeof(CgState)) + 256 + (resident ? res_slots_bytes(plan) : 0) +
                 (b3 ? align256(sizeof(int32_t) * (size_t)(nnz / 9 + 1)) + 256 + slices_scratch_bytes(n / 3)
                     : slices_scratch_bytes(n));
   AFEM_TRY(scratch_reserve(ctx, need));
@@ -736,6 +765,16 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
   AFEM_TRY(scratch_take(ctx, 3 * (size_t)nparts, &partials));
   AFEM_TRY(scratch_take(ctx, 1, &outer));
   AFEM_TRY(scratch_take(ctx, 1, &inner));
+  int* err;
+  ulonglong2* slots = nullptr;
+  AFEM_TRY(scratch_take(ctx, 2, &err));
+  if (resident && nnz > kResScatterEntries) {
+    bool scattered = false;
+    AFEM_TRY(res_scattered(ctx, n, rp, cols, err, &scattered));
+    resident = !scattered;
+  }
+  AFEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+  if (resident) AFEM_TRY(scratch_take(ctx, res_slots_bytes(plan) / sizeof(ulonglong2), &slots));
   AFEM_CUDA(cudaMemsetAsync(outer, 0, sizeof(CgState), ctx->stream));
   AFEM_CUDA(cudaMemsetAsync(inner, 0, sizeof(CgState), ctx->stream));
   int32_t* bcols = nullptr;
@@ -751,7 +790,9 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
   }
   // the FP32 matrix: the sliced copy, by 3x3 blocks or by scalar rows
   SlicedCopy<float> sliced;
-  if (b3)
+  if (resident && plan.fits)
+    ;   // filled into shared memory from the CSR rows
+  else if (b3)
     AFEM_TRY(build_slices3(ctx, n / 3, rp, (const int32_t*)bcols, vals, sliced));
   else
     AFEM_TRY(build_slices(ctx, n, rp, cols, vals, sliced));
@@ -763,7 +804,7 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
   const int chunk = opt.check_every > 0 ? opt.check_every : 16;
   // outer tolerance: needs ||b||, computed by the first residual pass
   GraphChunk gc;
-  AFEM_TRY(capture(ctx, gc, [&](cudaStream_t s) -> afem_status {
+  if (!resident) AFEM_TRY(capture(ctx, gc, [&](cudaStream_t s) -> afem_status {
     for (int k = 0; k < chunk; ++k) {
       if (b3)
         AFEM_TRY(launch_s(ctx, s, k_cgf_spmv_b3s, grid_b3, kSolveBlock, n / 3, (const int32_t*)sliced.soff,
@@ -826,7 +867,18 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
       break;
     }
     CgState hi{};
-    for (;;) {
+    if (resident) {
+      const CgfResident a{n, plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, b3 ? bcols : cols, vals,
+                          sliced.soff, sliced.cols, sliced.vals, dinv32, skip, x32, r32, z32, p32, q32, slots, err,
+                          inner};
+      AFEM_TRY(run_resident(ctx, inner, err, &hi, [&]() {
+        return dispatch_rows(plan.K, [&](auto k) {
+          constexpr int K = decltype(k)::value;
+          return b3 ? launch_resident(ctx, k_cgf_resident<K, true>, plan, a)
+                    : launch_resident(ctx, k_cgf_resident<K, false>, plan, a);
+        });
+      }));
+    } else for (;;) {
       AFEM_CUDA(cudaGraphLaunch(gc.exec, ctx->stream));
       ctx->launches += 2 * chunk;
       AFEM_CUDA(cudaMemcpyAsync(ctx->pinned, inner, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
