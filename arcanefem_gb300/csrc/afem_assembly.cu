@@ -825,12 +825,13 @@ __constant__ double kHexDN[8][3][8] = {
     {{-kHpm, kHpm, kHpp, -kHpp, -kHmm, kHmm, kHpm, -kHpm}, {-kHpm, -kHpp, kHpp, kHpm, -kHmm, -kHpm, kHpm, kHmm}, {-kHmm, -kHpm, -kHpp, -kHpm, kHmm, kHpm, kHpp, kHpm}},
     {{-kHmm, kHmm, kHpm, -kHpm, -kHpm, kHpm, kHpp, -kHpp}, {-kHmm, -kHpm, kHpm, kHmm, -kHpm, -kHpp, kHpp, kHpm}, {-kHmm, -kHpm, -kHpp, -kHpm, kHmm, kHpm, kHpp, kHpm}}};
 
-template <int F>
-__global__ void __launch_bounds__(128) k_elem_poisson_hexa8(int cell0, int nb_cell, const double* __restrict__ xyz,
-                                                            const int32_t* __restrict__ cn,
-                                                            const int32_t* __restrict__ inv,
-                                                            const double* __restrict__ coeff, double* __restrict__ er,
-                                                            int* __restrict__ bad) {
+// AFEM_FORMULATION_MINIMAL.
+__global__ void __launch_bounds__(128) k_elem_poisson_hexa8_minimal(int cell0, int nb_cell,
+                                                                    const double* __restrict__ xyz,
+                                                                    const int32_t* __restrict__ cn,
+                                                                    const int32_t* __restrict__ inv,
+                                                                    const double* __restrict__ coeff,
+                                                                    double* __restrict__ er, int* __restrict__ bad) {
   for (int64_t c = cell0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell;
        c += (int64_t)gridDim.x * blockDim.x) {
     double x[8], y[8], z[8];
@@ -842,99 +843,335 @@ __global__ void __launch_bounds__(128) k_elem_poisson_hexa8(int cell0, int nb_ce
       z[a] = __ldg(p + 2);
     }
     double K[8][8];
-    if constexpr (F != AFEM_FORMULATION_MINIMAL) {
-      const bool ok = ref::hexa8_matrix(x, y, z, kHexDnRef, K);
-      if (bad && !ok) atomicOr(bad, kFlagDegenerateCell);
-      if (coeff) scale_upper<8>(K, __ldg(coeff + c));
-      write_rows_q1<8>(K, inv + 8 * c, er);
-    } else {
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) K[a][b] = 0.0;
+    // The trilinear map's derivatives are bilinear in the other two reference
+    // coordinates: d x / d xi = m_xi + eta m_xieta + zeta m_xizeta + eta zeta m_xietazeta,
+    // and so on, with the moments m (signed sums of the 8 nodal coordinates, / 8)
+    // formed once per cell by a Walsh-Hadamard butterfly: 3 FMAs per Jacobian
+    // entry per Gauss point instead of 8.  Node a has reference signs
+    // (s_xi, s_eta, s_zeta) = (-,-,-) (+,-,-) (+,+,-) (-,+,-) (-,-,+) (+,-,+) (+,+,+) (-,+,+).
+    double mo[3][8];   // per component: [1, xi, eta, xi eta, zeta, xi zeta, eta zeta, xi eta zeta]
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double* v = q == 0 ? x : (q == 1 ? y : z);
+      // reorder to the binary order (xi bit 0, eta bit 1, zeta bit 2): nodes 0 1 3 2 4 5 7 6
+      const double u0 = v[0], u1 = v[1], u2 = v[3], u3 = v[2], u4 = v[4], u5 = v[5], u6 = v[7], u7 = v[6];
+      // stage xi
+      const double a0 = u1 + u0, a1 = u1 - u0, a2 = u3 + u2, a3 = u3 - u2;
+      const double a4 = u5 + u4, a5 = u5 - u4, a6 = u7 + u6, a7 = u7 - u6;
+      // stage eta
+      const double b0 = a2 + a0, b1 = a3 + a1, b2 = a2 - a0, b3 = a3 - a1;
+      const double b4 = a6 + a4, b5 = a7 + a5, b6 = a6 - a4, b7 = a7 - a5;
+      // stage zeta
+      mo[q][0] = 0.125 * (b4 + b0);
+      mo[q][1] = 0.125 * (b5 + b1);
+      mo[q][2] = 0.125 * (b6 + b2);
+      mo[q][3] = 0.125 * (b7 + b3);
+      mo[q][4] = 0.125 * (b4 - b0);
+      mo[q][5] = 0.125 * (b5 - b1);
+      mo[q][6] = 0.125 * (b6 - b2);
+      mo[q][7] = 0.125 * (b7 - b3);
+    }
+#pragma unroll 1
+    for (int g = 0; g < 8; ++g) {
+      const double* dxi = kHexDN[g][0];
+      const double* deta = kHexDN[g][1];
+      const double* dzeta = kHexDN[g][2];
+      const double xi = (g >> 2) ? kGauss : -kGauss, eta = ((g >> 1) & 1) ? kGauss : -kGauss,
+                   zeta = (g & 1) ? kGauss : -kGauss;
+      const double xe = (g >> 2) == ((g >> 1) & 1) ? kGauss * kGauss : -(kGauss * kGauss);
+      const double xz = (g >> 2) == (g & 1) ? kGauss * kGauss : -(kGauss * kGauss);
+      const double ez = ((g >> 1) & 1) == (g & 1) ? kGauss * kGauss : -(kGauss * kGauss);
+      double J[3][3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        J[0][q] = fma(ez, mo[q][7], fma(zeta, mo[q][5], fma(eta, mo[q][3], mo[q][1])));
+        J[1][q] = fma(xz, mo[q][7], fma(zeta, mo[q][6], fma(xi, mo[q][3], mo[q][2])));
+        J[2][q] = fma(xe, mo[q][7], fma(eta, mo[q][6], fma(xi, mo[q][5], mo[q][4])));
+      }
+      // determinant by the first row, inverse = adjugate / det
+      const double c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+      const double c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+      const double c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+      const double det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
+      if (bad && !ref::measure_ok(det)) atomicOr(bad, kFlagDegenerateCell);
+      const double id = 1.0 / det;
+      const double v00 = c00 * id, v10 = c01 * id, v20 = c02 * id;
+      const double v01 = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
+      const double v11 = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
+      const double v21 = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
+      const double v02 = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
+      const double v12 = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
+      const double v22 = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
+      // physical gradients, and the same scaled by det for the weighted products
+      double dx[8], dy[8], dz[8], sx[8], sy[8], sz[8];
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        dx[a] = v00 * dxi[a] + v01 * deta[a] + v02 * dzeta[a];
+        dy[a] = v10 * dxi[a] + v11 * deta[a] + v12 * dzeta[a];
+        dz[a] = v20 * dxi[a] + v21 * deta[a] + v22 * dzeta[a];
+        sx[a] = dx[a] * det;
+        sy[a] = dy[a] * det;
+        sz[a] = dz[a] * det;
+      }
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) K[a][b] = 0.0;
-      // The trilinear map's derivatives are bilinear in the other two reference
-      // coordinates: d x / d xi = m_xi + eta m_xieta + zeta m_xizeta + eta zeta m_xietazeta,
-      // and so on, with the moments m (signed sums of the 8 nodal coordinates, / 8)
-      // formed once per cell by a Walsh-Hadamard butterfly: 3 FMAs per Jacobian
-      // entry per Gauss point instead of 8.  Node a has reference signs
-      // (s_xi, s_eta, s_zeta) = (-,-,-) (+,-,-) (+,+,-) (-,+,-) (-,-,+) (+,-,+) (+,+,+) (-,+,+).
-      double mo[3][8];   // per component: [1, xi, eta, xi eta, zeta, xi zeta, eta zeta, xi eta zeta]
+        for (int b = a; b < 8; ++b) K[a][b] = fma(sx[a], dx[b], fma(sy[a], dy[b], fma(sz[a], dz[b], K[a][b])));
+    }
+    if (coeff) {
+      const double k = __ldg(coeff + c);
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const double* v = q == 0 ? x : (q == 1 ? y : z);
-        // reorder to the binary order (xi bit 0, eta bit 1, zeta bit 2): nodes 0 1 3 2 4 5 7 6
-        const double u0 = v[0], u1 = v[1], u2 = v[3], u3 = v[2], u4 = v[4], u5 = v[5], u6 = v[7], u7 = v[6];
-        // stage xi
-        const double a0 = u1 + u0, a1 = u1 - u0, a2 = u3 + u2, a3 = u3 - u2;
-        const double a4 = u5 + u4, a5 = u5 - u4, a6 = u7 + u6, a7 = u7 - u6;
-        // stage eta
-        const double b0 = a2 + a0, b1 = a3 + a1, b2 = a2 - a0, b3 = a3 - a1;
-        const double b4 = a6 + a4, b5 = a7 + a5, b6 = a6 - a4, b7 = a7 - a5;
-        // stage zeta
-        mo[q][0] = 0.125 * (b4 + b0);
-        mo[q][1] = 0.125 * (b5 + b1);
-        mo[q][2] = 0.125 * (b6 + b2);
-        mo[q][3] = 0.125 * (b7 + b3);
-        mo[q][4] = 0.125 * (b4 - b0);
-        mo[q][5] = 0.125 * (b5 - b1);
-        mo[q][6] = 0.125 * (b6 - b2);
-        mo[q][7] = 0.125 * (b7 - b3);
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int b = a; b < 8; ++b) K[a][b] *= k;
+    }
+    write_rows_q1<8>(K, inv + 8 * c, er);
+  }
+}
+
+// The reference-rounding hexahedron, its sums on the FP64 pipe and its products
+// and quotients on the integer pipes (afem_fp64_int.cuh), bit for bit the same.
+// Bound, as the tetrahedron's kernel, by the two pipes together: on the FP64
+// pipe alone a cell took 4704 instructions there.  Two things bring the count
+// down before the split.  The 24 derivative tables hold three magnitudes only
+// (0.125 (1 -+ p)(1 -+ p)), so that 72 products of a cell's coordinates serve
+// the Jacobians of all 8 Gauss points, and 27 of an inverse its gradients.  And
+// a Jacobian row depends on two of the three reference coordinates: 12 rows
+// instead of 24.  About 1600 sums a cell are left.
+//
+// Four threads share a cell, for shared memory of 440 B a thread instead of
+// 1.8 KB: thread t forms the products of nodes 2t and 2t + 1, the Jacobian rows
+// of one combination of two sides, then the inverse and the gradients of Gauss
+// points t and 4 + t, and the entries of rows t and 7 - t (9 of 36).  The sums
+// over Gauss points keep their order.  A warp holds 8 cells, lane = 8 t + cell;
+// nothing crosses a warp.  Measured, host coordinates to host values at 72^3:
+// 3.95 -> 1.71 ms; the assembly step at 90^3 9.23 -> 5.08 ms.
+constexpr int kHexBlock = 64;
+
+struct HexScratch {
+  static constexpr int kRows = 25;   // a Gauss point's rows: 3 x 8 gradients, the determinant
+  struct Factors {
+    uint2 sig[4 * kRows][8];
+    uint32_t se[4 * kRows][8];
+  };
+  union {
+    double prod[72][8];   // magnitude m of coordinate c of node a at [24 m + 8 c + a]
+    Factors f;
+  };
+  double jac[36][8];      // entry c of row r for the sides (s1, s2) at [3 (4 r + 2 s1 + s2) + c]
+  double K[36][8];        // thread t's entries at [9 t ..]
+  __device__ __forceinline__ ref::Val get(int q, int cs) const {
+    const uint2 s = f.sig[q][cs];
+    ref::Val v;
+    v.o = {s.x, s.y, f.se[q][cs]};
+    return v;
+  }
+  __device__ __forceinline__ void put(int q, int cs, const ref::Val& v) {
+    f.sig[q][cs] = make_uint2(v.o.lo, v.o.hi);
+    f.se[q][cs] = v.o.se;
+  }
+};
+
+// 0.125 times the products of 1 - p and 1 + p, by the number of 1 + p.  A node's
+// derivative at a Gauss point has the sign of the node's side in its own
+// coordinate and a 1 + p for each of the two others whose sides agree.
+constexpr double kHexLo = 1.0 - ref::kGaussPt, kHexHi = 1.0 + ref::kGaussPt;
+constexpr double kHexMag[3] = {0.125 * kHexLo * kHexLo, 0.125 * kHexLo * kHexHi, 0.125 * kHexHi * kHexHi};
+constexpr bool hex_magnitudes_hold() {
+  constexpr ref::HexDN dn = ref::make_hex_dn();
+  for (int g = 0; g < 8; ++g)
+    for (int a = 0; a < 8; ++a) {
+      const int side[3] = {(a ^ (a >> 1)) & 1, (a >> 1) & 1, a >> 2}, at[3] = {g >> 2, (g >> 1) & 1, g & 1};
+      for (int r = 0; r < 3; ++r) {
+        const int p = (r + 1) % 3, q = (r + 2) % 3;
+        const double m = kHexMag[(side[p] == at[p]) + (side[q] == at[q])];
+        if (dn.v[g][r][a] != (side[r] ? m : -m)) return false;
       }
-#pragma unroll 1
-      for (int g = 0; g < 8; ++g) {
-        const double* dxi = kHexDN[g][0];
-        const double* deta = kHexDN[g][1];
-        const double* dzeta = kHexDN[g][2];
-        const double xi = (g >> 2) ? kGauss : -kGauss, eta = ((g >> 1) & 1) ? kGauss : -kGauss,
-                     zeta = (g & 1) ? kGauss : -kGauss;
-        const double xe = (g >> 2) == ((g >> 1) & 1) ? kGauss * kGauss : -(kGauss * kGauss);
-        const double xz = (g >> 2) == (g & 1) ? kGauss * kGauss : -(kGauss * kGauss);
-        const double ez = ((g >> 1) & 1) == (g & 1) ? kGauss * kGauss : -(kGauss * kGauss);
-        double J[3][3];
+    }
+  return true;
+}
+static_assert(hex_magnitudes_hold(), "the derivative tables hold three magnitudes");
+
+// A hexahedron whose operands leave the integer path's range, on the FP64 pipe alone.
+__device__ __noinline__ void elem_hexa_cell_fp64(int64_t c, const double* xyz, const int32_t* cn, const int32_t* inv,
+                                                 const double* coeff, double* er, int* bad) {
+  double x[8], y[8], z[8];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          J[0][q] = fma(ez, mo[q][7], fma(zeta, mo[q][5], fma(eta, mo[q][3], mo[q][1])));
-          J[1][q] = fma(xz, mo[q][7], fma(zeta, mo[q][6], fma(xi, mo[q][3], mo[q][2])));
-          J[2][q] = fma(xe, mo[q][7], fma(eta, mo[q][6], fma(xi, mo[q][5], mo[q][4])));
-        }
-        // determinant by the first row, inverse = adjugate / det
-        const double c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-        const double c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-        const double c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-        const double det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
-        if (bad && !ref::measure_ok(det)) atomicOr(bad, kFlagDegenerateCell);
-        const double id = 1.0 / det;
-        const double v00 = c00 * id, v10 = c01 * id, v20 = c02 * id;
-        const double v01 = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
-        const double v11 = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
-        const double v21 = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
-        const double v02 = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
-        const double v12 = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
-        const double v22 = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
-        // physical gradients, and the same scaled by det for the weighted products
-        double dx[8], dy[8], dz[8], sx[8], sy[8], sz[8];
+  for (int a = 0; a < 8; ++a) {
+    const double* p = xyz + 3 * (int64_t)__ldg(cn + 8 * c + a);
+    x[a] = __ldg(p);
+    y[a] = __ldg(p + 1);
+    z[a] = __ldg(p + 2);
+  }
+  double K[8][8];
+  const bool ok = ref::hexa8_matrix(x, y, z, kHexDnRef, K);
+  if (bad && !ok) atomicOr(bad, kFlagDegenerateCell);
+  if (coeff) scale_upper<8>(K, __ldg(coeff + c));
+  write_rows_q1<8>(K, inv + 8 * c, er);
+}
+
+// Where entry (i, j) of the symmetric matrix is kept in HexScratch::K.
+__device__ __forceinline__ int hex_entry(int i, int j) {
+  const int lo = min(i, j), hi = max(i, j);
+  return lo < 4 ? 8 * lo + hi : 9 * (7 - lo) + hi + 1;   // 9 lo + (hi - lo); the second row of thread 7 - lo
+}
+
+template <bool COEFF>
+__global__ void __launch_bounds__(kHexBlock, 7)
+    k_elem_poisson_hexa8_ref(int cell0, int nb_cell, const double* __restrict__ xyz, const int32_t* __restrict__ cn,
+                             const int32_t* __restrict__ inv, const double* __restrict__ coeff, double* __restrict__ er,
+                             int* __restrict__ bad) {
+  using ref::add;
+  using ref::mul;
+  using ref::sub;
+  using V = ref::Val;
+  __shared__ HexScratch scratch[kHexBlock / 32];
+  HexScratch& sh = scratch[threadIdx.x >> 5];
+  const int cs = threadIdx.x & 7, t = (threadIdx.x >> 3) & 3;
+  constexpr double mag[3] = {kHexMag[0], kHexMag[1], kHexMag[2]};
+  for (int64_t c0 = cell0 + blockIdx.x * (int64_t)(kHexBlock / 4) + (threadIdx.x >> 5) * 8; c0 < nb_cell;
+       c0 += (int64_t)gridDim.x * (kHexBlock / 4)) {
+    const bool here = c0 + cs < nb_cell;
+    const int64_t c = here ? c0 + cs : nb_cell - 1;
+    bool ok = true;
+    __syncwarp();
+#pragma unroll 1
+    for (int a = 2 * t; a < 2 * t + 2; ++a) {
+      const double* p = xyz + 3 * (int64_t)__ldg(cn + 8 * c + a);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const double x = __ldg(p + k);
+        ok &= i64fp::in_window<ref::kCoordWindow>(__double2hiint(x), __double2loint(x));
+        const V v(x);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) sh.prod[24 * m + 8 * k + a][cs] = mul(v, V(mag[m]));
+      }
+    }
+    __syncwarp();
+    {
+      // node a's sides: xi 0 1 1 0 0 1 1 0, eta 0 0 1 1 0 0 1 1, zeta 0 0 0 0 1 1 1 1
+      const int s1 = t >> 1, s2 = t & 1;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        double J[3];
 #pragma unroll
         for (int a = 0; a < 8; ++a) {
-          dx[a] = v00 * dxi[a] + v01 * deta[a] + v02 * dzeta[a];
-          dy[a] = v10 * dxi[a] + v11 * deta[a] + v12 * dzeta[a];
-          dz[a] = v20 * dxi[a] + v21 * deta[a] + v22 * dzeta[a];
-          sx[a] = dx[a] * det;
-          sy[a] = dy[a] * det;
-          sz[a] = dz[a] * det;
+          const int sx = (a ^ (a >> 1)) & 1, sy = (a >> 1) & 1, sz = a >> 2;
+          const int side = r == 0 ? sx : r == 1 ? sy : sz;             // the sign of dN_a
+          const int f1 = r == 0 ? sy : sx, f2 = r == 2 ? sy : sz;      // its two factors' sides
+          const double* q = &sh.prod[24 * ((f1 == s1) + (f2 == s2)) + a][cs];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const double v = q[64 * k];
+            J[k] = a == 0 ? -v : side ? add(J[k], v) : sub(J[k], v);
+          }
         }
 #pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-          for (int b = a; b < 8; ++b) K[a][b] = fma(sx[a], dx[b], fma(sy[a], dy[b], fma(sz[a], dz[b], K[a][b])));
+        for (int k = 0; k < 3; ++k) sh.jac[3 * (4 * r + t) + k][cs] = J[k];
       }
-      if (coeff) {
-        const double k = __ldg(coeff + c);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      // Gauss point 4 half + t: its sides are half, t >> 1, t & 1
+      const int gy = t >> 1, gz = t & 1, row0 = HexScratch::kRows * t;
+      {
+        V J[3][3];
 #pragma unroll
-        for (int a = 0; a < 8; ++a)
+        for (int k = 0; k < 3; ++k) {
+          J[0][k] = V(sh.jac[3 * t + k][cs]);
+          J[1][k] = V(sh.jac[3 * (4 + 2 * half + gz) + k][cs]);
+          J[2][k] = V(sh.jac[3 * (8 + 2 * half + gy) + k][cs]);
+        }
+        auto minor = [&](int a, int b, int e, int f, int g, int h, int i, int j) {
+          return sub(mul(J[a][b], J[e][f]), mul(J[g][h], J[i][j]));
+        };
+        double num[3][3];
+        num[0][0] = minor(1, 1, 2, 2, 1, 2, 2, 1);
+        num[1][0] = minor(1, 0, 2, 2, 1, 2, 2, 0);
+        num[2][0] = minor(1, 0, 2, 1, 1, 1, 2, 0);
+        const double det = add(sub(mul(J[0][0], V(num[0][0])), mul(J[0][1], V(num[1][0]))), mul(J[0][2], V(num[2][0])));
+        num[1][0] = -num[1][0];
+        num[0][1] = minor(0, 2, 2, 1, 0, 1, 2, 2);
+        num[0][2] = minor(0, 1, 1, 2, 0, 2, 1, 1);
+        num[1][1] = minor(0, 0, 2, 2, 0, 2, 2, 0);
+        num[1][2] = minor(0, 2, 1, 0, 0, 0, 1, 2);
+        num[2][1] = minor(0, 1, 2, 0, 0, 0, 2, 1);
+        num[2][2] = minor(0, 0, 1, 1, 0, 1, 1, 0);
+        ok &= ref::measure_ok(det);
+        sh.put(row0 + 24, cs, V(det, ok));
+        const i64fp::Divisor by = i64fp::divisor(__double_as_longlong(det));
+        // the inverse, its columns with the sign of the Gauss point's side, kept where the gradients of a later
+        // dimension go: rows 8.. (d = 0), 16.. (1), 19.. (2)
 #pragma unroll
-          for (int b = a; b < 8; ++b) K[a][b] *= k;
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            V v(__longlong_as_double(i64fp::div(V(num[d][k]).o, by)), ok);
+            const int side = k == 0 ? half : k == 1 ? gy : gz;
+            v.o.se ^= side ? 0u : 0x80000000u;
+            sh.put(row0 + (d == 0 ? 8 : 13 + 3 * d) + k, cs, v);
+          }
       }
-      write_rows_q1<8>(K, inv + 8 * c, er);
+      // the node on the Gauss point's own sides; the others' indices differ from it by a constant pattern
+      const int own = 4 * gz + 2 * gy + (half ^ gy);
+#pragma unroll 1
+      for (int d = 0; d < 3; ++d) {
+        double P[3][3];   // [inverse column][magnitude]
+        {
+          const int at = row0 + (d == 0 ? 8 : 13 + 3 * d);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const V v = sh.get(at + k, cs);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) P[k][m] = mul(v, V(mag[m]));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {   // bits of q: on the Gauss point's side in xi, eta, zeta
+          const int x = q & 1, y = (q >> 1) & 1, z = q >> 2;
+          const double px = x ? P[0][y + z] : -P[0][y + z], py = y ? P[1][x + z] : -P[1][x + z],
+                       pz = z ? P[2][x + y] : -P[2][x + y];
+          const int flip = 4 * (1 - z) + 2 * (1 - y) + (x ^ y);
+          sh.put(row0 + 8 * d + (own ^ flip), cs, V(add(add(px, py), pz), ok));
+        }
+      }
+      __syncwarp();
+#pragma unroll 1
+      for (int s = 0; s < 9; ++s) {
+        const bool first = s < 8 - t;   // row t from its diagonal on, then row 7 - t
+        const int i = first ? t : 7 - t, j = first ? t + s : s - 1;
+        double k = half ? sh.K[9 * t + s][cs] : 0.0;
+#pragma unroll 2
+        for (int g = 0; g < 4; ++g) {
+          const int q = HexScratch::kRows * g;
+          const double x = mul(sh.get(q + i, cs), sh.get(q + j, cs));
+          const double y = mul(sh.get(q + 8 + i, cs), sh.get(q + 8 + j, cs));
+          const double z = mul(sh.get(q + 16 + i, cs), sh.get(q + 16 + j, cs));
+          k = add(k, mul(V(add(add(x, y), z)), sh.get(q + 24, cs)));
+        }
+        if constexpr (COEFF)
+          if (half) k = mul(__ldg(coeff + c), k);
+        sh.K[9 * t + s][cs] = k;
+      }
+      __syncwarp();
+    }
+    const unsigned all = __ballot_sync(0xffffffffu, ok);
+    if ((all >> cs & 0x01010101u) != 0x01010101u) {
+      if (here && t == 0) elem_hexa_cell_fp64(c, xyz, cn, inv, coeff, er, bad);
+    } else if (here) {
+      // row i: the diagonal, then the other nodes in increasing order; thread t its entries 2t and 2t + 1
+#pragma unroll 2
+      for (int i = 0; i < 8; ++i) {
+        const int e1 = 2 * t, e0 = e1 - 1;
+        const int j0 = t == 0 ? i : e0 + (e0 >= i), j1 = e1 + (e1 >= i);
+        reinterpret_cast<double2*>(er)[4 * (int64_t)__ldg(inv + 8 * c + i) + t] =
+            make_double2(sh.K[hex_entry(i, j0)][cs], sh.K[hex_entry(i, j1)][cs]);
+      }
     }
   }
 }
@@ -1202,9 +1439,10 @@ static afem_status launch_elem_q1(afem_context ctx, const afem_mesh_view* m, int
   int* bad = ctx->flags_d;
   const unsigned ge = grid_for(ctx, c1 - c0, 128, 16);
   if (m->dim == 3)
-    return minimal ? launch(ctx, k_elem_poisson_hexa8<AFEM_FORMULATION_MINIMAL>, ge, 128, 0, c0, c1, m->coords_d,
-                            m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad)
-                   : launch(ctx, k_elem_poisson_hexa8<AFEM_FORMULATION_REFERENCE>, ge, 128, 0, c0, c1, m->coords_d,
+    return minimal ? launch(ctx, k_elem_poisson_hexa8_minimal, ge, 128, 0, c0, c1, m->coords_d, m->cell_nodes_d,
+                            m->nc_inverse_d, coeff, ke, bad)
+                   : launch(ctx, coeff ? k_elem_poisson_hexa8_ref<true> : k_elem_poisson_hexa8_ref<false>,
+                            grid_for(ctx, (int64_t)(c1 - c0) * 4, kHexBlock, 28), kHexBlock, 0, c0, c1, m->coords_d,
                             m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad);
   return minimal ? launch(ctx, k_elem_poisson_quad4<AFEM_FORMULATION_MINIMAL>, ge, 128, 0, c0, c1, m->coords_d,
                           m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad)

@@ -62,3 +62,14 @@ def test_tetrahedra_over_the_operand_ranges(own_ctx, n, jitter, case):
     k = np.exp(np.random.default_rng(0).standard_normal(m.nb_cell))
     f.assemble_poisson(torch.as_tensor(k, device="cuda"))
     assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_TET4, coeff=k), "coefficient")
+
+
+@pytest.mark.parametrize("n,jitter,case", CASES)
+def test_hexahedra_over_the_operand_ranges(own_ctx, n, jitter, case):
+    m = moved_mesh(meshgen.unit_cube_hex, n, jitter, case)
+    f = build_format(own_ctx, m)
+    f.assemble_poisson()
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_HEXA8), "hexahedra")
+    k = np.exp(np.random.default_rng(0).standard_normal(m.nb_cell))
+    f.assemble_poisson(torch.as_tensor(k, device="cuda"))
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_HEXA8, coeff=k), "coefficient")
