@@ -342,13 +342,122 @@ __device__ __forceinline__ double elast_ref_entry(int a, int b, const double P[3
   return add(mul(mul(lambda, P[a][b]), vol), mul(mul(mu, P[b][a]), vol));
 }
 
+// The 78 entries of a cell with its products on the FP64 pipe alone.
+__device__ __noinline__ void elast_cell_fp64(int64_t c, const double* xyz, const int32_t* cn, double lambda, double mu,
+                                             double* my, int* bad) {
+  const int4 q = __ldg(reinterpret_cast<const int4*>(cn) + c);
+  const int32_t nid[4] = {q.x, q.y, q.z, q.w};
+  double n[4][3];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) n[a][k] = __ldg(xyz + 3 * (int64_t)nid[a] + k);
+  double g[3][4], vol;
+  const double v6 = ref::tet_gradients(n, g, &vol);
+  if (bad && !ref::measure_ok(v6)) atomicOr(bad, kFlagDegenerateCell);
+  const double l2m = ref::add(lambda, 2.0 * mu);
+#pragma unroll
+  for (int lo = 0; lo < 4; ++lo)
+#pragma unroll
+    for (int hi = lo; hi < 4; ++hi) {
+      double P[3][3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) P[a][b] = ref::mul(g[a][lo], g[b][hi]);
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+          if (lo != hi || a <= b) my[elast_packed(lo, hi, a, b)] = elast_ref_entry(a, b, P, l2m, lambda, mu, vol);
+    }
+}
+
+// The Lame factors' range on the integer pipe: with gradients and the volume
+// in +-kWindow, (mu (P + P)) vol stays normal, 2^-(553 + 200 + 250).
+constexpr int kLameWindow = 200;
+
+struct ElastFactors {
+  ref::Val l2m, lambda, mu;
+  bool ok;
+};
+__device__ __forceinline__ ElastFactors elast_factors(double lambda, double mu) {
+  const double l2m = ref::add(lambda, 2.0 * mu);
+  auto in = [](double x) { return i64fp::in_window<kLameWindow>(__double2hiint(x), __double2loint(x)); };
+  return {ref::Val(l2m), ref::Val(lambda), ref::Val(mu), in(l2m) && in(lambda) && in(mu)};
+}
+
+// The 78 entries from the gradients and the volume: elast_ref_entry with the
+// products of gradients and the sums on the FP64 pipe and the products by the
+// Lame factors and the volume on the integer pipes.  A cell's 636 rounded FP64
+// operations become 246 there and 372 products here, about the same time on
+// each: the element kernel 1.9 -> 1.25 ms for 1.5 M cells (a step 2.90 -> 2.26).
+// The loops over pairs and nodes stay loops for the instruction cache.
+__device__ __forceinline__ void elast_entries_int(const double g[3][4], const ref::Val& vol, const ElastFactors& f,
+                                                  double* my) {
+  using ref::add;
+  using ref::mul;
+  using V = ref::Val;
+  auto node = [&](int i, double out[3]) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) out[a] = i == 0 ? g[a][0] : i == 1 ? g[a][1] : i == 2 ? g[a][2] : g[a][3];
+  };
+  auto diagonal = [&](double p, double z) {
+    return add(mul(V(mul(f.l2m, V(p))), vol), mul(V(mul(f.mu, V(z))), vol));
+  };
+#pragma unroll 1
+  for (int pair = 0; pair < 6; ++pair) {
+    const int lo = pair < 3 ? 0 : pair < 5 ? 1 : 2, hi = pair < 3 ? pair + 1 : pair < 5 ? pair - 1 : 3;
+    double l[3], h[3], P[3][3];
+    node(lo, l);
+    node(hi, h);
+    double* out = my + 9 * pair;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) P[a][b] = mul(l[a], h[b]);
+    out[0] = diagonal(P[0][0], add(P[1][1], P[2][2]));
+    out[4] = diagonal(P[1][1], add(P[0][0], P[2][2]));
+    out[8] = diagonal(P[2][2], add(P[1][1], P[0][0]));
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = a + 1; b < 3; ++b) {
+        const V u(P[a][b]), v(P[b][a]);
+        out[3 * a + b] = add(mul(V(mul(f.lambda, u)), vol), mul(V(mul(f.mu, v)), vol));
+        out[3 * b + a] = add(mul(V(mul(f.lambda, v)), vol), mul(V(mul(f.mu, u)), vol));
+      }
+  }
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    double l[3];
+    node(i, l);
+    double* out = my + 54 + 6 * i;
+    const double p0 = mul(l[0], l[0]), p1 = mul(l[1], l[1]), p2 = mul(l[2], l[2]);
+    out[0] = diagonal(p0, add(p1, p2));
+    out[3] = diagonal(p1, add(p0, p2));
+    out[5] = diagonal(p2, add(p1, p0));
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = a + 1; b < 3; ++b) {
+        const V u(mul(l[a], l[b]));
+        out[2 * a + b] = add(mul(V(mul(f.lambda, u)), vol), mul(V(mul(f.mu, u)), vol));
+      }
+  }
+}
+
 template <int F>
 __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cell0, int nb_cell, const double* __restrict__ xyz,
                                                                          const int32_t* __restrict__ cn,
                                                                          const int32_t* __restrict__ inv,
                                                                          double lambda, double mu,
                                                                          double* __restrict__ er, int* __restrict__ bad) {
-  __shared__ double stage[kElastElemBlock][kElastPacked + 1];
+  // a warp's entries, in the place of its geometry
+  __shared__ union {
+    double entry[32][kElastPacked + 1];
+    ref::TetScratch<32> tet;
+  } stage[kElastElemBlock / 32];
   __shared__ int4 stage_p[kElastElemBlock];
   // src_tab[n][q]: packed positions of entries 2q and 2q + 1 of node n's row block
   __shared__ uint32_t src_tab[4][18];
@@ -369,55 +478,24 @@ __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cel
   const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
   for (int64_t base = cell0 + blockIdx.x * (int64_t)blockDim.x; base < nb_cell; base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t c = base + threadIdx.x;
-    double* my = stage[threadIdx.x];
-    if (c < nb_cell && F != AFEM_FORMULATION_MINIMAL) {
+    auto& warp = stage[threadIdx.x >> 5];
+    double* my = warp.entry[lane];
+    if constexpr (F != AFEM_FORMULATION_MINIMAL) {
       // reference rounding: gradients and volume of the reference, then the 78
       // distinct entries (6 node-pair blocks, 4 symmetric diagonal blocks)
-      const int4 q = __ldg(reinterpret_cast<const int4*>(cn) + c);
-      const int32_t nid[4] = {q.x, q.y, q.z, q.w};
-      double n[4][3];
+      const int64_t cc = c < nb_cell ? c : nb_cell - 1;
+      const ElastFactors f = elast_factors(lambda, mu);
+      bool ok = f.ok & ref::tet_gradients_int(xyz, __ldg(reinterpret_cast<const int4*>(cn) + cc), warp.tet, lane);
+      double g[3][4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const double* p = xyz + 3 * (int64_t)nid[a];
-        n[a][0] = __ldg(p);
-        n[a][1] = __ldg(p + 1);
-        n[a][2] = __ldg(p + 2);
-      }
-      double g[3][4], vol;
-      const double v6 = ref::tet_gradients(n, g, &vol);
-      if (bad && !ref::measure_ok(v6)) atomicOr(bad, kFlagDegenerateCell);
-      stage_p[threadIdx.x] = __ldg(reinterpret_cast<const int4*>(inv) + c);
-      const double l2m = ref::add(lambda, 2.0 * mu);
+      for (int d = 0; d < 3; ++d)
 #pragma unroll
-      for (int lo = 0; lo < 4; ++lo)
-#pragma unroll
-        for (int hi = lo + 1; hi < 4; ++hi) {
-          const int pair = lo * (7 - lo) / 2 + (hi - lo - 1);
-          double P[3][3];
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) P[a][b] = ref::mul(g[a][lo], g[b][hi]);
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b)
-              my[pair * 9 + a * 3 + b] = elast_ref_entry(a, b, P, l2m, lambda, mu, vol);
-        }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        double P[3][3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-          for (int b = a; b < 3; ++b) P[a][b] = P[b][a] = ref::mul(g[a][i], g[b][i]);
-        int k = 0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-          for (int b = a; b < 3; ++b, ++k)
-            my[54 + i * 6 + k] = elast_ref_entry(a, b, P, l2m, lambda, mu, vol);
-      }
+        for (int i = 0; i < 4; ++i) g[d][i] = warp.tet.gradient(d, i, lane).value();
+      const ref::Val vol = warp.tet.volume(lane);
+      stage_p[threadIdx.x] = __ldg(reinterpret_cast<const int4*>(inv) + cc);
+      __syncwarp();   // the entries take the geometry's place
+      if (ok) elast_entries_int(g, vol, f, my);
+      else if (c < nb_cell) elast_cell_fp64(c, xyz, cn, lambda, mu, my, bad);
     } else if (c < nb_cell) {
       // cofactors c_1..c_3 of the edges from node 0 and s = 1 / (6 |det|);
       // with G_n = s c_n the block of nodes (n, m) is
@@ -497,7 +575,7 @@ __global__ void __launch_bounds__(kElastElemBlock) k_elem_elasticity_tet(int cel
     // every pass adds 32 = 18 + 14 chunks
     int t = lane >= 18, q = lane - 18 * (lane >= 18);
     for (int k = lane; k < wcount * 18; k += 32) {
-      const double* src = stage[wbase + t];
+      const double* src = warp.entry[t];
       const int4 p4 = stage_p[wbase + t];
       const int pr[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll

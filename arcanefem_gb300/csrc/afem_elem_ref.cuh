@@ -48,6 +48,9 @@ struct Val {
   __device__ __forceinline__ Val(double x, bool& ok) : Val(x) {
     ok &= i64fp::in_window(__double2hiint(x), __double2loint(x));
   }
+  __device__ __forceinline__ double value() const {
+    return __hiloint2double((int)(o.se | ((o.hi >> 10) & 0xfffffu)), (int)((o.hi << 22) | (o.lo >> 10)));
+  }
 };
 __device__ __forceinline__ double mul(const Val& a, const Val& b) {
   return __longlong_as_double(i64fp::mul(a.o, b.o));

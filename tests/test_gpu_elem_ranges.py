@@ -73,3 +73,13 @@ def test_hexahedra_over_the_operand_ranges(own_ctx, n, jitter, case):
     k = np.exp(np.random.default_rng(0).standard_normal(m.nb_cell))
     f.assemble_poisson(torch.as_tensor(k, device="cuda"))
     assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_HEXA8, coeff=k), "coefficient")
+
+
+@pytest.mark.parametrize("lam,mu", [(1.3, 0.7), (0.0, 1.0), (2.0 ** 190, 2.0 ** -190), (2.0 ** 205, 1.0)])
+@pytest.mark.parametrize("n,jitter,case", CASES)
+def test_elasticity_over_the_operand_ranges(own_ctx, n, jitter, case, lam, mu):
+    m = moved_mesh(meshgen.unit_cube_tet, n, jitter, case)
+    f = build_format(own_ctx, m, 3)
+    f.assemble_elasticity(lam, mu)
+    ref = oracle_values(m, O.ELASTICITY_TET4, lam=lam, mu=mu)
+    assert_bit_exact(f.values.cpu().numpy(), ref, "elasticity")
