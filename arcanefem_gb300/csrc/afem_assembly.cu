@@ -391,8 +391,9 @@ __device__ __forceinline__ ElastFactors elast_factors(double lambda, double mu) 
 // products of gradients and the sums on the FP64 pipe and the products by the
 // Lame factors and the volume on the integer pipes.  A cell's 636 rounded FP64
 // operations become 246 there and 372 products here, about the same time on
-// each: the element kernel 1.9 -> 1.25 ms for 1.5 M cells (a step 2.90 -> 2.26).
-// The loops over pairs and nodes stay loops for the instruction cache.
+// each: the element kernel 1.9 -> 1.09 ms for 1.5 M cells (a step 2.90 -> 2.11);
+// with all 9 entries of a pair in a row 1.25, a third of its stalls waiting for
+// instructions.  The loops stay loops.
 __device__ __forceinline__ void elast_entries_int(const double g[3][4], const ref::Val& vol, const ElastFactors& f,
                                                   double* my) {
   using ref::add;
@@ -405,45 +406,50 @@ __device__ __forceinline__ void elast_entries_int(const double g[3][4], const re
   auto diagonal = [&](double p, double z) {
     return add(mul(V(mul(f.l2m, V(p))), vol), mul(V(mul(f.mu, V(z))), vol));
   };
+  // One step takes the diagonal entry (a, a) and the entries (a, b), (b, a), b after a cyclically; the components
+  // rotate through the registers.
+  auto rotate = [](double v[3]) {
+    const double f = v[0];
+    v[0] = v[1];
+    v[1] = v[2];
+    v[2] = f;
+  };
 #pragma unroll 1
   for (int pair = 0; pair < 6; ++pair) {
     const int lo = pair < 3 ? 0 : pair < 5 ? 1 : 2, hi = pair < 3 ? pair + 1 : pair < 5 ? pair - 1 : 3;
-    double l[3], h[3], P[3][3];
+    double l[3], h[3], p[3];
     node(lo, l);
     node(hi, h);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) p[a] = mul(l[a], h[a]);
     double* out = my + 9 * pair;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b) P[a][b] = mul(l[a], h[b]);
-    out[0] = diagonal(P[0][0], add(P[1][1], P[2][2]));
-    out[4] = diagonal(P[1][1], add(P[0][0], P[2][2]));
-    out[8] = diagonal(P[2][2], add(P[1][1], P[0][0]));
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = a + 1; b < 3; ++b) {
-        const V u(P[a][b]), v(P[b][a]);
-        out[3 * a + b] = add(mul(V(mul(f.lambda, u)), vol), mul(V(mul(f.mu, v)), vol));
-        out[3 * b + a] = add(mul(V(mul(f.lambda, v)), vol), mul(V(mul(f.mu, u)), vol));
-      }
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) {
+      const int b = a < 2 ? a + 1 : 0;
+      const V u(mul(l[0], h[1])), v(mul(l[1], h[0]));
+      out[4 * a] = diagonal(p[0], add(p[1], p[2]));
+      out[3 * a + b] = add(mul(V(mul(f.lambda, u)), vol), mul(V(mul(f.mu, v)), vol));
+      out[3 * b + a] = add(mul(V(mul(f.lambda, v)), vol), mul(V(mul(f.mu, u)), vol));
+      rotate(l);
+      rotate(h);
+      rotate(p);
+    }
   }
 #pragma unroll 1
   for (int i = 0; i < 4; ++i) {
-    double l[3];
+    double l[3], p[3];
     node(i, l);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) p[a] = mul(l[a], l[a]);
     double* out = my + 54 + 6 * i;
-    const double p0 = mul(l[0], l[0]), p1 = mul(l[1], l[1]), p2 = mul(l[2], l[2]);
-    out[0] = diagonal(p0, add(p1, p2));
-    out[3] = diagonal(p1, add(p0, p2));
-    out[5] = diagonal(p2, add(p1, p0));
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = a + 1; b < 3; ++b) {
-        const V u(mul(l[a], l[b]));
-        out[2 * a + b] = add(mul(V(mul(f.lambda, u)), vol), mul(V(mul(f.mu, u)), vol));
-      }
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) {   // upper triangle: 00 01 02 11 12 22
+      const V u(mul(l[0], l[1]));
+      out[a * (7 - a) / 2] = diagonal(p[0], add(p[1], p[2]));
+      out[a == 0 ? 1 : a == 1 ? 4 : 2] = add(mul(V(mul(f.lambda, u)), vol), mul(V(mul(f.mu, u)), vol));
+      rotate(l);
+      rotate(p);
+    }
   }
 }
 
