@@ -825,14 +825,13 @@ __device__ __forceinline__ void scale_upper(double (&K)[N][N], double k) {
     for (int b = a; b < N; ++b) K[a][b] = ref::mul(k, K[a][b]);
 }
 
-// F = AFEM_FORMULATION_MINIMAL: the fewest FP64 instructions (below);
-// otherwise the reference's own rounding (ref::quad4_matrix / hexa8_matrix).
-template <int F>
-__global__ void __launch_bounds__(128) k_elem_poisson_quad4(int cell0, int nb_cell, const double* __restrict__ xyz,
-                                                            const int32_t* __restrict__ cn,
-                                                            const int32_t* __restrict__ inv,
-                                                            const double* __restrict__ coeff, double* __restrict__ er,
-                                                            int* __restrict__ bad) {
+// AFEM_FORMULATION_MINIMAL: the fewest FP64 instructions.
+__global__ void __launch_bounds__(128) k_elem_poisson_quad4_minimal(int cell0, int nb_cell,
+                                                                    const double* __restrict__ xyz,
+                                                                    const int32_t* __restrict__ cn,
+                                                                    const int32_t* __restrict__ inv,
+                                                                    const double* __restrict__ coeff,
+                                                                    double* __restrict__ er, int* __restrict__ bad) {
   for (int64_t c = cell0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell;
        c += (int64_t)gridDim.x * blockDim.x) {
     double x[4], y[4];
@@ -843,52 +842,184 @@ __global__ void __launch_bounds__(128) k_elem_poisson_quad4(int cell0, int nb_ce
       y[a] = __ldg(p + 1);
     }
     double K[4][4];
-    if constexpr (F != AFEM_FORMULATION_MINIMAL) {
-      const bool ok = ref::quad4_matrix(x, y, kQuadDnRef, K);
-      if (bad && !ok) atomicOr(bad, kFlagDegenerateCell);
-      if (coeff) scale_upper<4>(K, __ldg(coeff + c));
-      write_rows_q1<4>(K, inv + 4 * c, er);
-    } else {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) K[a][b] = 0.0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const double xi = (g >> 1) ? kGauss : -kGauss, eta = (g & 1) ? kGauss : -kGauss;
+      const double dxi[4] = {-0.25 * (1.0 - eta), 0.25 * (1.0 - eta), 0.25 * (1.0 + eta), -0.25 * (1.0 + eta)};
+      const double deta[4] = {-0.25 * (1.0 - xi), -0.25 * (1.0 + xi), 0.25 * (1.0 + xi), 0.25 * (1.0 - xi)};
+      double j00 = 0.0, j01 = 0.0, j10 = 0.0, j11 = 0.0;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        j00 += dxi[a] * x[a];
+        j01 += dxi[a] * y[a];
+        j10 += deta[a] * x[a];
+        j11 += deta[a] * y[a];
+      }
+      const double det = j00 * j11 - j01 * j10;
+      if (bad && !ref::measure_ok(det)) atomicOr(bad, kFlagDegenerateCell);
+      const double i00 = j11 / det, i01 = -j01 / det, i10 = -j10 / det, i11 = j00 / det;
+      double dx[4], dy[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        dx[a] = i00 * dxi[a] + i01 * deta[a];
+        dy[a] = i10 * dxi[a] + i11 * deta[a];
+      }
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) K[a][b] = 0.0;
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const double xi = (g >> 1) ? kGauss : -kGauss, eta = (g & 1) ? kGauss : -kGauss;
-        const double dxi[4] = {-0.25 * (1.0 - eta), 0.25 * (1.0 - eta), 0.25 * (1.0 + eta), -0.25 * (1.0 + eta)};
-        const double deta[4] = {-0.25 * (1.0 - xi), -0.25 * (1.0 + xi), 0.25 * (1.0 + xi), 0.25 * (1.0 - xi)};
-        double j00 = 0.0, j01 = 0.0, j10 = 0.0, j11 = 0.0;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          j00 += dxi[a] * x[a];
-          j01 += dxi[a] * y[a];
-          j10 += deta[a] * x[a];
-          j11 += deta[a] * y[a];
-        }
-        const double det = j00 * j11 - j01 * j10;
-        if (bad && !ref::measure_ok(det)) atomicOr(bad, kFlagDegenerateCell);
-        const double i00 = j11 / det, i01 = -j01 / det, i10 = -j10 / det, i11 = j00 / det;
-        double dx[4], dy[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          dx[a] = i00 * dxi[a] + i01 * deta[a];
-          dy[a] = i10 * dxi[a] + i11 * deta[a];
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = a; b < 4; ++b) K[a][b] += (dx[a] * dx[b]) * det + (dy[a] * dy[b]) * det;
-      }
-      if (coeff) {
-        const double k = __ldg(coeff + c);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = a; b < 4; ++b) K[a][b] *= k;
-      }
-      write_rows_q1<4>(K, inv + 4 * c, er);
+        for (int b = a; b < 4; ++b) K[a][b] += (dx[a] * dx[b]) * det + (dy[a] * dy[b]) * det;
     }
+    if (coeff) {
+      const double k = __ldg(coeff + c);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = a; b < 4; ++b) K[a][b] *= k;
+    }
+    write_rows_q1<4>(K, inv + 4 * c, er);
+  }
+}
+
+// The reference-rounding quadrangle with its products and quotients on the
+// integer pipes, as k_elem_poisson_hexa8_ref below: two magnitudes
+// 0.25 (1 -+ p) in the derivative tables, so 16 products of a cell's
+// coordinates serve the Jacobians of all Gauss points, and a Jacobian row
+// depends on one side.  About 140 of a cell's 530 FP64 instructions are left.
+constexpr double kQuadMag[2] = {0.25 * (1.0 - ref::kGaussPt), 0.25 * (1.0 + ref::kGaussPt)};
+constexpr bool quad_magnitudes_hold() {
+  constexpr ref::QuadDN dn = ref::make_quad_dn();
+  for (int g = 0; g < 4; ++g)
+    for (int a = 0; a < 4; ++a) {
+      const int side[2] = {(a ^ (a >> 1)) & 1, a >> 1}, at[2] = {g >> 1, g & 1};
+      for (int r = 0; r < 2; ++r) {
+        const double m = kQuadMag[side[1 - r] == at[1 - r]];
+        if (dn.v[g][r][a] != (side[r] ? m : -m)) return false;
+      }
+    }
+  return true;
+}
+static_assert(quad_magnitudes_hold(), "the derivative tables hold two magnitudes");
+
+// Row 0 (d/dxi) for the side s of eta and row 1 (d/deta) for the side s of xi,
+// at [row][s][component].  False where a coordinate is out of range.
+__device__ __forceinline__ bool quad_jacobian_rows(int64_t c, const double* __restrict__ xyz,
+                                                   const int32_t* __restrict__ cn, double J[2][2][2]) {
+  constexpr double mag[2] = {kQuadMag[0], kQuadMag[1]};
+  bool ok = true;
+  double prod[2][4][2];   // [magnitude][node][component]
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const double* p = xyz + 3 * (int64_t)__ldg(cn + 4 * c + a);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double x = __ldg(p + k);
+      ok &= i64fp::in_window<ref::kCoordWindow>(__double2hiint(x), __double2loint(x));
+      const ref::Val v(x);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) prod[m][a][k] = ref::mul(v, ref::Val(mag[m]));
+    }
+  }
+  // node a's sides: xi 0 1 1 0, eta 0 0 1 1
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        double j = 0.0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const int side[2] = {(a ^ (a >> 1)) & 1, a >> 1};
+          const double v = prod[side[1 - r] == s][a][k];
+          j = a == 0 ? -v : side[r] ? ref::add(j, v) : ref::sub(j, v);
+        }
+        J[r][s][k] = j;
+      }
+  return ok;
+}
+
+// A quadrangle whose operands leave the integer path's range, on the FP64 pipe alone.
+__device__ __noinline__ void elem_quad_cell_fp64(int64_t c, const double* xyz, const int32_t* cn, const int32_t* inv,
+                                                 const double* coeff, double* er, int* bad) {
+  double x[4], y[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const double* p = xyz + 3 * (int64_t)__ldg(cn + 4 * c + a);
+    x[a] = __ldg(p);
+    y[a] = __ldg(p + 1);
+  }
+  double K[4][4];
+  const bool ok = ref::quad4_matrix(x, y, kQuadDnRef, K);
+  if (bad && !ok) atomicOr(bad, kFlagDegenerateCell);
+  if (coeff) scale_upper<4>(K, __ldg(coeff + c));
+  write_rows_q1<4>(K, inv + 4 * c, er);
+}
+
+template <bool COEFF>
+__global__ void __launch_bounds__(128) k_elem_poisson_quad4_ref(int cell0, int nb_cell, const double* __restrict__ xyz,
+                                                                const int32_t* __restrict__ cn,
+                                                                const int32_t* __restrict__ inv,
+                                                                const double* __restrict__ coeff,
+                                                                double* __restrict__ er, int* __restrict__ bad) {
+  using ref::add;
+  using ref::mul;
+  using V = ref::Val;
+  constexpr double mag[2] = {kQuadMag[0], kQuadMag[1]};
+  for (int64_t c = cell0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    double jac[2][2][2], K[4][4];
+    bool ok = quad_jacobian_rows(c, xyz, cn, jac);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) K[i][k] = 0.0;
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g) {
+      const int gx = g >> 1, gy = g & 1;
+      double j[2][2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        j[0][k] = gy ? jac[0][1][k] : jac[0][0][k];
+        j[1][k] = gx ? jac[1][1][k] : jac[1][0][k];
+      }
+      const double det = ref::sub(mul(V(j[0][0]), V(j[1][1])), mul(V(j[0][1]), V(j[1][0])));
+      ok &= ref::measure_ok(det);
+      const V w(det, ok);
+      const i64fp::Divisor by = i64fp::divisor(__double_as_longlong(det));
+      auto quotient = [&](double x) { return V(__longlong_as_double(i64fp::div(V(x).o, by)), ok); };
+      V d[2][4];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {   // the inverse's row, then the gradients' component
+        const V v0 = quotient(r == 0 ? j[1][1] : -j[1][0]), v1 = quotient(r == 0 ? -j[0][1] : j[0][0]);
+        double p0[2], p1[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          p0[m] = mul(v0, V(mag[m]));
+          p1[m] = mul(v1, V(mag[m]));
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const int sx = (a ^ (a >> 1)) & 1, sy = a >> 1;
+          const double x = sy == gy ? p0[1] : p0[0], y = sx == gx ? p1[1] : p1[0];
+          d[r][a] = V(add(sx ? x : -x, sy ? y : -y), ok);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = i; k < 4; ++k)
+          K[i][k] = add(K[i][k], add(mul(V(mul(d[0][i], d[0][k])), w), mul(V(mul(d[1][i], d[1][k])), w)));
+    }
+    if (!ok) {
+      elem_quad_cell_fp64(c, xyz, cn, inv, coeff, er, bad);
+      continue;
+    }
+    if constexpr (COEFF) scale_upper<4>(K, __ldg(coeff + c));
+    write_rows_q1<4>(K, inv + 4 * c, er);
   }
 }
 
@@ -1098,6 +1229,78 @@ __device__ __noinline__ void elem_hexa_cell_fp64(int64_t c, const double* xyz, c
   write_rows_q1<8>(K, inv + 8 * c, er);
 }
 
+// The products of a cell's coordinates and the 12 Jacobian rows, by its four
+// threads; false where a coordinate is out of range.  S: prod and jac of
+// HexScratch.
+template <class S>
+__device__ __forceinline__ bool hex_jacobian_rows(const double* __restrict__ xyz, const int32_t* __restrict__ cn,
+                                                  int64_t c, int cs, int t, S& sh) {
+  using ref::add;
+  using ref::mul;
+  using ref::sub;
+  using V = ref::Val;
+  constexpr double mag[3] = {kHexMag[0], kHexMag[1], kHexMag[2]};
+  bool ok = true;
+  __syncwarp();
+#pragma unroll 1
+  for (int a = 2 * t; a < 2 * t + 2; ++a) {
+    const double* p = xyz + 3 * (int64_t)__ldg(cn + 8 * c + a);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double x = __ldg(p + k);
+      ok &= i64fp::in_window<ref::kCoordWindow>(__double2hiint(x), __double2loint(x));
+      const V v(x);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) sh.prod[24 * m + 8 * k + a][cs] = mul(v, V(mag[m]));
+    }
+  }
+  __syncwarp();
+  {
+    // node a's sides: xi 0 1 1 0 0 1 1 0, eta 0 0 1 1 0 0 1 1, zeta 0 0 0 0 1 1 1 1
+    const int s1 = t >> 1, s2 = t & 1;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      double J[3];
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        const int sx = (a ^ (a >> 1)) & 1, sy = (a >> 1) & 1, sz = a >> 2;
+        const int side = r == 0 ? sx : r == 1 ? sy : sz;             // the sign of dN_a
+        const int f1 = r == 0 ? sy : sx, f2 = r == 2 ? sy : sz;      // its two factors' sides
+        const double* q = &sh.prod[24 * ((f1 == s1) + (f2 == s2)) + a][cs];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const double v = q[64 * k];
+          J[k] = a == 0 ? -v : side ? add(J[k], v) : sub(J[k], v);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sh.jac[3 * (4 * r + t) + k][cs] = J[k];
+    }
+  }
+  __syncwarp();
+  return ok;
+}
+
+// det J at the Gauss point of sides (gx, gy, gz), t = 2 gy + gz, its three
+// minors and the Jacobian.
+template <class S>
+__device__ __forceinline__ double hex_determinant(const S& sh, int cs, int gx, int gy, int gz, ref::Val (&J)[3][3],
+                                                  double (&m)[3]) {
+  using ref::mul;
+  using ref::sub;
+  using V = ref::Val;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    J[0][k] = V(sh.jac[3 * (2 * gy + gz) + k][cs]);
+    J[1][k] = V(sh.jac[3 * (4 + 2 * gx + gz) + k][cs]);
+    J[2][k] = V(sh.jac[3 * (8 + 2 * gx + gy) + k][cs]);
+  }
+  m[0] = sub(mul(J[1][1], J[2][2]), mul(J[1][2], J[2][1]));
+  m[1] = sub(mul(J[1][0], J[2][2]), mul(J[1][2], J[2][0]));
+  m[2] = sub(mul(J[1][0], J[2][1]), mul(J[1][1], J[2][0]));
+  return ref::add(sub(mul(J[0][0], V(m[0])), mul(J[0][1], V(m[1]))), mul(J[0][2], V(m[2])));
+}
+
 // Where entry (i, j) of the symmetric matrix is kept in HexScratch::K.
 __device__ __forceinline__ int hex_entry(int i, int j) {
   const int lo = min(i, j), hi = max(i, j);
@@ -1116,70 +1319,27 @@ __global__ void __launch_bounds__(kHexBlock, 7)
   __shared__ HexScratch scratch[kHexBlock / 32];
   HexScratch& sh = scratch[threadIdx.x >> 5];
   const int cs = threadIdx.x & 7, t = (threadIdx.x >> 3) & 3;
-  constexpr double mag[3] = {kHexMag[0], kHexMag[1], kHexMag[2]};
+  constexpr double mag[3] = {kHexMag[0], kHexMag[1], kHexMag[2]};   // in registers, not memory
+  const bool wide = ((uintptr_t)er & 15) == 0;   // a caller's buffer may start at any double
   for (int64_t c0 = cell0 + blockIdx.x * (int64_t)(kHexBlock / 4) + (threadIdx.x >> 5) * 8; c0 < nb_cell;
        c0 += (int64_t)gridDim.x * (kHexBlock / 4)) {
     const bool here = c0 + cs < nb_cell;
     const int64_t c = here ? c0 + cs : nb_cell - 1;
-    bool ok = true;
-    __syncwarp();
-#pragma unroll 1
-    for (int a = 2 * t; a < 2 * t + 2; ++a) {
-      const double* p = xyz + 3 * (int64_t)__ldg(cn + 8 * c + a);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double x = __ldg(p + k);
-        ok &= i64fp::in_window<ref::kCoordWindow>(__double2hiint(x), __double2loint(x));
-        const V v(x);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) sh.prod[24 * m + 8 * k + a][cs] = mul(v, V(mag[m]));
-      }
-    }
-    __syncwarp();
-    {
-      // node a's sides: xi 0 1 1 0 0 1 1 0, eta 0 0 1 1 0 0 1 1, zeta 0 0 0 0 1 1 1 1
-      const int s1 = t >> 1, s2 = t & 1;
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        double J[3];
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-          const int sx = (a ^ (a >> 1)) & 1, sy = (a >> 1) & 1, sz = a >> 2;
-          const int side = r == 0 ? sx : r == 1 ? sy : sz;             // the sign of dN_a
-          const int f1 = r == 0 ? sy : sx, f2 = r == 2 ? sy : sz;      // its two factors' sides
-          const double* q = &sh.prod[24 * ((f1 == s1) + (f2 == s2)) + a][cs];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const double v = q[64 * k];
-            J[k] = a == 0 ? -v : side ? add(J[k], v) : sub(J[k], v);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) sh.jac[3 * (4 * r + t) + k][cs] = J[k];
-      }
-    }
-    __syncwarp();
+    bool ok = hex_jacobian_rows(xyz, cn, c, cs, t, sh);
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
       // Gauss point 4 half + t: its sides are half, t >> 1, t & 1
       const int gy = t >> 1, gz = t & 1, row0 = HexScratch::kRows * t;
       {
         V J[3][3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          J[0][k] = V(sh.jac[3 * t + k][cs]);
-          J[1][k] = V(sh.jac[3 * (4 + 2 * half + gz) + k][cs]);
-          J[2][k] = V(sh.jac[3 * (8 + 2 * half + gy) + k][cs]);
-        }
+        double m[3], num[3][3];
+        const double det = hex_determinant(sh, cs, half, gy, gz, J, m);
         auto minor = [&](int a, int b, int e, int f, int g, int h, int i, int j) {
           return sub(mul(J[a][b], J[e][f]), mul(J[g][h], J[i][j]));
         };
-        double num[3][3];
-        num[0][0] = minor(1, 1, 2, 2, 1, 2, 2, 1);
-        num[1][0] = minor(1, 0, 2, 2, 1, 2, 2, 0);
-        num[2][0] = minor(1, 0, 2, 1, 1, 1, 2, 0);
-        const double det = add(sub(mul(J[0][0], V(num[0][0])), mul(J[0][1], V(num[1][0]))), mul(J[0][2], V(num[2][0])));
-        num[1][0] = -num[1][0];
+        num[0][0] = m[0];
+        num[1][0] = -m[1];
+        num[2][0] = m[2];
         num[0][1] = minor(0, 2, 2, 1, 0, 1, 2, 2);
         num[0][2] = minor(0, 1, 1, 2, 0, 2, 1, 1);
         num[1][1] = minor(0, 0, 2, 2, 0, 2, 2, 0);
@@ -1253,8 +1413,14 @@ __global__ void __launch_bounds__(kHexBlock, 7)
       for (int i = 0; i < 8; ++i) {
         const int e1 = 2 * t, e0 = e1 - 1;
         const int j0 = t == 0 ? i : e0 + (e0 >= i), j1 = e1 + (e1 >= i);
-        reinterpret_cast<double2*>(er)[4 * (int64_t)__ldg(inv + 8 * c + i) + t] =
-            make_double2(sh.K[hex_entry(i, j0)][cs], sh.K[hex_entry(i, j1)][cs]);
+        double* const out = er + 8 * (int64_t)__ldg(inv + 8 * c + i) + 2 * t;
+        const double v0 = sh.K[hex_entry(i, j0)][cs], v1 = sh.K[hex_entry(i, j1)][cs];
+        if (wide) {
+          *reinterpret_cast<double2*>(out) = make_double2(v0, v1);
+        } else {
+          out[0] = v0;
+          out[1] = v1;
+        }
       }
     }
   }
@@ -1269,37 +1435,119 @@ __global__ void __launch_bounds__(kHexBlock, 7)
 // cell, in Gauss-point order: the deterministic order of a sequential cell
 // loop.  Jacobians in the reference's rounding (afem_elem_ref.cuh).
 template <int N>
-__global__ void __launch_bounds__(128) k_cell_source_q1(int nb_cell, const double* __restrict__ xyz,
-                                                        const int32_t* __restrict__ cn,
-                                                        const int32_t* __restrict__ inv, double qdot,
-                                                        double* __restrict__ term) {
+__device__ __forceinline__ void cell_source_q1(int64_t c, const double* __restrict__ xyz,
+                                               const int32_t* __restrict__ cn, const int32_t* __restrict__ inv,
+                                               double qdot, double* __restrict__ term) {
   constexpr int NG = N;   // 4 Gauss points for Quad4, 8 for Hexa8
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell; c += (int64_t)gridDim.x * blockDim.x) {
-    double x[N], y[N], z[N];
-    int32_t pos[N];
+  double x[N], y[N], z[N];
+  int32_t pos[N];
 #pragma unroll
-    for (int a = 0; a < N; ++a) {
-      const double* p = xyz + 3 * (int64_t)__ldg(cn + N * c + a);
-      x[a] = __ldg(p);
-      y[a] = __ldg(p + 1);
-      z[a] = __ldg(p + 2);
-      pos[a] = __ldg(inv + N * c + a);
+  for (int a = 0; a < N; ++a) {
+    const double* p = xyz + 3 * (int64_t)__ldg(cn + N * c + a);
+    x[a] = __ldg(p);
+    y[a] = __ldg(p + 1);
+    z[a] = __ldg(p + 2);
+    pos[a] = __ldg(inv + N * c + a);
+  }
+#pragma unroll 1
+  for (int g = 0; g < NG; ++g) {
+    double det;
+    const double* Nf;
+    if constexpr (N == 4) {
+      double J[2][2];
+      det = ref::quad4_jacobian(x, y, kQuadDnRef, g, J);
+      Nf = kQuadDnRef.N[g];
+    } else {
+      double J[3][3], mm[3];
+      det = ref::hexa8_jacobian(x, y, z, kHexDnRef, g, J, mm);
+      Nf = kHexDnRef.N[g];
+    }
+#pragma unroll
+    for (int a = 0; a < N; ++a) term[(int64_t)pos[a] * NG + g] = ref::mul(ref::mul(Nf[a], qdot), det);
+  }
+}
+
+template <int N>
+__device__ __noinline__ void cell_source_fp64(int64_t c, const double* xyz, const int32_t* cn, const int32_t* inv,
+                                              double qdot, double* term) {
+  cell_source_q1<N>(c, xyz, cn, inv, qdot, term);
+}
+
+// N_a qdot of Gauss point g at [N g + a], for the block; N_a is between 2^-7
+// and 1.  Whether the products with a determinant stay in range.
+template <int N>
+__device__ __forceinline__ bool source_weights(const double (&shape)[N][N], double qdot, double* weight) {
+  for (int i = threadIdx.x; i < N * N; i += blockDim.x) weight[i] = ref::mul(shape[i / N][i % N], qdot);
+  __syncthreads();
+  return i64fp::in_window<i64fp::kWindow - 10>(__double2hiint(qdot), __double2loint(qdot));
+}
+
+// Quad4 and Hexa8 with the split of k_elem_poisson_quad4_ref / _hexa8_ref: the
+// Jacobian rows once, the products on the integer pipes; about 30 of a
+// quadrangle's 170 FP64 instructions and 290 of a hexahedron's 1330 are left.
+__global__ void __launch_bounds__(128) k_cell_source_quad4(int nb_cell, const double* __restrict__ xyz,
+                                                           const int32_t* __restrict__ cn,
+                                                           const int32_t* __restrict__ inv, double qdot,
+                                                           double* __restrict__ term) {
+  using V = ref::Val;
+  __shared__ double weight[16];
+  const bool q_ok = source_weights<4>(kQuadDnRef.N, qdot, weight);
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell; c += (int64_t)gridDim.x * blockDim.x) {
+    double jac[2][2][2];
+    bool ok = q_ok & quad_jacobian_rows(c, xyz, cn, jac);
+    V w[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const double *j0 = jac[0][g & 1], *j1 = jac[1][g >> 1];
+      w[g] = V(ref::sub(ref::mul(V(j0[0]), V(j1[1])), ref::mul(V(j0[1]), V(j1[0]))), ok);
+    }
+    if (!ok) {
+      cell_source_fp64<4>(c, xyz, cn, inv, qdot, term);
+      continue;
     }
 #pragma unroll 1
-    for (int g = 0; g < NG; ++g) {
-      double det;
-      const double* Nf;
-      if constexpr (N == 4) {
-        double J[2][2];
-        det = ref::quad4_jacobian(x, y, kQuadDnRef, g, J);
-        Nf = kQuadDnRef.N[g];
-      } else {
-        double J[3][3], mm[3];
-        det = ref::hexa8_jacobian(x, y, z, kHexDnRef, g, J, mm);
-        Nf = kHexDnRef.N[g];
-      }
+    for (int a = 0; a < 4; ++a) {
+      double* const out = term + 4 * (int64_t)__ldg(inv + 4 * c + a);
 #pragma unroll
-      for (int a = 0; a < N; ++a) term[(int64_t)pos[a] * NG + g] = ref::mul(ref::mul(Nf[a], qdot), det);
+      for (int g = 0; g < 4; ++g) out[g] = ref::mul(V(weight[4 * g + a]), w[g]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kHexBlock) k_cell_source_hexa8(int nb_cell, const double* __restrict__ xyz,
+                                                                 const int32_t* __restrict__ cn,
+                                                                 const int32_t* __restrict__ inv, double qdot,
+                                                                 double* __restrict__ term) {
+  using V = ref::Val;
+  __shared__ struct {
+    double prod[72][8], jac[36][8];
+  } scratch[kHexBlock / 32];
+  __shared__ double weight[64];
+  const bool q_ok = source_weights<8>(kHexDnRef.N, qdot, weight);
+  auto& sh = scratch[threadIdx.x >> 5];
+  const int cs = threadIdx.x & 7, t = (threadIdx.x >> 3) & 3;
+  for (int64_t c0 = blockIdx.x * (int64_t)(kHexBlock / 4) + (threadIdx.x >> 5) * 8; c0 < nb_cell;
+       c0 += (int64_t)gridDim.x * (kHexBlock / 4)) {
+    const bool here = c0 + cs < nb_cell;
+    const int64_t c = here ? c0 + cs : nb_cell - 1;
+    bool ok = q_ok & hex_jacobian_rows(xyz, cn, c, cs, t, sh);
+    V det[2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      V J[3][3];
+      double m[3];
+      det[half] = V(hex_determinant(sh, cs, half, t >> 1, t & 1, J, m), ok);
+    }
+    const unsigned all = __ballot_sync(0xffffffffu, ok);
+    if ((all >> cs & 0x01010101u) != 0x01010101u) {
+      if (here && t == 0) cell_source_fp64<8>(c, xyz, cn, inv, qdot, term);
+    } else if (here) {
+#pragma unroll 2
+      for (int a = 0; a < 8; ++a) {
+        double* out = term + 8 * (int64_t)__ldg(inv + 8 * c + a) + t;
+        out[0] = ref::mul(V(weight[8 * t + a]), det[0]);
+        out[4] = ref::mul(V(weight[8 * (4 + t) + a]), det[1]);
+      }
     }
   }
 }
@@ -1406,13 +1654,44 @@ __device__ __forceinline__ double cell_measure_ref(int dim, const double* __rest
   return ref::tet_volume(n);
 }
 
+// The volume of a tetrahedron (computeVolumeTetra4) with its products and the
+// quotient on the integer pipes: 14 of its 26 FP64 instructions are left, which
+// bind these kernels.  Coordinates outside that path's range: on the FP64 pipe.
+__device__ __forceinline__ bool tet_volume_int(const double* __restrict__ xyz, const int32_t* __restrict__ cn,
+                                               int64_t c, double* vol) {
+  const int4 q = __ldg(reinterpret_cast<const int4*>(cn) + c);
+  const int32_t nid[4] = {q.x, q.y, q.z, q.w};
+  double n[4][3];
+  bool ok = true;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      n[a][k] = __ldg(xyz + 3 * (int64_t)nid[a] + k);
+      ok &= i64fp::in_window<ref::kCoordWindow>(__double2hiint(n[a][k]), __double2loint(n[a][k]));
+    }
+  ref::Val v[3][3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[j][k] = ref::Val(ref::sub(n[j + 1][k], n[0][k]));
+  *vol = ref::div6(ref::Val(ref::tet_v6(v[0], v[1], v[2])));
+  return ok;
+}
+__device__ __forceinline__ double tet_volume_at(const double* __restrict__ xyz, const int32_t* __restrict__ cn,
+                                                int64_t c) {
+  double vol;
+  if (!tet_volume_int(xyz, cn, c, &vol)) vol = cell_measure_ref(3, xyz, cn, c);
+  return vol;
+}
+
 // w_c = (qdot * measure) / npc, each operation rounded as the reference's
 // sum += qdot * domain / nbItem rounds it (the division by 4 an exact
 // scaling, by 3 the corrected constant-reciprocal product).
 __global__ void k_cell_source_weight(int nb_cell, int dim, const double* __restrict__ xyz,
                                      const int32_t* __restrict__ cn, double qdot, double* __restrict__ w) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell; c += (int64_t)gridDim.x * blockDim.x) {
-    const double qm = __dmul_rn(qdot, cell_measure_ref(dim, xyz, cn, c));
+    const double qm = __dmul_rn(qdot, dim == 3 ? tet_volume_at(xyz, cn, c) : cell_measure_ref(dim, xyz, cn, c));
     w[c] = dim == 3 ? ref::div_const<4>(qm) : ref::div_const<3>(qm);
   }
 }
@@ -1437,7 +1716,7 @@ __global__ void k_node_sum(int nb_node, const int32_t* __restrict__ nc_ptr, cons
 __global__ void k_cell_volume(int nb_cell, const double* __restrict__ xyz, const int32_t* __restrict__ cn,
                               double* __restrict__ vol) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell; c += (int64_t)gridDim.x * blockDim.x)
-    vol[c] = cell_measure_ref(3, xyz, cn, c);
+    vol[c] = tet_volume_at(xyz, cn, c);
 }
 
 static afem_status check_mesh(const afem_mesh_view* m, const char* who) {
@@ -1528,10 +1807,10 @@ static afem_status launch_elem_q1(afem_context ctx, const afem_mesh_view* m, int
                    : launch(ctx, coeff ? k_elem_poisson_hexa8_ref<true> : k_elem_poisson_hexa8_ref<false>,
                             grid_for(ctx, (int64_t)(c1 - c0) * 4, kHexBlock, 28), kHexBlock, 0, c0, c1, m->coords_d,
                             m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad);
-  return minimal ? launch(ctx, k_elem_poisson_quad4<AFEM_FORMULATION_MINIMAL>, ge, 128, 0, c0, c1, m->coords_d,
-                          m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad)
-                 : launch(ctx, k_elem_poisson_quad4<AFEM_FORMULATION_REFERENCE>, ge, 128, 0, c0, c1, m->coords_d,
-                          m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad);
+  return minimal ? launch(ctx, k_elem_poisson_quad4_minimal, ge, 128, 0, c0, c1, m->coords_d, m->cell_nodes_d,
+                          m->nc_inverse_d, coeff, ke, bad)
+                 : launch(ctx, coeff ? k_elem_poisson_quad4_ref<true> : k_elem_poisson_quad4_ref<false>, ge, 128, 0,
+                          c0, c1, m->coords_d, m->cell_nodes_d, m->nc_inverse_d, coeff, ke, bad);
 }
 
 static afem_status launch_elem_elasticity(afem_context ctx, const afem_mesh_view* m, int c0, int c1, double lambda,
@@ -1912,10 +2191,10 @@ afem_status afem_rhs_constant_source_q1(afem_context ctx, const afem_mesh_view* 
   double* term;
   AFEM_TRY(scratch_take(ctx, npc * npc * (size_t)m->nb_cell, &term));
   if (m->dim == 3)
-    AFEM_TRY(launch(ctx, k_cell_source_q1<8>, grid_for(ctx, m->nb_cell, 128, 16), 128, 0, m->nb_cell, m->coords_d,
-                    m->cell_nodes_d, m->nc_inverse_d, qdot, term));
+    AFEM_TRY(launch(ctx, k_cell_source_hexa8, grid_for(ctx, (int64_t)m->nb_cell * 4, kHexBlock, 48), kHexBlock, 0,
+                    m->nb_cell, m->coords_d, m->cell_nodes_d, m->nc_inverse_d, qdot, term));
   else
-    AFEM_TRY(launch(ctx, k_cell_source_q1<4>, grid_for(ctx, m->nb_cell, 128, 16), 128, 0, m->nb_cell, m->coords_d,
+    AFEM_TRY(launch(ctx, k_cell_source_quad4, grid_for(ctx, m->nb_cell, 128, 16), 128, 0, m->nb_cell, m->coords_d,
                     m->cell_nodes_d, m->nc_inverse_d, qdot, term));
   return launch(ctx, k_incidence_sum, grid_for(ctx, m->nb_node, 256), 256, 0, m->nb_node, m->nc_ptr_d,
                 (const double*)term, (int)npc, nb_dof, rhs_d);

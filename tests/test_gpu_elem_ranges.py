@@ -83,3 +83,40 @@ def test_elasticity_over_the_operand_ranges(own_ctx, n, jitter, case, lam, mu):
     f.assemble_elasticity(lam, mu)
     ref = oracle_values(m, O.ELASTICITY_TET4, lam=lam, mu=mu)
     assert_bit_exact(f.values.cpu().numpy(), ref, "elasticity")
+
+
+MAKE = {"quad": meshgen.unit_square_quad, "tet": meshgen.unit_cube_tet, "hex": meshgen.unit_cube_hex}
+
+
+@pytest.mark.parametrize("n,jitter,case", CASES)
+def test_quadrangles_over_the_operand_ranges(own_ctx, n, jitter, case):
+    m = moved_mesh(meshgen.unit_square_quad, 3 * n, jitter, case)
+    f = build_format(own_ctx, m)
+    f.assemble_poisson()
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_QUAD4), "quadrangles")
+    k = np.exp(np.random.default_rng(0).standard_normal(m.nb_cell))
+    f.assemble_poisson(torch.as_tensor(k, device="cuda"))
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_QUAD4, coeff=k), "coefficient")
+
+
+@pytest.mark.parametrize("qdot", [-5.5, 0.0, 2.0 ** 245, 2.0 ** -243])
+@pytest.mark.parametrize("kind", list(MAKE))
+@pytest.mark.parametrize("n,jitter,case", CASES)
+def test_sources_over_the_operand_ranges(own_ctx, kind, n, jitter, case, qdot):
+    m = moved_mesh(MAKE[kind], n, jitter, case)
+    f = build_format(own_ctx, m)
+    rhs = torch.zeros(m.nb_node, dtype=torch.float64, device="cuda")
+    f.rhs_constant_source(qdot, rhs)
+    ptr, nc, _ = O.node_cell(m.nb_node, m.cells)
+    fn = O.rhs_constant_source if kind == "tet" else O.rhs_constant_source_q1
+    assert_bit_exact(rhs.cpu().numpy(), fn(m.dim, m.coords, m.cells, ptr, nc, qdot), "source")
+
+
+def test_hexahedra_into_a_buffer_at_an_odd_double(own_ctx):
+    m = meshgen.unit_cube_hex(3, jitter=0.15, seed=1)
+    f = build_format(own_ctx, m)
+    ke = torch.zeros(2 * f.element_buffer_size() + 2, dtype=torch.float64, device="cuda")
+    size = f.element_buffer_size()
+    f.element_matrices(ke[:size])
+    f.element_matrices(ke[size + 1:2 * size + 1])
+    assert torch.equal(ke[:size], ke[size + 1:2 * size + 1]) and float(ke[size]) == 0.0
