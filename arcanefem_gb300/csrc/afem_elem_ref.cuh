@@ -325,6 +325,30 @@ __device__ __forceinline__ double tri_gradients(const double n[3][3], double dx[
   return A2;
 }
 
+// Twice the signed area of a triangle whose nodes share one z, with its
+// products on the integer pipes.  Of the cross product only z is left then, and
+// it is the signed A2 too; the square root of its rounded square is its
+// magnitude exactly (radix 2, no overflow or underflow), so that the area is
+// |A2| / 2 bit for bit.  e: n1 - n0 and n2 - n0.  Returns false where z differs
+// or a coordinate is out of the integer path's range.
+__device__ __forceinline__ bool tri_planar(const double n[3][3], double e[2][2], double* A2) {
+  bool ok = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (k < 2) ok &= i64fp::in_window<kCoordWindow>(__double2hiint(n[a][k]), __double2loint(n[a][k]));
+      else
+        ok &= bexp(n[a][2]) != 2047 && __double_as_longlong(n[a][2]) == __double_as_longlong(n[0][2]);
+    }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) e[j][k] = sub(n[j + 1][k], n[0][k]);
+  *A2 = sub(mul(Val(e[0][0]), Val(e[1][1])), mul(Val(e[0][1]), Val(e[1][0])));
+  return ok;
+}
+
 // computeAreaTria3 (ArcaneFemFunctionsGpu.h:76-86): |(n1 - n0) x (n2 - n0)| / 2.
 __device__ __forceinline__ double tri_area(const double n[3][3]) {
   const double a0 = sub(n[1][0], n[0][0]), a1 = sub(n[1][1], n[0][1]), a2 = sub(n[1][2], n[0][2]);

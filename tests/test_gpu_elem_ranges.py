@@ -85,6 +85,24 @@ def test_elasticity_over_the_operand_ranges(own_ctx, n, jitter, case, lam, mu):
     assert_bit_exact(f.values.cpu().numpy(), ref, "elasticity")
 
 
+@pytest.mark.parametrize("bent", [False, True])
+@pytest.mark.parametrize("n,jitter,case", CASES)
+def test_triangles_over_the_operand_ranges(own_ctx, n, jitter, case, bent):
+    m = moved_mesh(meshgen.unit_square_tri, 3 * n, jitter, case)
+    if bent:                     # a third of the nodes out of the plane: their triangles take the general area
+        m.coords[::3, 2] = 0.3 * m.coords[::3, 0]
+    f = build_format(own_ctx, m)
+    f.assemble_poisson()
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_TRI3), "triangles")
+    k = np.exp(np.random.default_rng(0).standard_normal(m.nb_cell))
+    f.assemble_poisson(torch.as_tensor(k, device="cuda"))
+    assert_bit_exact(f.values.cpu().numpy(), oracle_values(m, O.POISSON_TRI3, coeff=k), "coefficient")
+    rhs = torch.zeros(m.nb_node, dtype=torch.float64, device="cuda")
+    f.rhs_constant_source(-5.5, rhs)
+    ptr, nc, _ = O.node_cell(m.nb_node, m.cells)
+    assert_bit_exact(rhs.cpu().numpy(), O.rhs_constant_source(2, m.coords, m.cells, ptr, nc, -5.5), "source")
+
+
 MAKE = {"quad": meshgen.unit_square_quad, "tet": meshgen.unit_cube_tet, "hex": meshgen.unit_cube_hex}
 
 
