@@ -11,13 +11,13 @@
 //    cost model (rows x sqrt(rows)^(exponent - 2): Jacobi CG needs ~N
 //    iterations on an N x N grid) so that the teams finish together; teams
 //    never wait on each other;
-//  * a team barrier is an arrival counter plus a generation word in global
-//    memory; every wait is bounded (spin limit) and sets a batch error flag
-//    when it runs out, after which all CTAs return;
-//  * team reductions are written as per-CTA partials and summed by every CTA
-//    in the same fixed order, so all CTAs of a team take the same decisions
-//    (alpha, beta, convergence) without a broadcast, and results are
-//    deterministic;
+//  * the CTAs of a team meet through 16-byte slots that carry a partial sum and
+//    the number of the exchange: the team's first CTA polls the others' slots,
+//    adds them in a fixed order, decides (alpha, beta, convergence) and
+//    publishes the decision in one line that the others poll, so all CTAs of a
+//    team agree and results are deterministic;
+//  * every wait is bounded (spin limit) and sets a batch error flag when it
+//    runs out, after which all CTAs return;
 //  * phase A assembles each row (thread per row, element rows recomputed from
 //    the incident cells in incidence order, exactly the arithmetic of the
 //    node-wise gather), applies Dirichlet row-column elimination as
@@ -34,19 +34,14 @@
 #include <cmath>
 #include <vector>
 
+#include "afem_fp64_int.cuh"
 #include "afem_krylov.cuh"
 
 namespace afem {
 
 constexpr int kBatchRhs = 4;
 constexpr int kBumps = 8;
-constexpr int kPartStride = 32;   // doubles of partials per CTA: 4 regions x 8
-
-struct __align__(128) TeamBar {
-  unsigned count;
-  unsigned gen;
-  unsigned pad[30];
-};
+constexpr int kTeamSlots = 16;    // slots of a CTA, and of a team's totals: 2 parities x 8 sums
 
 struct BatchInst {
   int n, nnz, ncell, cta0, ncta, pad0, pad1, pad2;
@@ -71,8 +66,8 @@ struct BatchInst {
   float4* p;
   float4* q;
   float4* d;
-  double* part;         // [ncta][kPartStride]
-  TeamBar* bar;
+  ulonglong2* part;     // [ncta][kTeamSlots]
+  ulonglong2* total;    // [kTeamSlots]
   afem_batch_result* res;
 };
 
@@ -80,6 +75,7 @@ struct BatchParams {
   double rtol, atol, inner_rtol;
   int max_inner, max_outer;
   long long spin_limit;
+  int own_rows;         // rows of a CTA whose q and d fit its shared memory
   int stall_cta;        // >= 0: that CTA leaves before its first barrier (failure-detection test)
 };
 
@@ -90,74 +86,133 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 }
 
 // ---------------------------------------------------------------------------
-// Team barrier and reductions.
+// The team's exchanges.  Slots alternate with the exchange's parity: a CTA
+// enters exchange e + 2 only after the totals of e + 1, for which every CTA has
+// left e.
 
-__device__ __forceinline__ bool team_sync(TeamBar* bar, int T, unsigned* gen_sh, int* err, long long limit) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned g = *gen_sh;
-    __threadfence();
-    if (atomicAdd(&bar->count, 1u) == (unsigned)T - 1u) {
-      atomicExch(&bar->count, 0u);
-      __threadfence();
-      atomicExch(&bar->gen, g + 1u);
-    } else {
-      long long spins = 0;
-      while (*(volatile unsigned*)&bar->gen == g) {
-        if (*(volatile int*)err) break;
-        if (++spins > limit) {
-          atomicCAS(err, 0, (int)AFEM_ERR_TIMEOUT);
-          break;
-        }
-        __nanosleep(128);
-      }
+// Poll a slot; false when the wait runs out.
+// PATIENCE polls go without a pause.
+template <int PATIENCE>
+__device__ __forceinline__ bool team_poll(const ulonglong2* s, unsigned epoch, int* err, long long limit, double* v) {
+  ulonglong2 got = slot_get(s);
+  long long spins = 0;
+  while (got.y != epoch) {
+    if (++spins > limit || ((spins & 255) == 0 && *(volatile int*)err)) {
+      atomicCAS(err, 0, (int)AFEM_ERR_TIMEOUT);
+      return false;
     }
-    __threadfence();
-    *gen_sh = g + 1u;
+    if (spins > PATIENCE) __nanosleep(32);   // leave the issue slots to the SM's other CTAs
+    got = slot_get(s);
   }
-  __syncthreads();
-  return *(volatile int*)err == 0;
-}
-
-// Sum v[0..M) over the block and then over the team (fixed order); the
-// results land in out[0..M) for every thread of every CTA of the team.
-// `region` (0..3) selects the partials slot (see the phase notes below).
-// T = float for the inner-solve dot products: per-thread and per-warp sums
-// stay on the FP32 pipe (GB300 issues FP64 at 1/74 of FP32, and the per-row
-// FP64 accumulation bound this kernel), only warp totals go to FP64.
-template <int BLOCK, int M, class T>
-__device__ __forceinline__ bool team_reduce(const T (&v)[M], double (&out)[M], const BatchInst& I, int rank,
-                                            int region, double (*red)[8], double* tres, unsigned* gen_sh, int* err,
-                                            long long limit) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < M; ++j) {
-    T s = v[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) red[warp][j] = (double)s;
-  }
-  __syncthreads();
-  if (threadIdx.x < M) {
-    double s = 0.0;
-    for (int w = 0; w < BLOCK / 32; ++w) s += red[w][threadIdx.x];
-    I.part[(int64_t)rank * kPartStride + region * 8 + threadIdx.x] = s;
-  }
-  if (!team_sync(I.bar, I.ncta, gen_sh, err, limit)) return false;
-  for (int j = warp; j < M; j += BLOCK / 32) {
-    double s = 0.0;
-    for (int k = lane; k < I.ncta; k += 32)
-      s += ((volatile const double*)I.part)[(int64_t)k * kPartStride + region * 8 + j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) tres[j] = s;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < M; ++j) out[j] = tres[j];
-  __syncthreads();
+  *v = __longlong_as_double(got.x);
   return true;
 }
+
+// Sums of v[0..M) over the block and then over the team, in a fixed order.  In
+// the team's first CTA, warp 0 calls decide(lane, total) with the total of sum
+// j in the lanes j, j + M, ...; the 8 bytes that it returns in lanes 0..3 reach
+// cast[0..4) of every CTA.  Only that CTA computes with the totals: an FP64
+// instruction takes an SM some 20 cycles however few lanes take part, and four
+// divisions in turn in each of an SM's four CTAs took longer than the rest of
+// the exchange (8 sums in a team of 2 CTAs: 17 000 cycles, 10 000 now; of 166
+// CTAs 21 000, 14 000 now, most of it the wait for the slowest CTA).
+// T = float for the inner-solve dot products: per-thread and per-warp sums
+// stay on the FP32 pipe, only warp totals go to FP64.
+// FENCE: what the team's threads wrote before is visible to all of them after.
+template <int BLOCK, int M, bool FENCE, class T, class F>
+__device__ __forceinline__ bool team_exchange(const T (&v)[M], const BatchInst& I, int rank, T (*red)[8],
+                                              double (*red64)[8], unsigned long long* cast, unsigned& epoch, int* err,
+                                              long long limit, F&& decide) {
+  constexpr int N = BLOCK / 32, G = 32 / M;   // warps; lanes that share a sum
+  static_assert(M == 1 || M == 4 || M == 8, "the lanes of a sum");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ++epoch;
+  const int parity = (epoch & 1) * 8;
+  {
+    // halve the sums a lane holds while there are several, then its partners: lane l ends with sum l / G
+    T w[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) w[j] = v[j];
+    int o = 16;
+#pragma unroll
+    for (int h = M / 2; h > 0; h >>= 1, o >>= 1)
+#pragma unroll
+      for (int j = 0; j < h; ++j) {
+        const bool up = (lane & o) != 0;
+        const T give = up ? w[j] : w[j + h], keep = up ? w[j + h] : w[j];
+        w[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+#pragma unroll
+    for (; o > 0; o >>= 1) w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
+    if (lane % G == 0) red[warp][lane / G] = w[0];
+  }
+  __syncthreads();
+  // lane l adds the warps l / M, l / M + G, ... of sum l % M
+  auto add_warps = [&](auto* r) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < N; w += G)
+      if (w + lane / M < N) s += (double)r[w + lane / M][lane % M];
+#pragma unroll
+    for (int o = 16; o >= M; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  };
+  if (warp == 0) {
+    const double s = add_warps(red);
+    if (lane < M) {
+      if constexpr (FENCE) __threadfence();
+      slot_put(I.part + (int64_t)rank * kTeamSlots + parity + lane, __double_as_longlong(s), epoch);
+    }
+  }
+  bool ok = true;
+  if (rank == 0) {
+    double s = 0.0;
+    for (int k = threadIdx.x / M; k < I.ncta && ok; k += BLOCK / M) {
+      double x = 0.0;
+      ok = team_poll<8>(I.part + (int64_t)k * kTeamSlots + parity + lane % M, epoch, err, limit, &x);
+      s += x;
+    }
+    if constexpr (FENCE) __threadfence();
+#pragma unroll
+    for (int o = 16; o >= M; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < M) red64[warp][lane] = s;
+    ok = __syncthreads_and(ok);
+    if (warp == 0 && ok) {
+      const unsigned long long d = decide(lane, add_warps(red64));
+      if (lane < 4) {
+        if constexpr (FENCE) __threadfence();
+        slot_put(I.total + parity + lane, d, epoch);
+        cast[lane] = d;
+      }
+    }
+  } else if (threadIdx.x < 4) {
+    double d = 0.0;
+    ok = team_poll<64>(I.total + parity + threadIdx.x, epoch, err, limit, &d);
+    cast[threadIdx.x] = __double_as_longlong(d);
+    if constexpr (FENCE) __threadfence();
+  }
+  return __syncthreads_and(ok);
+}
+
+// a / b rounded to nearest on the integer pipes (afem_fp64_int.cuh) where both
+// are in its range: an FP64 division is some ten dependent FP64 instructions.
+__device__ __forceinline__ double quotient(double a, double b) {
+  const int ah = __double2hiint(a), bh = __double2hiint(b);
+  if (!i64fp::in_window<400>(ah, __double2loint(a)) || !i64fp::in_window<400>(bh, __double2loint(b)) ||
+      (bh & 0x7ff00000) == 0)
+    return a / b;
+  return __longlong_as_double(i64fp::div(i64fp::operand(ah, __double2loint(a)),
+                                         i64fp::divisor(__double_as_longlong(b))));
+}
+
+// What the first CTA tells the others of a right-hand side: a float, whether
+// the side is active, and a flag that is the same for all four.
+__device__ __forceinline__ unsigned long long told(float v, bool active, bool flag) {
+  return (unsigned long long)__float_as_uint(v) | (unsigned long long)active << 32 | (unsigned long long)flag << 33;
+}
+__device__ __forceinline__ float told_value(unsigned long long c) { return __uint_as_float((unsigned)c); }
+__device__ __forceinline__ bool told_active(unsigned long long c) { return c >> 32 & 1; }
+__device__ __forceinline__ bool told_flag(unsigned long long c) { return c >> 33 & 1; }
 
 // ---------------------------------------------------------------------------
 // Phase A: one row of the Poisson operator, its elimination, the source.
@@ -228,12 +283,15 @@ __device__ __forceinline__ void assemble_row(const BatchInst& I, int row) {
 
 constexpr int kRowUnroll = 8;   // entries of a row loaded together in the FP32 SpMV (2D P1 rows hold ~7)
 
-// Per-CTA copy of the team's solver scalars (identical in every CTA of a team).
+__host__ __device__ __forceinline__ int rows_per_cta(int n, int ncta) {
+  return ((n + ncta - 1) / ncta + 31) / 32 * 32;
+}
+
+// The team's solver scalars, in its first CTA.
 struct SolveState {
   double bnorm2[kBatchRhs], tol2[kBatchRhs], rr64[kBatchRhs], itol2[kBatchRhs], rz[kBatchRhs], rzprev[kBatchRhs];
-  float alpha[kBatchRhs], beta[kBatchRhs], zc[kBatchRhs];
   int active[kBatchRhs], keep[kBatchRhs];
-  int any, all_done;
+  int status;
 };
 
 template <int BLOCK>
@@ -242,35 +300,47 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
                                                                int* err) {
   __shared__ BatchInst I;
   __shared__ SolveState S;
-  __shared__ double red[BLOCK / 32][8];
-  __shared__ double tres[8];
-  __shared__ unsigned gen_sh;
+  __shared__ float red[BLOCK / 32][8];
+  __shared__ double red64[BLOCK / 32][8], norms[BLOCK / 32][8];
+  __shared__ unsigned long long cast[4];
+  extern __shared__ __align__(16) float4 own_rows[];   // [2][own_rows]
+  unsigned epoch = 0;   // exchanges of the team so far
   const int team = cta_team[blockIdx.x];
   if (threadIdx.x == 0) {
     I = insts[team];
-    gen_sh = 0u;
+    S.status = AFEM_OK;
   }
   __syncthreads();
   const int rank = blockIdx.x - I.cta0;
-  const int nthr = I.ncta * BLOCK;
-  const int tid = rank * BLOCK + threadIdx.x;
+  // a CTA's rows are consecutive: neighbours gathered by several of them come from its L1
+  const int per = rows_per_cta(I.n, I.ncta);
+  const int row0 = min(I.n, rank * per) + (int)threadIdx.x, row1 = min(I.n, (rank + 1) * per);
+  // q and d, which no other CTA reads, in shared memory if the CTA's rows fit
+  const bool own = per <= prm.own_rows;
+  float4* const own_q = own ? own_rows : I.q;
+  float4* const own_d = own ? own_rows + prm.own_rows : I.d;
+  const int off = own ? rank * per : 0;
   const long long lim = prm.spin_limit;
   const unsigned long long t_start = globaltimer_ns();
   if ((int)blockIdx.x == prm.stall_cta) return;   // failure-detection test: this CTA never arrives
 
+  // the team's barrier
+  auto sync = [&]() {
+    const float none[1] = {0.f};
+    return team_exchange<BLOCK, 1, true>(none, I, rank, red, red64, cast, epoch, err, lim,
+                                         [](int, double) { return 0ull; });
+  };
+
   // ---- phase A: assembly
-  for (int row = tid; row < I.n; row += nthr) assemble_row(I, row);
-  if (!team_sync(I.bar, I.ncta, &gen_sh, err, lim)) return;
+  for (int row = row0; row < row1; row += BLOCK) assemble_row(I, row);
+  if (!sync()) return;
 
   // ---- phase B: FP64 refinement around FP32 Jacobi CG, 4 right-hand sides
-  // Partials regions: 0 = <p,q>, 1 = <r,z>,<r,r> (inner), 2 = outer residual
-  // norms, 3 = initial <r,z> of an inner solve.  Consecutive uses of one
-  // region are always separated by at least two team barriers.
-  int inner_total = 0, outer = 0, status = AFEM_OK;
+  int inner_total = 0, outer = 0;
   for (;; ++outer) {
     {
       double loc[2 * kBatchRhs] = {};
-      for (int row = tid; row < I.n; row += nthr) {
+      for (int row = row0; row < row1; row += BLOCK) {
         double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
         for (int32_t k = I.rp[row]; k < I.rp[row + 1]; ++k) {
           const double a = I.vals[k];
@@ -285,34 +355,34 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
         loc[0] += r0 * r0; loc[1] += r1 * r1; loc[2] += r2 * r2; loc[3] += r3 * r3;
         loc[4] += br[0] * br[0]; loc[5] += br[1] * br[1]; loc[6] += br[2] * br[2]; loc[7] += br[3] * br[3];
       }
-      double tot[2 * kBatchRhs];
-      if (!team_reduce<BLOCK, 2 * kBatchRhs>(loc, tot, I, rank, 2, red, tres, &gen_sh, err, lim)) return;
-      if (threadIdx.x == 0) {
-        int all = 1;
-        for (int j = 0; j < kBatchRhs; ++j) {
-          if (outer == 0) {
-            S.bnorm2[j] = tot[kBatchRhs + j];
-            S.tol2[j] = fmax(prm.rtol * prm.rtol * S.bnorm2[j], prm.atol * prm.atol);
-          }
-          // keep the direction when the last cycle at least halved the true
-          // residual and cycles are short enough for the FP32 recursive
-          // residual to stay close to the true one (inner_rtol >= 0.01)
-          S.keep[j] = outer > 0 && prm.inner_rtol >= 0.01 && tot[j] <= 0.25 * S.rr64[j];
-          S.rr64[j] = tot[j];
-          const int dn = !(tot[j] > S.tol2[j]);
-          S.active[j] = !dn;
-          S.itol2[j] = prm.inner_rtol * prm.inner_rtol * tot[j];
-          all = all && dn;
-        }
-        S.all_done = all;
-      }
-      __syncthreads();
+      // lanes j: ||r_j||^2, lanes 4 + j: ||b_j||^2
+      const bool first = outer == 0, last = outer >= prm.max_outer;
+      if (!team_exchange<BLOCK, 2 * kBatchRhs, false>(
+              loc, I, rank, norms, red64, cast, epoch, err, lim, [&](int lane, double t) {
+                const double bb = __shfl_down_sync(0xffffffffu, t, kBatchRhs);
+                const int j = lane & (kBatchRhs - 1);
+                if (lane < kBatchRhs) {
+                  if (first) {
+                    S.bnorm2[j] = bb;
+                    S.tol2[j] = fmax(prm.rtol * prm.rtol * bb, prm.atol * prm.atol);
+                  }
+                  // keep the direction when the last cycle at least halved the true
+                  // residual and cycles are short enough for the FP32 recursive
+                  // residual to stay close to the true one (inner_rtol >= 0.01)
+                  S.keep[j] = !first && prm.inner_rtol >= 0.01 && t <= 0.25 * S.rr64[j];
+                  S.rr64[j] = t;
+                  S.active[j] = t > S.tol2[j];
+                  S.itol2[j] = prm.inner_rtol * prm.inner_rtol * t;
+                }
+                __syncwarp();
+                const bool active = S.active[j];
+                const bool done = !__any_sync(0xffffffffu, active);
+                if (last && !done && lane == 0) S.status = AFEM_ERR_NOT_CONVERGED;
+                return told(0.f, active, done);
+              }))
+        return;
     }
-    if (S.all_done) break;
-    if (outer >= prm.max_outer) {
-      status = AFEM_ERR_NOT_CONVERGED;
-      break;
-    }
+    if (told_flag(cast[0]) || outer >= prm.max_outer) break;
     // FP32 CG on A32 d = r32 from d = 0 for the unconverged right-hand sides.
     // z = D^-1 r is never stored: the SpMV of each iteration forms the new
     // direction p = zc D^-1 r + beta p_old of every entry it gathers (and
@@ -326,38 +396,44 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
     // failed to halve the true residual.
     {
       float lrz[kBatchRhs] = {};
-      const bool a0 = S.active[0], a1 = S.active[1], a2 = S.active[2], a3 = S.active[3];
-      for (int row = tid; row < I.n; row += nthr) {
+      const bool a0 = told_active(cast[0]), a1 = told_active(cast[1]), a2 = told_active(cast[2]),
+                 a3 = told_active(cast[3]);
+      for (int row = row0; row < row1; row += BLOCK) {
         const double* rr = I.r64 + (int64_t)row * kBatchRhs;
         const float di = I.dinv[row];
         const float4 rv = make_float4(a0 ? (float)rr[0] : 0.f, a1 ? (float)rr[1] : 0.f, a2 ? (float)rr[2] : 0.f,
                                       a3 ? (float)rr[3] : 0.f);
         I.r[row] = rv;
         if (outer == 0) I.z[row] = make_float4(0.f, 0.f, 0.f, 0.f);   // p_old of the first iteration
-        I.d[row] = make_float4(0.f, 0.f, 0.f, 0.f);
+        own_d[row - off] = make_float4(0.f, 0.f, 0.f, 0.f);
         lrz[0] = fmaf(rv.x, di * rv.x, lrz[0]); lrz[1] = fmaf(rv.y, di * rv.y, lrz[1]);
         lrz[2] = fmaf(rv.z, di * rv.z, lrz[2]); lrz[3] = fmaf(rv.w, di * rv.w, lrz[3]);
       }
-      double trz[kBatchRhs];
-      if (!team_reduce<BLOCK, kBatchRhs>(lrz, trz, I, rank, 3, red, tres, &gen_sh, err, lim)) return;
-      if (threadIdx.x == 0)
-        for (int j = 0; j < kBatchRhs; ++j) {
-          S.beta[j] = S.keep[j] && S.active[j] ? (float)(trz[j] / S.rzprev[j]) : 0.f;
-          S.zc[j] = 1.f;
-          S.rz[j] = trz[j];
-        }
-      __syncthreads();
+      if (!team_exchange<BLOCK, kBatchRhs, true>(lrz, I, rank, red, red64, cast, epoch, err, lim,
+                                                 [&](int lane, double t) {
+                                                   const int j = lane & (kBatchRhs - 1);
+                                                   float beta = 0.f;
+                                                   if (lane < kBatchRhs) {
+                                                     if (S.keep[j] && S.active[j]) beta = (float)quotient(t, S.rzprev[j]);
+                                                     S.rz[j] = t;
+                                                   }
+                                                   return told(beta, true, false);
+                                                 }))
+        return;
     }
+    // cast holds beta and, in its active bit, the weight of z of the coming iteration
     for (int it = 0; it < prm.max_inner; ++it) {
       float4* const pold = (inner_total & 1) ? I.p : I.z;
       float4* const pnew = (inner_total & 1) ? I.z : I.p;
       // p = D^-1 r + beta p_old (on the fly), q = A32 p ; <p, q>.  Thread per
       // row; the row's column and value loads are issued together, then its gathers.
       {
-        const float b0 = S.beta[0], b1 = S.beta[1], b2 = S.beta[2], b3 = S.beta[3];
-        const float z0 = S.zc[0], z1 = S.zc[1], z2 = S.zc[2], z3 = S.zc[3];
+        const float b0 = told_value(cast[0]), b1 = told_value(cast[1]), b2 = told_value(cast[2]),
+                    b3 = told_value(cast[3]);
+        const float z0 = told_active(cast[0]), z1 = told_active(cast[1]), z2 = told_active(cast[2]),
+                    z3 = told_active(cast[3]);
         float lpq[kBatchRhs] = {};
-        for (int row = tid; row < I.n; row += nthr) {
+        for (int row = row0; row < row1; row += BLOCK) {
           const int32_t rb = I.rp[row], e = I.rp[row + 1];
           const int len = e - rb;
           int32_t c[kRowUnroll];
@@ -391,79 +467,81 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
           const float4 pr = make_float4(fmaf(b0, po.x, z0 * di * rv.x), fmaf(b1, po.y, z1 * di * rv.y),
                                         fmaf(b2, po.z, z2 * di * rv.z), fmaf(b3, po.w, z3 * di * rv.w));
           pnew[row] = pr;
-          I.q[row] = s;
+          own_q[row - off] = s;
           lpq[0] = fmaf(pr.x, s.x, lpq[0]); lpq[1] = fmaf(pr.y, s.y, lpq[1]);
           lpq[2] = fmaf(pr.z, s.z, lpq[2]); lpq[3] = fmaf(pr.w, s.w, lpq[3]);
         }
-        double pq[kBatchRhs];
-        if (!team_reduce<BLOCK, kBatchRhs>(lpq, pq, I, rank, 0, red, tres, &gen_sh, err, lim)) return;
-        if (threadIdx.x == 0) {
-          for (int j = 0; j < kBatchRhs; ++j) {
-            if (S.active[j] && !(pq[j] > 0.0)) {   // breakdown: stop this right-hand side
-              S.active[j] = 0;
-              status = AFEM_ERR_BREAKDOWN;
-            }
-            S.alpha[j] = S.active[j] ? (float)(S.rz[j] / pq[j]) : 0.f;
-          }
-        }
-        __syncthreads();
+        if (!team_exchange<BLOCK, kBatchRhs, false>(lpq, I, rank, red, red64, cast, epoch, err, lim,
+                                                    [&](int lane, double t) {
+                                                      const int j = lane & (kBatchRhs - 1);
+                                                      float alpha = 0.f;
+                                                      if (lane < kBatchRhs && S.active[j]) {
+                                                        if (t > 0.0) {
+                                                          alpha = (float)quotient(S.rz[j], t);
+                                                        } else {   // breakdown: stop this right-hand side
+                                                          S.active[j] = 0;
+                                                          S.status = AFEM_ERR_BREAKDOWN;
+                                                        }
+                                                      }
+                                                      return told(alpha, false, false);
+                                                    }))
+          return;
       }
       // d += alpha p ; r -= alpha q ; <r, D^-1 r>, <r, r>
       {
-        const float al0 = S.alpha[0], al1 = S.alpha[1], al2 = S.alpha[2], al3 = S.alpha[3];
+        const float al0 = told_value(cast[0]), al1 = told_value(cast[1]), al2 = told_value(cast[2]),
+                    al3 = told_value(cast[3]);
         float lrr[2 * kBatchRhs] = {};
-        for (int row = tid; row < I.n; row += nthr) {
-          const float4 pv = pnew[row], qv = I.q[row];
-          float4 dv = I.d[row], rv = I.r[row];
+        for (int row = row0; row < row1; row += BLOCK) {
+          const float4 pv = pnew[row], qv = own_q[row - off];
+          float4 dv = own_d[row - off], rv = I.r[row];
           dv.x = fmaf(al0, pv.x, dv.x); dv.y = fmaf(al1, pv.y, dv.y);
           dv.z = fmaf(al2, pv.z, dv.z); dv.w = fmaf(al3, pv.w, dv.w);
           rv.x = fmaf(-al0, qv.x, rv.x); rv.y = fmaf(-al1, qv.y, rv.y);
           rv.z = fmaf(-al2, qv.z, rv.z); rv.w = fmaf(-al3, qv.w, rv.w);
           const float di = I.dinv[row];
-          I.d[row] = dv;
+          own_d[row - off] = dv;
           I.r[row] = rv;
           lrr[0] = fmaf(rv.x, di * rv.x, lrr[0]); lrr[1] = fmaf(rv.y, di * rv.y, lrr[1]);
           lrr[2] = fmaf(rv.z, di * rv.z, lrr[2]); lrr[3] = fmaf(rv.w, di * rv.w, lrr[3]);
           lrr[4] = fmaf(rv.x, rv.x, lrr[4]); lrr[5] = fmaf(rv.y, rv.y, lrr[5]);
           lrr[6] = fmaf(rv.z, rv.z, lrr[6]); lrr[7] = fmaf(rv.w, rv.w, lrr[7]);
         }
-        double trr[2 * kBatchRhs];
-        if (!team_reduce<BLOCK, 2 * kBatchRhs>(lrr, trr, I, rank, 1, red, tres, &gen_sh, err, lim)) return;
-        if (threadIdx.x == 0) {
-          int any = 0;
-          for (int j = 0; j < kBatchRhs; ++j) {
-            if (S.active[j]) {
-              S.beta[j] = (float)(trr[j] / S.rz[j]);
-              S.rzprev[j] = S.rz[j];
-              S.rz[j] = trr[j];
-              if (!(trr[kBatchRhs + j] > S.itol2[j])) S.active[j] = 0;
-            }
-            if (!S.active[j]) {   // keep the direction for the next cycle
-              S.beta[j] = 1.f;
-              S.zc[j] = 0.f;
-            }
-            any = any || S.active[j];
-          }
-          S.any = any;
-        }
-        __syncthreads();
+        // lanes j: <r_j, z_j>, lanes 4 + j: <r_j, r_j>
+        if (!team_exchange<BLOCK, 2 * kBatchRhs, true>(
+                lrr, I, rank, red, red64, cast, epoch, err, lim, [&](int lane, double t) {
+                  const double rr = __shfl_down_sync(0xffffffffu, t, kBatchRhs);
+                  const int j = lane & (kBatchRhs - 1);
+                  float beta = 1.f;   // a side that is done keeps its direction for the next cycle
+                  bool active = false;
+                  if (lane < kBatchRhs && S.active[j]) {
+                    const float next = (float)quotient(t, S.rz[j]);
+                    S.rzprev[j] = S.rz[j];
+                    S.rz[j] = t;
+                    active = rr > S.itol2[j];
+                    S.active[j] = active;
+                    if (active) beta = next;
+                  }
+                  return told(beta, active, __any_sync(0xffffffffu, active));
+                }))
+          return;
       }
       ++inner_total;
-      if (!S.any) break;
+      if (!told_flag(cast[0])) break;
     }
     // x += d (FP64); the next residual reads neighbours' x
-    for (int row = tid; row < I.n; row += nthr) {
-      const float4 dv = I.d[row];
+    for (int row = row0; row < row1; row += BLOCK) {
+      const float4 dv = own_d[row - off];
       double* xr = I.x + (int64_t)row * kBatchRhs;
       xr[0] += (double)dv.x; xr[1] += (double)dv.y; xr[2] += (double)dv.z; xr[3] += (double)dv.w;
     }
-    if (!team_sync(I.bar, I.ncta, &gen_sh, err, lim)) return;
+    if (!sync()) return;
   }
   if (rank == 0 && threadIdx.x == 0) {
     I.res->finish_ms = (float)((double)(globaltimer_ns() - t_start) * 1e-6);
     I.res->inner_iterations = inner_total;
     I.res->refinements = outer;
-    I.res->status = status;
+    I.res->status = S.status;
     for (int j = 0; j < kBatchRhs; ++j)
       I.res->relres[j] = S.bnorm2[j] > 0.0 ? sqrt(S.rr64[j] / S.bnorm2[j]) : sqrt(S.rr64[j]);
   }
@@ -483,14 +561,15 @@ struct afem_batch_s {
   std::vector<BatchInst> dinst;     // host copy of the descriptors (device pointers)
   BatchInst* insts_d = nullptr;
   int32_t* cta_team_d = nullptr;
-  TeamBar* bars_d = nullptr;
   afem_batch_result* res_d = nullptr;
   int* err_d = nullptr;
-  double* part_d = nullptr;
+  ulonglong2* slots_d = nullptr;    // [max_grid][kTeamSlots], then the teams' totals [ninst][kTeamSlots]
+  size_t slots_bytes = 0;
   std::vector<void*> owned;
   afem_batch_config cfg{256, 4, 3.5f};
   std::vector<double> weights;      // empty: the cost model
   int grid = 0;
+  int own_rows = 0;                 // rows of a CTA whose q and d fit shared memory
   int max_teams = 0;
   // graph of the current configuration and options
   GraphChunk* graph = nullptr;
@@ -505,6 +584,9 @@ static afem_status batch_alloc(afem_batch b, size_t bytes, void** out) {
   b->owned.push_back(*out);
   return AFEM_OK;
 }
+
+constexpr size_t kOwnBytes = 150 * 1024;   // of an SM's shared memory, the rest is L1 for the gathers
+static size_t own_bytes(int rows) { return 2 * sizeof(float4) * (size_t)rows; }
 
 template <int BLOCK>
 static int max_blocks_per_sm() {
@@ -568,8 +650,18 @@ static afem_status batch_configure(afem_batch b) {
     b->dinst[i].ncta = sizes[i];
     for (int k = 0; k < sizes[i]; ++k) cta_team[c++] = i;
   }
-  // partials: one region block per CTA, laid out by team
-  for (int i = 0; i < b->ninst; ++i) b->dinst[i].part = b->part_d + (size_t)b->dinst[i].cta0 * kPartStride;
+  // q and d go to shared memory where a CTA's rows fit its share of kOwnBytes, if that holds for most CTAs
+  const int fit = (int)(kOwnBytes / bps / own_bytes(1));
+  int most = 0, served = 0;
+  for (int i = 0; i < b->ninst; ++i) {
+    const int per = rows_per_cta(b->inst[i].nb_node, sizes[i]);
+    if (per > fit) continue;
+    most = std::max(most, per);
+    served += sizes[i];
+  }
+  b->own_rows = 2 * served > grid ? most : 0;
+  // slots: one block per CTA, laid out by team
+  for (int i = 0; i < b->ninst; ++i) b->dinst[i].part = b->slots_d + (size_t)b->dinst[i].cta0 * kTeamSlots;
   AFEM_CUDA(cudaMemcpyAsync(b->insts_d, b->dinst.data(), sizeof(BatchInst) * b->ninst, cudaMemcpyHostToDevice,
                             ctx->stream));
   AFEM_CUDA(cudaMemcpyAsync(b->cta_team_d, cta_team.data(), sizeof(int32_t) * grid, cudaMemcpyHostToDevice,
@@ -585,8 +677,11 @@ static cudaError_t launch_batch(afem_batch b, cudaStream_t s, const BatchParams&
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(b->grid);
   lc.blockDim = dim3(BLOCK);
-  lc.dynamicSmemBytes = 0;
+  lc.dynamicSmemBytes = own_bytes(prm.own_rows);
   lc.stream = s;
+  const cudaError_t e = cudaFuncSetAttribute(k_batch<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)lc.dynamicSmemBytes);
+  if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
@@ -597,7 +692,7 @@ static cudaError_t launch_batch(afem_batch b, cudaStream_t s, const BatchParams&
 }
 
 static afem_status batch_enqueue(afem_batch b, cudaStream_t s, const BatchParams& prm) {
-  AFEM_CUDA(cudaMemsetAsync(b->bars_d, 0, sizeof(TeamBar) * b->ninst, s));
+  AFEM_CUDA(cudaMemsetAsync(b->slots_d, 0, b->slots_bytes, s));
   AFEM_CUDA(cudaMemsetAsync(b->err_d, 0, sizeof(int), s));
   AFEM_CUDA(cudaMemsetAsync(b->res_d, 0, sizeof(afem_batch_result) * b->ninst, s));
   cudaError_t e = cudaErrorInvalidValue;
@@ -618,18 +713,20 @@ static BatchParams batch_params(const afem_solver_options& opt) {
   prm.inner_rtol = opt.inner_rtol > 0 ? opt.inner_rtol : 0.1;
   prm.max_inner = opt.max_iter > 0 ? opt.max_iter : 1000;
   prm.max_outer = 30;
-  prm.spin_limit = 20000000LL;   // ~2.5 s of 128 ns sleeps
+  prm.spin_limit = 5000000LL;   // about 2.5 s of polls
   prm.stall_cta = -1;
   return prm;
 }
 
 static bool same_params(const BatchParams& a, const BatchParams& c) {
   return a.rtol == c.rtol && a.atol == c.atol && a.inner_rtol == c.inner_rtol && a.max_inner == c.max_inner &&
-         a.max_outer == c.max_outer && a.spin_limit == c.spin_limit && a.stall_cta == c.stall_cta;
+         a.max_outer == c.max_outer && a.spin_limit == c.spin_limit && a.own_rows == c.own_rows &&
+         a.stall_cta == c.stall_cta;
 }
 
-static afem_status batch_run(afem_batch b, const BatchParams& prm, bool use_graph, float* ms) {
+static afem_status batch_run(afem_batch b, BatchParams prm, bool use_graph, float* ms) {
   afem_context ctx = b->ctx;
+  prm.own_rows = b->own_rows;
   if (use_graph && (!b->graph_valid || !same_params(prm, b->graph_prm))) {
     delete b->graph;
     b->graph = new (std::nothrow) GraphChunk();
@@ -731,16 +828,15 @@ afem_status afem_batch_create(afem_context ctx, int nb_inst, const afem_batch_in
   b->insts_d = (BatchInst*)pv;
   if ((st = batch_alloc(b, sizeof(int32_t) * max_grid, &pv))) return cleanup(st);
   b->cta_team_d = (int32_t*)pv;
-  if ((st = batch_alloc(b, sizeof(TeamBar) * nb_inst, &pv))) return cleanup(st);
-  b->bars_d = (TeamBar*)pv;
   if ((st = batch_alloc(b, sizeof(afem_batch_result) * nb_inst, &pv))) return cleanup(st);
   b->res_d = (afem_batch_result*)pv;
   if ((st = batch_alloc(b, sizeof(int), &pv))) return cleanup(st);
   b->err_d = (int*)pv;
-  if ((st = batch_alloc(b, sizeof(double) * kPartStride * max_grid, &pv))) return cleanup(st);
-  b->part_d = (double*)pv;
+  b->slots_bytes = sizeof(ulonglong2) * kTeamSlots * ((size_t)max_grid + nb_inst);
+  if ((st = batch_alloc(b, b->slots_bytes, &pv))) return cleanup(st);
+  b->slots_d = (ulonglong2*)pv;
   for (int i = 0; i < nb_inst; ++i) {
-    b->dinst[i].bar = b->bars_d + i;
+    b->dinst[i].total = b->slots_d + (size_t)(max_grid + i) * kTeamSlots;
     b->dinst[i].res = b->res_d + i;
   }
   if ((st = batch_configure(b)) != AFEM_OK) return cleanup(st);

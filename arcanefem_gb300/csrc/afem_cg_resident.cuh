@@ -35,18 +35,6 @@ constexpr int kResSpins = 4000000;             // polls of a wait, about 2 s
 constexpr int kSlotStride = 8;                  // slots of 16 B a cache line of its own apart
 constexpr size_t kResSmem = 226 * 1024;        // dynamic shared memory of a block
 
-// A slot: the value's bits and the number of the exchange it belongs to.
-__device__ __forceinline__ void slot_put(ulonglong2* s, unsigned long long v, unsigned long long epoch) {
-  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], t;\n\t}"
-               :: "l"(v), "l"(epoch), "l"(s) : "memory");
-}
-__device__ __forceinline__ ulonglong2 slot_get(const ulonglong2* s) {
-  ulonglong2 r;
-  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-               : "=l"(r.x), "=l"(r.y) : "l"(s) : "memory");
-  return r;
-}
-
 // The blocks' exchanges.  Slots are double-buffered by the exchange's parity:
 // a block can be one exchange ahead of another's polling, never two.  FENCE:
 // what the block's threads wrote before is visible to every block afterwards

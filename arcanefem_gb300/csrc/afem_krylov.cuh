@@ -83,6 +83,21 @@ __device__ __forceinline__ double reduce_partials(const double* partials, int np
 }
 
 // ---------------------------------------------------------------------------
+// Exchanges between the blocks of a cooperative grid: one 16-byte access
+// carries a value's bits and the number of the exchange it belongs to, so that
+// a poll that sees the number has the value.
+__device__ __forceinline__ void slot_put(ulonglong2* s, unsigned long long v, unsigned long long epoch) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], t;\n\t}"
+               :: "l"(v), "l"(epoch), "l"(s) : "memory");
+}
+__device__ __forceinline__ ulonglong2 slot_get(const ulonglong2* s) {
+  ulonglong2 r;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(r.x), "=l"(r.y) : "l"(s) : "memory");
+  return r;
+}
+
+// ---------------------------------------------------------------------------
 // Host side.
 
 // FP64 rows: on GB300 a warp FP64 instruction costs the same whatever its
