@@ -633,6 +633,8 @@ static void team_sizes(const std::vector<afem_batch_instance>& inst, const std::
   for (int k = 0; k < spare - used; ++k) out[frac[k % n].second] += 1;
 }
 
+constexpr int64_t kFewRows = 1000, kManyRows = 15000;   // rows an SM of the default shapes, see afem_batch_create
+
 static afem_status batch_configure(afem_batch b) {
   afem_context ctx = b->ctx;
   const int occ = occupancy(b->cfg.block);
@@ -839,6 +841,15 @@ afem_status afem_batch_create(afem_context ctx, int nb_inst, const afem_batch_in
     b->dinst[i].total = b->slots_d + (size_t)(max_grid + i) * kTeamSlots;
     b->dinst[i].res = b->res_d + i;
   }
+  // The shape until the caller sets one.  Few rows an SM are bound by the exchanges, which cost less among fewer
+  // CTAs; many (out of L2) by the loads in flight, with more and smaller CTAs.  (256, 4), (512, 2), (512, 1), ms:
+  // 300 rows an SM 13.8, 9.6, 7.8; 820: 23.9, 16.6, 15.5; 2200: 37.6, 31.8, 32.5; 4400: 52.5, 51.2, 57.7;
+  // 11700: 126, 125, 185; 23000: 249, 262, 465.
+  int64_t rows = 0;
+  for (const afem_batch_instance& i : b->inst) rows += i.nb_node;
+  const int64_t per_sm = rows / ctx->sm_count;
+  if (per_sm <= kFewRows && nb_inst <= ctx->sm_count) b->cfg = {512, 1, 3.5f};
+  else if (per_sm <= kManyRows && nb_inst <= 2 * ctx->sm_count) b->cfg = {512, 2, 3.5f};
   if ((st = batch_configure(b)) != AFEM_OK) return cleanup(st);
   *out = b;
   return AFEM_OK;
