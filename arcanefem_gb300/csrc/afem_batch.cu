@@ -34,7 +34,6 @@
 #include <cmath>
 #include <vector>
 
-#include "afem_fp64_int.cuh"
 #include "afem_krylov.cuh"
 
 namespace afem {
@@ -192,17 +191,6 @@ __device__ __forceinline__ bool team_exchange(const T (&v)[M], const BatchInst& 
     if constexpr (FENCE) __threadfence();
   }
   return __syncthreads_and(ok);
-}
-
-// a / b rounded to nearest on the integer pipes (afem_fp64_int.cuh) where both
-// are in its range: an FP64 division is some ten dependent FP64 instructions.
-__device__ __forceinline__ double quotient(double a, double b) {
-  const int ah = __double2hiint(a), bh = __double2hiint(b);
-  if (!i64fp::in_window<400>(ah, __double2loint(a)) || !i64fp::in_window<400>(bh, __double2loint(b)) ||
-      (bh & 0x7ff00000) == 0)
-    return a / b;
-  return __longlong_as_double(i64fp::div(i64fp::operand(ah, __double2loint(a)),
-                                         i64fp::divisor(__double_as_longlong(b))));
 }
 
 // What the first CTA tells the others of a right-hand side: a float, whether

@@ -14,9 +14,12 @@
 //     other blocks gather it;
 //   * the blocks meet in all-to-all exchanges: a block publishes its partial
 //     sum and the exchange's number in one 16-byte slot, and each block polls
-//     all slots and adds them in the same fixed order.  Every block takes the
-//     same decisions, results are deterministic, and no exchange pays an
-//     atomic's queue or a second trip for a flag.
+//     all slots and adds them.  Every block takes the same decisions, results
+//     are deterministic, and no exchange pays an atomic's queue or a second
+//     trip for a flag;
+//   * the sums are made in fixed point (below): in FP64 each of an iteration's
+//     two sums is a chain of 20 dependent additions and a division, 3700 of an
+//     iteration's 19900 cycles (256^2 triangles; 9.7 -> 8.6 ms a solve).
 // Every wait is bounded; one that runs out sets *err and ends all blocks.
 #pragma once
 #include "afem_krylov.cuh"
@@ -35,76 +38,83 @@ constexpr int kResSpins = 4000000;             // polls of a wait, about 2 s
 constexpr int kSlotStride = 8;                  // slots of 16 B a cache line of its own apart
 constexpr size_t kResSmem = 226 * 1024;        // dynamic shared memory of a block
 
-// The blocks' exchanges.  Slots are double-buffered by the exchange's parity:
-// a block can be one exchange ahead of another's polling, never two.  FENCE:
-// what the block's threads wrote before is visible to every block afterwards
-// (a release before the put, an acquire after the polls).
-struct Grid {
-  ulonglong2* slots;          // [2 parities][2 values][gridDim.x] lines, zero at the launch
-  double* sh;                 // shared, res_scratch(gridDim.x) doubles
-  int* err;
-  unsigned long long epoch = 0;
+// Sums in fixed point.  Each partial sum becomes a 96-bit integer in units of
+// 2^(E - 69), E the exponent of the sum's last value, in five 22-bit limbs that
+// a warp adds in one instruction each (redux); integers add exactly, so the
+// order does not matter, and the total is rounded once.  Its error is that of
+// the conversions, half a unit a thread, against an FP64 tree's half ulp of
+// the running sums.  A partial sum of 2^(E + 9) or more (or not finite), or a
+// total below 2^(E - 4), sends that exchange to FP64 sums; so does a missing E.
+constexpr int kLimbs = 5, kLimbBits = 22;
+constexpr int kNoExponent = 1 << 20;
 
-  // Publish the values that threads 0 (and 32 for the second) of the block hold, poll everyone's into sh.
-  // Returns false in every thread if a wait ran out.  Ends with a block barrier.
-  template <int V, bool FENCE>
-  __device__ __forceinline__ bool meet(double v) {
-    ++epoch;
-    const int nb = gridDim.x;
-    ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
-    if constexpr (FENCE) __syncthreads();
-    if (threadIdx.x < 32 * V && (threadIdx.x & 31) == 0) {
-      if constexpr (FENCE) __threadfence();
-      slot_put(at + ((threadIdx.x >> 5) * nb + blockIdx.x) * kSlotStride, __double_as_longlong(v), epoch);
-    }
-    int bad = 0;
-    for (int i = threadIdx.x; i < V * nb; i += kResThreads) {
-      ulonglong2 s = slot_get(at + i * kSlotStride);
-      int spins = 0;
-      while (s.y != epoch) {
-        if (++spins >= kResSpins || ((spins & 1023) == 0 && *(volatile int*)err)) {
-          atomicCAS(err, 0, (int)AFEM_ERR_TIMEOUT);
-          bad = 1;
-          break;
-        }
-        s = slot_get(at + i * kSlotStride);
-      }
-      sh[i] = __longlong_as_double(s.x);
-    }
-    if constexpr (FENCE)
-      if (threadIdx.x < V * nb) __threadfence();   // the pollers acquire for the block
-    return __syncthreads_or(bad) == 0;
+__device__ __forceinline__ int sum_exponent(double total) {
+  const int e = (__double2hiint(total) >> 20 & 0x7ff) - 1023;
+  return abs(e) <= 900 ? e : kNoExponent;
+}
+
+// e: biased as a double's (0 for a zero), m: 53-bit significand, s: 0 or -1
+__device__ __forceinline__ bool to_limbs(int e, unsigned long long m, int s, int E, int (&l)[kLimbs]) {
+  int p = e - E - 1006;   // place of the significand's last bit
+  if (p < 0) {
+    m = p > -54 ? (m + (1ull << (-p - 1))) >> -p : 0ull;
+    p = 0;
   }
-
-  // total of sh[v * gridDim.x ..] for the warp v that calls it, in every lane
-  __device__ __forceinline__ double total(int v) const {
-    const int nb = gridDim.x, lane = threadIdx.x & 31;
-    double s = 0.0;
-    for (int i = lane; i < nb; i += 32) s += sh[v * nb + i];
+  const bool ok = e - 1023 - E <= 8;
+  if (!ok) p = 0;
+  const unsigned long long lo = m << p, hi = p ? m >> (64 - p) : 0ull;
+  constexpr int mask = (1 << kLimbBits) - 1;
+  const int u[kLimbs] = {(int)lo & mask, (int)(lo >> 22) & mask, (int)(lo >> 44 | hi << 20) & mask, (int)(hi >> 2) & mask,
+                         (int)(hi >> 24)};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
-  }
-};
+  for (int k = 0; k < kLimbs; ++k) l[k] = (u[k] ^ s) - s;
+  return ok;
+}
+__device__ __forceinline__ bool to_limbs(double v, int E, int (&l)[kLimbs]) {
+  const int h = __double2hiint(v), e = h >> 20 & 0x7ff;
+  const unsigned long long m = (unsigned long long)((h & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(v);
+  return to_limbs(e, e ? m : 0ull, h >> 31, E, l);
+}
+__device__ __forceinline__ bool to_limbs(float v, int E, int (&l)[kLimbs]) {
+  const int b = __float_as_int(v), e = b >> 23 & 0xff;
+  const unsigned long long m = (unsigned long long)((b & 0x7fffff) | 0x800000) << 29;
+  return to_limbs(e == 0 ? 0 : e == 255 ? 2047 : e + 896, e ? m : 0ull, b >> 31, E, l);
+}
 
-inline size_t res_scratch_doubles(unsigned grid) { return std::max<size_t>(2 * kResThreads, 2 * grid); }
+__device__ __forceinline__ __int128 from_limbs(const int (&l)[kLimbs]) {
+  return (__int128)((long long)l[0] + ((long long)l[1] << 22)) +
+         ((__int128)((long long)l[2] + ((long long)l[3] << 22)) << 44) + ((__int128)l[4] << 88);
+}
 
-// Block sums of V FP64 values a thread; value v's ends in the lanes of warp v.
+__device__ __forceinline__ double fixed_to_double(__int128 t, int E) {
+  if (t == 0) return 0.0;
+  const bool neg = t < 0;
+  unsigned __int128 m = neg ? -(unsigned __int128)t : (unsigned __int128)t;
+  const unsigned long long top = (unsigned long long)(m >> 64);
+  const int z = top ? __clzll((long long)top) : 64 + __clzll((long long)(unsigned long long)m);
+  m <<= z;
+  const unsigned long long lead = (unsigned long long)(m >> 64) | ((unsigned long long)m != 0);   // sticky
+  const double d = __ull2double_rn(lead);   // exponent 63 or 64
+  const int h = (__double2hiint(d) + (64 - z + E - 69) * (1 << 20)) | (neg ? (int)0x80000000 : 0);
+  return __hiloint2double(h, __double2loint(d));
+}
+
+// Block sums of V values a thread in FP64; value v's ends in the lanes of warp v.
 // GB300 takes as long for a warp's FP64 instruction however many lanes take
 // part, so the sums go through shared memory with full warps first.
-template <int V>
-__device__ __forceinline__ double res_block_sum(const double (&v)[V], double* sh) {
-  constexpr int T = kResThreads, W = 128 / V;   // four warps add, 128 / V threads per value
+template <int V, class T>
+__device__ __forceinline__ double res_block_sum(const T (&v)[V], double* sh) {
+  constexpr int B = kResThreads, W = 128 / V;   // four warps add, 128 / V threads per value
   const int t = threadIdx.x;
 #pragma unroll
-  for (int j = 0; j < V; ++j) sh[j * T + t] = v[j];
+  for (int j = 0; j < V; ++j) sh[j * B + t] = (double)v[j];
   __syncthreads();
   double s = 0.0;
   if (t < 128) {
-    const double* p = sh + (t / W) * T + t % W;
+    const double* p = sh + (t / W) * B + t % W;
     s = p[0];
 #pragma unroll
-    for (int m = 1; m < T / W; ++m) s += p[m * W];
+    for (int m = 1; m < B / W; ++m) s += p[m * W];
   }
   __syncthreads();
   if (t < 128) sh[t] = s;
@@ -121,31 +131,174 @@ __device__ __forceinline__ double res_block_sum(const double (&v)[V], double* sh
   return s;
 }
 
-// The same of FP32 values, warps summed in FP32 and their totals in FP64.
-template <int V>
-__device__ __forceinline__ double res_block_sum_f(const float (&v)[V], double* sh) {
-  constexpr int NW = kResThreads / 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// The blocks' exchanges.  Slots are double-buffered by the exchange's parity:
+// a block can be one exchange ahead of another's polling, never two.  FENCE:
+// what the block's threads wrote before is visible to every block afterwards
+// (a release before the put, an acquire after the polls).
+struct Grid {
+  ulonglong2* slots;          // [2 parities][2 values][gridDim.x] lines, zero at the launch
+  double* sh;                 // shared, res_scratch(gridDim.x) doubles
+  int* err;
+  unsigned long long epoch = 0;
+
+  // Publish the values that threads 0 (and 32 for the second) of the block hold, poll everyone's into sh.
+  // Returns false in every thread if a wait ran out.  Ends with a block barrier.
+  template <int V>
+  __device__ __forceinline__ bool meet(double v) {
+    ++epoch;
+    const int nb = gridDim.x;
+    ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
+    if (threadIdx.x < 32 * V && (threadIdx.x & 31) == 0)
+      slot_put(at + ((threadIdx.x >> 5) * nb + blockIdx.x) * kSlotStride, __double_as_longlong(v), epoch);
+    int bad = 0;
+    for (int i = threadIdx.x; i < V * nb; i += kResThreads) {
+      ulonglong2 s;
+      if (!poll(at + i * kSlotStride, &s)) bad = 1;
+      sh[i] = __longlong_as_double(s.x);
+    }
+    return __syncthreads_or(bad) == 0;
+  }
+
+  // What the blocks wrote before is visible to all of them after.
+  __device__ __forceinline__ bool barrier() {
+    ++epoch;
+    const int nb = gridDim.x;
+    ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      slot_put(at + blockIdx.x * kSlotStride, 0, epoch);
+    }
+    int bad = 0;
+    if (threadIdx.x < nb) {   // the pollers acquire for the block
+      ulonglong2 s;
+      for (int i = threadIdx.x; i < nb; i += kResThreads)
+        if (!poll(at + i * kSlotStride, &s)) bad = 1;
+      __threadfence();
+    }
+    return __syncthreads_or(bad) == 0;
+  }
+
+  __device__ __forceinline__ bool poll(const ulonglong2* s, ulonglong2* got) {
+    *got = slot_get(s);
+    for (int spins = 0; (unsigned)got->y != (unsigned)epoch; *got = slot_get(s))
+      if (++spins >= kResSpins || ((spins & 1023) == 0 && *(volatile int*)err)) {
+        atomicCAS(err, 0, (int)AFEM_ERR_TIMEOUT);
+        return false;
+      }
+    return true;
+  }
+
+  // The grid's V sums of v in each of the block's threads: done(j, total) in lane 0 of warp j < V (again, with FP64
+  // sums, where those in fixed point cannot be used), and total[j] for all.  Returns false in every thread if a
+  // wait ran out.  Ends with a block barrier.
+  template <int V, bool FENCE, class T, class F>
+  __device__ __forceinline__ bool sum(const T (&v)[V], const int (&E)[V], double* total, int* slow, F&& done) {
+    constexpr int W = kResThreads / 32, P = W / V;   // warps, warps that poll a sum's slots
+    int (*part)[kLimbs + 1] = reinterpret_cast<int (*)[kLimbs + 1]>(sh);   // [V * W], the last word: taking part
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = gridDim.x;
+    bool ok = true;
 #pragma unroll
-  for (int j = 0; j < V; ++j) {
-    float s = v[j];
+    for (int j = 0; j < V; ++j) {
+      int l[kLimbs] = {};
+      ok &= E[j] != kNoExponent;
+      if (E[j] != kNoExponent) ok &= to_limbs(v[j], E[j], l);
+#pragma unroll
+      for (int k = 0; k < kLimbs; ++k) {
+        l[k] = __reduce_add_sync(0xffffffffu, l[k]);
+        if (lane == 0) part[j * W + w][k] = l[k];
+      }
+    }
+    ok = __syncthreads_and(ok);
+    ++epoch;
+    ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
+    if (w < V) {
+      int l[kLimbs];
+#pragma unroll
+      for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, lane < W ? part[w * W + lane][k] : 0);
+      if (lane == 0) {
+        const __int128 t = from_limbs(l);
+        // the high word's lowest value stands for a block that cannot take part
+        const unsigned hi = ok ? (unsigned)(t >> 64) : 0x80000000u;
+        if constexpr (FENCE) __threadfence();
+        slot_put(at + (w * nb + blockIdx.x) * kSlotStride, (unsigned long long)t,
+                 (unsigned long long)hi << 32 | (unsigned)epoch);
+      }
+    }
+    __syncthreads();   // part is read
+    int bad = 0;
+    {
+      const int j = w / P;
+      int l[kLimbs + 1] = {};
+      l[kLimbs] = 1;
+      for (int i = (w - j * P) * 32 + lane; i < nb; i += P * 32) {
+        ulonglong2 got;
+        if (!poll(at + (j * nb + i) * kSlotStride, &got)) bad = 1;
+        const int hi = (int)(got.y >> 32);
+        constexpr int mask = (1 << kLimbBits) - 1;
+        if ((unsigned)hi == 0x80000000u) l[kLimbs] = 0;
+        l[0] += (int)got.x & mask;
+        l[1] += (int)(got.x >> 22) & mask;
+        l[2] += (int)((got.x >> 44) | ((unsigned long long)(unsigned)hi << 20)) & mask;
+        l[3] += (hi >> 2) & mask;
+        l[4] += hi >> 24;
+      }
+      if constexpr (FENCE)
+        if ((w - j * P) * 32 < nb) __threadfence();   // the pollers acquire for the block
+#pragma unroll
+      for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, l[k]);
+      l[kLimbs] = __all_sync(0xffffffffu, l[kLimbs]);
+      if (lane == 0)
+#pragma unroll
+        for (int k = 0; k <= kLimbs; ++k) part[w][k] = l[k];
+    }
+    if (__syncthreads_or(bad)) return false;
+    if (w < V) {
+      int l[kLimbs];
+#pragma unroll
+      for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, lane < P ? part[w * P + lane][k] : 0);
+      ok = __all_sync(0xffffffffu, lane < P ? part[w * P + lane][kLimbs] : 1);
+      const int e0 = V == 1 || w == 0 ? E[0] : E[V - 1];
+      const double t = ok ? fixed_to_double(from_limbs(l), e0) : 0.0;
+      if (lane == 0) {
+        const bool no = !ok || (__double2hiint(t) >> 20 & 0x7ff) - 1023 < e0 - 4;
+        total[w] = t;
+        slow[w] = no;
+        if (!no) done(w, t);
+      }
+    }
+    __syncthreads();
+    if (slow[0] || slow[V - 1]) {   // the same in every block
+      const double b = res_block_sum<V>(v, sh);
+      if (!meet<V>(b)) return false;
+      if (w < V) {
+        const double t = this->total(w);
+        if (lane == 0) {
+          total[w] = t;
+          done(w, t);
+        }
+      }
+      __syncthreads();
+    }
+    return true;
+  }
+
+  // total of sh[v * gridDim.x ..] for the warp v that calls it, in every lane
+  __device__ __forceinline__ double total(int v) const {
+    const int nb = gridDim.x, lane = threadIdx.x & 31;
+    double s = 0.0;
+    for (int i = lane; i < nb; i += 32) s += sh[v * nb + i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) sh[j * NW + w] = (double)s;
+    return s;
   }
-  __syncthreads();
-  double s = 0.0;
-  if (w < V) {
-    s = sh[w * NW + (lane & (NW - 1))];
-#pragma unroll
-    for (int o = NW / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  }
-  __syncthreads();
-  return s;
-}
+};
+
+inline size_t res_scratch_doubles(unsigned grid) { return std::max<size_t>(2 * kResThreads, 2 * grid); }
 
 struct ResCtl {
-  double alpha, beta;
+  double total[2], alpha, beta;
+  int slow[2];
   int done, status;
 };
 
@@ -293,9 +446,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident
     }
   }
   __syncthreads();
-  double rz = a.st->rz;                  // thread 0's is the one in use
+  double rz = a.st->rz;
   const double tol2 = a.st->tol2;
   const int max_iter = a.st->max_iter, iter0 = a.st->iter;
+  int epq = kNoExponent, erz = sum_exponent(rz), err = sum_exponent(a.st->rr);   // of the sums' last values
   int it = 0;
   for (;;) {
     // q = A p ; <p, q> -> alpha
@@ -315,19 +469,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident
         if (row < r1) pq[0] += (kAll ? p[kAll ? k : 0] : a.p[row]) * q[k];
       }
     }
-    const double bpq = res_block_sum<1>(pq, grid.sh);
-    if (!grid.template meet<1, false>(bpq)) return;
-    if (threadIdx.x < 32) {
-      const double t = grid.total(0);
-      if (threadIdx.x == 0) {
-        const bool ok = t > 0.0 && isfinite(t);
-        ctl.alpha = ok ? rz / t : 0.0;
-        ctl.status = ok ? AFEM_OK : AFEM_ERR_BREAKDOWN;
-        ctl.done = !ok;
-        if (blockIdx.x == 0) a.st->pq = t;
-      }
-    }
-    __syncthreads();
+    if (!grid.template sum<1, false>(pq, {epq}, ctl.total, ctl.slow, [&](int, double t) {
+          const bool ok = t > 0.0 && isfinite(t);
+          ctl.alpha = ok ? quotient(rz, t) : 0.0;
+          ctl.status = ok ? AFEM_OK : AFEM_ERR_BREAKDOWN;
+          ctl.done = !ok;
+        }))
+      return;
+    epq = sum_exponent(ctl.total[0]);
     if (ctl.done) break;
     // x += alpha p ; r -= alpha q ; z = D^-1 r ; <r, z>, <r, r> -> beta, stop test
     const double alpha = ctl.alpha;
@@ -344,31 +493,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident
         if (counted >> k & 1) rs[1] += r[k] * r[k];
       }
     }
-    const double brs = res_block_sum<2>(rs, grid.sh);
-    if (!grid.template meet<2, false>(brs)) return;
     ++it;
-    if (threadIdx.x < 64) {
-      const double t = grid.total(threadIdx.x >> 5);
-      if (threadIdx.x == 0) {
-        ctl.beta = t / rz;
-        rz = t;
-      } else if (threadIdx.x == 32) {
-        int done = 0, status = AFEM_OK;
-        if (!isfinite(t)) {
-          status = AFEM_ERR_BREAKDOWN;
-          done = 1;
-        } else if (t <= tol2) {
-          done = 1;
-        } else if (iter0 + it >= max_iter) {
-          status = AFEM_ERR_NOT_CONVERGED;
-          done = 1;
-        }
-        ctl.done = done;
-        ctl.status = status;
-        if (blockIdx.x == 0) a.st->rr = t;
-      }
-    }
-    __syncthreads();
+    if (!grid.template sum<2, false>(rs, {erz, err}, ctl.total, ctl.slow, [&](int j, double t) {
+          if (j == 0) {
+            ctl.beta = quotient(t, rz);
+            return;
+          }
+          ctl.done = !isfinite(t) || t <= tol2 || iter0 + it >= max_iter;
+          ctl.status = !isfinite(t) ? AFEM_ERR_BREAKDOWN
+                                    : t > tol2 && iter0 + it >= max_iter ? AFEM_ERR_NOT_CONVERGED : AFEM_OK;
+        }))
+      return;
+    rz = ctl.total[0];
+    erz = sum_exponent(rz);
+    err = sum_exponent(ctl.total[1]);
     if (ctl.done) break;
     // p = z + beta p
     const double beta = ctl.beta;
@@ -382,7 +520,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident
       }
     }
     if (it == a.iters) break;
-    if (!grid.template meet<1, true>(0.0)) return;
+    if (!grid.barrier()) return;
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
@@ -394,6 +532,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.st->rz = rz;
+    if (it > 0) a.st->rr = ctl.total[1];
     a.st->iter = iter0 + it;
     a.st->status = ctl.status;
     a.st->done = ctl.done;
@@ -544,11 +683,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfReside
     }
   }
   __syncthreads();
-  double rz = a.st->rz, rz_prev = 0.0, rr = 0.0;   // threads 0 (rz) and 32 (rr) keep them
+  double rz = a.st->rz, rz_prev = 0.0;
   float beta = (float)a.st->beta;
-  double beta64 = 0.0;
   const double tol2 = a.st->tol2;
   const int max_iter = a.st->max_iter, iter0 = a.st->iter;
+  int epq = kNoExponent, erz = sum_exponent(rz), err = sum_exponent(a.st->rr);   // of the sums' last values
   int it = 0;
   for (;;) {
     float pq[1] = {0.f};
@@ -580,18 +719,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfReside
         }
       }
     }
-    const double bpq = res_block_sum_f<1>(pq, grid.sh);
-    if (!grid.template meet<1, false>(bpq)) return;
-    if (threadIdx.x < 32) {
-      const double t = grid.total(0);
-      if (threadIdx.x == 0) {
-        const bool ok = t > 0.0 && isfinite(t);
-        ctl.alpha = ok ? rz / t : 0.0;
-        ctl.status = ok ? AFEM_OK : AFEM_ERR_BREAKDOWN;
-        ctl.done = !ok;
-      }
-    }
-    __syncthreads();
+    if (!grid.template sum<1, false>(pq, {epq}, ctl.total, ctl.slow, [&](int, double t) {
+          const bool ok = t > 0.0 && isfinite(t);
+          ctl.alpha = ok ? quotient(rz, t) : 0.0;
+          ctl.status = ok ? AFEM_OK : AFEM_ERR_BREAKDOWN;
+          ctl.done = !ok;
+        }))
+      return;
+    epq = sum_exponent(ctl.total[0]);
     if (ctl.done) break;
     const float alpha = (float)ctl.alpha;
     float rs[2] = {0.f, 0.f};
@@ -607,23 +742,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfReside
         if (counted >> k & 1) rs[1] = fmaf(r[k], r[k], rs[1]);
       }
     }
-    const double brs = res_block_sum_f<2>(rs, grid.sh);
-    if (!grid.template meet<2, true>(brs)) return;
     ++it;
-    if (threadIdx.x < 64) {
-      const double t = grid.total(threadIdx.x >> 5);
-      if (threadIdx.x == 0) {
-        beta64 = t / rz;
-        ctl.beta = beta64;
-        rz_prev = rz;
-        rz = t;
-      } else if (threadIdx.x == 32) {
-        rr = t;
-        ctl.status = isfinite(t) ? AFEM_OK : AFEM_ERR_BREAKDOWN;
-        ctl.done = !isfinite(t) || t <= tol2 || iter0 + it >= max_iter;
-      }
-    }
-    __syncthreads();
+    if (!grid.template sum<2, true>(rs, {erz, err}, ctl.total, ctl.slow, [&](int j, double t) {
+          if (j == 0) {
+            ctl.beta = quotient(t, rz);
+            return;
+          }
+          ctl.done = !isfinite(t) || t <= tol2 || iter0 + it >= max_iter;
+          ctl.status = isfinite(t) ? AFEM_OK : AFEM_ERR_BREAKDOWN;
+        }))
+      return;
+    rz_prev = rz;
+    rz = ctl.total[0];
+    erz = sum_exponent(rz);
+    err = sum_exponent(ctl.total[1]);
     beta = (float)ctl.beta;
     if (ctl.done || it == a.iters) break;
   }
@@ -637,12 +769,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfReside
       a.q[row] = q[k];
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 32 && it > 0) a.st->rr = rr;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (it > 0) {
-      a.st->beta = beta64;
+      a.st->beta = ctl.beta;
       a.st->pad0 = rz_prev;
       a.st->rz = rz;
+      a.st->rr = ctl.total[1];
     }
     a.st->iter = iter0 + it;
     a.st->status = ctl.status;
@@ -666,10 +798,10 @@ struct ResPlan {
 // Where the line lies: one block an SM has the loads in flight for what the
 // shared memory leaves over of a matrix up to about 80 MB (L2-resident), and
 // registers for 6 rows a thread.  A solve, three launches an iteration against
-// this form: 2D triangles 256^2 19.2 -> 9.6 ms, 600^2 98.5 -> 43.2; tetrahedra
-// 57^3 8.8 -> 4.3, 75^3 17.7 -> 9.7; hexahedra 69^3 (34 MB left over)
-// 11.2 -> 7.1; elasticity 40^3 (77 MB left over) 50.8 -> 30.1, mixed
-// 35.1 -> 15.1.  Above, with 8 rows a thread: tetrahedra 84^3 23.7 -> 20.2, but
+// this form: 2D triangles 256^2 19.2 -> 8.6 ms, 600^2 98.5 -> 41.8; tetrahedra
+// 57^3 8.8 -> 4.0, 75^3 17.7 -> 9.7; hexahedra 69^3 (34 MB left over)
+// 11.2 -> 7.1; elasticity 40^3 (77 MB left over) 50.8 -> 29.1, mixed
+// 35.1 -> 14.7.  Above, with 8 rows a thread: tetrahedra 84^3 23.7 -> 20.2, but
 // renumbered at random 28.1 -> 34.2; hexahedra 84^3 17.9 -> 20.4.
 // A matrix whose rows gather at random lives on what the L1 keeps of the
 // gathered vector, and here shared memory takes most of the L1: with

@@ -5,6 +5,7 @@
 #pragma once
 #include <type_traits>
 
+#include "afem_fp64_int.cuh"
 #include "afem_internal.cuh"
 
 namespace afem {
@@ -80,6 +81,17 @@ __device__ __forceinline__ double reduce_partials(const double* partials, int np
   double s = 0.0;
   for (int k = threadIdx.x; k < nparts; k += blockDim.x) s += ((volatile const double*)partials)[(int64_t)k * W + w];
   return block_sum(s, sh);
+}
+
+// a / b rounded to nearest on the integer pipes (afem_fp64_int.cuh) where both
+// are in its range: an FP64 division is some ten dependent FP64 instructions.
+__device__ __forceinline__ double quotient(double a, double b) {
+  const int ah = __double2hiint(a), bh = __double2hiint(b);
+  if (!i64fp::in_window<400>(ah, __double2loint(a)) || !i64fp::in_window<400>(bh, __double2loint(b)) ||
+      (bh & 0x7ff00000) == 0)
+    return a / b;
+  return __longlong_as_double(i64fp::div(i64fp::operand(ah, __double2loint(a)),
+                                         i64fp::divisor(__double_as_longlong(b))));
 }
 
 // ---------------------------------------------------------------------------
