@@ -61,11 +61,11 @@ __device__ __forceinline__ double row_dot(int row, const int32_t* __restrict__ r
 }
 
 // ---------------------------------------------------------------------------
-// Last-block finalize helper: every block publishes partials[blockIdx.x * W + w];
+// Last-block finalize helper: the first lanes of a block's warps publish its partials (block_partials, or thread 0);
 // returns true in the (single) last block, after which all partials are visible.
 __device__ __forceinline__ bool last_block(unsigned int* ticket) {
   __shared__ bool is_last;
-  __threadfence();
+  if ((threadIdx.x & 31) == 0) __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned int t = atomicAdd(ticket, 1u);
@@ -76,11 +76,50 @@ __device__ __forceinline__ bool last_block(unsigned int* ticket) {
   return is_last;
 }
 
-// Fixed-order sum of partials[k * W + w], k < nparts (valid in thread 0).
-__device__ __forceinline__ double reduce_partials(const double* partials, int nparts, int W, int w, double* sh) {
-  double s = 0.0;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) s += ((volatile const double*)partials)[(int64_t)k * W + w];
-  return block_sum(s, sh);
+// Block sums of V values a thread (blocks of kSolveBlock) into partials[blockIdx.x * V + j].  An FP64 instruction
+// takes an SM about 19 cycles however few lanes take part, so the block's values go through shared memory and one
+// warp a sum adds them, 12 warp instructions; shuffles in every warp were 45, and the three kernels of a CG iteration
+// lost 10 of 104 us to them (128^3 tetrahedra).  sh: V * kSolveBlock doubles.
+template <int V>
+__device__ __forceinline__ void block_partials(const double (&v)[V], double* sh, double* partials) {
+  const int t = threadIdx.x, w = t >> 5;
+#pragma unroll
+  for (int j = 0; j < V; ++j) sh[j * kSolveBlock + t] = v[j];
+  __syncthreads();
+  if (w < V) {
+    const double* p = sh + w * kSolveBlock + (t & 31);
+    double s = p[0];
+#pragma unroll
+    for (int m = 1; m < kSolveBlock / 32; ++m) s += p[32 * m];
+    s = warp_sum(s);
+    if ((t & 31) == 0) partials[blockIdx.x * V + w] = s;
+  }
+}
+
+// Fixed-order sums of partials[k * V + j], k < nparts, for the threads of the last block (out valid in thread 0).
+template <int V>
+__device__ __forceinline__ void total_partials(const double* partials, int nparts, double* sh, double (&out)[V]) {
+  const int t = threadIdx.x, w = t >> 5;
+  __syncthreads();
+  double s[V] = {};
+  for (int k = t; k < nparts; k += kSolveBlock)
+#pragma unroll
+    for (int j = 0; j < V; ++j) s[j] += ((volatile const double*)partials)[(int64_t)k * V + j];
+#pragma unroll
+  for (int j = 0; j < V; ++j) sh[j * kSolveBlock + t] = s[j];
+  __syncthreads();
+  if (w < V) {
+    double* p = sh + w * kSolveBlock;
+    double r = p[t & 31];
+#pragma unroll
+    for (int m = 1; m < kSolveBlock / 32; ++m) r += p[(t & 31) + 32 * m];
+    r = warp_sum(r);
+    __syncwarp();
+    if ((t & 31) == 0) p[0] = r;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < V; ++j) out[j] = sh[j * kSolveBlock];
 }
 
 // a / b rounded to nearest on the integer pipes (afem_fp64_int.cuh) where both

@@ -2173,7 +2173,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_init(int n, const int32_t* 
                                                           float* __restrict__ r32, double* partials, FcgState* st,
                                                           double rtol, double atol, int max_iter,
                                                           const uint8_t* __restrict__ skip) {
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[2 * kSolveBlock];
   const int lane = threadIdx.x & (G - 1);
   const int groups = gridDim.x * (blockDim.x / G);
   const int nr = n + ((groups - n % groups) % groups);
@@ -2195,15 +2195,13 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_init(int n, const int32_t* 
       }
     }
   }
-  rr = block_sum(rr, sh);
-  bb = block_sum(bb, sh);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x * 2] = rr;
-    partials[blockIdx.x * 2 + 1] = bb;
-  }
+  const double sums[2] = {rr, bb};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[0])) {
-    const double trr = reduce_partials(partials, gridDim.x, 2, 0, sh);
-    const double tbb = reduce_partials(partials, gridDim.x, 2, 1, sh);
+    double tot[2];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double trr = tot[0];
+    const double tbb = tot[1];
     if (threadIdx.x == 0) {
       st->rr = trr;
       st->bnorm2 = tbb;
@@ -2226,7 +2224,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_spmv(int n, const int32_t* 
   pdl_trigger();
   pdl_wait();
   if (((volatile FcgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[2 * kSolveBlock];
   const int lane = threadIdx.x & (G - 1);
   const int groups = gridDim.x * (blockDim.x / G);
   const int nr = n + ((groups - n % groups) % groups);
@@ -2245,15 +2243,13 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_spmv(int n, const int32_t* 
       rpd += r[row] * pi;
     }
   }
-  pq = block_sum(pq, sh);
-  rpd = block_sum(rpd, sh);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x * 2] = pq;
-    partials[blockIdx.x * 2 + 1] = rpd;
-  }
+  const double sums[2] = {pq, rpd};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[1])) {
-    const double tpq = reduce_partials(partials, gridDim.x, 2, 0, sh);
-    const double trp = reduce_partials(partials, gridDim.x, 2, 1, sh);
+    double tot[2];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double tpq = tot[0];
+    const double trp = tot[1];
     if (threadIdx.x == 0) {
       st->pq = tpq;
       st->rp = trp;
@@ -2276,7 +2272,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_update(int n, double* __res
   pdl_trigger();
   pdl_wait();
   if (((volatile FcgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[kSolveBlock];
   const double alpha = ((volatile FcgState*)st)->alpha;
   double rr = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -2286,10 +2282,12 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_update(int n, double* __res
     r32[i] = (float)ri;
     if (!(skip && skip[i])) rr += ri * ri;
   }
-  rr = block_sum(rr, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x * 2] = rr;
+  const double sums[1] = {rr};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[2])) {
-    const double trr = reduce_partials(partials, gridDim.x, 2, 0, sh);
+    double tot[1];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double trr = tot[0];
     if (threadIdx.x == 0) {
       st->rr = trr;
       st->iter += 1;
@@ -2307,50 +2305,50 @@ __global__ void __launch_bounds__(kSolveBlock) k_fcg_update(int n, double* __res
   }
 }
 
-// first != 0: p = z32 (the initial direction).  Otherwise z = z32 and
-// <z, q> -> beta = -<z, q> / <p, q>.
-__global__ void __launch_bounds__(kSolveBlock) k_fcg_widen(int n, const float* __restrict__ z32, double* __restrict__ z,
-                                                           const double* __restrict__ q, double* __restrict__ p,
-                                                           int first, double* partials, FcgState* st) {
+// p = z32, the initial direction.
+__global__ void __launch_bounds__(kSolveBlock) k_fcg_first(int n, const float* __restrict__ z32, double* __restrict__ p,
+                                                           const FcgState* st) {
+  if (((volatile const FcgState*)st)->done) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = (double)z32[i];
+}
+
+// <z, q> -> beta = -<z, q> / <p, q>
+__global__ void __launch_bounds__(kSolveBlock) k_fcg_beta(int n, const float* __restrict__ z32,
+                                                          const double* __restrict__ q, double* partials,
+                                                          FcgState* st) {
   pdl_trigger();
   pdl_wait();
   if (((volatile FcgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[kSolveBlock];
   double zq = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double zi = (double)z32[i];
-    if (first) {
-      p[i] = zi;
-    } else {
-      z[i] = zi;
-      zq += zi * q[i];
-    }
-  }
-  if (first) return;
-  zq = block_sum(zq, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x * 2] = zq;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) zq += (double)z32[i] * q[i];
+  const double sums[1] = {zq};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[3])) {
-    const double t = reduce_partials(partials, gridDim.x, 2, 0, sh);
+    double tot[1];
+    total_partials(partials, gridDim.x, sh, tot);
     if (threadIdx.x == 0) {
-      st->beta = -t / st->pq;
+      st->beta = -tot[0] / st->pq;
       st->ticket[3] = 0;
     }
   }
 }
 
-__global__ void __launch_bounds__(kSolveBlock) k_fcg_dir(int n, const double* __restrict__ z, double* __restrict__ p,
+// p = z + beta p
+__global__ void __launch_bounds__(kSolveBlock) k_fcg_dir(int n, const float* __restrict__ z32, double* __restrict__ p,
                                                          const FcgState* st) {
   pdl_trigger();
   pdl_wait();
   if (((volatile const FcgState*)st)->done) return;
   const double beta = ((volatile const FcgState*)st)->beta;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = z[i] + beta * p[i];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    p[i] = (double)z32[i] + beta * p[i];
 }
 
 // Solver buffers and the captured iteration graph, kept with the network and
 // rebuilt when the operator or solution pointers change.
 struct FcgWork {
-  double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *partials = nullptr;
+  double *r = nullptr, *p = nullptr, *q = nullptr, *partials = nullptr;
   FcgState* st = nullptr;
   int nparts = 0;
   const void* key[5] = {};
@@ -2375,7 +2373,6 @@ static afem_status fcg_work(afem_mpnn net, FcgWork** out) {
     w->nparts = (int)std::max<unsigned>(grid_for(net->ctx, (int64_t)n * 32, kSolveBlock, 8),
                                         grid_for(net->ctx, (int64_t)n, kSolveBlock, 8));
     AFEM_TRY(dalloc(net, n, &w->r));
-    AFEM_TRY(dalloc(net, n, &w->z));
     AFEM_TRY(dalloc(net, n, &w->p));
     AFEM_TRY(dalloc(net, n, &w->q));
     AFEM_TRY(dalloc(net, (size_t)2 * w->nparts, &w->partials));
@@ -2422,8 +2419,8 @@ afem_status afem::fcg_solve(afem_context ctx, int n, const int32_t* rp, const in
   int32_t nnz32 = 0;
   AFEM_TRY(read_scalar(ctx, rp + n, &nnz32));
   const int G = lanes_per_row_fp64(n, nnz32);
-  const unsigned grid_rows = grid_for(ctx, (int64_t)n * G, kSolveBlock, 8);
-  const unsigned grid_vec = grid_for(ctx, n, kSolveBlock, 8);
+  const unsigned grid_rows = grid_for(ctx, (int64_t)n * G, kSolveBlock, 4);
+  const unsigned grid_vec = grid_for(ctx, n, kSolveBlock, 4);
   FcgWork* w = nullptr;
   AFEM_TRY(fcg_work(net, &w));
   if (!net->scalings_valid) AFEM_TRY(features_forward(net));
@@ -2450,9 +2447,9 @@ afem_status afem::fcg_solve(afem_context ctx, int n, const int32_t* rp, const in
         AFEM_TRY(launch_pdl(ctx, s, k_fcg_update, dim3(grid_vec), kSolveBlock, n, x, w->r, net->r32,
                             (const double*)w->p, (const double*)w->q, w->partials, w->st, skip));
         AFEM_TRY(apply_on(net, s));
-        AFEM_TRY(launch_pdl(ctx, s, k_fcg_widen, dim3(grid_vec), kSolveBlock, n, (const float*)net->z32, w->z,
-                            (const double*)w->q, w->p, 0, w->partials, w->st));
-        AFEM_TRY(launch_pdl(ctx, s, k_fcg_dir, dim3(grid_vec), kSolveBlock, n, (const double*)w->z, w->p,
+        AFEM_TRY(launch_pdl(ctx, s, k_fcg_beta, dim3(grid_vec), kSolveBlock, n, (const float*)net->z32,
+                            (const double*)w->q, w->partials, w->st));
+        AFEM_TRY(launch_pdl(ctx, s, k_fcg_dir, dim3(grid_vec), kSolveBlock, n, (const float*)net->z32, w->p,
                             (const FcgState*)w->st));
       }
       return AFEM_OK;
@@ -2478,8 +2475,7 @@ afem_status afem::fcg_solve(afem_context ctx, int n, const int32_t* rp, const in
   });
   if (st == AFEM_OK) st = apply(net, 1, net->r32, net->z32);
   if (st == AFEM_OK)
-    st = launch(ctx, k_fcg_widen, grid_vec, kSolveBlock, 0, n, (const float*)net->z32, w->z, (const double*)w->q,
-                w->p, 1, w->partials, w->st);
+    st = launch(ctx, k_fcg_first, grid_vec, kSolveBlock, 0, n, (const float*)net->z32, w->p, (const FcgState*)w->st);
   // Chunks of `chunk` iterations while at least that many remain, then single
   // iterations: the remaining count is predicted from the residual's
   // reduction since the previous read-back (iterations past convergence

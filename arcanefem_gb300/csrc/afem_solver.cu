@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_cg_init(int n, const int32_t* _
                                                          const uint8_t* __restrict__ skip, double* __restrict__ r,
                                                          double* __restrict__ z, double* __restrict__ p,
                                                          double* partials, CgState* st, double rtol, double atol) {
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[3 * kSolveBlock];
   const int lane = threadIdx.x & (G - 1);
   const int groups = gridDim.x * (blockDim.x / G);
   double rz = 0.0, rr = 0.0, bb = 0.0;
@@ -89,18 +89,14 @@ __global__ void __launch_bounds__(kSolveBlock) k_cg_init(int n, const int32_t* _
       }
     }
   }
-  rz = block_sum(rz, sh);
-  rr = block_sum(rr, sh);
-  bb = block_sum(bb, sh);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x * 3 + 0] = rz;
-    partials[blockIdx.x * 3 + 1] = rr;
-    partials[blockIdx.x * 3 + 2] = bb;
-  }
+  const double sums[3] = {rz, rr, bb};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[0])) {
-    double trz = reduce_partials(partials, gridDim.x, 3, 0, sh);
-    double trr = reduce_partials(partials, gridDim.x, 3, 1, sh);
-    double tbb = reduce_partials(partials, gridDim.x, 3, 2, sh);
+    double tot[3];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double trz = tot[0];
+    const double trr = tot[1];
+    const double tbb = tot[2];
     if (threadIdx.x == 0) {
       st->rz = trz;
       st->rr = trr;
@@ -125,7 +121,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_cg_update(int n, double* __rest
                                                            const uint8_t* __restrict__ skip, double* partials,
                                                            CgState* st) {
   if (((volatile CgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[2 * kSolveBlock];
   const double alpha = ((volatile CgState*)st)->alpha;
   double rz = 0.0, rr = 0.0;
   // two elements per thread and pass (16-byte accesses: every vector here is
@@ -162,15 +158,13 @@ __global__ void __launch_bounds__(kSolveBlock) k_cg_update(int n, double* __rest
     rz += ri * zi;
     if (!(skip && skip[i])) rr += ri * ri;
   }
-  rz = block_sum(rz, sh);
-  rr = block_sum(rr, sh);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x * 2 + 0] = rz;
-    partials[blockIdx.x * 2 + 1] = rr;
-  }
+  const double sums[2] = {rz, rr};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[2])) {
-    double trz = reduce_partials(partials, gridDim.x, 2, 0, sh);
-    double trr = reduce_partials(partials, gridDim.x, 2, 1, sh);
+    double tot[2];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double trz = tot[0];
+    const double trr = tot[1];
     if (threadIdx.x == 0) {
       st->beta = trz / st->rz;
       st->rz = trz;
@@ -235,7 +229,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_cg_spmv_sl(int n, const int32_t
                                                             const double* __restrict__ p, double* __restrict__ q,
                                                             double* partials, CgState* st) {
   if (((volatile CgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[kSolveBlock];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;   // a multiple of 32: a warp is one slice
   const int64_t nr = ((int64_t)n + kSlice - 1) / kSlice * kSlice;
   double pq = 0.0;
@@ -249,10 +243,12 @@ __global__ void __launch_bounds__(kSolveBlock) k_cg_spmv_sl(int n, const int32_t
       pq += p[row] * acc;
     }
   }
-  pq = block_sum(pq, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = pq;
+  const double sums[1] = {pq};
+  block_partials(sums, sh, partials);
   if (last_block(&st->ticket[1])) {
-    double t = reduce_partials(partials, gridDim.x, 1, 0, sh);
+    double tot[1];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double t = tot[0];
     if (threadIdx.x == 0) {
       st->pq = t;
       if (!(t > 0.0) || !isfinite(t)) {
@@ -280,7 +276,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_cgf_spmv_sl(int n, const int32_
                                                              const float* __restrict__ z, float* __restrict__ p,
                                                              float* __restrict__ q, double* partials, CgState* st) {
   if (((volatile CgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[kSolveBlock];
   const float beta = (float)((volatile CgState*)st)->beta;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;   // a multiple of 32: a warp is one slice
   const int64_t nr = ((int64_t)n + kSlice - 1) / kSlice * kSlice;
@@ -302,7 +298,9 @@ __global__ void __launch_bounds__(kSolveBlock) k_cgf_spmv_sl(int n, const int32_
   const double pq = block_sum_f(pqf, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = pq;
   if (last_block(&st->ticket[1])) {
-    double t = reduce_partials(partials, gridDim.x, 1, 0, sh);
+    double tot[1];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double t = tot[0];
     if (threadIdx.x == 0) {
       st->pq = t;
       if (!(t > 0.0) || !isfinite(t)) {
@@ -396,7 +394,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_cgf_spmv_b3s(int nb, const int3
                                                               const float* __restrict__ z, float* __restrict__ p,
                                                               float* __restrict__ q, double* partials, CgState* st) {
   if (((volatile CgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[kSolveBlock];
   const float beta = (float)((volatile CgState*)st)->beta;
   const int lane = threadIdx.x & 31;
   const int64_t nslice = ((int64_t)nb + kSlice - 1) / kSlice;
@@ -442,7 +440,9 @@ __global__ void __launch_bounds__(kSolveBlock) k_cgf_spmv_b3s(int nb, const int3
   const double pq = block_sum_f(pqf, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = pq;
   if (last_block(&st->ticket[1])) {
-    double t = reduce_partials(partials, gridDim.x, 1, 0, sh);
+    double tot[1];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double t = tot[0];
     if (threadIdx.x == 0) {
       st->pq = t;
       if (!(t > 0.0) || !isfinite(t)) {
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_cgf_update(int n, float* __rest
                                                             const uint8_t* __restrict__ skip, double* partials,
                                                             CgState* st) {
   if (((volatile CgState*)st)->done) return;
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[2 * kSolveBlock];
   const float alpha = (float)((volatile CgState*)st)->alpha;
   float rzf = 0.f, rrf = 0.f;
   // four elements per thread and pass (16-byte accesses: the vectors are the
@@ -513,8 +513,10 @@ __global__ void __launch_bounds__(kSolveBlock) k_cgf_update(int n, float* __rest
     partials[blockIdx.x * 2 + 1] = rr;
   }
   if (last_block(&st->ticket[2])) {
-    double trz = reduce_partials(partials, gridDim.x, 2, 0, sh);
-    double trr = reduce_partials(partials, gridDim.x, 2, 1, sh);
+    double tot[2];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double trz = tot[0];
+    const double trr = tot[1];
     if (threadIdx.x == 0) {
       st->beta = trz / st->rz;
       st->pad0 = st->rz;   // <r, z> before this step, for a reliable update that keeps p
@@ -543,7 +545,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_ir_residual(
     const double* __restrict__ b, const double* __restrict__ x, const float* __restrict__ dinv32,
     const uint8_t* __restrict__ skip, float* __restrict__ r32, float* __restrict__ x32, float* __restrict__ z32,
     double* partials, CgState* outer, CgState* inner, double inner_rtol, int inner_max, int restart) {
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[3 * kSolveBlock];
   const int lane = threadIdx.x & (G - 1);
   const int groups = gridDim.x * (blockDim.x / G);
   const int nr = n + ((groups - n % groups) % groups);
@@ -570,18 +572,14 @@ __global__ void __launch_bounds__(kSolveBlock) k_ir_residual(
       }
     }
   }
-  rz = block_sum(rz, sh);
-  rr = block_sum(rr, sh);
-  bb = block_sum(bb, sh);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x * 3 + 0] = rz;
-    partials[blockIdx.x * 3 + 1] = rr;
-    partials[blockIdx.x * 3 + 2] = bb;
-  }
+  const double sums[3] = {rz, rr, bb};
+  block_partials(sums, sh, partials);
   if (last_block(&outer->ticket[0])) {
-    double trz = reduce_partials(partials, gridDim.x, 3, 0, sh);
-    double trr = reduce_partials(partials, gridDim.x, 3, 1, sh);
-    double tbb = reduce_partials(partials, gridDim.x, 3, 2, sh);
+    double tot[3];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double trz = tot[0];
+    const double trr = tot[1];
+    const double tbb = tot[2];
     if (threadIdx.x == 0) {
       outer->rr = trr;
       outer->bnorm2 = tbb;
@@ -910,7 +908,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_true_residual(int n, const int3
                                                                const double* __restrict__ x,
                                                                const uint8_t* __restrict__ skip, double* partials,
                                                                unsigned int* ticket, double* out) {
-  __shared__ double sh[kSolveBlock / 32];
+  __shared__ double sh[2 * kSolveBlock];
   const int lane = threadIdx.x & (G - 1);
   const int groups = gridDim.x * (blockDim.x / G);
   const int nr = n + ((groups - n % groups) % groups);
@@ -928,15 +926,13 @@ __global__ void __launch_bounds__(kSolveBlock) k_true_residual(int n, const int3
       bb += b[row] * b[row];
     }
   }
-  rr = block_sum(rr, sh);
-  bb = block_sum(bb, sh);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x * 2] = rr;
-    partials[blockIdx.x * 2 + 1] = bb;
-  }
+  const double sums[2] = {rr, bb};
+  block_partials(sums, sh, partials);
   if (last_block(ticket)) {
-    double a = reduce_partials(partials, gridDim.x, 2, 0, sh);
-    double c = reduce_partials(partials, gridDim.x, 2, 1, sh);
+    double tot[2];
+    total_partials(partials, gridDim.x, sh, tot);
+    const double a = tot[0];
+    const double c = tot[1];
     if (threadIdx.x == 0) {
       out[0] = a;
       out[1] = c;
