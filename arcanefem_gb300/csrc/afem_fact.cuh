@@ -352,40 +352,35 @@ __global__ void k_fact_dc(FactView f, const float* __restrict__ m, const float* 
 __global__ void k_fact_edge_backward(FactView f, const float* __restrict__ z, const float* __restrict__ a_low,
                                      const float* __restrict__ gl_low, const bf16* __restrict__ o,
                                      float* __restrict__ dz, float* __restrict__ part) {
-  __shared__ float sh[kF + 1][8];
-  float acc[kF + 1];
-#pragma unroll
-  for (int c = 0; c <= kF; ++c) acc[c] = 0.f;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < f.nlow; e += gridDim.x * blockDim.x) {
-    const int32_t i = f.lo_row[e], j = f.lo_col[e];
-    const float th = tanhf(z[e]);
-    const float sj = f.sq[j];
-    const float g = gl_low[e] * a_low[e] * f.sq[i] * sj * sj * 2.f * (1.f - th * th);
-    dz[e] = g;
-    const __nv_bfloat162* oi = reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)i * kF);
-    const __nv_bfloat162* oj = reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)j * kF);
-#pragma unroll
-    for (int c = 0; c < kF / 2; ++c) {
-      const float2 a = __bfloat1622float2(oi[c]), b = __bfloat1622float2(oj[c]);
-      acc[2 * c] = fmaf(g * a.x, b.x, acc[2 * c]);
-      acc[2 * c + 1] = fmaf(g * a.y, b.y, acc[2 * c + 1]);
+  // a warp takes 32 edges: their dz one a lane, then edge by edge the two rows of o, two features a lane
+  float a0 = 0.f, a1 = 0.f, gs = 0.f;
+  const int lane = threadIdx.x & 31;
+  for (int64_t e0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; e0 < f.nlow;
+       e0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t e = e0 + lane;
+    int32_t i = 0, j = 0;
+    float g = 0.f;
+    if (e < f.nlow) {
+      i = f.lo_row[e];
+      j = f.lo_col[e];
+      const float th = tanhf(z[e]);
+      const float sj = f.sq[j];
+      g = gl_low[e] * a_low[e] * f.sq[i] * sj * sj * 2.f * (1.f - th * th);
+      dz[e] = g;
     }
-    acc[kF] += g;
+    const int count = (int)min((int64_t)32, f.nlow - e0);
+#pragma unroll 4
+    for (int k = 0; k < count; ++k) {
+      const float gk = __shfl_sync(0xffffffffu, g, k);
+      const int32_t ik = __shfl_sync(0xffffffffu, i, k), jk = __shfl_sync(0xffffffffu, j, k);
+      const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)ik * kF)[lane]);
+      const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)jk * kF)[lane]);
+      a0 = fmaf(gk * a.x, b.x, a0);
+      a1 = fmaf(gk * a.y, b.y, a1);
+      gs += gk;
+    }
   }
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-#pragma unroll
-  for (int c = 0; c <= kF; ++c) {
-    float v = acc[c];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) sh[c][wp] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x <= kF) {
-    float s = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[threadIdx.x][k];
-    part[(int64_t)blockIdx.x * (kF + 1) + threadIdx.x] = s;
-  }
+  column_partials<true>(a0, a1, gs, part);
 }
 
 // dO_i += sum over the edges e of node i (as row and as column) of dz_e ew * o_other; one warp per node,

@@ -430,12 +430,23 @@ __global__ void __launch_bounds__(128) k_dw_grad(const __grid_constant__ CUtenso
 // (warp w takes b = w, w + kSumWarps, ..., four loads in flight), and warp 0
 // adds the warp sums in warp order.
 constexpr int kSumWarps = 32;
-__global__ void __launch_bounds__(32 * kSumWarps) k_sum_partials(int nparts, int nelem,
-                                                                 const float* __restrict__ partial,
-                                                                 float* __restrict__ out, int accumulate) {
-  __shared__ float sh[kSumWarps][33];
+
+// k_sum_partials_many does it for several arrays in one launch: block b belongs to the job with
+// block0 <= b < the next one's.
+struct SumJob {
+  const float* part;
+  float* out;
+  int nparts, nelem, block0;
+};
+constexpr int kSumJobs = 40;
+struct SumJobs {
+  SumJob job[kSumJobs];
+  int count;
+};
+
+__device__ __forceinline__ float sum_column(const float* __restrict__ partial, int nparts, int nelem, int e,
+                                            float (*sh)[33]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int e = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (e < nelem) {
     int b = w;
@@ -453,10 +464,46 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum_partials(int nparts, int
   }
   sh[w][lane] = s;
   __syncthreads();
-  if (w == 0 && e < nelem) {
-    float t = 0.f;
+  float t = 0.f;
+  if (w == 0)
     for (int k = 0; k < kSumWarps; ++k) t += sh[k][lane];
-    out[e] = accumulate ? out[e] + t : t;
+  return t;   // in warp 0
+}
+
+__global__ void __launch_bounds__(32 * kSumWarps) k_sum_partials(int nparts, int nelem,
+                                                                 const float* __restrict__ partial,
+                                                                 float* __restrict__ out, int accumulate) {
+  __shared__ float sh[kSumWarps][33];
+  const int e = blockIdx.x * 32 + (threadIdx.x & 31);
+  const float t = sum_column(partial, nparts, nelem, e, sh);
+  if (threadIdx.x < 32 && e < nelem) out[e] = accumulate ? out[e] + t : t;
+}
+
+__global__ void __launch_bounds__(32 * kSumWarps) k_sum_partials_many(const SumJobs jobs) {
+  __shared__ float sh[kSumWarps][33];
+  int j = 0;
+  while (j + 1 < jobs.count && (int)blockIdx.x >= jobs.job[j + 1].block0) ++j;
+  const SumJob& q = jobs.job[j];
+  const int e = ((int)blockIdx.x - q.block0) * 32 + (threadIdx.x & 31);
+  const float t = sum_column(q.part, q.nparts, q.nelem, e, sh);
+  if (threadIdx.x < 32 && e < q.nelem) q.out[e] = t;
+}
+
+// Column sums of a block whose lanes hold two features (and a scalar, the same in a warp's lanes) of their warps'
+// rows: part[block][0..kF) and, with SCALAR, part[block][kF].
+template <bool SCALAR>
+__device__ __forceinline__ void column_partials(float a0, float a1, float g, float* __restrict__ part) {
+  __shared__ float sh[kF + 1][9];
+  constexpr int C = kF + (SCALAR ? 1 : 0);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  sh[2 * lane][w] = a0;
+  sh[2 * lane + 1][w] = a1;
+  if (SCALAR && lane == 0) sh[kF][w] = g;
+  __syncthreads();
+  if (threadIdx.x < C) {
+    float s = 0.f;
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[threadIdx.x][k];
+    part[(int64_t)blockIdx.x * C + threadIdx.x] = s;
   }
 }
 
@@ -915,9 +962,10 @@ __global__ void k_l1cap(int n, const int32_t* __restrict__ rp, const double* __r
 }
 
 // per-sample energy sums: sums[b*4+0] += e . (A e), sums[b*4+1] += (e - z) . (A (e - z))
-__global__ void k_energy_sums(int n, const float* __restrict__ z, const float* __restrict__ e,
-                              const float* __restrict__ Ae, const float* __restrict__ Av, double* __restrict__ sums) {
-  __shared__ double sh[32];
+__global__ void __launch_bounds__(256) k_energy_sums(int n, const float* __restrict__ z, const float* __restrict__ e,
+                                                     const float* __restrict__ Ae, const float* __restrict__ Av,
+                                                     double* __restrict__ sums) {
+  __shared__ double sh[2 * 256];
   const int64_t b = blockIdx.y;
   double ee = 0, vv = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -926,11 +974,16 @@ __global__ void k_energy_sums(int n, const float* __restrict__ z, const float* _
     ee += ei * (double)Ae[k];
     vv += (ei - (double)z[k]) * (double)Av[k];
   }
-  ee = block_sum(ee, sh);
-  vv = block_sum(vv, sh);
-  if (threadIdx.x == 0) {
-    atomicAdd(&sums[b * 4], ee);
-    atomicAdd(&sums[b * 4 + 1], vv);
+  const int t = threadIdx.x, w = t >> 5;
+  sh[t] = ee;
+  sh[256 + t] = vv;
+  __syncthreads();
+  if (w < 2) {   // a warp a sum: FP64 instructions cost the same however few lanes take part
+    double s = 0.0;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) s += sh[w * 256 + (t & 31) + 32 * m];
+    s = warp_sum(s);
+    if ((t & 31) == 0) atomicAdd(&sums[b * 4 + w], s);
   }
 }
 
@@ -943,8 +996,13 @@ __global__ void k_sub(int64_t n, const float* __restrict__ e, const float* __res
 // dL/dz = -2 A (e - z) / (e . A e  B), in place over Av
 __global__ void k_energy_grad(int n, int batch, const double* __restrict__ sums, float* __restrict__ Av) {
   const int64_t b = blockIdx.y;
-  const double ee = sums[b * 4] > 0 ? sums[b * 4] : 1e-300;
-  const float scale = (float)(-2.0 / (ee * batch));
+  __shared__ float scale_sh;   // one FP64 division a block: in every thread they took 22 of the kernel's 26 us
+  if (threadIdx.x == 0) {
+    const double ee = sums[b * 4] > 0 ? sums[b * 4] : 1e-300;
+    scale_sh = (float)(-2.0 / (ee * batch));
+  }
+  __syncthreads();
+  const float scale = scale_sh;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) Av[b * n + i] *= scale;
 }
 
@@ -965,48 +1023,32 @@ __global__ void k_dc_vcycle(int n, int batch, const float* __restrict__ d, const
   }
 }
 
-// head backward: d o = dc (x) w (FP32 [n][64]); partials of dw = sum_i dc_i o_i and dbeta = sum_i dc_i
+// head backward: d o = dc (x) w (FP32 [n][64]); partials of dw = sum_i dc_i o_i and dbeta = sum_i dc_i.  A warp per
+// row, two features a lane: its loads and stores are whole lines (a thread per row with 65 sums took 11 us a level
+// on average in a training step at 257^2, this 4).
 __global__ void k_head_backward(int n, const float* __restrict__ dc, const bf16* __restrict__ o,
                                 const float* __restrict__ w, float* __restrict__ dO, float* __restrict__ part) {
-  __shared__ float sh[kF + 1][8];
-  float acc[kF + 1];
-#pragma unroll
-  for (int c = 0; c <= kF; ++c) acc[c] = 0.f;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float g = dc[i];
-    const __nv_bfloat162* row = reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)i * kF);
-    float2* drow = reinterpret_cast<float2*>(dO + (int64_t)i * kF);
-#pragma unroll
-    for (int c = 0; c < kF / 2; ++c) {
-      const __nv_bfloat162 v = row[c];
-      acc[2 * c] = fmaf(g, __low2float(v), acc[2 * c]);
-      acc[2 * c + 1] = fmaf(g, __high2float(v), acc[2 * c + 1]);
-      drow[c] = make_float2(g * w[2 * c], g * w[2 * c + 1]);
-    }
-    acc[kF] += g;
+  float a0 = 0.f, a1 = 0.f, gs = 0.f;
+  const int lane = threadIdx.x & 31;
+  const float w0 = w[2 * lane], w1 = w[2 * lane + 1];
+#pragma unroll 4
+  for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; row < n;
+       row += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const float g = dc[row];
+    const float2 v = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(o + row * kF)[lane]);
+    reinterpret_cast<float2*>(dO + row * kF)[lane] = make_float2(g * w0, g * w1);
+    a0 = fmaf(g, v.x, a0);
+    a1 = fmaf(g, v.y, a1);
+    gs += g;
   }
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-#pragma unroll
-  for (int c = 0; c <= kF; ++c) {
-    float v = acc[c];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) sh[c][wp] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x <= kF) {
-    float s = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[threadIdx.x][k];
-    part[(int64_t)blockIdx.x * (kF + 1) + threadIdx.x] = s;
-  }
+  column_partials<true>(a0, a1, gs, part);
 }
 
 // G = dO (x) [O > 0] in BF16, and per-block column sums (db)
 __global__ void k_relu_grad(int64_t M, const float* __restrict__ dO, const bf16* __restrict__ O,
                             bf16* __restrict__ G, float* __restrict__ db_part) {
-  __shared__ float sh[kF][8];
   float acc0 = 0.f, acc1 = 0.f;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; row < M;
        row += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const __nv_bfloat162 o = reinterpret_cast<const __nv_bfloat162*>(O + row * kF)[lane];
@@ -1016,14 +1058,7 @@ __global__ void k_relu_grad(int64_t M, const float* __restrict__ dO, const bf16*
     acc0 += g0;
     acc1 += g1;
   }
-  sh[2 * lane][w] = acc0;
-  sh[2 * lane + 1][w] = acc1;
-  __syncthreads();
-  if (threadIdx.x < kF) {
-    float s = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[threadIdx.x][k];
-    db_part[(int64_t)blockIdx.x * kF + threadIdx.x] = s;
-  }
+  column_partials<false>(acc0, acc1, 0.f, db_part);
 }
 
 // input layer backward: G_in = da (x) [a > 0]; partials of dW_in = x0^T G_in (2 x 64) and db_in
@@ -1164,6 +1199,8 @@ struct afem_mpnn_s {
   double* sums = nullptr;                    // [B][4]
   float* part = nullptr;                     // partial sums (dW, db)
   int64_t part_cap = 0;
+  int64_t part_used = 0;                     // of the sums still to be made
+  SumJobs sums_due{};
   float* a32 = nullptr;                      // A in FP32 on the level-0 graph (training loss)
   CsrLevel Aop;
   float* tmpB = nullptr;                     // [B][n0]
@@ -1634,11 +1671,41 @@ static afem_status apply_adjoint(afem_mpnn net, int batch) {
   return AFEM_OK;
 }
 
-static afem_status ensure_part(afem_mpnn net, int64_t count) {
-  if (count <= net->part_cap) return AFEM_OK;
-  AFEM_TRY(dalloc(net, (size_t)count, &net->part));
-  net->part_cap = count;
+// The partial sums of a backward pass (one array a use) are added up together
+// in sums_flush: one launch instead of some twenty of 3 us each.
+static afem_status sums_flush(afem_mpnn net) {
+  SumJobs& due = net->sums_due;
+  if (due.count > 0) {
+    const SumJob& last = due.job[due.count - 1];
+    AFEM_TRY(launch(net->ctx, k_sum_partials_many, (unsigned)(last.block0 + (last.nelem + 31) / 32), 32 * kSumWarps, 0,
+                    due));
+  }
+  due.count = 0;
+  net->part_used = 0;
   return AFEM_OK;
+}
+
+// Room for `count` partial sums that stay until the next sums_flush (which this calls if the buffer is full; it then
+// grows, so that a pass of the same size fits the next time).
+static afem_status part_take(afem_mpnn net, int64_t count, float** out) {
+  if (net->part_used + count > net->part_cap || net->sums_due.count == kSumJobs) {
+    const int64_t want = 2 * net->part_cap + count;
+    const bool full = net->part_used + count > net->part_cap;
+    AFEM_TRY(sums_flush(net));
+    if (full) {
+      AFEM_TRY(dalloc(net, (size_t)want, &net->part));
+      net->part_cap = want;
+    }
+  }
+  *out = net->part + net->part_used;
+  net->part_used += (count + 31) / 32 * 32;
+  return AFEM_OK;
+}
+
+static void sum_later(afem_mpnn net, int nparts, int nelem, const float* part, float* dst) {
+  SumJobs& due = net->sums_due;
+  const int block0 = due.count ? due.job[due.count - 1].block0 + (due.job[due.count - 1].nelem + 31) / 32 : 0;
+  due.job[due.count++] = {part, dst, nparts, nelem, block0};
 }
 
 static afem_status sum_partials(afem_context ctx, int nparts, int nelem, const float* part, float* dst,
@@ -1655,7 +1722,7 @@ static int dw_grad_parts(afem_context ctx, int64_t M) {
 
 // part: dw_grad_parts(ctx, M) x 2 x 64 x 64 floats
 static afem_status dw_grad_launch(afem_context ctx, int* err, float* part, int64_t M, const bf16* X1,
-                                  const bf16* X2, const bf16* G, float* dst) {
+                                  const bf16* X2, const bf16* G) {
   if (M <= 0) return AFEM_OK;
   const int nb = dw_grad_parts(ctx, M);
   CUtensorMap m1, m2, mg;
@@ -1669,12 +1736,17 @@ static afem_status dw_grad_launch(afem_context ctx, int* err, float* part, int64
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_dw_grad", __FILE__, __LINE__);
   ++ctx->launches;
-  return sum_partials(ctx, nb, 2 * kF * kF, (const float*)part, dst, 0);
+  return AFEM_OK;
 }
 
 static afem_status dw_gemm2(afem_mpnn net, int64_t M, const bf16* X1, const bf16* X2, const bf16* G, float* dst) {
-  AFEM_TRY(ensure_part(net, (int64_t)dw_grad_parts(net->ctx, M) * 2 * kF * kF));
-  return dw_grad_launch(net->ctx, net->tc_err, net->part, M, X1, X2, G, dst);
+  if (M <= 0) return AFEM_OK;
+  const int nb = dw_grad_parts(net->ctx, M);
+  float* part;
+  AFEM_TRY(part_take(net, (int64_t)nb * 2 * kF * kF, &part));
+  AFEM_TRY(dw_grad_launch(net->ctx, net->tc_err, part, M, X1, X2, G));
+  sum_later(net, nb, 2 * kF * kF, part, dst);
+  return AFEM_OK;
 }
 
 // loss and gradients of the mean relative squared error over (r, e)
@@ -1694,13 +1766,14 @@ static afem_status fact_backward(afem_mpnn net, int batch) {
     const float* rl = l == 0 ? net->t0 : net->t[l];
     const CsrLevel& A = net->Ac[l];
     const unsigned nbk = grid_for(ctx, nl, 256, 2);
-    AFEM_TRY(ensure_part(net, std::max<int64_t>(nbk, (int64_t)grid_for(ctx, std::max(f.nlow, 1), 256, 2) * (kF + 1))));
+    float* part;
+    AFEM_TRY(part_take(net, nbk, &part));
     // the coarsest level's single use out = G r enters as a pre-smoothing with x1b = g
     AFEM_TRY(launch(ctx, k_fact_grad, nbk, 256, 0, fv, batch, rl, last ? (const float*)net->s[l] : net->x1b[l],
                     (const float*)f.wpre, (const float*)f.gpre, last ? (const float*)nullptr : net->u[l],
                     (const float*)net->s[l], (const float*)f.wpost, (const float*)f.gpost, f.gl_diag, f.gl_low,
-                    net->part));
-    AFEM_TRY(sum_partials(ctx, (int)nbk, 1, (const float*)net->part, f.scal + 2, 0));
+                    part));
+    AFEM_TRY(sum_partials(ctx, (int)nbk, 1, (const float*)part, f.scal + 2, 0));
     AFEM_TRY(launch(ctx, k_fact_theta_grad, 1, 32, 0, fv, (const int32_t*)A.rp, (const int32_t*)A.cols,
                     (const float*)A.w, (const float*)(f.scal + 1), (const int*)f.istar, (const float*)(f.scal + 2),
                     f.gl_diag, f.gl_low));
@@ -1709,10 +1782,11 @@ static afem_status fact_backward(afem_mpnn net, int batch) {
                     (const float*)net->base[l], net->dc[l]));
     float* gedge = net->grads + off_edge(net->NL, L, f.k);
     if (f.nlow) {
-      const unsigned nbe = grid_for(ctx, f.nlow, 256, 2);
+      const unsigned nbe = grid_for(ctx, f.nlow, 256, 4);
+      AFEM_TRY(part_take(net, (int64_t)nbe * (kF + 1), &part));
       AFEM_TRY(launch(ctx, k_fact_edge_backward, nbe, 256, 0, fv, (const float*)f.z, (const float*)f.a_low,
-                      (const float*)f.gl_low, (const bf16*)net->o[l], f.dz, net->part));
-      AFEM_TRY(sum_partials(ctx, (int)nbe, kF + 1, (const float*)net->part, gedge, 0));
+                      (const float*)f.gl_low, (const bf16*)net->o[l], f.dz, part));
+      sum_later(net, (int)nbe, kF + 1, part, gedge);
     }
   }
   return AFEM_OK;
@@ -1722,6 +1796,8 @@ static afem_status loss_and_gradients(afem_mpnn net, int batch, const float* r, 
   afem_context ctx = net->ctx;
   cudaStream_t s = ctx->stream;
   const int n0 = net->n0, L = net->L;
+  net->sums_due.count = 0;
+  net->part_used = 0;
   if (!net->scalings_valid) AFEM_TRY(features_forward(net));
   AFEM_TRY(apply(net, batch, r, nullptr));
   AFEM_CUDA(cudaMemsetAsync(net->sums, 0, sizeof(double) * 4 * batch, s));
@@ -1732,7 +1808,8 @@ static afem_status loss_and_gradients(afem_mpnn net, int batch, const float* r, 
   AFEM_TRY(sweep(net, &net->Aop, batch, net->tmpB, nullptr, nullptr, net->s[0], n0));
   AFEM_TRY(sweep(net, &net->Aop, batch, e, nullptr, nullptr, net->tmpB, n0));
   {
-    dim3 g(grid_for(ctx, n0, 256, 2), batch);
+    // about four blocks an SM over all vectors
+    dim3 g(std::min(grid_for(ctx, n0, 256, 2), std::max(1u, 4u * (unsigned)ctx->sm_count / (unsigned)batch)), batch);
     k_energy_sums<<<g, 256, 0, s>>>(n0, net->w[0], e, net->tmpB, net->s[0], net->sums);
     k_energy_grad<<<g, 256, 0, s>>>(n0, batch, net->sums, net->s[0]);
     cudaError_t ce = cudaGetLastError();
@@ -1744,12 +1821,12 @@ static afem_status loss_and_gradients(afem_mpnn net, int batch, const float* r, 
   AFEM_TRY(fact_backward(net, batch));
   for (int l = 0; l < L; ++l) {
     const int nl = net->n[l];
-    const unsigned nbk = grid_for(ctx, nl, 256, 2);
-    AFEM_TRY(ensure_part(net, (int64_t)nbk * (kF + 1)));
+    const unsigned nbk = grid_for(ctx, (int64_t)nl * 32, 256, 4);
+    float* part;
+    AFEM_TRY(part_take(net, (int64_t)nbk * (kF + 1), &part));
     AFEM_TRY(launch(ctx, k_head_backward, nbk, 256, 0, nl, (const float*)net->dc[l], (const bf16*)net->o[l],
-                    (const float*)(net->params + off_head(net->NL, l)), net->dO[l], net->part));
-    AFEM_TRY(sum_partials(ctx, (int)nbk, kF + 1, (const float*)net->part,
-                    net->grads + off_head(net->NL, l), 0));
+                    (const float*)(net->params + off_head(net->NL, l)), net->dO[l], part));
+    sum_later(net, (int)nbk, kF + 1, part, net->grads + off_head(net->NL, l));
     const auto& f = net->fl[l];
     if (f.on && f.nlow)   // + the edge head's d o
       AFEM_TRY(launch(ctx, k_fact_dO, grid_for(ctx, (int64_t)nl * 32, 256, 8), 256, 0, fact_view(net, l),
@@ -1764,10 +1841,11 @@ static afem_status loss_and_gradients(afem_mpnn net, int batch, const float* r, 
       continue;
     }
     const unsigned nbk = grid_for(ctx, M * 32, 256, 4);
-    AFEM_TRY(ensure_part(net, std::max<int64_t>((int64_t)nbk * kF, (int64_t)ctx->sm_count * 2 * kF * kF)));
+    float* part;
+    AFEM_TRY(part_take(net, (int64_t)nbk * kF, &part));
     AFEM_TRY(launch(ctx, k_relu_grad, nbk, 256, 0, M, (const float*)net->dO[l], (const bf16*)net->o[l], net->Gb,
-                    net->part));
-    AFEM_TRY(sum_partials(ctx, (int)nbk, kF, (const float*)net->part, net->grads + off_b(l), 0));
+                    part));
+    sum_later(net, (int)nbk, kF, part, net->grads + off_b(l));
     AFEM_TRY(dw_gemm2(net, M, net->h[l], net->m[l], net->Gb, net->grads + off_w1(l)));   // dW2 at off_w2 = off_w1 + 64^2
     // dh_l = G W1^T + S_l^T (G W2^T)   (S_l symmetric)
     AFEM_TRY((row_gemm<false, false>(net, M, net->Gb, net->Wn + (2 * l) * kF * kF, nullptr, nullptr, nullptr,
@@ -1779,11 +1857,12 @@ static afem_status loss_and_gradients(afem_mpnn net, int batch, const float* r, 
   }
   {
     const unsigned nbk = grid_for(ctx, (int64_t)n0 * 32, 256, 4);
-    AFEM_TRY(ensure_part(net, (int64_t)nbk * 3 * kF));
+    float* part;
+    AFEM_TRY(part_take(net, (int64_t)nbk * 3 * kF, &part));
     AFEM_TRY(launch(ctx, k_input_backward, nbk, 256, 0, (int64_t)n0, (const float*)net->dH[0],
-                    (const bf16*)net->a_in, (const float*)net->x0, net->part));
-    AFEM_TRY(sum_partials(ctx, (int)nbk, 3 * kF, (const float*)net->part,
-                    net->grads + off_win(), 0));
+                    (const bf16*)net->a_in, (const float*)net->x0, part));
+    sum_later(net, (int)nbk, 3 * kF, part, net->grads + off_win());
+    AFEM_TRY(sums_flush(net));
   }
   if (loss_h) {
     std::vector<double> hs(4 * batch);
@@ -2132,7 +2211,8 @@ afem_status afem_tc_weight_grad(afem_context ctx, int64_t M, const void* X1, con
   AFEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
   if (M == 0) AFEM_CUDA(cudaMemsetAsync(dW, 0, sizeof(float) * 2 * kF * kF, ctx->stream));
   AFEM_TRY(dw_grad_launch(ctx, err, part, M, static_cast<const bf16*>(X1), static_cast<const bf16*>(X2),
-                          static_cast<const bf16*>(G), dW));
+                          static_cast<const bf16*>(G)));
+  if (M > 0) AFEM_TRY(sum_partials(ctx, nb, 2 * kF * kF, (const float*)part, dW, 0));
   int h = 0;
   AFEM_TRY(read_scalar(ctx, err, &h));
   if (h) return fail(AFEM_ERR_TIMEOUT, "afem_tc_weight_grad: a tensor-core mbarrier wait ran out");
@@ -2153,8 +2233,8 @@ afem_status afem_tc_weight_grad(afem_context ctx, int64_t M, const void* X1, con
 //   K1  q = A p ; <p, q>, <r, p>            -> alpha = <r, p> / <p, q>
 //   K2  x += alpha p ; r -= alpha q ; r32   -> <r, r>, stop test
 //   M   z32 = M r32 (one V-cycle)
-//   K3  z = z32 ; <z, q>                    -> beta = -<z, q> / <p, q>
-//   K4  p = z + beta p
+//   K3  <z32, q>                            -> beta = -<z, q> / <p, q>
+//   K4  p = z32 + beta p
 
 namespace afem {
 
