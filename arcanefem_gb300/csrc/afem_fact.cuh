@@ -36,8 +36,8 @@ struct FactView {
 };
 
 // w = L x
-__device__ __forceinline__ void fact_lower(int i0, int st, const FactView& f, const float* __restrict__ x,
-                                           float* __restrict__ w) {
+__device__ __forceinline__ void fact_lower(int i0, int st, const FactView& f, const float* x,
+                                           float* w) {
   for (int i = i0; i < f.n; i += st) {
     float acc = f.sq[i] * x[i];
     for (int32_t e = f.low_rp[i]; e < f.low_rp[i + 1]; ++e) acc = fmaf(f.lval[e], x[f.lo_col[e]], acc);
@@ -46,9 +46,9 @@ __device__ __forceinline__ void fact_lower(int i0, int st, const FactView& f, co
 }
 
 // out = (base ? base : 0) + theta L^T (w1 + (w2 ? w2 : 0))
-__device__ __forceinline__ void fact_upper(int i0, int st, const FactView& f, const float* __restrict__ w1,
-                                           const float* __restrict__ w2, const float* __restrict__ base,
-                                           float* __restrict__ out) {
+__device__ __forceinline__ void fact_upper(int i0, int st, const FactView& f, const float* w1,
+                                           const float* w2, const float* base,
+                                           float* out) {
   const float th = *f.theta;
   for (int j = i0; j < f.n; j += st) {
     float acc = f.sq[j] * (w2 ? w1[j] + w2[j] : w1[j]);
@@ -63,8 +63,8 @@ __device__ __forceinline__ void fact_upper(int i0, int st, const FactView& f, co
 // out = r - A x
 __device__ __forceinline__ void vc_res(int i0, int st, int n, const int32_t* __restrict__ rp,
                                        const int32_t* __restrict__ cols, const float* __restrict__ w,
-                                       const float* __restrict__ r, const float* __restrict__ x,
-                                       float* __restrict__ out) {
+                                       const float* r, const float* x,
+                                       float* out) {
   for (int i = i0; i < n; i += st) {
     float acc = r[i];
     for (int32_t k = rp[i]; k < rp[i + 1]; ++k) acc = fmaf(-w[k], x[cols[k]], acc);

@@ -635,13 +635,15 @@ __global__ void k_sweep(int nrow, int ncol, const int32_t* __restrict__ rp, cons
 // V-cycle kernels (FP32).  The row operations below are shared by the
 // per-level kernels (grid-stride over the rows of one vector, the vector in
 // grid.y) and the coarse-levels kernels (block-stride, one block per vector).
-// Pointers are already offset to the vector.
+// Pointers are already offset to the vector; those of vectors are not
+// __restrict__, since in the coarse kernels other blocks write them between
+// two steps.
 
 // s = r - A (d .* r)     (forward pre-smoothing residual; backward x2b = g - A (d .* g))
 __device__ __forceinline__ void vc_smooth_res(int i0, int st, int n, const int32_t* __restrict__ rp,
                                               const int32_t* __restrict__ cols, const float* __restrict__ w,
-                                              const float* __restrict__ d, const float* __restrict__ r,
-                                              float* __restrict__ s) {
+                                              const float* __restrict__ d, const float* r,
+                                              float* s) {
   for (int i = i0; i < n; i += st) {
     float acc = r[i];
     for (int32_t k = rp[i]; k < rp[i + 1]; ++k) {
@@ -655,8 +657,8 @@ __device__ __forceinline__ void vc_smooth_res(int i0, int st, int n, const int32
 // y = (d ? d .* t : 0) + M x
 __device__ __forceinline__ void vc_spmv(int i0, int st, int n, const int32_t* __restrict__ rp,
                                         const int32_t* __restrict__ cols, const float* __restrict__ w,
-                                        const float* __restrict__ x, const float* __restrict__ d,
-                                        const float* __restrict__ t, float* __restrict__ y) {
+                                        const float* x, const float* __restrict__ d,
+                                        const float* t, float* y) {
   for (int i = i0; i < n; i += st) {
     float acc = d ? d[i] * t[i] : 0.f;
     for (int32_t k = rp[i]; k < rp[i + 1]; ++k) acc = fmaf(w[k], x[cols[k]], acc);
@@ -667,8 +669,8 @@ __device__ __forceinline__ void vc_spmv(int i0, int st, int n, const int32_t* __
 // y = add + M x
 __device__ __forceinline__ void vc_spmv_add(int i0, int st, int n, const int32_t* __restrict__ rp,
                                             const int32_t* __restrict__ cols, const float* __restrict__ w,
-                                            const float* __restrict__ x, const float* __restrict__ add,
-                                            float* __restrict__ y) {
+                                            const float* x, const float* add,
+                                            float* y) {
   for (int i = i0; i < n; i += st) {
     float acc = add[i];
     for (int32_t k = rp[i]; k < rp[i + 1]; ++k) acc = fmaf(w[k], x[cols[k]], acc);
@@ -679,8 +681,8 @@ __device__ __forceinline__ void vc_spmv_add(int i0, int st, int n, const int32_t
 // u = r - A x2 ; y = x2 + d .* u   (post-smoothing; u kept for the backward when non-null)
 __device__ __forceinline__ void vc_post(int i0, int st, int n, const int32_t* __restrict__ rp,
                                         const int32_t* __restrict__ cols, const float* __restrict__ w,
-                                        const float* __restrict__ d, const float* __restrict__ r,
-                                        const float* __restrict__ x2, float* __restrict__ u, float* __restrict__ y) {
+                                        const float* __restrict__ d, const float* r,
+                                        const float* x2, float* u, float* y) {
   for (int i = i0; i < n; i += st) {
     float acc = r[i];
     for (int32_t k = rp[i]; k < rp[i + 1]; ++k) acc = fmaf(-w[k], x2[cols[k]], acc);
@@ -692,9 +694,9 @@ __device__ __forceinline__ void vc_post(int i0, int st, int n, const int32_t* __
 // adjoint of the pre-smoothing: x1b = x2b - A sb ; rb = d .* (g + x1b) + sb
 __device__ __forceinline__ void vc_pre_adjoint(int i0, int st, int n, const int32_t* __restrict__ rp,
                                                const int32_t* __restrict__ cols, const float* __restrict__ w,
-                                               const float* __restrict__ d, const float* __restrict__ g,
-                                               const float* __restrict__ x2b, const float* __restrict__ sb,
-                                               float* __restrict__ x1b, float* __restrict__ rb) {
+                                               const float* __restrict__ d, const float* g,
+                                               const float* x2b, const float* sb,
+                                               float* x1b, float* rb) {
   for (int i = i0; i < n; i += st) {
     float acc = x2b[i];
     for (int32_t k = rp[i]; k < rp[i + 1]; ++k) acc = fmaf(-w[k], sb[cols[k]], acc);
@@ -737,12 +739,20 @@ __global__ void k_vc_pre_adjoint(int n, const int32_t* __restrict__ rp, const in
 
 namespace afem {
 
-// The coarse end of the V-cycle in ONE block per vector: levels lo..L-1 are
-// small (<= kCoarseRows rows each), so their steps run back to back with
-// block barriers instead of one launch each.
+// The coarse end of the V-cycle in ONE cluster of blocks per vector: levels
+// lo..L-1 are small (<= kCoarseRows rows each), so their steps run back to
+// back with cluster barriers instead of one launch each.  Eight blocks of 512
+// threads: in one block of 1024 a step of the 1089-row level was two passes
+// of one SM (513^2, 289 rows solved exactly: 26 -> 22 us a cycle).
 constexpr int kCoarseRows = 2048;
 constexpr int kExactRows = 320;   // the first level below the finest of at most this many rows is solved exactly
-constexpr int kCoarseBlock = 1024;
+constexpr int kCoarseBlock = 512;
+constexpr int kCoarseCluster = 8;
+
+// What the cluster's threads wrote before is visible to all of them after.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 struct CoarseLevel {
   int n;
@@ -764,9 +774,9 @@ struct CoarsePlan {
 };
 
 // y = M x for a dense row-major n x n M, one warp per row
-__device__ __forceinline__ void dense_matvec(int n, const float* __restrict__ M, const float* __restrict__ x,
-                                             float* __restrict__ y) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+__device__ __forceinline__ void dense_matvec(int i0, int st, int n, const float* __restrict__ M, const float* x,
+                                             float* y) {
+  const int lane = threadIdx.x & 31, w = i0 >> 5, nw = st >> 5;
   for (int i = w; i < n; i += nw) {
     const float* row = M + (int64_t)i * n;
     float acc = 0.f;
@@ -779,12 +789,13 @@ __device__ __forceinline__ void dense_matvec(int n, const float* __restrict__ M,
 
 // forward: x_lo = V_lo(r_lo), keeping t, u (and the factored smoothers' L r,
 // L u) per level for the backward
-__global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse(CoarsePlan plan, const float* __restrict__ r_lo,
-                                                            float* __restrict__ x_lo) {
+__global__ void __cluster_dims__(kCoarseCluster, 1, 1) __launch_bounds__(kCoarseBlock)
+    k_vc_coarse(CoarsePlan plan, const float* r_lo, float* x_lo) {
   pdl_trigger();
   pdl_wait();
   const int64_t b = blockIdx.y;
-  const int lo = plan.lo, L = plan.L, i0 = threadIdx.x, st = blockDim.x;
+  const int lo = plan.lo, L = plan.L, i0 = blockIdx.x * blockDim.x + threadIdx.x,
+            st = kCoarseCluster * blockDim.x;
   for (int l = lo; l + 1 < L; ++l) {   // pre-smoothing residual, restriction
     const CoarseLevel& A = plan.lev[l];
     const CoarseLevel& C = plan.lev[l + 1];
@@ -793,16 +804,16 @@ __global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse(CoarsePlan plan, con
     float* s = A.vs + o;
     if (A.fact) {   // x1 = G r, s = r - A x1
       fact_lower(i0, st, A.f, r, A.wpre + o);
-      __syncthreads();
+      cluster_sync();
       fact_upper(i0, st, A.f, A.wpre + o, nullptr, nullptr, A.x1 + o);
-      __syncthreads();
+      cluster_sync();
       vc_res(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, r, A.x1 + o, s);
     } else {
       vc_smooth_res(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, A.d, r, s);
     }
-    __syncthreads();
+    cluster_sync();
     vc_spmv(i0, st, C.n, A.pt_rp, A.pt_cols, A.pt_w, s, nullptr, nullptr, C.t + b * C.n);
-    __syncthreads();
+    cluster_sync();
   }
   {
     const CoarseLevel& C = plan.lev[L - 1];
@@ -810,15 +821,15 @@ __global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse(CoarsePlan plan, con
     const float* r = (L - 1 == lo ? r_lo : C.t) + o;
     float* x = (L - 1 == lo ? x_lo : C.w) + o;
     if (plan.minv) {   // the exact level
-      dense_matvec(C.n, plan.minv, r, x);
+      dense_matvec(i0, st, C.n, plan.minv, r, x);
     } else if (C.fact) {
       fact_lower(i0, st, C.f, r, C.wpre + o);
-      __syncthreads();
+      cluster_sync();
       fact_upper(i0, st, C.f, C.wpre + o, nullptr, nullptr, x);
     } else {
       for (int i = i0; i < C.n; i += st) x[i] = C.d[i] * r[i];
     }
-    __syncthreads();
+    cluster_sync();
   }
   for (int l = L - 2; l >= lo; --l) {   // prolongation + x1, post-smoothing
     const CoarseLevel& A = plan.lev[l];
@@ -829,28 +840,29 @@ __global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse(CoarsePlan plan, con
     float* y = (l == lo ? x_lo : A.w) + o;
     if (A.fact) {   // x2 = x1 + P x_{l+1}; u = r - A x2; y = x2 + G u
       vc_spmv_add(i0, st, A.n, A.p_rp, A.p_cols, A.p_w, C.w + b * C.n, A.x1 + o, x2);
-      __syncthreads();
+      cluster_sync();
       vc_res(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, r, x2, A.u + o);
-      __syncthreads();
+      cluster_sync();
       fact_lower(i0, st, A.f, A.u + o, A.wpost + o);
-      __syncthreads();
+      cluster_sync();
       fact_upper(i0, st, A.f, A.wpost + o, nullptr, x2, y);
     } else {
       vc_spmv(i0, st, A.n, A.p_rp, A.p_cols, A.p_w, C.w + b * C.n, A.d, r, x2);
-      __syncthreads();
+      cluster_sync();
       vc_post(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, A.d, r, x2, A.u + o, y);
     }
-    __syncthreads();
+    cluster_sync();
   }
 }
 
 // backward: from the adjoint g_lo of x_lo, rb_lo (the adjoint of r_lo), and
 // per level g (the adjoint of the level's output) and x1b for the weights;
 // on factored levels also L g (gpost) and L x1b (gpre)
-__global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse_adjoint(CoarsePlan plan, const float* __restrict__ g_lo,
-                                                                    float* __restrict__ rb_lo) {
+__global__ void __cluster_dims__(kCoarseCluster, 1, 1) __launch_bounds__(kCoarseBlock)
+    k_vc_coarse_adjoint(CoarsePlan plan, const float* g_lo, float* rb_lo) {
   const int64_t b = blockIdx.y;
-  const int lo = plan.lo, L = plan.L, i0 = threadIdx.x, st = blockDim.x;
+  const int lo = plan.lo, L = plan.L, i0 = blockIdx.x * blockDim.x + threadIdx.x,
+            st = kCoarseCluster * blockDim.x;
   for (int l = lo; l + 1 < L; ++l) {   // adjoint of the post-smoothing, then of the prolongation
     const CoarseLevel& A = plan.lev[l];
     const CoarseLevel& C = plan.lev[l + 1];
@@ -859,16 +871,16 @@ __global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse_adjoint(CoarsePlan p
     float* x2b = A.x2 + o;
     if (A.fact) {   // x2b = g - A G g
       fact_lower(i0, st, A.f, g, A.gpost + o);
-      __syncthreads();
+      cluster_sync();
       fact_upper(i0, st, A.f, A.gpost + o, nullptr, nullptr, A.tmp + o);
-      __syncthreads();
+      cluster_sync();
       vc_res(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, g, A.tmp + o, x2b);
     } else {
       vc_smooth_res(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, A.d, g, x2b);
     }
-    __syncthreads();
+    cluster_sync();
     vc_spmv(i0, st, C.n, A.pt_rp, A.pt_cols, A.pt_w, x2b, nullptr, nullptr, C.g + b * C.n);
-    __syncthreads();
+    cluster_sync();
   }
   {
     const CoarseLevel& C = plan.lev[L - 1];
@@ -876,15 +888,15 @@ __global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse_adjoint(CoarsePlan p
     const float* g = (L - 1 == lo ? g_lo : C.g) + o;
     float* rb = (L - 1 == lo ? rb_lo : C.w) + o;
     if (plan.minv) {   // the exact level: rb = minv g (symmetric), no parameter
-      dense_matvec(C.n, plan.minv, g, rb);
+      dense_matvec(i0, st, C.n, plan.minv, g, rb);
     } else if (C.fact) {   // one use, out = G r: its adjoint terms as a pre-smoothing with x1b = g
       fact_lower(i0, st, C.f, g, C.gpre + o);
-      __syncthreads();
+      cluster_sync();
       fact_upper(i0, st, C.f, C.gpre + o, nullptr, nullptr, rb);
     } else {
       for (int i = i0; i < C.n; i += st) rb[i] = C.d[i] * g[i];
     }
-    __syncthreads();
+    cluster_sync();
   }
   for (int l = L - 2; l >= lo; --l) {   // adjoint of the restriction, then of the pre-smoothing
     const CoarseLevel& A = plan.lev[l];
@@ -894,18 +906,18 @@ __global__ void __launch_bounds__(kCoarseBlock) k_vc_coarse_adjoint(CoarsePlan p
     float* sb = A.vs + o;
     float* rb = (l == lo ? rb_lo : A.w) + o;
     vc_spmv(i0, st, A.n, A.p_rp, A.p_cols, A.p_w, C.w + b * C.n, nullptr, nullptr, sb);
-    __syncthreads();
+    cluster_sync();
     if (A.fact) {   // x1b = x2b - A sb ; rb = sb + G (g + x1b)
       vc_pre_adjoint(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, A.d, g, A.x2 + o, sb, A.x1b + o, nullptr);
-      __syncthreads();
+      cluster_sync();
       fact_lower(i0, st, A.f, A.x1b + o, A.gpre + o);
-      __syncthreads();
+      cluster_sync();
       if (rb_lo || l != lo) fact_upper(i0, st, A.f, A.gpost + o, A.gpre + o, sb, rb);
     } else {
       vc_pre_adjoint(i0, st, A.n, A.a_rp, A.a_cols, A.a_w, A.d, g, A.x2 + o, sb, A.x1b + o,
                      (l == lo && !rb_lo) ? nullptr : rb);
     }
-    __syncthreads();
+    cluster_sync();
   }
 }
 
@@ -1577,10 +1589,10 @@ static afem_status apply(afem_mpnn net, int batch, const float* r, float* z) {
   }
   float* x0 = z ? z : net->w[0];
   if (net->pdl) {
-    AFEM_TRY(launch_pdl(net->ctx, net->ctx->stream, k_vc_coarse, dim3(1, batch), kCoarseBlock, coarse_plan(net),
+    AFEM_TRY(launch_pdl(net->ctx, net->ctx->stream, k_vc_coarse, dim3(kCoarseCluster, batch), kCoarseBlock, coarse_plan(net),
                         lo == 0 ? r : (const float*)net->t[lo], lo == 0 ? x0 : net->w[lo]));
   } else {
-    k_vc_coarse<<<dim3(1, batch), kCoarseBlock, 0, net->ctx->stream>>>(coarse_plan(net), lo == 0 ? r : net->t[lo],
+    k_vc_coarse<<<dim3(kCoarseCluster, batch), kCoarseBlock, 0, net->ctx->stream>>>(coarse_plan(net), lo == 0 ? r : net->t[lo],
                                                                       lo == 0 ? x0 : net->w[lo]);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "k_vc_coarse", __FILE__, __LINE__);
@@ -1633,7 +1645,7 @@ static afem_status apply_adjoint(afem_mpnn net, int batch) {
     AFEM_TRY(sweep(net, &net->Pt[l], batch, net->x2[l], nullptr, nullptr, net->s[l + 1], net->n[l + 1]));
   }
   {
-    k_vc_coarse_adjoint<<<dim3(1, batch), kCoarseBlock, 0, ctx->stream>>>(coarse_plan(net), net->s[lo], net->w[lo]);
+    k_vc_coarse_adjoint<<<dim3(kCoarseCluster, batch), kCoarseBlock, 0, ctx->stream>>>(coarse_plan(net), net->s[lo], net->w[lo]);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "k_vc_coarse_adjoint", __FILE__, __LINE__);
     ++ctx->launches;

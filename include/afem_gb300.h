@@ -551,7 +551,7 @@ afem_status afem_mpnn_set_operator(afem_mpnn net, int n, const int32_t* row_ptr_
 /* z = M r for `batch` FP32 vectors stored one after the other. */
 afem_status afem_mpnn_forward(afem_mpnn net, int batch, const float* r_d, float* z_d);
 /* Levels of at most `rows` rows (default 2048) run their V-cycle steps in
- * one block per vector with block barriers; larger levels one grid-wide
+ * one cluster of blocks per vector with cluster barriers; larger levels one grid-wide
  * launch per step. */
 afem_status afem_mpnn_set_coarse_rows(afem_mpnn net, int rows);
 /* The level-l smoother weights d_l (level_rows[l] floats). */
