@@ -100,10 +100,23 @@ __global__ void k_scan_tile_sums(const int32_t* __restrict__ in, int64_t n, int3
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// Phase 3: scan inside each tile, offset by the scanned tile sum.
-__global__ void k_scan_tiles(const int32_t* __restrict__ in, int64_t n, const int32_t* __restrict__ offsets,
-                             int32_t* __restrict__ out, int write_total) {
+// Phase 3: scan inside each tile, offset by the scanned tile sum, or (raw) by
+// the sum of the tile sums before it, which the block adds itself: up to
+// kScanRaw tiles that is a microsecond, where a launch to scan them is four.
+constexpr int kScanRaw = 8192;
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t* __restrict__ in, int64_t n,
+                                                             const int32_t* __restrict__ offsets, int raw,
+                                                             int32_t* __restrict__ out, int write_total) {
   __shared__ int32_t sh[32];
+  int32_t before = 0;
+  if (raw) {
+    int32_t s = 0, total;
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += kScanThreads) s += offsets[t];
+    block_exclusive_scan(s, sh, &total);
+    before = total;
+  } else if (offsets) {
+    before = offsets[blockIdx.x];
+  }
   int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   int32_t v[kScanItems];
   int32_t s = 0;
@@ -113,7 +126,7 @@ __global__ void k_scan_tiles(const int32_t* __restrict__ in, int64_t n, const in
     s += v[i];
   }
   int32_t total;
-  int32_t pre = block_exclusive_scan(s, sh, &total) + (offsets ? offsets[blockIdx.x] : 0);
+  int32_t pre = block_exclusive_scan(s, sh, &total) + before;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i < n) out[base + i] = pre;
@@ -138,13 +151,15 @@ afem_status exclusive_scan_i32(afem_context ctx, const int32_t* in, int32_t* out
     return AFEM_OK;
   }
   int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  if (tiles == 1) return launch(ctx, k_scan_tiles, 1, kScanThreads, 0, in, n, (const int32_t*)nullptr, out, 1);
+  if (tiles == 1) return launch(ctx, k_scan_tiles, 1, kScanThreads, 0, in, n, (const int32_t*)nullptr, 0, out, 1);
   int32_t *sums, *offs;
   AFEM_TRY(scratch_take(ctx, (size_t)tiles + 1, &sums));
   AFEM_TRY(scratch_take(ctx, (size_t)tiles + 1, &offs));
   AFEM_TRY(launch(ctx, k_scan_tile_sums, (unsigned)tiles, kScanThreads, 0, in, n, sums));
+  if (tiles <= kScanRaw)
+    return launch(ctx, k_scan_tiles, (unsigned)tiles, kScanThreads, 0, in, n, (const int32_t*)sums, 1, out, 1);
   AFEM_TRY(exclusive_scan_i32(ctx, sums, offs, tiles));
-  return launch(ctx, k_scan_tiles, (unsigned)tiles, kScanThreads, 0, in, n, (const int32_t*)offs, out, 1);
+  return launch(ctx, k_scan_tiles, (unsigned)tiles, kScanThreads, 0, in, n, (const int32_t*)offs, 0, out, 1);
 }
 
 }  // namespace afem

@@ -37,18 +37,53 @@ namespace afem {
 // ---------------------------------------------------------------------------
 // node -> cell
 
+// The nodes of cell c (one or two 16-byte loads when cn is 16-byte aligned).
+template <int NPC>
+__device__ __forceinline__ void load_cell(const int32_t* __restrict__ cn, bool vec, int32_t c, int32_t (&v)[NPC]) {
+  const int32_t* cp = cn + (int64_t)c * NPC;
+  if constexpr (NPC == 4 || NPC == 8) {
+    if (vec) {
+#pragma unroll
+      for (int k = 0; k < NPC / 4; ++k) {
+        const int4 q = __ldg(reinterpret_cast<const int4*>(cp) + k);
+        v[4 * k] = q.x;
+        v[4 * k + 1] = q.y;
+        v[4 * k + 2] = q.z;
+        v[4 * k + 3] = q.w;
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NPC; ++j) v[j] = __ldg(cp + j);
+}
+
 // Histogram of incidences per node; each incidence keeps the count its
 // atomic returned (its rank among the node's incidences, in arbitrary order),
-// so that the scatter needs no second atomic.
-__global__ void k_nc_count(const int32_t* __restrict__ cn, int64_t total, int nb_node, int32_t* __restrict__ cnt,
+// so that the scatter needs no second atomic.  A thread takes a cell, its
+// atomics in flight together (a thread an incidence: 305 us at 128^3
+// tetrahedra, this 225).
+template <int NPC>
+__global__ void k_nc_count(const int32_t* __restrict__ cn, int nb_cell, int nb_node, int32_t* __restrict__ cnt,
                            int32_t* __restrict__ rank, int* __restrict__ err) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t n = cn[i];
-    if (n < 0 || n >= nb_node) {
-      atomicOr(err, 1);
-      continue;
+  const bool vec = (reinterpret_cast<uintptr_t>(cn) & 15) == 0;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell; c += (int64_t)gridDim.x * blockDim.x) {
+    int32_t n[NPC], r[NPC];
+    load_cell<NPC>(cn, vec, (int32_t)c, n);
+#pragma unroll
+    for (int j = 0; j < NPC; ++j) {
+      const bool in = (unsigned)n[j] < (unsigned)nb_node;
+      r[j] = in ? atomicAdd(&cnt[n[j]], 1) : 0;
+      if (!in) atomicOr(err, 1);
     }
-    rank[i] = atomicAdd(&cnt[n], 1);
+    if constexpr (NPC % 4 == 0) {   // rank is scratch, 256-byte aligned
+#pragma unroll
+      for (int k = 0; k < NPC / 4; ++k)
+        reinterpret_cast<int4*>(rank + c * NPC)[k] = make_int4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NPC; ++j) rank[c * NPC + j] = r[j];
+    }
   }
 }
 
@@ -275,27 +310,6 @@ __device__ __forceinline__ void defer_node(int n, int32_t* defer, int32_t* defer
   defer[atomicAdd(defer_count, 1)] = n;
 }
 
-// The nodes of cell c (one or two 16-byte loads when cn is 16-byte aligned).
-template <int NPC>
-__device__ __forceinline__ void load_cell(const int32_t* __restrict__ cn, bool vec, int32_t c, int32_t (&v)[NPC]) {
-  const int32_t* cp = cn + (int64_t)c * NPC;
-  if constexpr (NPC == 4 || NPC == 8) {
-    if (vec) {
-#pragma unroll
-      for (int k = 0; k < NPC / 4; ++k) {
-        const int4 q = __ldg(reinterpret_cast<const int4*>(cp) + k);
-        v[4 * k] = q.x;
-        v[4 * k + 1] = q.y;
-        v[4 * k + 2] = q.z;
-        v[4 * k + 3] = q.w;
-      }
-      return;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NPC; ++j) v[j] = __ldg(cp + j);
-}
-
 // The cells of incidences b, b + 1, ... < e in order: the nodes (and the
 // local index of the row's node) two incidences ahead, the cell ids three
 // ahead, so that a thread's dependent loads overlap its work on the earlier
@@ -383,18 +397,19 @@ __global__ void __launch_bounds__(kThreadBlock)
       b = __ldg(nc_ptr + n);
       e = __ldg(nc_ptr + n + 1);
     }
-    const bool light = n < nb_node && e - b <= TT::max_deg;   // the others are k_sparsity_rows_warp's
+    const bool light = n < nb_node && e - b <= TT::max_deg;
     const unsigned lights = __ballot_sync(0xffffffffu, light);
-    if (__popc(lights) < kThreadMinLanes) {
-      // too few light nodes to keep this warp's lanes busy (the boundary of a
-      // dense mesh): they go to the warp kernel's list
+    // to the warp kernel's list: the heavy nodes, and all of a warp with too
+    // few light ones to keep its lanes busy (the boundary of a dense mesh)
+    const bool pass = n < nb_node && (!light || __popc(lights) < kThreadMinLanes);
+    const unsigned passed = __ballot_sync(0xffffffffu, pass);
+    if (passed) {
       int base = 0;
-      if (lane == 0 && lights) base = atomicAdd(defer_count, __popc(lights));
+      if (lane == 0) base = atomicAdd(defer_count, __popc(passed));
       base = __shfl_sync(0xffffffffu, base, 0);
-      if (light) defer[base + __popc(lights & ((1u << lane) - 1u))] = n;
-      continue;
+      if (pass) defer[base + __popc(passed & ((1u << lane) - 1u))] = n;
     }
-    if (!light) continue;
+    if (pass || n >= nb_node) continue;
     int D = 0;   // distinct neighbours; above DMAX the row is deferred
     bool bad = false;
     {
@@ -517,10 +532,9 @@ __global__ void __launch_bounds__(kThreadBlock)
   }
 }
 
-// The nodes in more than `min_deg` cells (every node when -1, none when
-// INT_MAX), and the rows k_sparsity_thread or k_sparsity_rows_sub deferred
-// (more distinct neighbours than their tables hold), listed
-// in `list[0 .. *list_count)`: one warp per node, lanes over its incidences
+// The nodes k_sparsity_thread or k_sparsity_rows_sub passed on (in more cells,
+// or with more distinct neighbours, than they take), listed in
+// `list[0 .. *list_count)`: one warp per node, lanes over its incidences
 // (chunks of 32).  The row's own node is inserted into the warp's hash set
 // first, then every lane inserts the nodes of its cell: a node met again
 // (the row's own included) finds its slot, so the number of first insertions
@@ -535,8 +549,7 @@ __global__ void __launch_bounds__(kThreadBlock)
 // k_sparsity_thread.
 template <int NPC, bool FILL>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-    k_sparsity_rows_warp(int nb_node, int min_deg, const int32_t* __restrict__ list,
-                         const int32_t* __restrict__ list_count,
+    k_sparsity_rows_warp(int nb_node, const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
                          const int32_t* __restrict__ cn, const int32_t* __restrict__ nc_ptr,
                          const int32_t* __restrict__ nc_cell, const uint8_t* __restrict__ nc_local,
                          const int32_t* __restrict__ row_ptr, int self_last, int packed_slots,
@@ -555,13 +568,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const bool vec = (reinterpret_cast<uintptr_t>(cn) & 15) == 0;
-  const int direct = min_deg == INT_MAX ? 0 : nb_node;   // INT_MAX: the list alone
-  const int count = direct + *list_count;
+  const int count = *list_count;
   for (int it = wid; it < count; it += nwarps) {
-    const int n = it < direct ? it : __ldg(list + (it - direct));
+    const int n = __ldg(list + it);
     const int32_t b = __ldg(nc_ptr + n);
     const int deg = __ldg(nc_ptr + n + 1) - b;
-    if (it < direct && deg <= min_deg) continue;   // k_sparsity_thread's
     if (lane == 0) {
       const int h = tab_hash(n);
       t.key[h] = n;
@@ -1004,7 +1015,8 @@ afem_status afem_node_cell_build(afem_context ctx, int nb_node, int nb_cell, int
   AFEM_TRY(scratch_take(ctx, 1, &err));
   AFEM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nb_node + 1), ctx->stream));
   AFEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
-  AFEM_TRY(launch(ctx, k_nc_count, grid_for(ctx, total, 256), 256, 0, cell_nodes_d, total, nb_node, cnt, rank, err));
+  AFEM_TRY(launch(ctx, npc == 2 ? k_nc_count<2> : npc == 3 ? k_nc_count<3> : npc == 4 ? k_nc_count<4> : k_nc_count<8>,
+                  grid_for(ctx, nb_cell, 256), 256, 0, cell_nodes_d, nb_cell, nb_node, cnt, rank, err));
   AFEM_TRY(exclusive_scan_i32(ctx, cnt, nc_ptr_d, nb_node));
   AFEM_TRY(launch(ctx, k_nc_scatter, grid_for(ctx, total, 256), 256, 0, cell_nodes_d, total, npc, nb_node,
                   (const int32_t*)nc_ptr_d, (const int32_t*)rank, key));
@@ -1060,14 +1072,13 @@ static afem_status launch_rows(afem_context ctx, bool dense, int nb_node, const 
     AFEM_TRY(launch(ctx, k_sparsity_rows_sub<NPC, FILL, kSubLanes>, g1, kWarpsPerBlock * 32, 0, nb_node, cn, nc_ptr,
                     nc_cell, nc_local, row_ptr, self_last, packed, row_len, cols, slot, defer, defer_count, err));
   }
-  // the rows the thread or sub-warp kernel passed on (and, after the thread
-  // kernel, the heavy ones): the grid covers the worst case and each warp
-  // reads the list's length on the device
+  // the rows the thread or sub-warp kernel passed on: the grid covers the
+  // worst case and each warp reads the list's length on the device
   const unsigned g2 = (unsigned)std::min<int64_t>((nb_node + kWarpsPerBlock - 1) / kWarpsPerBlock,
                                                   (int64_t)ctx->sm_count * per_sm_warp);
   return launch(ctx, k_sparsity_rows_warp<NPC, FILL>, g2, kWarpsPerBlock * 32, 0, nb_node,
-                dense ? INT_MAX : ThreadTable<NPC>::max_deg, (const int32_t*)defer, (const int32_t*)defer_count, cn,
-                nc_ptr, nc_cell, nc_local, row_ptr, self_last, packed, row_len, cols, slot, err);
+                (const int32_t*)defer, (const int32_t*)defer_count, cn, nc_ptr, nc_cell, nc_local, row_ptr, self_last,
+                packed, row_len, cols, slot, err);
 }
 
 static afem_status launch_sparsity_rows(afem_context ctx, bool fill, int nb_node, int npc, int64_t incidences,
