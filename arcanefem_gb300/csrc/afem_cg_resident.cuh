@@ -35,6 +35,7 @@ struct CgState {
 constexpr int kResThreads = 512;
 constexpr int kResMaxRows = 6;                 // rows a thread owns at most
 constexpr int kResSpins = 4000000;             // polls of a wait, about 2 s
+constexpr int kResCluster = 8;                 // blocks of a system small enough for one cluster
 constexpr int kSlotStride = 8;                  // slots of 16 B a cache line of its own apart
 constexpr size_t kResSmem = 226 * 1024;        // dynamic shared memory of a block
 
@@ -135,11 +136,33 @@ __device__ __forceinline__ double res_block_sum(const T (&v)[V], double* sh) {
 // a block can be one exchange ahead of another's polling, never two.  FENCE:
 // what the block's threads wrote before is visible to every block afterwards
 // (a release before the put, an acquire after the polls).
+// CL: the grid is one cluster.  A block then writes its slot into every
+// block's shared memory and the cluster's barrier stands for the polls and
+// the fences (an exchange through L2 takes 1400 to 2500 cycles among 5 blocks;
+// res_plan has the solves' times).  That barrier needs no bound: every block
+// takes the same branches, decided from the same totals.
+template <bool CL>
 struct Grid {
-  ulonglong2* slots;          // [2 parities][2 values][gridDim.x] lines, zero at the launch
+  ulonglong2* slots;          // [2 parities][2 values][gridDim.x] lines, zero at the launch; CL: shared, [2][2][8]
   double* sh;                 // shared, res_scratch(gridDim.x) doubles
   int* err;
   unsigned long long epoch = 0;
+
+  // CL: {lo, hi} as this block's slot of value w in every block of the cluster, lane i in block i
+  __device__ __forceinline__ void spread(int w, unsigned long long lo, unsigned long long hi) {
+    const unsigned lane = threadIdx.x & 31;
+    if (lane < gridDim.x) {
+      const unsigned at = (unsigned)__cvta_generic_to_shared(slots + ((epoch & 1) * 2 + w) * kResCluster + blockIdx.x);
+      asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\t"
+                   "st.shared::cluster.v2.u64 [a], {%2, %3};\n\t}"
+                   :: "r"(at), "r"(lane), "l"(lo), "l"(hi) : "memory");
+    }
+  }
+  __device__ __forceinline__ ulonglong2 spread_slot(int w, int i) const {
+    const volatile unsigned long long* q =
+        reinterpret_cast<const volatile unsigned long long*>(slots + ((epoch & 1) * 2 + w) * kResCluster + i);
+    return make_ulonglong2(q[0], q[1]);
+  }
 
   // Publish the values that threads 0 (and 32 for the second) of the block hold, poll everyone's into sh.
   // Returns false in every thread if a wait ran out.  Ends with a block barrier.
@@ -147,6 +170,14 @@ struct Grid {
   __device__ __forceinline__ bool meet(double v) {
     ++epoch;
     const int nb = gridDim.x;
+    if constexpr (CL) {   // every lane of warp j holds value j
+      const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      if (w < V) spread(w, __double_as_longlong(v), 0);
+      cluster_sync();
+      if (w < V && lane < nb) sh[w * nb + lane] = __longlong_as_double(spread_slot(w, lane).x);
+      __syncthreads();
+      return true;
+    }
     ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
     if (threadIdx.x < 32 * V && (threadIdx.x & 31) == 0)
       slot_put(at + ((threadIdx.x >> 5) * nb + blockIdx.x) * kSlotStride, __double_as_longlong(v), epoch);
@@ -161,6 +192,10 @@ struct Grid {
 
   // What the blocks wrote before is visible to all of them after.
   __device__ __forceinline__ bool barrier() {
+    if constexpr (CL) {
+      cluster_sync();
+      return true;
+    }
     ++epoch;
     const int nb = gridDim.x;
     ulonglong2* at = slots + (epoch & 1) * 2 * nb * kSlotStride;
@@ -216,24 +251,30 @@ struct Grid {
       int l[kLimbs];
 #pragma unroll
       for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, lane < W ? part[w * W + lane][k] : 0);
-      if (lane == 0) {
+      if (CL || lane == 0) {
         const __int128 t = from_limbs(l);
         // the high word's lowest value stands for a block that cannot take part
         const unsigned hi = ok ? (unsigned)(t >> 64) : 0x80000000u;
-        if constexpr (FENCE) __threadfence();
-        slot_put(at + (w * nb + blockIdx.x) * kSlotStride, (unsigned long long)t,
-                 (unsigned long long)hi << 32 | (unsigned)epoch);
+        const unsigned long long word = (unsigned long long)hi << 32 | (unsigned)epoch;
+        if constexpr (CL) {
+          spread(w, (unsigned long long)t, word);
+        } else {
+          if constexpr (FENCE) __threadfence();
+          slot_put(at + (w * nb + blockIdx.x) * kSlotStride, (unsigned long long)t, word);
+        }
       }
     }
-    __syncthreads();   // part is read
+    if constexpr (CL) cluster_sync();
+    else __syncthreads();   // part is read
     int bad = 0;
-    {
+    if (!CL || w % P == 0) {
       const int j = w / P;
       int l[kLimbs + 1] = {};
       l[kLimbs] = 1;
       for (int i = (w - j * P) * 32 + lane; i < nb; i += P * 32) {
         ulonglong2 got;
-        if (!poll(at + (j * nb + i) * kSlotStride, &got)) bad = 1;
+        if constexpr (CL) got = spread_slot(j, i);
+        else if (!poll(at + (j * nb + i) * kSlotStride, &got)) bad = 1;
         const int hi = (int)(got.y >> 32);
         constexpr int mask = (1 << kLimbBits) - 1;
         if ((unsigned)hi == 0x80000000u) l[kLimbs] = 0;
@@ -243,7 +284,7 @@ struct Grid {
         l[3] += (hi >> 2) & mask;
         l[4] += hi >> 24;
       }
-      if constexpr (FENCE)
+      if constexpr (FENCE && !CL)
         if ((w - j * P) * 32 < nb) __threadfence();   // the pollers acquire for the block
 #pragma unroll
       for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, l[k]);
@@ -253,11 +294,13 @@ struct Grid {
         for (int k = 0; k <= kLimbs; ++k) part[w][k] = l[k];
     }
     if (__syncthreads_or(bad)) return false;
+    constexpr int kParts = CL ? 1 : P;   // warps that took slots of a value
     if (w < V) {
       int l[kLimbs];
 #pragma unroll
-      for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, lane < P ? part[w * P + lane][k] : 0);
-      ok = __all_sync(0xffffffffu, lane < P ? part[w * P + lane][kLimbs] : 1);
+      for (int k = 0; k < kLimbs; ++k)
+        l[k] = __reduce_add_sync(0xffffffffu, lane < kParts ? part[w * P + lane][k] : 0);
+      ok = __all_sync(0xffffffffu, lane < kParts ? part[w * P + lane][kLimbs] : 1);
       const int e0 = V == 1 || w == 0 ? E[0] : E[V - 1];
       const double t = ok ? fixed_to_double(from_limbs(l), e0) : 0.0;
       if (lane == 0) {
@@ -407,15 +450,17 @@ struct CgResident {
   CgState* st;
 };
 
-template <int K>
+template <int K, bool CL>
 __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ ResCtl ctl;
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
   if (((volatile CgState*)a.st)->done) return;
   const int nb = gridDim.x, lane = threadIdx.x & 31;
-  Grid grid;
-  grid.slots = a.slots;
+  __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster : 1];
+  if constexpr (CL) cluster_sync();   // every block runs before one writes into another
+  Grid<CL> grid;
+  grid.slots = CL ? cluster_slots : a.slots;
   grid.sh = reinterpret_cast<double*>(dyn);
   grid.err = a.err;
   ResMatrix<double> mat;
@@ -636,15 +681,17 @@ struct CgfResident {
   CgState* st;
 };
 
-template <int K, bool B3>
+template <int K, bool B3, bool CL>
 __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfResident a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ ResCtl ctl;
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
   if (((volatile CgState*)a.st)->done) return;
   const int nb = gridDim.x, lane = threadIdx.x & 31;
-  Grid grid;
-  grid.slots = a.slots;
+  __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster : 1];
+  if constexpr (CL) cluster_sync();   // every block runs before one writes into another
+  Grid<CL> grid;
+  grid.slots = CL ? cluster_slots : a.slots;
   grid.sh = reinterpret_cast<double*>(dyn);
   grid.err = a.err;
   std::conditional_t<B3, ResMatrix3, ResMatrix<float>> mat;
@@ -791,6 +838,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfReside
 struct ResPlan {
   unsigned grid = 0;
   int rows_pb = 0, K = 0, steps = 0;
+  bool cluster = false;  // one cluster of blocks
   bool fits = false;     // every slice is likely to fit the shared memory
   bool take = false;     // this form rather than the launches per iteration
 };
@@ -811,13 +859,28 @@ struct ResPlan {
 constexpr int64_t kResScatterEntries = 3300000;
 constexpr int64_t kResStreamBytes = 80ll << 20;
 
+constexpr int kResClusterUnits = 384;
+constexpr int64_t kResClusterBytes = 1200 << 10;
+
 inline ResPlan res_plan(afem_context ctx, int rows, int C, int64_t nnz, size_t step_bytes) {
   ResPlan p;
-  const int64_t want = std::min<int64_t>(ctx->sm_count, ((int64_t)rows * C + 127) / 128);
-  const int64_t pb = (rows + want - 1) / want;
-  p.rows_pb = (int)((pb + 31) / 32 * 32);
-  p.grid = (unsigned)((rows + p.rows_pb - 1) / p.rows_pb);
-  p.K = (int)(((int64_t)C * p.rows_pb + kResThreads - 1) / kResThreads);
+  auto split = [&](int64_t blocks) {
+    const int64_t pb = (rows + blocks - 1) / blocks;
+    p.rows_pb = (int)((pb + 31) / 32 * 32);
+    p.grid = (unsigned)((rows + p.rows_pb - 1) / p.rows_pb);
+    p.K = (int)(((int64_t)C * p.rows_pb + kResThreads - 1) / kResThreads);
+  };
+  // One cluster up to 384 rows a block and two thirds of its shared memory.  Eight blocks hold fewer rows at once
+  // than the grid of 128 a block, but meet sooner (Grid): whole solves in FP64 1.36 -> 1.16 ms at 45^2 triangles,
+  // 0.57 -> 0.52 at 12^3 tetrahedra, 2.10 -> 1.93 at 8^3 with three unknowns a node (1.0 MB of matrix); but
+  // 2.35 -> 2.37 at 9^3 (1.4 MB), and with 512 rows a block 0.67 -> 0.69 at 15^3, 2.53 -> 3.07 at 10^3 with three.
+  int64_t blocks = 1;
+  while (blocks < kResCluster && blocks * 64 < (int64_t)rows * C) blocks *= 2;
+  split(blocks);
+  p.cluster = (int64_t)C * p.rows_pb <= kResClusterUnits &&
+              nnz / (C * C) * (int64_t)(step_bytes / 32) <= kResClusterBytes;
+  if (p.cluster) p.grid = (unsigned)blocks;
+  else split(std::min<int64_t>(ctx->sm_count, ((int64_t)rows * C + 127) / 128));
   p.steps = (int)((kResSmem - sizeof(double) * res_scratch_doubles(p.grid)) / step_bytes);
   // rows of a slice differ in length and the last block may be short: one step in ten for the padding
   p.take = p.K <= kResMaxRows &&
@@ -877,8 +940,13 @@ afem_status launch_resident(afem_context ctx, void (*k)(const Args), const ResPl
   lc.dynamicSmemBytes = kResSmem;
   lc.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
+  if (p.cluster) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {p.grid, 1, 1};
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
   lc.attrs = attr;
   lc.numAttrs = 1;
   AFEM_CUDA(cudaLaunchKernelEx(&lc, k, a));

@@ -133,6 +133,11 @@ __device__ __forceinline__ double quotient(double a, double b) {
                                          i64fp::divisor(__double_as_longlong(b))));
 }
 
+// What the cluster's threads wrote before is visible to all of them after.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Exchanges between the blocks of a cooperative grid: one 16-byte access
 // carries a value's bits and the number of the exchange it belongs to, so that

@@ -749,10 +749,6 @@ constexpr int kExactRows = 320;   // the first level below the finest of at most
 constexpr int kCoarseBlock = 512;
 constexpr int kCoarseCluster = 8;
 
-// What the cluster's threads wrote before is visible to all of them after.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 struct CoarseLevel {
   int n;

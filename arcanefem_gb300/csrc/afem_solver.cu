@@ -689,8 +689,9 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
     const CgResident a{n,    plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, cols, vals, sliced.soff,
                        sliced.cols, sliced.vals, dv, skip, x, r, p, slots, err, st};
     AFEM_TRY(run_resident(ctx, st, err, &hs, [&]() {
+      if (plan.cluster) return launch_resident(ctx, k_cg_resident<1, true>, plan, a);
       return dispatch_rows(plan.K, [&](auto k) {
-        return launch_resident(ctx, k_cg_resident<decltype(k)::value>, plan, a);
+        return launch_resident(ctx, k_cg_resident<decltype(k)::value, false>, plan, a);
       });
     }));
     AFEM_CUDA(cudaMemcpyAsync(x_user, x, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -870,10 +871,13 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
                           sliced.soff, sliced.cols, sliced.vals, dinv32, skip, x32, r32, z32, p32, q32, slots, err,
                           inner};
       AFEM_TRY(run_resident(ctx, inner, err, &hi, [&]() {
+        if (plan.cluster)
+          return b3 ? launch_resident(ctx, k_cgf_resident<1, true, true>, plan, a)
+                    : launch_resident(ctx, k_cgf_resident<1, false, true>, plan, a);
         return dispatch_rows(plan.K, [&](auto k) {
           constexpr int K = decltype(k)::value;
-          return b3 ? launch_resident(ctx, k_cgf_resident<K, true>, plan, a)
-                    : launch_resident(ctx, k_cgf_resident<K, false>, plan, a);
+          return b3 ? launch_resident(ctx, k_cgf_resident<K, true, false>, plan, a)
+                    : launch_resident(ctx, k_cgf_resident<K, false, false>, plan, a);
         });
       }));
     } else for (;;) {

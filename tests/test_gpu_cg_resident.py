@@ -74,9 +74,10 @@ def dev(A):
             torch.as_tensor(A.indices.astype(np.int32), device="cuda"), torch.as_tensor(A.data, device="cuda"))
 
 
-@pytest.mark.parametrize("n,longest", [(1, 7), (2, 7), (31, 7), (33, 7), (129, 7), (5000, 7), (FULL, 7),
+@pytest.mark.parametrize("n,longest", [(1, 7), (2, 7), (31, 7), (33, 7), (129, 7), (257, 7), (3072, 7), (3073, 7),
+                                       (5000, 7), (FULL, 7),
                                        (FULL + 1, 7), (2 * FULL + 33, 7), (4 * FULL + 1, 7), (6 * FULL, 7),
-                                       (6 * FULL + 1, 7), (20000, 200), (300001, 120)])
+                                       (6 * FULL + 1, 7), (3000, 300), (20000, 200), (300001, 120)])
 def test_iterates_match_numpy(cuda_ctx, n, longest):
     A = matrix(n, min(longest, n), seed=n % 97)
     b = np.random.default_rng(n).standard_normal(n)
@@ -93,7 +94,7 @@ def test_iterates_match_numpy(cuda_ctx, n, longest):
     assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
 
 
-@pytest.mark.parametrize("n,longest", [(33, 7), (5000, 7), (FULL + 1, 7), (6 * FULL, 7), (300001, 120)])
+@pytest.mark.parametrize("n,longest", [(33, 7), (3000, 300), (5000, 7), (FULL + 1, 7), (6 * FULL, 7), (300001, 120)])
 def test_mixed_reaches_its_tolerance(cuda_ctx, n, longest):
     A = matrix(n, longest, seed=3)
     b = np.random.default_rng(n).standard_normal(n)
@@ -103,7 +104,7 @@ def test_mixed_reaches_its_tolerance(cuda_ctx, n, longest):
     assert np.linalg.norm(b - A @ x.cpu().numpy()) <= 1.01e-11 * np.linalg.norm(b)
 
 
-@pytest.mark.parametrize("nb", [1, 11, 1700, FULL // 3 + 1, 60000])
+@pytest.mark.parametrize("nb", [1, 11, 160, 1024, 1025, 1700, FULL // 3 + 1, 60000])
 def test_mixed_blocks_reach_their_tolerance(cuda_ctx, nb):
     A = block_matrix(nb)
     n = 3 * nb
