@@ -717,6 +717,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 // rounds, ranks and slot bytes.  Nodes in more than 4 G cells, or with more
 // than 3/4 of a table's slots in distinct neighbours, go to
 // k_sparsity_rows_warp through the node list.  Errors as k_sparsity_thread.
+// Instruction issue binds it (72 % of the slots, the integer pipe 62 %): a
+// cell's nodes are turned once to the order of the rounds and a round without
+// a first insertion skips the list (128^3 tetrahedra 655 -> 570 us).
 constexpr int kSubLanes = 8;   // lanes per node of k_sparsity_rows_sub
 
 template <int G>
@@ -734,6 +737,27 @@ constexpr bool kKeepSlots = NPC <= 4;
 
 template <int TS, int BITS>
 __device__ __forceinline__ int sub_hash(int32_t v) { return (int)(((uint32_t)v * 2654435761u) >> (32 - BITS)); }
+
+// v turned so that w[r] is the cell node r + 1 places after the local index li, w[NPC - 1] the one at li.
+template <int NPC>
+__device__ __forceinline__ void turn_after(const int32_t (&v)[NPC], int li, int32_t (&w)[NPC]) {
+  if constexpr ((NPC & (NPC - 1)) == 0) {
+    int32_t t[NPC];
+#pragma unroll
+    for (int r = 0; r < NPC; ++r) w[r] = v[(r + 1) % NPC];
+#pragma unroll
+    for (int k = 1; k < NPC; k <<= 1) {   // by one bit of li at a time
+      const bool on = li & k;
+#pragma unroll
+      for (int r = 0; r < NPC; ++r) t[r] = on ? w[(r + k) % NPC] : w[r];
+#pragma unroll
+      for (int r = 0; r < NPC; ++r) w[r] = t[r];
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < NPC; ++r) w[r] = pick<NPC>(v, li + 1 + r >= NPC ? li + 1 + r - NPC : li + 1 + r);
+  }
+}
 
 template <int NPC, bool FILL, int G>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
@@ -793,40 +817,43 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       const int kb = c * G;
       if (kb >= maxdeg) break;
       const bool act = mine && kb + gl < deg;
-      int32_t v[NPC];
+      int32_t v[NPC], x[NPC];
       int li = 0;
       if (act) {
         load_cell<NPC>(cn, vec, __ldg(nc_cell + b + kb + gl), v);
-        if (FILL && nc_local) {
-          li = __ldg(nc_local + b + kb + gl);
-        } else if (FILL) {
-          li = local_index<NPC>(v, n, err);
-        } else {
+        // the local index, that of n's first occurrence
 #pragma unroll
-          for (int j = NPC - 1; j > 0; --j)
-            if (v[j] == n) li = j;
+        for (int j = NPC - 1; j > 0; --j)
+          if (v[j] == n) li = j;
+        if (v[0] == n) li = 0;
+        if (FILL && nc_local) li = __ldg(nc_local + b + kb + gl);
+        uint32_t top = 0;
+#pragma unroll
+        for (int j = 0; j < NPC; ++j) top = max(top, (uint32_t)v[j]);
+        bad |= top >= (uint32_t)nb_node;
+        turn_after<NPC>(v, li, x);
+        if (FILL && !nc_local) {   // as local_index
+          bool odd = x[NPC - 1] != n;
+#pragma unroll
+          for (int r = 0; r + 1 < NPC; ++r) odd |= x[r] == n;
+          if (odd) atomicOr(err, 16);
         }
-#pragma unroll
-        for (int j = 0; j < NPC; ++j) bad |= (unsigned)v[j] >= (unsigned)nb_node;
       }
 #pragma unroll
       for (int r = 0; r + 1 < NPC; ++r) {
-        int j = li + 1 + r;
-        j -= j >= NPC ? NPC : 0;
         bool fresh = false;
         int h = 0;
         if (act) {
-          const int32_t x = pick<NPC>(v, j);
-          h = sub_hash<TS, BITS>(x);
-          const int32_t old = atomicCAS(key + h, -1, x);
+          h = sub_hash<TS, BITS>(x[r]);
+          const int32_t old = atomicCAS(key + h, -1, x[r]);
           fresh = old == -1;
-          if (!fresh && old != x) {
+          if (!fresh && old != x[r]) {
             h = -1;
 #pragma unroll 1
             for (int p = 1; p < TS; ++p) {
-              const int hp = (sub_hash<TS, BITS>(x) + p) & (TS - 1);
-              const int32_t o = atomicCAS(key + hp, -1, x);
-              if (o == -1 || o == x) {
+              const int hp = (sub_hash<TS, BITS>(x[r]) + p) & (TS - 1);
+              const int32_t o = atomicCAS(key + hp, -1, x[r]);
+              if (o == -1 || o == x[r]) {
                 fresh = o == -1;
                 h = hp;
                 break;
@@ -836,16 +863,18 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
           }
         }
         const unsigned fb = __ballot_sync(0xffffffffu, fresh);
-        if (fresh) {
-          const int a = D + __popc(fb & gbelow);
-          if (a < DMAX) {
-            at[a] = (int16_t)h;
-            if (FILL) val[a] = pick<NPC>(v, j);
-          } else {
-            full = true;
+        if (fb) {
+          if (fresh) {
+            const int a = D + __popc(fb & gbelow);
+            if (a < DMAX) {
+              at[a] = (int16_t)h;
+              if (FILL) val[a] = x[r];
+            } else {
+              full = true;
+            }
           }
+          D += __popc(fb & gmask);
         }
-        D += __popc(fb & gmask);
         if (kKeepSlots<NPC>) kept[c] |= (uint32_t)(h & 0xff) << (8 * r);
       }
       if (kKeepSlots<NPC>) kept[c] |= (uint32_t)li << 24;
@@ -910,13 +939,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         using Word = typename std::conditional<(NPC > 4), uint64_t, uint32_t>::type;
         Word word = (Word)pn;
         if constexpr (kKeepSlots<NPC>) {
+          // the positions in the order of the rounds, those past the last local index (the last li) then first
           const int li = (int)(kept[c] >> 24);
+          uint32_t turned = 0;
 #pragma unroll
-          for (int r = 0; r + 1 < NPC; ++r) {
-            int j = li + 1 + r;
-            j -= j >= NPC ? NPC : 0;
-            word |= (Word)pos[(kept[c] >> (8 * r)) & 0xffu] << (8 * (j < li ? j + 1 : j));
-          }
+          for (int r = 0; r + 1 < NPC; ++r) turned |= (uint32_t)pos[(kept[c] >> (8 * r)) & 0xffu] << (8 * r);
+          constexpr uint32_t kMask = (1u << (8 * (NPC - 1))) - 1;
+          turned = (turned << (8 * li) | turned >> (8 * (NPC - 1 - li))) & kMask;
+          word |= (Word)(turned << 8);
         } else {
           int32_t v[NPC];
           load_cell<NPC>(cn, vec, __ldg(nc_cell + b + kb + gl), v);
