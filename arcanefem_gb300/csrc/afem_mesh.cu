@@ -58,14 +58,17 @@ __device__ __forceinline__ void load_cell(const int32_t* __restrict__ cn, bool v
   for (int j = 0; j < NPC; ++j) v[j] = __ldg(cp + j);
 }
 
-// Histogram of incidences per node; each incidence keeps the count its
-// atomic returned (its rank among the node's incidences, in arbitrary order),
-// so that the scatter needs no second atomic.  A thread takes a cell, its
-// atomics in flight together (a thread an incidence: 305 us at 128^3
-// tetrahedra, this 225).
+// Incidences of each node counted and put in the node's bucket: `cap` keys
+// (cell << 3 | local; cells < 2^28 checked by the caller, local < 8) in the
+// order the atomics return.  The incidences of a node in more than cap cells
+// go to a list (k_nc_spill).  A thread takes a cell, its atomics in flight
+// together.  Scattered accesses to L2 bind it: an atomic and a 4-byte write
+// an incidence, against which counting first and writing each key to its
+// place after the scan also wrote and read a rank and read the nodes again.
 template <int NPC>
-__global__ void k_nc_count(const int32_t* __restrict__ cn, int nb_cell, int nb_node, int32_t* __restrict__ cnt,
-                           int32_t* __restrict__ rank, int* __restrict__ err) {
+__global__ void k_nc_bucket(const int32_t* __restrict__ cn, int nb_cell, int nb_node, int cap, int32_t* __restrict__ cnt,
+                            int32_t* __restrict__ bucket, int32_t* __restrict__ spill, int* __restrict__ spilled,
+                            int* __restrict__ err) {
   const bool vec = (reinterpret_cast<uintptr_t>(cn) & 15) == 0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nb_cell; c += (int64_t)gridDim.x * blockDim.x) {
     int32_t n[NPC], r[NPC];
@@ -73,30 +76,48 @@ __global__ void k_nc_count(const int32_t* __restrict__ cn, int nb_cell, int nb_n
 #pragma unroll
     for (int j = 0; j < NPC; ++j) {
       const bool in = (unsigned)n[j] < (unsigned)nb_node;
-      r[j] = in ? atomicAdd(&cnt[n[j]], 1) : 0;
+      r[j] = in ? atomicAdd(&cnt[n[j]], 1) : -1;
       if (!in) atomicOr(err, 1);
     }
-    if constexpr (NPC % 4 == 0) {   // rank is scratch, 256-byte aligned
 #pragma unroll
-      for (int k = 0; k < NPC / 4; ++k)
-        reinterpret_cast<int4*>(rank + c * NPC)[k] = make_int4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < NPC; ++j) rank[c * NPC + j] = r[j];
+    for (int j = 0; j < NPC; ++j) {
+      if (r[j] < 0) continue;
+      if (r[j] < cap) {
+        bucket[(int64_t)n[j] * cap + r[j]] = ((int32_t)c << 3) | j;
+      } else {   // one atomic for the lanes that come here together
+        const unsigned here = __activemask();
+        const int lane = threadIdx.x & 31, first = __ffs(here) - 1;
+        int at = 0;
+        if (lane == first) at = atomicAdd(spilled, __popc(here));
+        at = __shfl_sync(here, at, first) + __popc(here & ((1u << lane) - 1u));
+        spill[at] = (int32_t)(c * NPC + j);
+      }
     }
   }
 }
 
-__global__ void k_nc_scatter(const int32_t* __restrict__ cn, int64_t total, int npc, int nb_node,
-                             const int32_t* __restrict__ nc_ptr, const int32_t* __restrict__ rank,
-                             int32_t* __restrict__ key) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t n = cn[i];
-    if (n < 0 || n >= nb_node) continue;
-    int32_t pos = nc_ptr[n] + rank[i];
-    int32_t cell = (int32_t)(i / npc);
-    int32_t local = (int32_t)(i - (int64_t)cell * npc);
-    key[pos] = (cell << 3) | local;  // cells < 2^28 checked by the caller; local < 8
+// The listed incidences' keys to the places past the bucket's in their node's
+// range of nc_cell.  cnt counts down from the node's incidences.
+__global__ void k_nc_spill(const int32_t* __restrict__ cn, int npc, const int32_t* __restrict__ spill,
+                           const int* __restrict__ spilled, const int32_t* __restrict__ nc_ptr,
+                           int32_t* __restrict__ cnt, int32_t* __restrict__ nc_cell) {
+  const int m = *spilled;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t i = spill[k], n = cn[i], cell = i / npc;
+    nc_cell[nc_ptr[n] + atomicSub(&cnt[n], 1) - 1] = (cell << 3) | (i - cell * npc);
+  }
+}
+
+// Ascending insertion sort in place
+__device__ __forceinline__ void insertion_sort(int32_t* key, int m) {
+  for (int i = 1; i < m; ++i) {
+    const int32_t v = key[i];
+    int j = i - 1;
+    while (j >= 0 && key[j] > v) {
+      key[j + 1] = key[j];
+      --j;
+    }
+    key[j + 1] = v;
   }
 }
 
@@ -121,20 +142,37 @@ __device__ __forceinline__ void bitonic_sort(uint32_t (&a)[M]) {
 }
 
 // Per-node sort of the (cell << 3 | local) keys, then split; the inverse map
-// records, for each (cell, local), its incidence index.  One thread per node
+// records, for each (cell, local), its incidence index.  The first `cap` keys
+// come from the node's bucket (cap a multiple of 8), others from its range of
+// nc_cell.  One thread per node
 // (meshes of at most 16 cells per node on average: triangles, hexahedra):
 // up to 32 keys are sorted by a bitonic network in registers; longer lists
 // (rare hubs) by an insertion sort in place.
-__global__ void k_nc_sort_thread(int nb_node, int npc, const int32_t* __restrict__ nc_ptr, int32_t* __restrict__ key,
-                          int32_t* __restrict__ nc_cell, uint8_t* __restrict__ nc_local,
-                          int32_t* __restrict__ nc_inverse) {
+__global__ void k_nc_sort_thread(int nb_node, int npc, int cap, const int32_t* __restrict__ nc_ptr,
+                          const int32_t* __restrict__ bucket, int32_t* __restrict__ nc_cell,
+                          uint8_t* __restrict__ nc_local, int32_t* __restrict__ nc_inverse) {
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nb_node; n += gridDim.x * blockDim.x) {
     const int32_t b = nc_ptr[n], e = nc_ptr[n + 1];
     const int deg = e - b;
+    const int32_t* own = bucket + (int64_t)n * cap;
     if (deg <= 32) {
       uint32_t a[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) a[i] = i < deg ? (uint32_t)key[b + i] : 0xffffffffu;
+      for (int i = 0; i < 32; i += 4) {
+        int4 q = make_int4(-1, -1, -1, -1);
+        if (i < deg && i < cap) {
+          q = __ldg(reinterpret_cast<const int4*>(own + i));
+        } else if (i < deg) {
+          q.x = nc_cell[b + i];
+          if (i + 1 < deg) q.y = nc_cell[b + i + 1];
+          if (i + 2 < deg) q.z = nc_cell[b + i + 2];
+          if (i + 3 < deg) q.w = nc_cell[b + i + 3];
+        }
+        a[i] = i < deg ? (uint32_t)q.x : 0xffffffffu;
+        a[i + 1] = i + 1 < deg ? (uint32_t)q.y : 0xffffffffu;
+        a[i + 2] = i + 2 < deg ? (uint32_t)q.z : 0xffffffffu;
+        a[i + 3] = i + 3 < deg ? (uint32_t)q.w : 0xffffffffu;
+      }
       bitonic_sort<32>(a);
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
@@ -146,17 +184,10 @@ __global__ void k_nc_sort_thread(int nb_node, int npc, const int32_t* __restrict
         }
       }
     } else {
-      for (int32_t i = b + 1; i < e; ++i) {
-        const int32_t v = key[i];
-        int32_t j = i - 1;
-        while (j >= b && key[j] > v) {
-          key[j + 1] = key[j];
-          --j;
-        }
-        key[j + 1] = v;
-      }
+      for (int i = 0; i < min(deg, cap); ++i) nc_cell[b + i] = own[i];
+      insertion_sort(nc_cell + b, deg);
       for (int32_t i = b; i < e; ++i) {
-        const int32_t v = key[i];
+        const int32_t v = nc_cell[i];
         nc_cell[i] = v >> 3;
         nc_local[i] = (uint8_t)(v & 7);
         if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = i;
@@ -171,9 +202,9 @@ constexpr int kWarpsPerBlock = 8;
 // average: its loads and stores stay coalesced over the node's list):
 // up to 32 keys are sorted by a bitonic network on registers (shuffles);
 // longer lists (rare) by an insertion sort in lane 0.
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_node, int npc,
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_node, int npc, int cap,
                                                                  const int32_t* __restrict__ nc_ptr,
-                                                                 int32_t* __restrict__ key,
+                                                                 const int32_t* __restrict__ bucket,
                                                                  int32_t* __restrict__ nc_cell,
                                                                  uint8_t* __restrict__ nc_local,
                                                                  int32_t* __restrict__ nc_inverse) {
@@ -183,8 +214,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_nod
   for (int n = wid; n < nb_node; n += nwarps) {
     const int32_t b = nc_ptr[n], e = nc_ptr[n + 1];
     const int deg = e - b;
+    const int32_t* own = bucket + (int64_t)n * cap;
+    // with the node's range, not after it: past the node's own keys it holds anything
+    int32_t v = lane < cap ? __ldg(own + lane) : INT_MAX;
     if (deg <= 32) {
-      int32_t v = lane < deg ? key[b + lane] : INT_MAX;
+      if (lane >= deg) v = INT_MAX;
+      else if (lane >= cap) v = nc_cell[b + lane];
 #pragma unroll
       for (int k = 2; k <= 32; k <<= 1) {
 #pragma unroll
@@ -194,21 +229,19 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_nod
           v = keep_min ? min(v, o) : max(v, o);
         }
       }
-      if (lane < deg) key[b + lane] = v;
-    } else if (lane == 0) {
-      for (int32_t i = b + 1; i < e; ++i) {
-        int32_t v = key[i];
-        int32_t j = i - 1;
-        while (j >= b && key[j] > v) {
-          key[j + 1] = key[j];
-          --j;
-        }
-        key[j + 1] = v;
+      if (lane < deg) {
+        nc_cell[b + lane] = v >> 3;
+        nc_local[b + lane] = (uint8_t)(v & 7);
+        if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = b + lane;
       }
+      continue;
     }
+    for (int i = lane; i < min(deg, cap); i += 32) nc_cell[b + i] = own[i];
+    __syncwarp();
+    if (lane == 0) insertion_sort(nc_cell + b, deg);
     __syncwarp();
     for (int32_t i = b + lane; i < e; i += 32) {
-      int32_t v = key[i];
+      v = nc_cell[i];
       nc_cell[i] = v >> 3;
       nc_local[i] = (uint8_t)(v & 7);
       if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = i;
@@ -1034,31 +1067,36 @@ afem_status afem_node_cell_build(afem_context ctx, int nb_node, int nb_cell, int
   AFEM_CHECK_ARG(cell_nodes_d && nc_ptr_d && nc_cell_d && nc_local_d, "afem_node_cell_build: null buffer");
   int64_t total = (int64_t)nb_cell * npc;
   AFEM_CHECK_ARG(total < INT_MAX, "afem_node_cell_build: too many incidences");
-  size_t need = align256(sizeof(int32_t) * ((size_t)nb_node + 1)) + 2 * align256(sizeof(int32_t) * total) + 256 +
-                scan_scratch_bytes(nb_node);
+  // keys of a bucket: half again the average, so that few nodes of a mesh spill, in whole sectors
+  const int cap = (int)(std::min<int64_t>(total * 3 / (2 * (int64_t)nb_node) + 8, 64) / 8 * 8);
+  const size_t nbucket = (size_t)cap * nb_node;
+  size_t need = align256(sizeof(int32_t) * ((size_t)nb_node + 1)) + align256(sizeof(int32_t) * nbucket) +
+                align256(sizeof(int32_t) * total) + 256 + scan_scratch_bytes(nb_node);
   AFEM_TRY(scratch_reserve(ctx, need));
-  int32_t *cnt, *rank, *key;
-  int* err;
+  int32_t *cnt, *bucket, *spill;
+  int* err;   // err[0] error bits, err[1] spilled incidences
   AFEM_TRY(scratch_take(ctx, (size_t)nb_node + 1, &cnt));
-  AFEM_TRY(scratch_take(ctx, (size_t)total, &rank));
-  AFEM_TRY(scratch_take(ctx, (size_t)total, &key));
-  AFEM_TRY(scratch_take(ctx, 1, &err));
+  AFEM_TRY(scratch_take(ctx, nbucket, &bucket));
+  AFEM_TRY(scratch_take(ctx, (size_t)total, &spill));
+  AFEM_TRY(scratch_take(ctx, 2, &err));
   AFEM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nb_node + 1), ctx->stream));
-  AFEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
-  AFEM_TRY(launch(ctx, npc == 2 ? k_nc_count<2> : npc == 3 ? k_nc_count<3> : npc == 4 ? k_nc_count<4> : k_nc_count<8>,
-                  grid_for(ctx, nb_cell, 256), 256, 0, cell_nodes_d, nb_cell, nb_node, cnt, rank, err));
+  AFEM_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(int), ctx->stream));
+  AFEM_TRY(launch(ctx,
+                  npc == 2 ? k_nc_bucket<2> : npc == 3 ? k_nc_bucket<3> : npc == 4 ? k_nc_bucket<4> : k_nc_bucket<8>,
+                  grid_for(ctx, nb_cell, 256), 256, 0, cell_nodes_d, nb_cell, nb_node, cap, cnt, bucket, spill, err + 1,
+                  err));
   AFEM_TRY(exclusive_scan_i32(ctx, cnt, nc_ptr_d, nb_node));
-  AFEM_TRY(launch(ctx, k_nc_scatter, grid_for(ctx, total, 256), 256, 0, cell_nodes_d, total, npc, nb_node,
-                  (const int32_t*)nc_ptr_d, (const int32_t*)rank, key));
+  AFEM_TRY(launch(ctx, k_nc_spill, grid_for(ctx, total, 256, 2), 256, 0, cell_nodes_d, npc, (const int32_t*)spill,
+                  (const int*)(err + 1), (const int32_t*)nc_ptr_d, cnt, nc_cell_d));
   // measured at 128^3 tetrahedra (24 cells per node): warp 0.37 ms, thread 0.77 ms (its per-thread
   // stores are uncoalesced); Hexa8 96^3 and triangles 1024^2: the thread sort is the faster
   if (total > (int64_t)16 * nb_node)
     AFEM_TRY(launch(ctx, k_nc_sort_warp, grid_for(ctx, (int64_t)nb_node * 32, kWarpsPerBlock * 32, 8),
-                    kWarpsPerBlock * 32, 0, nb_node, npc, (const int32_t*)nc_ptr_d, key, nc_cell_d, nc_local_d,
-                    nc_inverse_d));
+                    kWarpsPerBlock * 32, 0, nb_node, npc, cap, (const int32_t*)nc_ptr_d, (const int32_t*)bucket,
+                    nc_cell_d, nc_local_d, nc_inverse_d));
   else
-    AFEM_TRY(launch(ctx, k_nc_sort_thread, grid_for(ctx, nb_node, 128), 128, 0, nb_node, npc,
-                    (const int32_t*)nc_ptr_d, key, nc_cell_d, nc_local_d, nc_inverse_d));
+    AFEM_TRY(launch(ctx, k_nc_sort_thread, grid_for(ctx, nb_node, 128), 128, 0, nb_node, npc, cap,
+                    (const int32_t*)nc_ptr_d, (const int32_t*)bucket, nc_cell_d, nc_local_d, nc_inverse_d));
   int herr = 0;
   AFEM_TRY(read_scalar(ctx, err, &herr));
   if (herr) return fail(AFEM_ERR_MESH, "afem_node_cell_build: node id out of range [0, %d) in cell_nodes", nb_node);
