@@ -75,6 +75,7 @@ struct BatchParams {
   int max_inner, max_outer;
   long long spin_limit;
   int own_rows;         // rows of a CTA whose q and d fit its shared memory
+  int together;         // the other CTAs of a team go through its rows together
   int stall_cta;        // >= 0: that CTA leaves before its first barrier (failure-detection test)
 };
 
@@ -300,11 +301,18 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
   }
   __syncthreads();
   const int rank = blockIdx.x - I.cta0;
-  // a CTA's rows are consecutive: neighbours gathered by several of them come from its L1
+  // A CTA's rows are consecutive, so that neighbours gathered by several of them come from its L1 -- but small CTAs
+  // with more rows than their shared memory takes go through the team's rows together: as many fronts as CTAs, each
+  // far apart, miss L2.  64 instances (39800 rows an SM) with 8 CTAs of 128 an SM 547 -> 463 ms, 4 of 256 486 -> 467;
+  // 2 of 512 take 464 to 476 with consecutive rows and 481 to 488 together.  The step is a run-time value in every
+  // shape: as a constant of the 512-thread form it measured slower (12 instances, 8800 rows an SM 102 -> 107 ms).
   const int per = rows_per_cta(I.n, I.ncta);
-  const int row0 = min(I.n, rank * per) + (int)threadIdx.x, row1 = min(I.n, (rank + 1) * per);
   // q and d, which no other CTA reads, in shared memory if the CTA's rows fit
   const bool own = per <= prm.own_rows;
+  const bool together = prm.together && !own;
+  const int step = together ? I.ncta * BLOCK : BLOCK;
+  const int row0 = (together ? rank * BLOCK : min(I.n, rank * per)) + (int)threadIdx.x;
+  const int row1 = together ? I.n : min(I.n, (rank + 1) * per);
   float4* const own_q = own ? own_rows : I.q;
   float4* const own_d = own ? own_rows + prm.own_rows : I.d;
   const int off = own ? rank * per : 0;
@@ -320,7 +328,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
   };
 
   // ---- phase A: assembly
-  for (int row = row0; row < row1; row += BLOCK) assemble_row(I, row);
+  for (int row = row0; row < row1; row += step) assemble_row(I, row);
   if (!sync()) return;
 
   // ---- phase B: FP64 refinement around FP32 Jacobi CG, 4 right-hand sides
@@ -328,7 +336,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
   for (;; ++outer) {
     {
       double loc[2 * kBatchRhs] = {};
-      for (int row = row0; row < row1; row += BLOCK) {
+      for (int row = row0; row < row1; row += step) {
         double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
         for (int32_t k = I.rp[row]; k < I.rp[row + 1]; ++k) {
           const double a = I.vals[k];
@@ -386,7 +394,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
       float lrz[kBatchRhs] = {};
       const bool a0 = told_active(cast[0]), a1 = told_active(cast[1]), a2 = told_active(cast[2]),
                  a3 = told_active(cast[3]);
-      for (int row = row0; row < row1; row += BLOCK) {
+      for (int row = row0; row < row1; row += step) {
         const double* rr = I.r64 + (int64_t)row * kBatchRhs;
         const float di = I.dinv[row];
         const float4 rv = make_float4(a0 ? (float)rr[0] : 0.f, a1 ? (float)rr[1] : 0.f, a2 ? (float)rr[2] : 0.f,
@@ -421,7 +429,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
         const float z0 = told_active(cast[0]), z1 = told_active(cast[1]), z2 = told_active(cast[2]),
                     z3 = told_active(cast[3]);
         float lpq[kBatchRhs] = {};
-        for (int row = row0; row < row1; row += BLOCK) {
+        for (int row = row0; row < row1; row += step) {
           const int32_t rb = I.rp[row], e = I.rp[row + 1];
           const int len = e - rb;
           int32_t c[kRowUnroll];
@@ -480,7 +488,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
         const float al0 = told_value(cast[0]), al1 = told_value(cast[1]), al2 = told_value(cast[2]),
                     al3 = told_value(cast[3]);
         float lrr[2 * kBatchRhs] = {};
-        for (int row = row0; row < row1; row += BLOCK) {
+        for (int row = row0; row < row1; row += step) {
           const float4 pv = pnew[row], qv = own_q[row - off];
           float4 dv = own_d[row - off], rv = I.r[row];
           dv.x = fmaf(al0, pv.x, dv.x); dv.y = fmaf(al1, pv.y, dv.y);
@@ -518,7 +526,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch(const BatchInst* 
       if (!told_flag(cast[0])) break;
     }
     // x += d (FP64); the next residual reads neighbours' x
-    for (int row = row0; row < row1; row += BLOCK) {
+    for (int row = row0; row < row1; row += step) {
       const float4 dv = own_d[row - off];
       double* xr = I.x + (int64_t)row * kBatchRhs;
       xr[0] += (double)dv.x; xr[1] += (double)dv.y; xr[2] += (double)dv.z; xr[3] += (double)dv.w;
@@ -711,12 +719,13 @@ static BatchParams batch_params(const afem_solver_options& opt) {
 static bool same_params(const BatchParams& a, const BatchParams& c) {
   return a.rtol == c.rtol && a.atol == c.atol && a.inner_rtol == c.inner_rtol && a.max_inner == c.max_inner &&
          a.max_outer == c.max_outer && a.spin_limit == c.spin_limit && a.own_rows == c.own_rows &&
-         a.stall_cta == c.stall_cta;
+         a.together == c.together && a.stall_cta == c.stall_cta;
 }
 
 static afem_status batch_run(afem_batch b, BatchParams prm, bool use_graph, float* ms) {
   afem_context ctx = b->ctx;
   prm.own_rows = b->own_rows;
+  prm.together = b->cfg.block <= 256;
   if (use_graph && (!b->graph_valid || !same_params(prm, b->graph_prm))) {
     delete b->graph;
     b->graph = new (std::nothrow) GraphChunk();

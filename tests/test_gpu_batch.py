@@ -149,3 +149,31 @@ def test_barrier_wait_runs_out_and_context_survives(small_batch):
     assert status == 5   # AFEM_ERR_TIMEOUT
     res, _ = bt.solve(fem.solver_options(rtol=1e-8, inner_rtol=0.1, max_iter=20000))
     assert all(r.status == 0 for r in res)
+
+
+# more rows a CTA than its shared memory takes: small CTAs go through a team's rows together, large ones each through
+# their own; 310^2 and a ragged 307^2 beside a team of few rows.  A row's assembly does not depend on the CTA that
+# takes it: matrices and right-hand sides bit for bit as with one CTA an SM.
+@pytest.mark.parametrize("block,per_sm", [(128, 8), (256, 4), (512, 2)])
+def test_rows_beyond_shared_memory(block, per_sm):
+    ctx = fem.Context()
+    sizes = [310, 307, 310, 310, 310, 310, 310, 310, 310, 5]
+    bt = B.Batch(ctx, sizes, seed=4, jitter=0.2)
+    options = fem.solver_options(rtol=1e-8, inner_rtol=0.1, max_iter=20000)
+    bt.set_config(512, 1, 3.0)
+    bt.solve(options)
+    kept = [(f.values.clone(), b.clone()) for f, b in zip(bt.fmts, bt.rhs)]
+    for f, b in zip(bt.fmts, bt.rhs):
+        f.values.fill_(np.nan)
+        b.fill_(np.nan)
+    bt.set_config(block, per_sm, 3.0)
+    res, _ = bt.solve(options)
+    for i, (v, b) in enumerate(kept):
+        f = bt.fmts[i]
+        assert torch.equal(f.values, v) and torch.equal(bt.rhs[i], b), i
+        assert res[i].status == 0
+        rp, cols, vg, bg = (t.cpu().numpy() for t in (f.row_ptr, f.cols, v, b))
+        for j in range(4):
+            r = bg[:, j] - O.spmv(rp, cols, vg, bt.x[i].cpu().numpy()[:, j])
+            assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(bg[:, j])
+    bt.close()
