@@ -317,10 +317,10 @@ def kernel_names(name, mesh, formulation):
     if w["nb_dof"] == 3:
         return "k_elem_elasticity_tet + k_gather_elasticity"
     if w.get("cell") == "hex":
-        return "k_elem_poisson_hexa8 + k_gather_scalar<8>"
+        return f"k_elem_poisson_hexa8_{'minimal' if formulation == 'minimal' else 'ref'} + k_gather_scalar<8>"
     if formulation == "minimal":
         return f"k_elem_poisson_{'tet' if mesh.dim == 3 else 'tri'} + k_gather_scalar<{mesh.npc}>"
-    return f"k_elem_poisson_p1_ref<{mesh.npc}> + k_gather_scalar<{mesh.npc}>"
+    return f"k_elem_poisson_{'tet' if mesh.dim == 3 else 'tri'}_ref + k_gather_scalar<{mesh.npc}>"
 
 
 def measure_workload(args, name, n, ctx, rank, world, local, main):
