@@ -64,7 +64,8 @@ __device__ __forceinline__ void load_cell(const int32_t* __restrict__ cn, bool v
 // go to a list (k_nc_spill).  A thread takes a cell, its atomics in flight
 // together.  Scattered accesses to L2 bind it: an atomic and a 4-byte write
 // an incidence, against which counting first and writing each key to its
-// place after the scan also wrote and read a rank and read the nodes again.
+// place after the scan also wrote and read a rank and read the nodes again
+// (128^3 tetrahedra: 225 + 190 us, this 330 to 380, and the sort 366 -> 348).
 template <int NPC>
 __global__ void k_nc_bucket(const int32_t* __restrict__ cn, int nb_cell, int nb_node, int cap, int32_t* __restrict__ cnt,
                             int32_t* __restrict__ bucket, int32_t* __restrict__ spill, int* __restrict__ spilled,

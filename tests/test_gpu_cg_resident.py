@@ -94,6 +94,30 @@ def test_iterates_match_numpy(cuda_ctx, n, longest):
     assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
 
 
+# blocks that gather from few others, which the barrier alone waits for: none (a diagonal), the next ones, and a slow
+# block with long rows that its neighbours leave behind
+@pytest.mark.parametrize("n,width,heavy", [(5000, 0, 0), (FULL + 1, 1, 0), (2 * FULL + 33, 1, 40), (20000, 300, 0),
+                                           (20000, 1, 64)])
+def test_iterates_of_band_matrices_match_numpy(cuda_ctx, n, width, heavy):
+    rng = np.random.default_rng(n + width)
+    A = sp.diags([-rng.uniform(0.5, 1.0, n - width)], [width], shape=(n, n)) if width else sp.csr_matrix((n, n))
+    if heavy:
+        i, j = np.repeat(np.arange(heavy), 1500), np.tile(np.arange(heavy, heavy + 1500), heavy)
+        A = A + sp.coo_matrix((-rng.uniform(0.0, 0.01, i.size), (i, j)), shape=(n, n))
+    A = (A + A.T).tocsr()
+    A = (A + sp.diags(np.asarray(abs(A).sum(1)).ravel() + rng.uniform(1.0, 3.0, n))).tocsr()
+    A.sort_indices()
+    b = rng.standard_normal(n)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    try:
+        info = fem.cg_solve_csr(cuda_ctx, *dev(A), torch.as_tensor(b, device="cuda"), x,
+                                options=fem.solver_options(rtol=0.0, atol=1e-300, max_iter=10 if width or heavy else 1))
+    except fem.AfemError as e:
+        info = e.info
+    want = cg(A, b, info.iterations)
+    assert np.max(np.abs(x.cpu().numpy() - want)) <= 1e-12 * np.max(np.abs(want))
+
+
 @pytest.mark.parametrize("n,longest", [(33, 7), (3000, 300), (5000, 7), (FULL + 1, 7), (6 * FULL, 7), (300001, 120)])
 def test_mixed_reaches_its_tolerance(cuda_ctx, n, longest):
     A = matrix(n, longest, seed=3)
