@@ -33,6 +33,7 @@ struct CgState {
 };
 
 constexpr int kResThreads = 512;
+constexpr int kResWarps = kResThreads / 32;
 constexpr int kResMaxRows = 6;                 // rows a thread owns at most
 constexpr int kResSpins = 4000000;             // polls of a wait, about 2 s
 constexpr int kResCluster = 8;                 // blocks of a system small enough for one cluster
@@ -140,31 +141,34 @@ __device__ __forceinline__ double res_block_sum(const T (&v)[V], double* sh) {
 // three, so slots are kept apart for four.  FENCE:
 // what the block's threads wrote before is visible to every block afterwards
 // (a release before the put, an acquire after the polls).
-// CL: the grid is one cluster.  A block then writes its slot into every
-// block's shared memory and the cluster's barrier stands for the polls and
-// the fences (an exchange through L2 takes 1400 to 2500 cycles among 5 blocks;
-// res_plan has the solves' times).  That barrier needs no bound: every block
-// takes the same branches, decided from the same totals.
+// CL: the grid is one cluster.  Every warp then writes its sum into every
+// block's shared memory (by way of a block's sum 45^2 triangles took 1.17 ms,
+// now 1.09) and the cluster's barrier stands for the polls and the fences (an
+// exchange through L2 takes 1400 to 2500 cycles among 5 blocks; res_plan has
+// the solves' times).  That barrier needs no bound: every block takes the same
+// branches, decided from the same totals.
 template <bool CL>
 struct Grid {
-  ulonglong2* slots;          // [4 exchanges][2 values][gridDim.x] lines, zero at the launch; CL: shared, [2][2][8]
+  ulonglong2* slots;          // [4 exchanges][2 values][gridDim.x] lines, zero at the launch; CL: shared, [2][2][8][16]
   double* sh;                 // shared, res_scratch(gridDim.x) doubles
   int* err;
   unsigned long long epoch = 0;
 
-  // CL: {lo, hi} as this block's slot of value w in every block of the cluster, lane i in block i
-  __device__ __forceinline__ void spread(int w, unsigned long long lo, unsigned long long hi) {
+  // CL: {lo, hi} as the slot `sub` of value w of this block in every block of the cluster, lane i in block i
+  __device__ __forceinline__ void spread(int w, int sub, unsigned long long lo, unsigned long long hi) {
     const unsigned lane = threadIdx.x & 31;
     if (lane < gridDim.x) {
-      const unsigned at = (unsigned)__cvta_generic_to_shared(slots + ((epoch & 1) * 2 + w) * kResCluster + blockIdx.x);
+      const unsigned at = (unsigned)__cvta_generic_to_shared(
+          slots + (((epoch & 1) * 2 + w) * kResCluster + blockIdx.x) * kResWarps + sub);
       asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\t"
                    "st.shared::cluster.v2.u64 [a], {%2, %3};\n\t}"
                    :: "r"(at), "r"(lane), "l"(lo), "l"(hi) : "memory");
     }
   }
+  // slot i of value w, counted over the blocks' kResWarps each
   __device__ __forceinline__ ulonglong2 spread_slot(int w, int i) const {
-    const volatile unsigned long long* q =
-        reinterpret_cast<const volatile unsigned long long*>(slots + ((epoch & 1) * 2 + w) * kResCluster + i);
+    const volatile unsigned long long* q = reinterpret_cast<const volatile unsigned long long*>(
+        slots + ((epoch & 1) * 2 + w) * kResCluster * kResWarps + i);
     return make_ulonglong2(q[0], q[1]);
   }
 
@@ -176,9 +180,9 @@ struct Grid {
     const int nb = gridDim.x;
     if constexpr (CL) {   // every lane of warp j holds value j
       const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      if (w < V) spread(w, __double_as_longlong(v), 0);
+      if (w < V) spread(w, 0, __double_as_longlong(v), 0);
       cluster_sync();
-      if (w < V && lane < nb) sh[w * nb + lane] = __longlong_as_double(spread_slot(w, lane).x);
+      if (w < V && lane < nb) sh[w * nb + lane] = __longlong_as_double(spread_slot(w, lane * kResWarps).x);
       __syncthreads();
       return true;
     }
@@ -234,10 +238,25 @@ struct Grid {
   // wait ran out.  Ends with a block barrier.
   template <int V, bool FENCE, class T, class F>
   __device__ __forceinline__ bool sum(const T (&v)[V], const int (&E)[V], double* total, int* slow, F&& done) {
-    constexpr int W = kResThreads / 32, P = W / V;   // warps, warps that poll a sum's slots
+    constexpr int W = kResWarps, P = W / V;   // warps, warps that poll a sum's slots
     int (*part)[kLimbs + 1] = reinterpret_cast<int (*)[kLimbs + 1]>(sh);   // [V * W], the last word: taking part
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = gridDim.x;
     bool ok = true;
+    // a slot's words from limbs and back; the high word's lowest value stands for one that cannot take part
+    auto word = [&](const __int128 t) {
+      return (unsigned long long)(ok ? (unsigned)(t >> 64) : 0x80000000u) << 32 | (unsigned)epoch;
+    };
+    auto take = [](const ulonglong2 got, int (&l)[kLimbs], int& in) {
+      const int hi = (int)(got.y >> 32);
+      constexpr int mask = (1 << kLimbBits) - 1;
+      if ((unsigned)hi == 0x80000000u) in = 0;
+      l[0] += (int)got.x & mask;
+      l[1] += (int)(got.x >> 22) & mask;
+      l[2] += (int)((got.x >> 44) | ((unsigned long long)(unsigned)hi << 20)) & mask;
+      l[3] += (hi >> 2) & mask;
+      l[4] += hi >> 24;
+    };
+    if constexpr (CL) ++epoch;
 #pragma unroll
     for (int j = 0; j < V; ++j) {
       int l[kLimbs] = {};
@@ -246,66 +265,63 @@ struct Grid {
 #pragma unroll
       for (int k = 0; k < kLimbs; ++k) {
         l[k] = __reduce_add_sync(0xffffffffu, l[k]);
-        if (lane == 0) part[j * W + w][k] = l[k];
+        if (!CL && lane == 0) part[j * W + w][k] = l[k];
+      }
+      if constexpr (CL) {   // every warp's sum straight to all blocks
+        ok = __all_sync(0xffffffffu, ok);
+        const __int128 t = from_limbs(l);
+        spread(j, w, (unsigned long long)t, word(t));
       }
     }
-    ok = __syncthreads_and(ok);
-    ++epoch;
-    ulonglong2* at = slots + (epoch % kSlotBuffers) * 2 * nb * kSlotStride;
-    if (w < V) {
-      int l[kLimbs];
+    int bad = 0;
+    if constexpr (CL) {
+      cluster_sync();
+    } else {
+      ok = __syncthreads_and(ok);
+      ++epoch;
+      ulonglong2* at = slots + (epoch % kSlotBuffers) * 2 * nb * kSlotStride;
+      if (w < V) {
+        int l[kLimbs];
 #pragma unroll
-      for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, lane < W ? part[w * W + lane][k] : 0);
-      if (CL || lane == 0) {
-        const __int128 t = from_limbs(l);
-        // the high word's lowest value stands for a block that cannot take part
-        const unsigned hi = ok ? (unsigned)(t >> 64) : 0x80000000u;
-        const unsigned long long word = (unsigned long long)hi << 32 | (unsigned)epoch;
-        if constexpr (CL) {
-          spread(w, (unsigned long long)t, word);
-        } else {
+        for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, lane < W ? part[w * W + lane][k] : 0);
+        if (lane == 0) {
+          const __int128 t = from_limbs(l);
           if constexpr (FENCE) __threadfence();
-          slot_put(at + (w * nb + blockIdx.x) * kSlotStride, (unsigned long long)t, word);
+          slot_put(at + (w * nb + blockIdx.x) * kSlotStride, (unsigned long long)t, word(t));
         }
       }
-    }
-    if constexpr (CL) cluster_sync();
-    else __syncthreads();   // part is read
-    int bad = 0;
-    if (!CL || w % P == 0) {
+      __syncthreads();   // part is read
       const int j = w / P;
-      int l[kLimbs + 1] = {};
-      l[kLimbs] = 1;
+      int l[kLimbs] = {}, in = 1;
       for (int i = (w - j * P) * 32 + lane; i < nb; i += P * 32) {
         ulonglong2 got;
-        if constexpr (CL) got = spread_slot(j, i);
-        else if (!poll(at + (j * nb + i) * kSlotStride, &got)) bad = 1;
-        const int hi = (int)(got.y >> 32);
-        constexpr int mask = (1 << kLimbBits) - 1;
-        if ((unsigned)hi == 0x80000000u) l[kLimbs] = 0;
-        l[0] += (int)got.x & mask;
-        l[1] += (int)(got.x >> 22) & mask;
-        l[2] += (int)((got.x >> 44) | ((unsigned long long)(unsigned)hi << 20)) & mask;
-        l[3] += (hi >> 2) & mask;
-        l[4] += hi >> 24;
+        if (!poll(at + (j * nb + i) * kSlotStride, &got)) bad = 1;
+        take(got, l, in);
       }
-      if constexpr (FENCE && !CL)
+      if constexpr (FENCE)
         if ((w - j * P) * 32 < nb) __threadfence();   // the pollers acquire for the block
 #pragma unroll
       for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, l[k]);
-      l[kLimbs] = __all_sync(0xffffffffu, l[kLimbs]);
-      if (lane == 0)
+      in = __all_sync(0xffffffffu, in);
+      if (lane == 0) {
 #pragma unroll
-        for (int k = 0; k <= kLimbs; ++k) part[w][k] = l[k];
+        for (int k = 0; k < kLimbs; ++k) part[w][k] = l[k];
+        part[w][kLimbs] = in;
+      }
+      if (__syncthreads_or(bad)) return false;
     }
-    if (__syncthreads_or(bad)) return false;
-    constexpr int kParts = CL ? 1 : P;   // warps that took slots of a value
     if (w < V) {
-      int l[kLimbs];
+      int l[kLimbs] = {}, in = 1;
+      if constexpr (CL) {
+        for (int i = lane; i < nb * W; i += 32) take(spread_slot(w, i), l, in);
+      } else if (lane < P) {
 #pragma unroll
-      for (int k = 0; k < kLimbs; ++k)
-        l[k] = __reduce_add_sync(0xffffffffu, lane < kParts ? part[w * P + lane][k] : 0);
-      ok = __all_sync(0xffffffffu, lane < kParts ? part[w * P + lane][kLimbs] : 1);
+        for (int k = 0; k < kLimbs; ++k) l[k] = part[w * P + lane][k];
+        in = part[w * P + lane][kLimbs];
+      }
+#pragma unroll
+      for (int k = 0; k < kLimbs; ++k) l[k] = __reduce_add_sync(0xffffffffu, l[k]);
+      ok = __all_sync(0xffffffffu, in);
       const int e0 = V == 1 || w == 0 ? E[0] : E[V - 1];
       const double t = ok ? fixed_to_double(from_limbs(l), e0) : 0.0;
       if (lane == 0) {
@@ -462,7 +478,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
   if (((volatile CgState*)a.st)->done) return;
   const int nb = gridDim.x, lane = threadIdx.x & 31;
-  __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster : 1];
+  __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster * kResWarps : 1];
   if constexpr (CL) cluster_sync();   // every block runs before one writes into another
   Grid<CL> grid;
   grid.slots = CL ? cluster_slots : a.slots;
@@ -704,7 +720,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfReside
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
   if (((volatile CgState*)a.st)->done) return;
   const int nb = gridDim.x, lane = threadIdx.x & 31;
-  __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster : 1];
+  __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster * kResWarps : 1];
   if constexpr (CL) cluster_sync();   // every block runs before one writes into another
   Grid<CL> grid;
   grid.slots = CL ? cluster_slots : a.slots;
@@ -855,6 +871,8 @@ struct ResPlan {
   unsigned grid = 0;
   int rows_pb = 0, K = 0, steps = 0;
   bool cluster = false;  // one cluster of blocks
+  // dynamic shared memory: the cluster form's slots are static
+  size_t smem() const { return kResSmem - (cluster ? sizeof(ulonglong2) * 4 * kResCluster * kResWarps : 0); }
   bool fits = false;     // every slice is likely to fit the shared memory
   bool take = false;     // this form rather than the launches per iteration
 };
@@ -887,9 +905,10 @@ inline ResPlan res_plan(afem_context ctx, int rows, int C, int64_t nnz, size_t s
     p.K = (int)(((int64_t)C * p.rows_pb + kResThreads - 1) / kResThreads);
   };
   // One cluster up to 384 rows a block and two thirds of its shared memory.  Eight blocks hold fewer rows at once
-  // than the grid of 128 a block, but meet sooner (Grid): whole solves in FP64 1.36 -> 1.16 ms at 45^2 triangles,
-  // 0.57 -> 0.52 at 12^3 tetrahedra, 2.10 -> 1.93 at 8^3 with three unknowns a node (1.0 MB of matrix); but
-  // 2.35 -> 2.37 at 9^3 (1.4 MB), and with 512 rows a block 0.67 -> 0.69 at 15^3, 2.53 -> 3.07 at 10^3 with three.
+  // than the grid of 128 a block, but meet sooner (Grid): whole solves in FP64 1.36 -> 1.09 ms at 45^2 triangles,
+  // 0.60 -> 0.54 at 13^3 tetrahedra, 2.10 -> 1.84 at 8^3 with three unknowns a node (1.0 MB of matrix); but, with
+  // the sums still going by way of the blocks', 2.35 -> 2.37 at 9^3 (1.4 MB), and with 512 rows a block 0.67 -> 0.69
+  // at 15^3, 2.53 -> 3.07 at 10^3 with three.
   int64_t blocks = 1;
   while (blocks < kResCluster && blocks * 64 < (int64_t)rows * C) blocks *= 2;
   split(blocks);
@@ -897,7 +916,7 @@ inline ResPlan res_plan(afem_context ctx, int rows, int C, int64_t nnz, size_t s
               nnz / (C * C) * (int64_t)(step_bytes / 32) <= kResClusterBytes;
   if (p.cluster) p.grid = (unsigned)blocks;
   else split(std::min<int64_t>(std::min(ctx->sm_count, kResGrid), ((int64_t)rows * C + 127) / 128));
-  p.steps = (int)((kResSmem - sizeof(double) * res_scratch_doubles(p.grid)) / step_bytes);
+  p.steps = (int)((p.smem() - sizeof(double) * res_scratch_doubles(p.grid)) / step_bytes);
   // rows of a slice differ in length and the last block may be short: one step in ten for the padding
   p.take = p.K <= kResMaxRows &&
            (int64_t)(nnz / (C * C) * (step_bytes / 32)) - (int64_t)p.grid * (int64_t)kResSmem <= kResStreamBytes;
@@ -949,11 +968,11 @@ inline int res_launch_iters(int n, int64_t nnz) {
 template <class Args>
 afem_status launch_resident(afem_context ctx, void (*k)(const Args), const ResPlan& p, const Args& a) {
   AFEM_CUDA(cudaMemsetAsync(a.slots, 0, res_slots_bytes(p), ctx->stream));
-  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
+  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem()));
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(p.grid);
   lc.blockDim = dim3(kResThreads);
-  lc.dynamicSmemBytes = kResSmem;
+  lc.dynamicSmemBytes = p.smem();
   lc.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
   if (p.cluster) {
