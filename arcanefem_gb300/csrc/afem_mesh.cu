@@ -1071,17 +1071,15 @@ afem_status afem_node_cell_build(afem_context ctx, int nb_node, int nb_cell, int
   // keys of a bucket: half again the average, so that few nodes of a mesh spill, in whole sectors
   const int cap = (int)(std::min<int64_t>(total * 3 / (2 * (int64_t)nb_node) + 8, 64) / 8 * 8);
   const size_t nbucket = (size_t)cap * nb_node;
-  size_t need = align256(sizeof(int32_t) * ((size_t)nb_node + 1)) + align256(sizeof(int32_t) * nbucket) +
-                align256(sizeof(int32_t) * total) + 256 + scan_scratch_bytes(nb_node);
+  size_t need = align256(sizeof(int32_t) * ((size_t)nb_node + 3)) + align256(sizeof(int32_t) * nbucket) +
+                align256(sizeof(int32_t) * total) + scan_scratch_bytes(nb_node);
   AFEM_TRY(scratch_reserve(ctx, need));
   int32_t *cnt, *bucket, *spill;
-  int* err;   // err[0] error bits, err[1] spilled incidences
-  AFEM_TRY(scratch_take(ctx, (size_t)nb_node + 1, &cnt));
+  AFEM_TRY(scratch_take(ctx, (size_t)nb_node + 3, &cnt));
+  int* err = cnt + nb_node + 1;   // err[0] error bits, err[1] spilled incidences; zeroed with the counts
   AFEM_TRY(scratch_take(ctx, nbucket, &bucket));
   AFEM_TRY(scratch_take(ctx, (size_t)total, &spill));
-  AFEM_TRY(scratch_take(ctx, 2, &err));
-  AFEM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nb_node + 1), ctx->stream));
-  AFEM_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(int), ctx->stream));
+  AFEM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)nb_node + 3), ctx->stream));
   AFEM_TRY(launch(ctx,
                   npc == 2 ? k_nc_bucket<2> : npc == 3 ? k_nc_bucket<3> : npc == 4 ? k_nc_bucket<4> : k_nc_bucket<8>,
                   grid_for(ctx, nb_cell, 256), 256, 0, cell_nodes_d, nb_cell, nb_node, cap, cnt, bucket, spill, err + 1,
