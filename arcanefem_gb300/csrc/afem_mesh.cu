@@ -109,16 +109,40 @@ __global__ void k_nc_spill(const int32_t* __restrict__ cn, int npc, const int32_
   }
 }
 
-// Ascending insertion sort in place
-__device__ __forceinline__ void insertion_sort(int32_t* key, int m) {
-  for (int i = 1; i < m; ++i) {
-    const int32_t v = key[i];
-    int j = i - 1;
-    while (j >= 0 && key[j] > v) {
-      key[j + 1] = key[j];
-      --j;
+// Ascending sort of m keys in place by a warp: the bitonic network whose merges first compare mirrored places, so that
+// every comparison puts the smaller key first and places past m take no part.
+__device__ __forceinline__ void warp_sort(int32_t* key, unsigned m) {
+  const unsigned lane = threadIdx.x & 31;
+  for (unsigned half = 1; half < m; half <<= 1) {   // sorted runs of this many keys merge in pairs
+    for (unsigned j = half; j > 0; j >>= 1) {
+      for (unsigned t = lane; 2 * (t & ~(j - 1)) < m; t += 32) {
+        const unsigned at = t & (j - 1), i = 2 * t - at, l = j == half ? i + 2 * (half - at) - 1 : i + j;
+        if (l >= m) continue;
+        const int32_t x = key[i], y = key[l];
+        if (x > y) {
+          key[i] = y;
+          key[l] = x;
+        }
+      }
+      __syncwarp();
     }
-    key[j + 1] = v;
+  }
+}
+
+// The keys of a node in more than 32 cells, sorted and split by a warp in the node's range of nc_cell.  An insertion
+// sort by one thread is quadratic wherever the atomics' order of arrival is not the cells': a node in 3000 tetrahedra
+// took 93 ms (30 to 68 with the keys in that order), in 3000 triangles 97, and 0.4 so.
+__device__ __noinline__ void sort_long_list(const int32_t* own, int cap, int32_t b, int deg, int npc, int32_t* nc_cell,
+                                            uint8_t* nc_local, int32_t* nc_inverse) {
+  const int lane = threadIdx.x & 31;
+  for (int i = lane; i < min(deg, cap); i += 32) nc_cell[b + i] = own[i];
+  __syncwarp();
+  warp_sort(nc_cell + b, deg);
+  for (int i = lane; i < deg; i += 32) {
+    const int32_t v = nc_cell[b + i];
+    nc_cell[b + i] = v >> 3;
+    nc_local[b + i] = (uint8_t)(v & 7);
+    if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = b + i;
   }
 }
 
@@ -147,14 +171,17 @@ __device__ __forceinline__ void bitonic_sort(uint32_t (&a)[M]) {
 // come from the node's bucket (cap a multiple of 8), others from its range of
 // nc_cell.  One thread per node
 // (meshes of at most 16 cells per node on average: triangles, hexahedra):
-// up to 32 keys are sorted by a bitonic network in registers; longer lists
-// (rare hubs) by an insertion sort in place.
+// up to 32 keys are sorted by a bitonic network in registers; the longer lists
+// (rare hubs) of a warp's nodes one after the other by the whole warp.
 __global__ void k_nc_sort_thread(int nb_node, int npc, int cap, const int32_t* __restrict__ nc_ptr,
                           const int32_t* __restrict__ bucket, int32_t* __restrict__ nc_cell,
                           uint8_t* __restrict__ nc_local, int32_t* __restrict__ nc_inverse) {
-  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nb_node; n += gridDim.x * blockDim.x) {
-    const int32_t b = nc_ptr[n], e = nc_ptr[n + 1];
-    const int deg = e - b;
+  const int lane = threadIdx.x & 31;
+  for (int64_t n0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); n0 < nb_node;
+       n0 += (int64_t)gridDim.x * blockDim.x) {   // whole warps in every pass
+    const int n = (int)(n0 + lane < nb_node ? n0 + lane : n0);
+    const int32_t b = nc_ptr[n];
+    const int deg = n0 + lane < nb_node ? nc_ptr[n + 1] - b : 0;
     const int32_t* own = bucket + (int64_t)n * cap;
     if (deg <= 32) {
       uint32_t a[32];
@@ -184,15 +211,11 @@ __global__ void k_nc_sort_thread(int nb_node, int npc, int cap, const int32_t* _
           if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = b + i;
         }
       }
-    } else {
-      for (int i = 0; i < min(deg, cap); ++i) nc_cell[b + i] = own[i];
-      insertion_sort(nc_cell + b, deg);
-      for (int32_t i = b; i < e; ++i) {
-        const int32_t v = nc_cell[i];
-        nc_cell[i] = v >> 3;
-        nc_local[i] = (uint8_t)(v & 7);
-        if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = i;
-      }
+    }
+    for (unsigned lists = __ballot_sync(0xffffffffu, deg > 32); lists; lists &= lists - 1) {
+      const int src = __ffs(lists) - 1;
+      sort_long_list(bucket + (n0 + src) * cap, cap, __shfl_sync(0xffffffffu, b, src),
+                     __shfl_sync(0xffffffffu, deg, src), npc, nc_cell, nc_local, nc_inverse);
     }
   }
 }
@@ -202,8 +225,9 @@ constexpr int kWarpsPerBlock = 8;
 // The same with one warp per node (meshes of more than 16 cells per node on
 // average: its loads and stores stay coalesced over the node's list):
 // up to 32 keys are sorted by a bitonic network on registers (shuffles);
-// longer lists (rare) by an insertion sort in lane 0.
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_node, int npc, int cap,
+// longer lists (rare) in place (sort_long_list).  Eight blocks an SM: without
+// the bound the call costs 48 registers (128^3 tetrahedra 1.76 -> 1.85 ms).
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_nc_sort_warp(int nb_node, int npc, int cap,
                                                                  const int32_t* __restrict__ nc_ptr,
                                                                  const int32_t* __restrict__ bucket,
                                                                  int32_t* __restrict__ nc_cell,
@@ -213,8 +237,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_nod
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int n = wid; n < nb_node; n += nwarps) {
-    const int32_t b = nc_ptr[n], e = nc_ptr[n + 1];
-    const int deg = e - b;
+    const int32_t b = nc_ptr[n];
+    const int deg = nc_ptr[n + 1] - b;
     const int32_t* own = bucket + (int64_t)n * cap;
     // with the node's range, not after it: past the node's own keys it holds anything
     int32_t v = lane < cap ? __ldg(own + lane) : INT_MAX;
@@ -237,16 +261,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_nod
       }
       continue;
     }
-    for (int i = lane; i < min(deg, cap); i += 32) nc_cell[b + i] = own[i];
-    __syncwarp();
-    if (lane == 0) insertion_sort(nc_cell + b, deg);
-    __syncwarp();
-    for (int32_t i = b + lane; i < e; i += 32) {
-      v = nc_cell[i];
-      nc_cell[i] = v >> 3;
-      nc_local[i] = (uint8_t)(v & 7);
-      if (nc_inverse) nc_inverse[(int64_t)(v >> 3) * npc + (v & 7)] = i;
-    }
+    sort_long_list(own, cap, b, deg, npc, nc_cell, nc_local, nc_inverse);
   }
 }
 
