@@ -304,7 +304,9 @@ __device__ __noinline__ void elem_tri_cell_fp64(int64_t c, const double* xyz, co
 // integer pipes.  A planar triangle (every 2D mesh) needs no square root and
 // one cross product component: 16 of 91 FP64 instructions are left, against 27
 // products and 6 quotients on the integer pipes.  An assembly step of 2.9 M
-// triangles 0.98 -> 0.47 ms.
+// triangles 0.98 -> 0.47 ms.  A triangle that shares no z leaves before the
+// products: behind the quotients a curved surface of 2.9 M paid 0.71 ms for
+// its matrix, now the FP64 path's 0.65 (planar 0.27).
 template <bool COEFF>
 __global__ void __launch_bounds__(128) k_elem_poisson_tri_ref(int cell0, int nb_cell, const double* __restrict__ xyz,
                                                               const int32_t* __restrict__ cn,
@@ -322,6 +324,10 @@ __global__ void __launch_bounds__(128) k_elem_poisson_tri_ref(int cell0, int nb_
       for (int k = 0; k < 3; ++k) n[a][k] = __ldg(p + k);
     }
     bool ok = ref::tri_planar(n, e, &A2);
+    if (!ok) {
+      elem_tri_cell_fp64(c, xyz, cn, inv, coeff, er, bad);
+      continue;
+    }
     ok &= ref::measure_ok(A2);
     const V area(ref::mul(V(fabs(A2)), V(0.5)), ok);
     const i64fp::Divisor by = i64fp::divisor(__double_as_longlong(A2));

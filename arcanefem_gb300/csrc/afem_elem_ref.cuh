@@ -341,12 +341,13 @@ __device__ __forceinline__ bool tri_planar(const double n[3][3], double e[2][2],
       else
         ok &= bexp(n[a][2]) != 2047 && __double_as_longlong(n[a][2]) == __double_as_longlong(n[0][2]);
     }
+  if (!ok) return false;   // before the products: a curved surface's triangles all leave here
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int k = 0; k < 2; ++k) e[j][k] = sub(n[j + 1][k], n[0][k]);
   *A2 = sub(mul(Val(e[0][0]), Val(e[1][1])), mul(Val(e[0][1]), Val(e[1][0])));
-  return ok;
+  return true;
 }
 
 // computeAreaTria3 (ArcaneFemFunctionsGpu.h:76-86): |(n1 - n0) x (n2 - n0)| / 2.
