@@ -353,7 +353,7 @@ __global__ void k_fact_edge_backward(FactView f, const float* __restrict__ z, co
                                      const float* __restrict__ gl_low, const bf16* __restrict__ o,
                                      float* __restrict__ dz, float* __restrict__ part) {
   // a warp takes 32 edges: their dz one a lane, then edge by edge the two rows of o, two features a lane
-  float a0 = 0.f, a1 = 0.f, gs = 0.f;
+  Sum32 a0, a1, gs;   // gs: of the lane's own edges
   const int lane = threadIdx.x & 31;
   for (int64_t e0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32; e0 < f.nlow;
        e0 += (int64_t)gridDim.x * blockDim.x) {
@@ -367,6 +367,7 @@ __global__ void k_fact_edge_backward(FactView f, const float* __restrict__ z, co
       const float sj = f.sq[j];
       g = gl_low[e] * a_low[e] * f.sq[i] * sj * sj * 2.f * (1.f - th * th);
       dz[e] = g;
+      gs.add(g);
     }
     const int count = (int)min((int64_t)32, f.nlow - e0);
 #pragma unroll 4
@@ -375,12 +376,14 @@ __global__ void k_fact_edge_backward(FactView f, const float* __restrict__ z, co
       const int32_t ik = __shfl_sync(0xffffffffu, i, k), jk = __shfl_sync(0xffffffffu, j, k);
       const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)ik * kF)[lane]);
       const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(o + (int64_t)jk * kF)[lane]);
-      a0 = fmaf(gk * a.x, b.x, a0);
-      a1 = fmaf(gk * a.y, b.y, a1);
-      gs += gk;
+      a0.add_product(gk * a.x, b.x);
+      a1.add_product(gk * a.y, b.y);
     }
   }
-  column_partials<true>(a0, a1, gs, part);
+  float g = gs.value();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+  column_partials<true>(a0.value(), a1.value(), g, part);
 }
 
 // dO_i += sum over the edges e of node i (as row and as column) of dz_e ew * o_other; one warp per node,

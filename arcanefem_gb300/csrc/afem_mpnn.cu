@@ -45,6 +45,7 @@
 #include <cmath>
 #include <vector>
 
+#include "afem_fp32_sum.cuh"
 #include "afem_krylov.cuh"
 
 namespace afem {
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(128) k_dw_grad(const __grid_constant__ CUtenso
 // covers 32 consecutive elements, one per lane, so that every warp load is
 // one coalesced 128-byte row segment; its kSumWarps warps split the partials
 // (warp w takes b = w, w + kSumWarps, ..., four loads in flight), and warp 0
-// adds the warp sums in warp order.
+// adds the warp sums in pairs.
 constexpr int kSumWarps = 32;
 
 // k_sum_partials_many does it for several arrays in one launch: block b belongs to the job with
@@ -455,19 +456,13 @@ __device__ __forceinline__ float sum_column(const float* __restrict__ partial, i
       const float a1 = partial[(int64_t)(b + kSumWarps) * nelem + e];
       const float a2 = partial[(int64_t)(b + 2 * kSumWarps) * nelem + e];
       const float a3 = partial[(int64_t)(b + 3 * kSumWarps) * nelem + e];
-      s += a0;
-      s += a1;
-      s += a2;
-      s += a3;
+      s += (a0 + a1) + (a2 + a3);
     }
     for (; b < nparts; b += kSumWarps) s += partial[(int64_t)b * nelem + e];
   }
   sh[w][lane] = s;
   __syncthreads();
-  float t = 0.f;
-  if (w == 0)
-    for (int k = 0; k < kSumWarps; ++k) t += sh[k][lane];
-  return t;   // in warp 0
+  return w == 0 ? pair_sum<kSumWarps, 33>(&sh[0][lane]) : 0.f;
 }
 
 __global__ void __launch_bounds__(32 * kSumWarps) k_sum_partials(int nparts, int nelem,
@@ -489,22 +484,20 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum_partials_many(const SumJ
   if (threadIdx.x < 32 && e < q.nelem) q.out[e] = t;
 }
 
-// Column sums of a block whose lanes hold two features (and a scalar, the same in a warp's lanes) of their warps'
-// rows: part[block][0..kF) and, with SCALAR, part[block][kF].
+// Column sums of a block of 8 warps whose lanes hold two features (and a scalar, the same in a warp's lanes) of their
+// warps' rows: part[block][0..kF) and, with SCALAR, part[block][kF].
+constexpr int kColumnBlock = 256;
 template <bool SCALAR>
 __device__ __forceinline__ void column_partials(float a0, float a1, float g, float* __restrict__ part) {
-  __shared__ float sh[kF + 1][9];
+  __shared__ float sh[kF + 1][kColumnBlock / 32 + 1];
   constexpr int C = kF + (SCALAR ? 1 : 0);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   sh[2 * lane][w] = a0;
   sh[2 * lane + 1][w] = a1;
   if (SCALAR && lane == 0) sh[kF][w] = g;
   __syncthreads();
-  if (threadIdx.x < C) {
-    float s = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[threadIdx.x][k];
-    part[(int64_t)blockIdx.x * C + threadIdx.x] = s;
-  }
+  if (threadIdx.x < C)
+    part[(int64_t)blockIdx.x * C + threadIdx.x] = pair_sum<kColumnBlock / 32>(sh[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1036,7 +1029,7 @@ __global__ void k_dc_vcycle(int n, int batch, const float* __restrict__ d, const
 // on average in a training step at 257^2, this 4).
 __global__ void k_head_backward(int n, const float* __restrict__ dc, const bf16* __restrict__ o,
                                 const float* __restrict__ w, float* __restrict__ dO, float* __restrict__ part) {
-  float a0 = 0.f, a1 = 0.f, gs = 0.f;
+  Sum32 a0, a1, gs;
   const int lane = threadIdx.x & 31;
   const float w0 = w[2 * lane], w1 = w[2 * lane + 1];
 #pragma unroll 4
@@ -1045,11 +1038,11 @@ __global__ void k_head_backward(int n, const float* __restrict__ dc, const bf16*
     const float g = dc[row];
     const float2 v = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(o + row * kF)[lane]);
     reinterpret_cast<float2*>(dO + row * kF)[lane] = make_float2(g * w0, g * w1);
-    a0 = fmaf(g, v.x, a0);
-    a1 = fmaf(g, v.y, a1);
-    gs += g;
+    a0.add_product(g, v.x);
+    a1.add_product(g, v.y);
+    gs.add(g);
   }
-  column_partials<true>(a0, a1, gs, part);
+  column_partials<true>(a0.value(), a1.value(), gs.value(), part);
 }
 
 // G = dO (x) [O > 0] in BF16, and per-block column sums (db)
