@@ -104,6 +104,7 @@ SIGNATURES = {
     "afem_solver_options_default": (None, [C.POINTER(SolverOptions)]),
     "afem_cg_solve_csr": (C.c_int, [_P, C.c_int, _P, _P, _P, _P, _P, _P, C.POINTER(SolverOptions),
                                     C.POINTER(SolveInfo)]),
+    "afem_cg_failure_test": (C.c_int, [_P, C.c_int, _P, _P, _P, _P, _P, C.POINTER(SolverOptions), C.c_int, C.c_int]),
     "afem_ls_solve": (C.c_int, [_P, C.POINTER(SolverOptions), C.POINTER(SolveInfo)]),
     "afem_ls_set_learned_preconditioner": (C.c_int, [_P, _P]),
     "afem_spmv_csr": (C.c_int, [_P, C.c_int, _P, _P, _P, _P, _P]),

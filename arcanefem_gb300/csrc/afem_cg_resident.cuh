@@ -20,11 +20,19 @@
 //   * the sums are made in fixed point (below): in FP64 each of an iteration's
 //     two sums is a chain of 20 dependent additions and a division, 3700 of an
 //     iteration's 19900 cycles (256^2 triangles; 9.7 -> 8.6 ms a solve).
-// Every wait is bounded; one that runs out sets *err and ends all blocks.
+// Every poll is bounded; one that runs out sets *err and ends all blocks.  (A
+// system small enough for one cluster of blocks has no polls: it meets at the
+// hardware's cluster barrier, Grid with CL.)
 #pragma once
 #include "afem_krylov.cuh"
 
 namespace afem {
+
+// Of the failure-detection test (kernels with TEST): how long a poll goes on, and the block that leaves before its
+// first exchange.  A limit at run time in the solves themselves cost 2 % at 256^2 triangles and 5 % at 40^3 elasticity.
+struct ResWaits {
+  int spins, stall;
+};
 
 struct CgState {
   double rz, rr, pq, alpha, beta, bnorm2, tol2, pad0;
@@ -147,11 +155,12 @@ __device__ __forceinline__ double res_block_sum(const T (&v)[V], double* sh) {
 // exchange through L2 takes 1400 to 2500 cycles among 5 blocks; res_plan has
 // the solves' times).  That barrier needs no bound: every block takes the same
 // branches, decided from the same totals.
-template <bool CL>
+template <bool CL, bool TEST>
 struct Grid {
   ulonglong2* slots;          // [4 exchanges][2 values][gridDim.x] lines, zero at the launch; CL: shared, [2][2][8][16]
   double* sh;                 // shared, res_scratch(gridDim.x) doubles
   int* err;
+  int spins;                  // polls of a wait in a TEST
   unsigned long long epoch = 0;
 
   // CL: {lo, hi} as the slot `sub` of value w of this block in every block of the cluster, lane i in block i
@@ -225,8 +234,8 @@ struct Grid {
 
   __device__ __forceinline__ bool poll(const ulonglong2* s, ulonglong2* got) {
     *got = slot_get(s);
-    for (int spins = 0; (unsigned)got->y != (unsigned)epoch; *got = slot_get(s))
-      if (++spins >= kResSpins || ((spins & 1023) == 0 && *(volatile int*)err)) {
+    for (int n = 0; (unsigned)got->y != (unsigned)epoch; *got = slot_get(s))
+      if (++n >= (TEST ? spins : kResSpins) || ((n & 1023) == 0 && *(volatile int*)err)) {
         atomicCAS(err, 0, (int)AFEM_ERR_TIMEOUT);
         return false;
       }
@@ -469,21 +478,26 @@ struct CgResident {
   ulonglong2* slots;
   int* err;
   CgState* st;
+  ResWaits waits;
 };
 
-template <int K, bool CL>
+template <int K, bool CL, bool TEST = false>
 __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ ResCtl ctl;
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
   if (((volatile CgState*)a.st)->done) return;
+  if constexpr (TEST)
+    if ((int)blockIdx.x == a.waits.stall) return;
+  static_assert(!(CL && TEST), "the cluster's barrier has no bound: no block may stay away");
   const int nb = gridDim.x, lane = threadIdx.x & 31;
   __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster * kResWarps : 1];
   if constexpr (CL) cluster_sync();   // every block runs before one writes into another
-  Grid<CL> grid;
+  Grid<CL, TEST> grid;
   grid.slots = CL ? cluster_slots : a.slots;
   grid.sh = reinterpret_cast<double*>(dyn);
   grid.err = a.err;
+  if constexpr (TEST) grid.spins = a.waits.spins;
   ResMatrix<double> mat;
   mat.off = soff_sh;
   mat.vals = grid.sh + (2 * kResThreads > 2 * nb ? 2 * kResThreads : 2 * nb);
@@ -711,21 +725,26 @@ struct CgfResident {
   ulonglong2* slots;
   int* err;
   CgState* st;
+  ResWaits waits;
 };
 
-template <int K, bool B3, bool CL>
+template <int K, bool B3, bool CL, bool TEST = false>
 __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfResident a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ ResCtl ctl;
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
   if (((volatile CgState*)a.st)->done) return;
+  if constexpr (TEST)
+    if ((int)blockIdx.x == a.waits.stall) return;
+  static_assert(!(CL && TEST), "the cluster's barrier has no bound: no block may stay away");
   const int nb = gridDim.x, lane = threadIdx.x & 31;
   __shared__ ulonglong2 cluster_slots[CL ? 4 * kResCluster * kResWarps : 1];
   if constexpr (CL) cluster_sync();   // every block runs before one writes into another
-  Grid<CL> grid;
+  Grid<CL, TEST> grid;
   grid.slots = CL ? cluster_slots : a.slots;
   grid.sh = reinterpret_cast<double*>(dyn);
   grid.err = a.err;
+  if constexpr (TEST) grid.spins = a.waits.spins;
   std::conditional_t<B3, ResMatrix3, ResMatrix<float>> mat;
   mat.off = soff_sh;
   mat.vals = reinterpret_cast<float*>(grid.sh + (2 * kResThreads > 2 * nb ? 2 * kResThreads : 2 * nb));

@@ -634,7 +634,7 @@ static afem_status build_slices3(afem_context ctx, int nb, const int32_t* rp, co
 
 afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals, int64_t nnz,
                     const double* b, double* x, const uint8_t* skip, const afem_solver_options& opt,
-                    afem_solve_info* info) {
+                    afem_solve_info* info, const ResWaits* test) {
   const int G = lanes_per_row_fp64(n, nnz);
   const unsigned grid_rows = grid_for(ctx, (int64_t)n * G, kSolveBlock, 8);
   const unsigned grid_vec = grid_for(ctx, n, kSolveBlock, 8);
@@ -643,6 +643,9 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
                 align256(sizeof(CgState)) + slices_scratch_bytes(n) + 256;
   const ResPlan plan = res_plan(ctx, n, 1, nnz, 32 * (sizeof(double) + sizeof(int32_t)));
   bool resident = plan.take;
+  AFEM_CHECK_ARG(!test || (resident && !plan.cluster && plan.K == 1 && test->stall < (int)plan.grid &&
+                           nnz <= kResScatterEntries),
+                 "afem_cg_failure_test: no block %d that other blocks poll", test->stall);
   if (resident) need += res_slots_bytes(plan);
   AFEM_TRY(scratch_reserve(ctx, need));
   double *r, *z, *p, *q, *dinv, *partials;
@@ -687,8 +690,9 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
   CgState hs{};
   if (resident) {
     const CgResident a{n,    plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, cols, vals, sliced.soff,
-                       sliced.cols, sliced.vals, dv, skip, x, r, p, slots, err, st};
+                       sliced.cols, sliced.vals, dv, skip, x, r, p, slots, err, st, test ? *test : ResWaits{}};
     AFEM_TRY(run_resident(ctx, st, err, &hs, [&]() {
+      if (test) return launch_resident(ctx, k_cg_resident<1, false, true>, plan, a);
       if (plan.cluster) return launch_resident(ctx, k_cg_resident<1, true>, plan, a);
       return dispatch_rows(plan.K, [&](auto k) {
         return launch_resident(ctx, k_cg_resident<decltype(k)::value, false>, plan, a);
@@ -734,7 +738,7 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
 
 afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals, int64_t nnz,
                      const double* b, double* x, const uint8_t* skip, const afem_solver_options& opt,
-                     afem_solve_info* info) {
+                     afem_solve_info* info, const ResWaits* test) {
   const int G64 = lanes_per_row_fp64(n, nnz);   // FP64 outer residual
   const bool b3 = opt.block_size == 3;          // FP32 3x3-block SpMV, else the sliced-ELL scalar SpMV
   AFEM_CHECK_ARG(!b3 || n % 3 == 0, "block_size 3 needs a multiple of 3 rows (%d)", n);
@@ -747,6 +751,9 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
   // a step of the resident form: 32 entries, or 32 blocks of nine values
   const ResPlan plan = res_plan(ctx, b3 ? n / 3 : n, b3 ? 3 : 1, nnz, b3 ? 32 * 40 : 32 * 8);
   bool resident = plan.take;
+  AFEM_CHECK_ARG(!test || (resident && !plan.cluster && plan.K == 1 && test->stall < (int)plan.grid &&
+                           nnz <= kResScatterEntries),
+                 "afem_cg_failure_test: no block %d that other blocks poll", test->stall);
   size_t need = 6 * align256(sizeof(float) * (size_t)n) + align256(sizeof(double) * 3 * nparts) +
                 2 * align256(sizeof(CgState)) + 256 + (resident ? res_slots_bytes(plan) : 0) +
                 (b3 ? align256(sizeof(int32_t) * (size_t)(nnz / 9 + 1)) + 256 + slices_scratch_bytes(n / 3)
@@ -869,8 +876,11 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
     if (resident) {
       const CgfResident a{n, plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, b3 ? bcols : cols, vals,
                           sliced.soff, sliced.cols, sliced.vals, dinv32, skip, x32, r32, z32, p32, q32, slots, err,
-                          inner};
+                          inner, test ? *test : ResWaits{}};
       AFEM_TRY(run_resident(ctx, inner, err, &hi, [&]() {
+        if (test)
+          return b3 ? launch_resident(ctx, k_cgf_resident<1, true, false, true>, plan, a)
+                    : launch_resident(ctx, k_cgf_resident<1, false, false, true>, plan, a);
         if (plan.cluster)
           return b3 ? launch_resident(ctx, k_cgf_resident<1, true, true>, plan, a)
                     : launch_resident(ctx, k_cgf_resident<1, false, true>, plan, a);
@@ -967,9 +977,9 @@ afem_status true_relres(afem_context ctx, int n, const int32_t* rp, const int32_
   return AFEM_OK;
 }
 
-afem_status solve_csr(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals,
-                      const double* b, double* x, const uint8_t* forced, const afem_solver_options* opt_in,
-                      afem_solve_info* info) {
+static afem_status solve_with(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals,
+                              const double* b, double* x, const uint8_t* forced, const afem_solver_options* opt_in,
+                              afem_solve_info* info, const ResWaits* test) {
   AFEM_CHECK_ARG(ctx && n > 0 && rp && cols && vals && b && x, "afem_cg_solve_csr: bad arguments");
   afem_solver_options opt;
   if (opt_in) opt = *opt_in;
@@ -984,8 +994,8 @@ afem_status solve_csr(afem_context ctx, int n, const int32_t* rp, const int32_t*
   AFEM_CUDA(cudaEventCreate(&e0));
   AFEM_CUDA(cudaEventCreate(&e1));
   AFEM_CUDA(cudaEventRecord(e0, ctx->stream));
-  afem_status st = opt.precision == AFEM_PRECISION_MIXED ? cg_mixed(ctx, n, rp, cols, vals, nnz, b, x, skip, opt, info)
-                                                         : cg_fp64(ctx, n, rp, cols, vals, nnz, b, x, skip, opt, info);
+  afem_status st = opt.precision == AFEM_PRECISION_MIXED ? cg_mixed(ctx, n, rp, cols, vals, nnz, b, x, skip, opt, info, test)
+                                                         : cg_fp64(ctx, n, rp, cols, vals, nnz, b, x, skip, opt, info, test);
   cudaEventRecord(e1, ctx->stream);
   cudaEventSynchronize(e1);
   float ms = 0.f;
@@ -1004,6 +1014,12 @@ afem_status solve_csr(afem_context ctx, int n, const int32_t* rp, const int32_t*
   if (st == AFEM_ERR_NOT_CONVERGED) return fail(st, "CG did not reach the tolerance (relres %.3e)", rel);
   if (st == AFEM_ERR_BREAKDOWN) return fail(st, "CG breakdown (<p, A p> <= 0 or non-finite)");
   return AFEM_OK;
+}
+
+afem_status solve_csr(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals,
+                      const double* b, double* x, const uint8_t* forced, const afem_solver_options* opt,
+                      afem_solve_info* info) {
+  return solve_with(ctx, n, rp, cols, vals, b, x, forced, opt, info, nullptr);
 }
 
 afem_status spmv_fp64(afem_context ctx, int n, int64_t nnz, const int32_t* rp, const int32_t* cols,
@@ -1038,6 +1054,14 @@ afem_status afem_cg_solve_csr(afem_context ctx, int n, const int32_t* rp, const 
                               const double* b, double* x, const uint8_t* forced, const afem_solver_options* opt,
                               afem_solve_info* info) {
   return solve_csr(ctx, n, rp, cols, vals, b, x, forced, opt, info);
+}
+
+afem_status afem_cg_failure_test(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals,
+                                 const double* b, double* x, const afem_solver_options* opt, int stall_block,
+                                 int spin_limit) {
+  AFEM_CHECK_ARG(stall_block >= 0 && spin_limit > 0, "afem_cg_failure_test: bad arguments");
+  const ResWaits test = {spin_limit, stall_block};
+  return solve_with(ctx, n, rp, cols, vals, b, x, nullptr, opt, nullptr, &test);
 }
 
 afem_status afem_spmv_csr(afem_context ctx, int n, const int32_t* rp, const int32_t* cols, const double* vals,

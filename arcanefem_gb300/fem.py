@@ -465,6 +465,14 @@ def cg_solve_csr(ctx: Context, row_ptr, cols, values, b, x, forced_info=None, op
                       _ptr(x), _ptr(forced_info), C.byref(opt), C.byref(info))
 
 
+def cg_failure_test(ctx: Context, row_ptr, cols, values, b, x, options: SolverOptions, stall_block: int,
+                    spin_limit: int) -> int:
+    """Status of a solve one of whose blocks never arrives (see afem_cg_failure_test)."""
+    return int(_capi.lib().afem_cg_failure_test(ctx.handle, int(row_ptr.numel()) - 1, _ptr(row_ptr), _ptr(cols),
+                                                _ptr(values), _ptr(b), _ptr(x), C.byref(options), stall_block,
+                                                spin_limit))
+
+
 FACE_SCALAR, FACE_NORMAL, FACE_VECTOR = 0, 1, 2
 
 

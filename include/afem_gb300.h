@@ -464,6 +464,15 @@ afem_status afem_cg_solve_csr(afem_context ctx, int n, const int32_t* row_ptr_d,
                               const double* values_d, const double* b_d, double* x_d, const uint8_t* forced_info_d,
                               const afem_solver_options* opt, afem_solve_info* info);
 
+/* Failure-detection test of the one-launch form: block `stall_block` leaves
+ * before its first exchange, so the waits of the others run out after
+ * `spin_limit` polls and the call returns AFEM_ERR_TIMEOUT, with x as it was and
+ * the context still usable.  AFEM_ERR_BAD_ARG where the system has no such block
+ * (it meets in one cluster, or has more than a row a thread). */
+afem_status afem_cg_failure_test(afem_context ctx, int n, const int32_t* row_ptr_d, const int32_t* cols_d,
+                                 const double* values_d, const double* b_d, double* x_d,
+                                 const afem_solver_options* opt, int stall_block, int spin_limit);
+
 /* IDoFLinearSystemImpl::solve: solves the linear system's matrix view for
  * its rhs into its solution variable (applyLinearSystemTransformationAndSolve
  * calls the two transformations first, femutils/DoFLinearSystem.cc:487-493).
