@@ -1,16 +1,23 @@
-"""The one-launch CG where a block never arrives."""
+"""The one-launch CG where it can fail without a wrong number: a block that
+never arrives, iterates asked for and not made, and inner solves that take more
+than one launch.  Sizes follow the device's SM count."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 import torch
 
 from arcanefem_gb300 import fem
-from test_gpu_cg_resident import block_matrix, dev, matrix
+from test_gpu_cg_resident import block_matrix, cg, dev, matrix
 
 pytestmark = pytest.mark.gpu
 
-BAD_ARG, TIMEOUT = 1, 5
+BAD_ARG, NOT_CONVERGED, TIMEOUT = 1, 3, 5
 OPTIONS = {"fp64": dict(precision=fem.PRECISION_FP64), "mixed": dict(precision=fem.PRECISION_MIXED),
            "blocks": dict(precision=fem.PRECISION_MIXED, block_size=3)}
+
+
+def rows_of_one_a_thread():
+    return min(torch.cuda.get_device_properties(0).multi_processor_count, 256) * 512
 
 
 # 40 blocks of 128 rows, or 27 of 64 block rows
@@ -39,3 +46,55 @@ def test_systems_without_polls_have_no_failure_test(cuda_ctx):
     b = torch.ones(5000, dtype=torch.float64, device="cuda")
     x = torch.zeros_like(b)
     assert fem.cg_failure_test(cuda_ctx, *dev(A), b, x, fem.solver_options(), 40, 1000) == BAD_ARG
+
+
+def solve_exactly(ctx, A, b, iters):
+    """x after `iters` iterations; anything else that the solve says is an error."""
+    x = torch.zeros(A.shape[0], dtype=torch.float64, device="cuda")
+    with pytest.raises(fem.AfemError) as e:
+        fem.cg_solve_csr(ctx, *dev(A), torch.as_tensor(b, device="cuda"), x,
+                         options=fem.solver_options(rtol=0.0, atol=1e-300, max_iter=iters))
+    assert e.value.status == NOT_CONVERGED and e.value.info.iterations == iters
+    return x.cpu().numpy()
+
+
+# the device's edges of one, four and six rows a thread, and the first system past them; iterates as in
+# test_gpu_cg_resident.py, to its 1e-12
+@pytest.mark.parametrize("rows,more", [(1, 0), (1, 1), (2, 33), (4, 1), (6, 0), (6, 1)])
+def test_iterates_at_the_splits_of_this_device(cuda_ctx, rows, more):
+    n = rows * rows_of_one_a_thread() + more
+    A = matrix(n, seed=n % 97)
+    b = np.random.default_rng(n).standard_normal(n)
+    want = cg(A, b, 6)
+    assert np.max(np.abs(solve_exactly(cuda_ctx, A, b, 6) - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("n,width,heavy", [(5000, 1, 0), (20000, 300, 0), (20000, 1, 64), (170000, 1, 40)])
+def test_band_matrices_make_the_iterations_asked_for(cuda_ctx, n, width, heavy):
+    rng = np.random.default_rng(n + width)
+    A = sp.diags([-rng.uniform(0.5, 1.0, n - width)], [width], shape=(n, n))
+    if heavy:
+        i, j = np.repeat(np.arange(heavy), 1500), np.tile(np.arange(heavy, heavy + 1500), heavy)
+        A = A + sp.coo_matrix((-rng.uniform(0.0, 0.01, i.size), (i, j)), shape=(n, n))
+    A = (A + A.T).tocsr()
+    A = (A + sp.diags(np.asarray(abs(A).sum(1)).ravel() + rng.uniform(1.0, 3.0, n))).tocsr()
+    A.sort_indices()
+    b = rng.standard_normal(n)
+    want = cg(A, b, 10)
+    assert np.max(np.abs(solve_exactly(cuda_ctx, A, b, 10) - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("n", [2000, 5000])
+def test_mixed_inner_solves_span_several_launches(cuda_ctx, n):
+    """A shifted chain: in numpy the FP32 cycles take 3000 to 4500 iterations at 5000 rows; a launch makes 1890
+    there, 1930 at 2000."""
+    A = sp.diags([-np.ones(n - 1), (2.0 + 1e-6) * np.ones(n), -np.ones(n - 1)], [-1, 0, 1]).tocsr()
+    b = np.random.default_rng(0).standard_normal(n)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    info = fem.cg_solve_csr(cuda_ctx, *dev(A), torch.as_tensor(b, device="cuda"), x,
+                            options=fem.solver_options(rtol=1e-8, max_iter=200000, inner_rtol=1e-3,
+                                                       precision=fem.PRECISION_MIXED))
+    assert info.status == 0
+    if n == 5000:
+        assert info.iterations > 2000 * info.refinements
+    assert np.linalg.norm(b - A @ x.cpu().numpy()) <= 1.01e-8 * np.linalg.norm(b)
