@@ -677,8 +677,10 @@ static cudaError_t launch_batch(afem_batch b, cudaStream_t s, const BatchParams&
   lc.blockDim = dim3(BLOCK);
   lc.dynamicSmemBytes = own_bytes(prm.own_rows);
   lc.stream = s;
+  // the same limit in every call, whatever this batch takes: the attribute is the function's, and other threads launch
+  // batches of their own between this call and the launch
   const cudaError_t e = cudaFuncSetAttribute(k_batch<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)lc.dynamicSmemBytes);
+                                             (int)kOwnBytes);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
