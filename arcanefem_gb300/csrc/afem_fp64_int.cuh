@@ -1,4 +1,4 @@
-// FP64 add, multiply and divide on the integer pipe, rounded to nearest even.
+// FP64 multiply and divide on the integer pipe, rounded to nearest even.
 //
 // GB300 issues FP64 slowly: measured 0.5 T FMA/s, about 1.7 FP64 lane
 // operations per clock and SM, while an SM issues up to four warp
@@ -17,9 +17,10 @@
 // integer products / aligned sums of the 53-bit significands with guard and
 // sticky bits, normalisation, round to nearest with ties to even.
 //
-// First the operations on packed operands, for any operands: normal ones with
-// a normal (or exactly zero) result.  Zeros, subnormals, infinities, NaN and
-// results that would overflow or underflow return false.
+// What the kernels use are the products and quotients of unpacked operands and
+// mulhi.  The multiply and add of packed operands before them, for any operands
+// (zeros, subnormals, infinities, NaN and results that would overflow or
+// underflow return false), have no caller but their host check.
 #pragma once
 
 #include <cstdint>
