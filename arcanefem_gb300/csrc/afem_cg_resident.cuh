@@ -33,6 +33,12 @@ namespace afem {
 struct ResWaits {
   int spins, stall;
 };
+template <class Args>
+struct WithWaits : Args {
+  ResWaits waits;
+};
+template <bool TEST, class Args>
+using ResArgs = std::conditional_t<TEST, WithWaits<Args>, Args>;
 
 struct CgState {
   double rz, rr, pq, alpha, beta, bnorm2, tol2, pad0;
@@ -478,11 +484,10 @@ struct CgResident {
   ulonglong2* slots;
   int* err;
   CgState* st;
-  ResWaits waits;
 };
 
 template <int K, bool CL, bool TEST = false>
-__global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const CgResident a) {
+__global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const ResArgs<TEST, CgResident> a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ ResCtl ctl;
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];
@@ -725,11 +730,10 @@ struct CgfResident {
   ulonglong2* slots;
   int* err;
   CgState* st;
-  ResWaits waits;
 };
 
 template <int K, bool B3, bool CL, bool TEST = false>
-__global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const CgfResident a) {
+__global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const ResArgs<TEST, CgfResident> a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ ResCtl ctl;
   __shared__ int32_t soff_sh[K * kResThreads / 32 + 1];

@@ -690,9 +690,9 @@ afem_status cg_fp64(afem_context ctx, int n, const int32_t* rp, const int32_t* c
   CgState hs{};
   if (resident) {
     const CgResident a{n,    plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, cols, vals, sliced.soff,
-                       sliced.cols, sliced.vals, dv, skip, x, r, p, slots, err, st, test ? *test : ResWaits{}};
+                       sliced.cols, sliced.vals, dv, skip, x, r, p, slots, err, st};
     AFEM_TRY(run_resident(ctx, st, err, &hs, [&]() {
-      if (test) return launch_resident(ctx, k_cg_resident<1, false, true>, plan, a);
+      if (test) return launch_resident(ctx, k_cg_resident<1, false, true>, plan, WithWaits<CgResident>{a, *test});
       if (plan.cluster) return launch_resident(ctx, k_cg_resident<1, true>, plan, a);
       return dispatch_rows(plan.K, [&](auto k) {
         return launch_resident(ctx, k_cg_resident<decltype(k)::value, false>, plan, a);
@@ -876,11 +876,13 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
     if (resident) {
       const CgfResident a{n, plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, b3 ? bcols : cols, vals,
                           sliced.soff, sliced.cols, sliced.vals, dinv32, skip, x32, r32, z32, p32, q32, slots, err,
-                          inner, test ? *test : ResWaits{}};
+                          inner};
       AFEM_TRY(run_resident(ctx, inner, err, &hi, [&]() {
-        if (test)
-          return b3 ? launch_resident(ctx, k_cgf_resident<1, true, false, true>, plan, a)
-                    : launch_resident(ctx, k_cgf_resident<1, false, false, true>, plan, a);
+        if (test) {
+          const WithWaits<CgfResident> w{a, *test};
+          return b3 ? launch_resident(ctx, k_cgf_resident<1, true, false, true>, plan, w)
+                    : launch_resident(ctx, k_cgf_resident<1, false, false, true>, plan, w);
+        }
         if (plan.cluster)
           return b3 ? launch_resident(ctx, k_cgf_resident<1, true, true>, plan, a)
                     : launch_resident(ctx, k_cgf_resident<1, false, true>, plan, a);
