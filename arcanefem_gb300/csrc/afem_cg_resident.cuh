@@ -455,15 +455,14 @@ __device__ __forceinline__ T res_row_dot(const int32_t* c, const T* a, int m, co
   return acc;
 }
 // straight from the CSR row (slices that do not fit where no sliced copy was made)
-template <class T>
-__device__ __forceinline__ T res_row_dot_csr(int row, const int32_t* __restrict__ rp,
-                                             const int32_t* __restrict__ cols, const double* __restrict__ vals,
-                                             const T* x) {
-  T acc = T(0);
+__device__ __forceinline__ double res_row_dot_csr(int row, const int32_t* __restrict__ rp,
+                                                  const int32_t* __restrict__ cols, const double* __restrict__ vals,
+                                                  const double* x) {
+  double acc = 0.0;
   const int32_t e = __ldg(rp + row + 1);
   for (int32_t k = __ldg(rp + row); k < e; ++k) {
     const int32_t c = __ldg(cols + k);
-    if (c >= 0) acc = fma((T)__ldg(vals + k), x[c], acc);
+    if (c >= 0) acc = fma(__ldg(vals + k), x[c], acc);
   }
   return acc;
 }
@@ -561,7 +560,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const ResArgs<TE
           const int64_t at = (int64_t)kSlice * __ldg(a.soff + (row >> 5)) + lane;
           q[k] = res_row_dot<kSlice, false>(a.scols + at, a.svals + at, m, a.p);
         } else if (row < r1)
-          q[k] = res_row_dot_csr<double>(row, a.rp, a.cols, a.vals, a.p);
+          q[k] = res_row_dot_csr(row, a.rp, a.cols, a.vals, a.p);
         if (row < r1) pq[0] += (kAll ? p[kAll ? k : 0] : a.p[row]) * q[k];
       }
     }
@@ -704,16 +703,6 @@ __device__ __forceinline__ float res_row_dot3(const int32_t* c, const float* v, 
   return acc;
 }
 
-__device__ __forceinline__ float res_row_dot3_csr(int I, int c, const int32_t* __restrict__ rp,
-                                                  const int32_t* __restrict__ bcols, const double* __restrict__ vals,
-                                                  const float* z) {
-  float acc = 0.f;
-  const int32_t b0 = __ldg(rp + 3 * I), b = __ldg(rp + 3 * I + c), len = __ldg(rp + 3 * I + 1) - b0;
-  for (int32_t k = 0; k < len; ++k)
-    acc = fmaf((float)__ldg(vals + b + k), z[3 * __ldg(bcols + b0 / 9 + k / 3) + k % 3], acc);
-  return acc;
-}
-
 // The FP32 inner CG of the mixed solver, up to `iters` iterations: the
 // arithmetic of k_cgf_spmv_sl / k_cgf_spmv_b3s (w = A z, p = z + beta p,
 // q = w + beta q) and k_cgf_update row by row.  B3: a warp takes one
@@ -803,12 +792,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgf_resident(const ResArgs<T
           const int32_t* mc = mat.cols + 32 * (size_t)mat.off[s] + lane;
           if constexpr (B3) w = res_row_dot3<true>(mc, mat.vals + 288 * (size_t)mat.off[s] + 96 * c + lane, m, a.z);
           else w = res_row_dot<32, true>(mc, mat.vals + 32 * mat.off[s] + lane, m, a.z);
-        } else if (!a.scols) {
-          w = 0.f;
-          if (I < r1) {
-            if constexpr (B3) w = res_row_dot3_csr(I, c, a.rp, a.cols, a.vals, a.z);
-            else w = res_row_dot_csr<float>(I, a.rp, a.cols, a.vals, a.z);
-          }
         } else {
           const int64_t at = (int64_t)kSlice * __ldg(a.soff + (r0 >> 5) + s);
           if constexpr (B3) w = res_row_dot3<false>(a.scols + at + lane, a.svals + 9 * at + 96 * c + lane, m, a.z);
@@ -896,7 +879,7 @@ struct ResPlan {
   bool cluster = false;  // one cluster of blocks
   // dynamic shared memory: the cluster form's slots are static
   size_t smem() const { return kResSmem - (cluster ? sizeof(ulonglong2) * 4 * kResCluster * kResWarps : 0); }
-  bool fits = false;     // every slice is likely to fit the shared memory
+  bool fits = false;     // every slice is likely to fit the shared memory (exactly: k_res_unfit)
   bool take = false;     // this form rather than the launches per iteration
 };
 
@@ -945,6 +928,27 @@ inline ResPlan res_plan(afem_context ctx, int rows, int C, int64_t nnz, size_t s
            (int64_t)(nnz / (C * C) * (step_bytes / 32)) - (int64_t)p.grid * (int64_t)kResSmem <= kResStreamBytes;
   p.fits = (double)nnz / (C * C) <= 0.9 * 32.0 * p.steps * p.grid;
   return p;
+}
+
+// Whether the slices of a block's rows (C scalar rows each) are more than `steps` long together, in any block: a block
+// of the solve a block here, a warp a slice.  res_plan's `fits` expects slices of about equal rows; a node with far more
+// neighbours than the others makes its slice as long as its row.  The mixed solver reads the answer with its first
+// residual and makes the sliced copy then: walked in the CSR row, entry by entry with the values' conversions, a row of
+// 5000 entries among 140^2 cost 190 ms a solve, from the copy 107 (launches per iteration 157 to 166).
+static __global__ void __launch_bounds__(kResThreads) k_res_unfit(int rows, int rows_pb, int C, int steps,
+                                                                  const int32_t* __restrict__ rp, int* unfit) {
+  __shared__ int total;
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  const int r0 = blockIdx.x * rows_pb, r1 = min(rows, r0 + rows_pb);
+  for (int s = threadIdx.x >> 5; 32 * s < r1 - r0; s += kResWarps) {
+    const int I = r0 + 32 * s + (threadIdx.x & 31);
+    const int len = I < r1 ? (__ldg(rp + C * I + 1) - __ldg(rp + C * I)) / C : 0;
+    const int m = __reduce_max_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&total, m);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && total > steps) *unfit = 1;
 }
 
 // Samples slices of 32 rows: counts[0] entries seen, counts[1] those more than

@@ -779,7 +779,8 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
     AFEM_TRY(res_scattered(ctx, n, rp, cols, err, &scattered));
     resident = !scattered;
   }
-  AFEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+  AFEM_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(int), ctx->stream));
+  int* const unfit = err + 1;
   if (resident) AFEM_TRY(scratch_take(ctx, res_slots_bytes(plan) / sizeof(ulonglong2), &slots));
   AFEM_CUDA(cudaMemsetAsync(outer, 0, sizeof(CgState), ctx->stream));
   AFEM_CUDA(cudaMemsetAsync(inner, 0, sizeof(CgState), ctx->stream));
@@ -796,12 +797,16 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
   }
   // the FP32 matrix: the sliced copy, by 3x3 blocks or by scalar rows
   SlicedCopy<float> sliced;
-  if (resident && plan.fits)
-    ;   // filled into shared memory from the CSR rows
-  else if (b3)
-    AFEM_TRY(build_slices3(ctx, n / 3, rp, (const int32_t*)bcols, vals, sliced));
+  auto slices = [&]() {
+    return b3 ? build_slices3(ctx, n / 3, rp, (const int32_t*)bcols, vals, sliced)
+              : build_slices(ctx, n, rp, cols, vals, sliced);
+  };
+  const bool from_rows = resident && plan.fits;   // filled into shared memory from the CSR rows, if they do fit
+  if (from_rows)
+    AFEM_TRY(launch(ctx, k_res_unfit, plan.grid, kResThreads, 0, b3 ? n / 3 : n, plan.rows_pb, b3 ? 3 : 1, plan.steps,
+                    rp, unfit));
   else
-    AFEM_TRY(build_slices(ctx, n, rp, cols, vals, sliced));
+    AFEM_TRY(slices());
   AFEM_TRY(launch(ctx, k_inv_diag, grid_vec, kSolveBlock, 0, n, rp, cols, vals, (double*)nullptr, dinv32));
   if (opt.precond != AFEM_PRECOND_JACOBI)  // unpreconditioned inner solve: D^-1 = 1
     AFEM_TRY(launch(ctx, k_fill_f32, grid_for(ctx, n, 256), 256, 0, (int64_t)n, 1.0f, dinv32));
@@ -840,9 +845,18 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
                     inner_rtol, remaining, restart ? 1 : 0);
     }));
     CgState ho{};
-    AFEM_CUDA(cudaMemcpyAsync(ctx->pinned, outer, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+    struct First {
+      CgState s;
+      int unfit;
+    };
+    auto* const h = reinterpret_cast<First*>(ctx->pinned);
+    h->unfit = 0;
+    AFEM_CUDA(cudaMemcpyAsync(&h->s, outer, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+    if (from_rows && outer_steps == 0)
+      AFEM_CUDA(cudaMemcpyAsync(&h->unfit, unfit, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     AFEM_CUDA(cudaStreamSynchronize(ctx->stream));
-    ho = *reinterpret_cast<CgState*>(ctx->pinned);
+    ho = h->s;
+    const bool copy_now = h->unfit != 0;
     if (!restart && !(ho.rr <= 0.25 * rr_prev && inner_rtol >= 0.01)) {
       // the true residual did not halve: redo this update with a fresh direction
       restart = true;
@@ -872,6 +886,7 @@ afem_status cg_mixed(afem_context ctx, int n, const int32_t* rp, const int32_t* 
       status = AFEM_ERR_NOT_CONVERGED;
       break;
     }
+    if (copy_now) AFEM_TRY(slices());
     CgState hi{};
     if (resident) {
       const CgfResident a{n, plan.rows_pb, res_launch_iters(n, nnz), plan.steps, rp, b3 ? bcols : cols, vals,
