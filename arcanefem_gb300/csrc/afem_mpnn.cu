@@ -736,12 +736,14 @@ namespace afem {
 // lo..L-1 are small (<= kCoarseRows rows each), so their steps run back to
 // back with cluster barriers instead of one launch each.  Eight blocks of 512
 // threads: in one block of 1024 a step of the 1089-row level was two passes
-// of one SM (513^2, 289 rows solved exactly: 26 -> 22 us a cycle).
+// of one SM (513^2, 289 rows solved exactly: 26 -> 22 us a cycle).  Four for
+// more vectors than the chip holds clusters of eight at once (36): 64 vectors
+// of a 33^2 cycle 39 us, 55 with eight (39 with one block of 1024), 513^2 0.32
+// ms, 0.34 with eight.
 constexpr int kCoarseRows = 2048;
 constexpr int kExactRows = 320;   // the first level below the finest of at most this many rows is solved exactly
 constexpr int kCoarseBlock = 512;
 constexpr int kCoarseCluster = 8;
-
 
 struct CoarseLevel {
   int n;
@@ -778,13 +780,14 @@ __device__ __forceinline__ void dense_matvec(int i0, int st, int n, const float*
 
 // forward: x_lo = V_lo(r_lo), keeping t, u (and the factored smoothers' L r,
 // L u) per level for the backward
-__global__ void __cluster_dims__(kCoarseCluster, 1, 1) __launch_bounds__(kCoarseBlock)
+template <int CLUSTER>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(kCoarseBlock)
     k_vc_coarse(CoarsePlan plan, const float* r_lo, float* x_lo) {
   pdl_trigger();
   pdl_wait();
   const int64_t b = blockIdx.y;
   const int lo = plan.lo, L = plan.L, i0 = blockIdx.x * blockDim.x + threadIdx.x,
-            st = kCoarseCluster * blockDim.x;
+            st = CLUSTER * blockDim.x;
   for (int l = lo; l + 1 < L; ++l) {   // pre-smoothing residual, restriction
     const CoarseLevel& A = plan.lev[l];
     const CoarseLevel& C = plan.lev[l + 1];
@@ -847,11 +850,12 @@ __global__ void __cluster_dims__(kCoarseCluster, 1, 1) __launch_bounds__(kCoarse
 // backward: from the adjoint g_lo of x_lo, rb_lo (the adjoint of r_lo), and
 // per level g (the adjoint of the level's output) and x1b for the weights;
 // on factored levels also L g (gpost) and L x1b (gpre)
-__global__ void __cluster_dims__(kCoarseCluster, 1, 1) __launch_bounds__(kCoarseBlock)
+template <int CLUSTER>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(kCoarseBlock)
     k_vc_coarse_adjoint(CoarsePlan plan, const float* g_lo, float* rb_lo) {
   const int64_t b = blockIdx.y;
   const int lo = plan.lo, L = plan.L, i0 = blockIdx.x * blockDim.x + threadIdx.x,
-            st = kCoarseCluster * blockDim.x;
+            st = CLUSTER * blockDim.x;
   for (int l = lo; l + 1 < L; ++l) {   // adjoint of the post-smoothing, then of the prolongation
     const CoarseLevel& A = plan.lev[l];
     const CoarseLevel& C = plan.lev[l + 1];
@@ -1188,6 +1192,7 @@ struct afem_mpnn_s {
   float* t[kMaxLevels] = {};                 // level input r_l [B][n_l] (level 0: the caller's r, t0)
   const float* t0 = nullptr;
   int coarse_lo = 0;                         // levels coarse_lo..Lv-1 run in the coarse-levels kernels
+  int coarse_clusters = 0;                   // their clusters of eight blocks that the device runs at once
   int ex = -1;                               // the level solved exactly (-1: none)
   int Lv = 0;                                // levels the V-cycle uses: ex + 1, or L
   float* minv = nullptr;                     // FP32 inverse of A_ex's nonzero rows' block [n_ex][n_ex]
@@ -1577,12 +1582,15 @@ static afem_status apply(afem_mpnn net, int batch, const float* r, float* z) {
     AFEM_TRY(sweep(net, &net->Pt[l], batch, net->vs[l], nullptr, nullptr, net->t[l + 1], net->n[l + 1]));
   }
   float* x0 = z ? z : net->w[0];
+  const bool wide = batch <= net->coarse_clusters;
+  const dim3 coarse_grid(wide ? kCoarseCluster : kCoarseCluster / 2, batch);
+  const auto coarse = wide ? k_vc_coarse<kCoarseCluster> : k_vc_coarse<kCoarseCluster / 2>;
   if (net->pdl) {
-    AFEM_TRY(launch_pdl(net->ctx, net->ctx->stream, k_vc_coarse, dim3(kCoarseCluster, batch), kCoarseBlock, coarse_plan(net),
+    AFEM_TRY(launch_pdl(net->ctx, net->ctx->stream, coarse, coarse_grid, kCoarseBlock, coarse_plan(net),
                         lo == 0 ? r : (const float*)net->t[lo], lo == 0 ? x0 : net->w[lo]));
   } else {
-    k_vc_coarse<<<dim3(kCoarseCluster, batch), kCoarseBlock, 0, net->ctx->stream>>>(coarse_plan(net), lo == 0 ? r : net->t[lo],
-                                                                      lo == 0 ? x0 : net->w[lo]);
+    coarse<<<coarse_grid, kCoarseBlock, 0, net->ctx->stream>>>(coarse_plan(net), lo == 0 ? r : net->t[lo],
+                                                               lo == 0 ? x0 : net->w[lo]);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "k_vc_coarse", __FILE__, __LINE__);
     ++net->ctx->launches;
@@ -1634,7 +1642,10 @@ static afem_status apply_adjoint(afem_mpnn net, int batch) {
     AFEM_TRY(sweep(net, &net->Pt[l], batch, net->x2[l], nullptr, nullptr, net->s[l + 1], net->n[l + 1]));
   }
   {
-    k_vc_coarse_adjoint<<<dim3(kCoarseCluster, batch), kCoarseBlock, 0, ctx->stream>>>(coarse_plan(net), net->s[lo], net->w[lo]);
+    const bool wide = batch <= net->coarse_clusters;
+    const auto coarse = wide ? k_vc_coarse_adjoint<kCoarseCluster> : k_vc_coarse_adjoint<kCoarseCluster / 2>;
+    coarse<<<dim3(wide ? kCoarseCluster : kCoarseCluster / 2, batch), kCoarseBlock, 0, ctx->stream>>>(
+        coarse_plan(net), net->s[lo], net->w[lo]);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "k_vc_coarse_adjoint", __FILE__, __LINE__);
     ++ctx->launches;
@@ -1934,6 +1945,18 @@ afem_status afem_mpnn_create(afem_context ctx, int nb_levels, int nb_layers, con
   net->Lv = net->ex >= 0 ? net->ex + 1 : nb_levels;
   net->coarse_lo = net->Lv - 1;
   while (net->coarse_lo > 0 && level_rows[net->coarse_lo - 1] <= kCoarseRows) --net->coarse_lo;
+  {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {kCoarseCluster, 1, 1};
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(kCoarseCluster, kMaxBatch);
+    lc.blockDim = dim3(kCoarseBlock);
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&net->coarse_clusters, k_vc_coarse<kCoarseCluster>, &lc);
+    if (e != cudaSuccess) return cleanup(cuda_fail(e, "cudaOccupancyMaxActiveClusters", __FILE__, __LINE__));
+  }
   if (net->ex >= 0 && (st = dalloc(net, (size_t)level_rows[net->ex] * level_rows[net->ex], &net->minv)) != AFEM_OK)
     return cleanup(st);
   for (int l = 0; l < net->Lv; ++l) {
