@@ -23,9 +23,12 @@ Two more sections ride on the same line (rank 0):
            assembled and solved to 1e-8 in one persistent launch.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gb300|reference]
-                  [--workload poisson3d|elasticity3d|poisson2d]
+                  [--workload poisson3d|elasticity3d|poisson2d] [--record FILE]
 
-One JSON line on rank 0.  ``value`` is device-timed (CUDA events, L2 flushed
+One JSON line of a few kilobytes on rank 0: the metric, its end-to-end value,
+clocks, roofline and a summary of the sections; --record FILE keeps the whole
+record (rooflines, transfers, CPU baselines and oracle checks of every
+workload).  ``value`` is device-timed (CUDA events, L2 flushed
 between steps); ``e2e`` is the same metric through the public API with host
 buffers (mesh in from pinned host memory, connectivity + sparsity + assembly,
 CSR back to pinned host memory) inside the timed region.  ``--impl
@@ -94,6 +97,7 @@ def parse_args():
                    help="auto: autotune (JSON cache); none: the library's default configuration")
     p.add_argument("--no-extra-workloads", action="store_true",
                    help="measure the main workload only (skip " + ", ".join(EXTRA_WORKLOADS) + ")")
+    p.add_argument("--record", metavar="FILE", help="write the whole record to FILE; the printed line is a summary")
     a = p.parse_args()
     if a.n <= 0:
         a.n = WORKLOADS[a.workload]["n"]
@@ -428,6 +432,49 @@ def measure_workload(args, name, n, ctx, rank, world, local, main):
     return out
 
 
+def pick(d, *keys):
+    """The entries of d that there are, numbers to six digits."""
+    d = d or {}
+    return {k: float(f"{d[k]:.6g}") if isinstance(d[k], float) else d[k] for k in keys if k in d}
+
+
+def headline(out):
+    """The printed line: everything of the metric itself, and the sections' figures alone."""
+    line = {k: out[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                                "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config",
+                                "gpu_launches", "clocks")}
+    if "e2e" in out:
+        line["e2e"] = {k: out["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step",
+                                                   "ms_per_step") if k in out["e2e"]}
+    line["nnz"] = out["nnz"]
+    line["roofline"] = pick(out["roofline"], "bound", "achieved", "peak", "unit", "frac", "kernel")
+    line["cpu_baseline"] = pick(out.get("cpu_baseline"), "value", "unit", "cores", "kind", "sample",
+                                "bit_exact_vs_gpu")
+
+    def section(w):
+        solve = w.get("solve") or {}
+        return {"element_ms": w["element_ms"], "gather_ms": w["gather_ms"],
+                "minimal_ms": (w.get("minimal_formulation") or {}).get("ms_per_step"),
+                **pick(w.get("structure"), "node_cell_ms", "sparsity_ms"),
+                "solve": {k: pick(solve.get(k), "solve_ms", "iterations", "true_relres")
+                          for k in ("fp64", "mixed") if k in solve}}
+
+    def rounded(x):
+        if isinstance(x, dict):
+            return {k: rounded(v) for k, v in x.items()}
+        return float(f"{x:.6g}") if isinstance(x, float) else x
+
+    line["sections"] = rounded({
+        "main": section(out),
+        **{k: {"ms_per_step": w["ms_per_step"], "value": w["value"], "e2e_ms": (w.get("e2e") or {}).get("ms_per_step"),
+               **section(w)} for k, w in out["workloads"].items()},
+        "learned": {k: pick(out["learned"][k], "solve_ms", "iterations") for k in
+                    ("plain_fp64_cg_jacobi", "fcg_vcycle_untrained", "fcg_learned")} if out["learned"] else None,
+        "batched": pick(out["batched"], "instances", "rhs_per_instance", "batch_ms", "max_relres") or None,
+    })
+    return line
+
+
 def run_gpu(args):
     import torch
     import torch.distributed as dist
@@ -463,7 +510,10 @@ def run_gpu(args):
         out["workloads"] = extras
         out["learned"] = learned
         out["batched"] = batched
-        print(json.dumps(out), flush=True)
+        if args.record:
+            with open(args.record, "w") as f:
+                json.dump(out, f, indent=1)
+        print(json.dumps(headline(out)), flush=True)
     if world > 1:
         dist.destroy_process_group()
 
