@@ -132,8 +132,8 @@ __device__ __forceinline__ void warp_sort(int32_t* key, unsigned m) {
 // The keys of a node in more than 32 cells, sorted and split by a warp in the node's range of nc_cell.  An insertion
 // sort by one thread is quadratic wherever the atomics' order of arrival is not the cells': a node in 3000 tetrahedra
 // took 93 ms (30 to 68 with the keys in that order), in 3000 triangles 97, and 0.4 so.
-__device__ __noinline__ void sort_long_list(const int32_t* own, int cap, int32_t b, int deg, int npc, int32_t* nc_cell,
-                                            uint8_t* nc_local, int32_t* nc_inverse) {
+__device__ __forceinline__ void sort_long_list(const int32_t* own, int cap, int32_t b, int deg, int npc,
+                                               int32_t* nc_cell, uint8_t* nc_local, int32_t* nc_inverse) {
   const int lane = threadIdx.x & 31;
   for (int i = lane; i < min(deg, cap); i += 32) nc_cell[b + i] = own[i];
   __syncwarp();
@@ -225,9 +225,9 @@ constexpr int kWarpsPerBlock = 8;
 // The same with one warp per node (meshes of more than 16 cells per node on
 // average: its loads and stores stay coalesced over the node's list):
 // up to 32 keys are sorted by a bitonic network on registers (shuffles);
-// longer lists (rare) in place (sort_long_list).  Eight blocks an SM: without
-// the bound the call costs 48 registers (128^3 tetrahedra 1.76 -> 1.85 ms).
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) k_nc_sort_warp(int nb_node, int npc, int cap,
+// longer lists (rare) in place (sort_long_list: inlined, since a call costs 48
+// registers for 32, 128^3 tetrahedra 1.75 -> 1.85 ms).
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_nc_sort_warp(int nb_node, int npc, int cap,
                                                                  const int32_t* __restrict__ nc_ptr,
                                                                  const int32_t* __restrict__ bucket,
                                                                  int32_t* __restrict__ nc_cell,
