@@ -17,7 +17,7 @@
 // vanish on Dirichlet nodes (rows of fine and columns of coarse boundary
 // nodes), so that the coarse spaces satisfy the boundary condition.
 // Fine levels run one kernel per step; the levels of <= kCoarseRows rows run
-// in ONE block per vector with block barriers.
+// in ONE cluster of blocks per vector with cluster barriers.
 //
 // Network (message-passing layers of width 64, BF16 weights and activations,
 // FP32 accumulation) on the coefficient features x0 = [1, log(A_ii / mean)]:
@@ -627,7 +627,7 @@ __global__ void k_sweep(int nrow, int ncol, const int32_t* __restrict__ rp, cons
 // ---------------------------------------------------------------------------
 // V-cycle kernels (FP32).  The row operations below are shared by the
 // per-level kernels (grid-stride over the rows of one vector, the vector in
-// grid.y) and the coarse-levels kernels (block-stride, one block per vector).
+// grid.y) and the coarse-levels kernels (cluster-stride, one cluster per vector).
 // Pointers are already offset to the vector; those of vectors are not
 // __restrict__, since in the coarse kernels other blocks write them between
 // two steps.
@@ -2640,8 +2640,8 @@ afem_status afem::fcg_solve(afem_context ctx, int n, const int32_t* rp, const in
   return AFEM_OK;
 }
 
-// Levels of at most `rows` rows run in the coarse-levels kernel (one block
-// per vector); the others one launch per V-cycle step.
+// Levels of at most `rows` rows run in the coarse-levels kernel (one cluster
+// of blocks per vector); the others one launch per V-cycle step.
 extern "C" afem_status afem_mpnn_set_coarse_rows(afem_mpnn net, int rows) {
   AFEM_CHECK_ARG(net && rows >= 0, "afem_mpnn_set_coarse_rows: bad arguments");
   net->coarse_lo = net->Lv - 1;

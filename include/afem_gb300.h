@@ -85,7 +85,10 @@ afem_status afem_device_fp64_fma_rate(afem_context ctx, double* gfma_per_s_h);
  * of (cell, local node i) in that list (nullable).  Buffers:
  * nc_ptr_d[nb_node+1], nc_cell_d, nc_local_d and
  * nc_inverse_d[nb_cell*nodes_per_cell].  Deterministic.  nodes_per_cell:
- * 3 or 4 for cells; 2 also serves boundary edges (node -> face lists). */
+ * 3 or 4 for cells; 2 also serves boundary edges (node -> face lists).
+ * Scratch of the context: 4 bytes an incidence, and for each node 4 and a
+ * bucket of 8 to 64 keys of 4 bytes (half again the average, rounded down to
+ * eights, plus 8: 32 bytes for a node in no cell of a sparse numbering). */
 afem_status afem_node_cell_build(afem_context ctx, int nb_node, int nb_cell, int nodes_per_cell,
                                  const int32_t* cell_nodes_d, int32_t* nc_ptr_d, int32_t* nc_cell_d,
                                  uint8_t* nc_local_d, int32_t* nc_inverse_d);
@@ -439,7 +442,8 @@ typedef struct {
   int skip_forced_rows;   /* leave penalty (forced) rows out of both norms of the stop test */
   double inner_rtol;      /* MIXED and batch: FP32 residual reduction between reliable updates
                              (<= 0: 0.1) */
-  int check_every;        /* iterations between host convergence checks (default 16) */
+  int check_every;        /* iterations between host convergence checks (default 16) of a solve in launches per
+                             iteration; a solve in one launch tests every iteration on the device */
   int block_size;         /* MIXED: 3 = the CSR holds 3x3 blocks (the per-row layout of a 3-DoF
                              BSR matrix): the FP32 SpMV then reads one column index per block
                              (the FP32 BSR SpMV); 0 or 1: scalar rows */
@@ -459,7 +463,17 @@ void afem_solver_options_default(afem_solver_options* opt);
  * Replaces IDoFLinearSystemImpl::solve of the HYPRE / PETSc / Aleph / Arcane
  * MatVec backends (HypreDoFLinearSystem.cc:265-858, DoFLinearSystem.cc:146-159).
  * forced_info_d (nullable) marks rows left out of the stop test when
- * opt->skip_forced_rows.  Synchronous (returns after convergence). */
+ * opt->skip_forced_rows.  Synchronous (returns after convergence).
+ *
+ * Systems whose vectors fit the register files (up to 6 rows a thread, 467 k
+ * rows on 152 SMs) run in one launch, a block of 226 KB of shared memory an SM:
+ * AFEM_ERR_TIMEOUT if a block's wait for the others runs out (about 2 s), x
+ * then as it was (MIXED: as of the last refinement).  Up to 3072 rows take
+ * eight SMs; above, an SM for every 128 rows or, at most, each SM, so that from
+ * half the chip on (about 9.7 k rows) solves of several threads run one after
+ * the other.  A solve of 256^2 triangles from 1, 2 and 4 threads: 8.2, 8.1 and
+ * 8.1 ms (in launches per iteration 20.4, 11.8 and 7.2); of 100^2 2.8, 2.7 and
+ * 2.7 (6.9, 3.9 and 1.9); of 45^2 1.09, 0.57 and 0.29 (3.3, 1.8 and 0.95). */
 afem_status afem_cg_solve_csr(afem_context ctx, int n, const int32_t* row_ptr_d, const int32_t* cols_d,
                               const double* values_d, const double* b_d, double* x_d, const uint8_t* forced_info_d,
                               const afem_solver_options* opt, afem_solve_info* info);
@@ -560,8 +574,9 @@ afem_status afem_mpnn_set_operator(afem_mpnn net, int n, const int32_t* row_ptr_
 /* z = M r for `batch` FP32 vectors stored one after the other. */
 afem_status afem_mpnn_forward(afem_mpnn net, int batch, const float* r_d, float* z_d);
 /* Levels of at most `rows` rows (default 2048) run their V-cycle steps in
- * one cluster of blocks per vector with cluster barriers; larger levels one grid-wide
- * launch per step. */
+ * one cluster of blocks per vector with cluster barriers (eight blocks, four
+ * for more vectors than the device runs clusters of eight at once); larger
+ * levels one grid-wide launch per step. */
 afem_status afem_mpnn_set_coarse_rows(afem_mpnn net, int rows);
 /* The level-l smoother weights d_l (level_rows[l] floats). */
 afem_status afem_mpnn_scalings(afem_mpnn net, int level, float* d_d);
@@ -632,6 +647,8 @@ typedef struct {
 } afem_batch_instance;
 
 typedef struct {
+  /* Until one is set: by the rows an SM, {512, 1, 3.5} up to 1000, {512, 2, 3.5} up to 15000, {256, 4, 3.5} above
+   * (or with more instances than CTAs of the smaller grids). */
   int block;                    /* threads per CTA: 128, 256 or 512 */
   int blocks_per_sm;            /* CTAs per SM (clamped to the occupancy) */
   float cost_exponent;          /* team size ~ rows^(cost_exponent / 2) */
