@@ -71,7 +71,7 @@ __device__ __forceinline__ int sum_exponent(double total) {
   return abs(e) <= 900 ? e : kNoExponent;
 }
 
-// e: biased as a double's (0 for a zero), m: 53-bit significand, s: 0 or -1
+// e: biased as a double's, m: significand of up to 53 bits, 0 for a zero, s: 0 or -1
 __device__ __forceinline__ bool to_limbs(int e, unsigned long long m, int s, int E, int (&l)[kLimbs]) {
   int p = e - E - 1006;   // place of the significand's last bit
   if (p < 0) {
@@ -93,10 +93,11 @@ __device__ __forceinline__ bool to_limbs(double v, int E, int (&l)[kLimbs]) {
   const unsigned long long m = (unsigned long long)((h & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(v);
   return to_limbs(e, e ? m : 0ull, h >> 31, E, l);
 }
+// Subnormal numbers take part: an FP32 sum of tiny terms is made of them long before its total leaves FP32's range.
 __device__ __forceinline__ bool to_limbs(float v, int E, int (&l)[kLimbs]) {
   const int b = __float_as_int(v), e = b >> 23 & 0xff;
-  const unsigned long long m = (unsigned long long)((b & 0x7fffff) | 0x800000) << 29;
-  return to_limbs(e == 0 ? 0 : e == 255 ? 2047 : e + 896, e ? m : 0ull, b >> 31, E, l);
+  const unsigned long long m = (unsigned long long)((b & 0x7fffff) | (e ? 0x800000 : 0)) << 29;
+  return to_limbs(e == 255 ? 2047 : max(e, 1) + 896, m, b >> 31, E, l);
 }
 
 __device__ __forceinline__ __int128 from_limbs(const int (&l)[kLimbs]) {

@@ -140,3 +140,26 @@ def test_a_long_row_costs_fp32_no_more_than_fp64(cuda_ctx):
                                                                                     **OPTIONS[form]))
             best[form] = min(best.get(form, np.inf), info.solve_ms / info.iterations)
     assert best["mixed"] <= 1.1 * best["fp64"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("side", [30, 100])
+def test_tiny_systems_converge_as_their_multiples(cuda_ctx, side, precision):
+    """The same problem at 2^-k: powers of two change no digit in FP64, nor in FP32 until the squares of the residual's
+    entries (2^-64 at 2^-44 and 1e-6) leave its normal numbers; they keep 13 bits and more down to 2^-48."""
+    T = sp.diags([-np.ones(side - 1), 2.0 * np.ones(side), -np.ones(side - 1)], [-1, 0, 1])
+    A = (sp.kron(T, sp.identity(side)) + sp.kron(sp.identity(side), T)).tocsr()
+    A.sort_indices()
+    sys, b0 = dev(A), np.random.default_rng(0).standard_normal(side * side)
+    iters = {}
+    for k in (0, 40, 44, 46, 48) + ((200, 400, 460, 480) if precision == "fp64" else ()):
+        b = b0 * 2.0 ** -k
+        x = torch.zeros(side * side, dtype=torch.float64, device="cuda")
+        info = fem.cg_solve_csr(cuda_ctx, *sys, torch.as_tensor(b, device="cuda"), x,
+                                options=fem.solver_options(rtol=1e-6, max_iter=1000, **OPTIONS[precision]))
+        assert info.status == 0
+        iters[k] = info.iterations
+        scaled = x.cpu().numpy() * 2.0 ** k
+        assert np.linalg.norm(b0 - A @ scaled) <= 1.01e-6 * np.linalg.norm(b0)
+    spread = 1.05 if precision == "mixed" else 1.0
+    assert max(iters.values()) <= spread * iters[0]
